@@ -11,8 +11,15 @@
 // runs in parallel: one thread per chunk.
 //
 // One thread-block cluster serves one row of logits: each CTA keeps a contiguous slice of the distribution in shared
-// memory (float32), reads the other slices through distributed shared memory where a chunk straddles CTAs, and the
-// cluster meets at hardware barriers; no global scratch is used.
+// memory (float32) and the head of the next CTA's slice behind it, so that the chunk and the block that straddle the
+// border are added up where they begin, from local memory; the cluster meets at hardware barriers; no global scratch.
+//
+// What bounds a call is the length of the chains of dependent additions (V / 256 for a sum, 256 per block of a cumulative
+// sum, 256 and V / 256 for the totals), at one add per 4 cycles, and the cluster barriers.  The chains therefore run from
+// local shared memory with the loads of several steps in flight, on every CTA of the cluster at once, and the slice is
+// laid out with one word of padding per 256 (`slot`), which puts chains that start a block apart on different banks.
+// 128256 logits, one row, k = 0: 320 us with the chains of CTA 0 reading the peers' slices element by element, 23 us
+// now; k = 40: 274 and 78 us.
 #include <math.h>
 
 #include <cooperative_groups.h>
@@ -35,33 +42,82 @@ struct SampleArgs {
   const float* u;        // [B] uniform samples in [0, 1)
   int32_t* counter;      // [B][V] alpha counters, or null
   int32_t* tokens;       // [B]
-  int V, k, per;         // per: elements of the distribution held by one CTA
+  int V, k, per, ext;    // per: elements of the distribution held by one CTA; ext: the same with the head of the next slice
   int div, len;          // reductions over V: `div` chunks of `len` (div = 0: one sequential pass)
   float inv_temp, thr, af, ap;
 };
 
-// Walks the distribution, which is spread over the CTAs' shared-memory slices, in ascending index order.
-struct SliceCursor {
-  float* const* base;
-  int per, owner, off;
-  __device__ SliceCursor(float* const* b, int per_, int j) : base(b), per(per_), owner(j / per_), off(j % per_) {}
-  __device__ __forceinline__ float load() const { return base[owner][off]; }
-  __device__ __forceinline__ void store(float v) const { base[owner][off] = v; }
-  __device__ __forceinline__ void next() { if (++off == per) { off = 0; owner++; } }
+// Word of a slice that holds its element i: chains that start 256 elements apart begin on neighbouring banks.
+__host__ __device__ __forceinline__ int smp_slot(int i) { return i + (i >> 8); }
+
+// Part of a row's distribution as one CTA sees it: its own slice and `ext - per` elements of the next one in local memory,
+// anything beyond through distributed shared memory.
+struct SliceView {
+  float* const* base;  // the CTAs' slices
+  const float* local;
+  int per, ext, j0;
+  __device__ __forceinline__ float load(int j) const {
+    const int i = j - j0;
+    if (i >= 0 && i < ext) return local[smp_slot(i)];
+    return base[j / per][smp_slot(j % per)];
+  }
+  // s + t(j) + t(j + 1) + ... + t(j + n - 1), added in that order; t(x) = x * scale rounded once (scale 1: x)
+  __device__ __forceinline__ float add_up(float s, int j, int n, float scale) const {
+    const int i = j - j0;
+    return i >= 0 && i + n <= ext ? chain(s, n, scale, [&](int k) { return local[smp_slot(i + k)]; })  // no test per element
+                                  : chain(s, n, scale, [&](int k) { return load(j + k); });
+  }
+  template <typename F>
+  __device__ __forceinline__ static float chain(float s, int n, float scale, F at) {
+    constexpr int U = 16;
+    int k = 0;
+#pragma unroll 1
+    for (; k + U <= n; k += U) {
+      float v[U];
+#pragma unroll
+      for (int q = 0; q < U; q++) v[q] = at(k + q);
+#pragma unroll
+      for (int q = 0; q < U; q++) s = __fadd_rn(s, __fmul_rn(v[q], scale));
+    }
+    for (; k < n; k++) s = __fadd_rn(s, __fmul_rn(at(k), scale));
+    return s;
+  }
 };
+
+// s + p[0] + ... + p[n - 1] in that order (p in local shared memory); `prefix`, where given, receives the sum before each entry
+__device__ __forceinline__ float chain_sum(float s, const float* p, int n, float* prefix) {
+  constexpr int U = 16;
+  int k = 0;
+  for (; k + U <= n; k += U) {
+    float v[U];
+#pragma unroll
+    for (int q = 0; q < U; q++) v[q] = p[k + q];
+#pragma unroll
+    for (int q = 0; q < U; q++) {
+      if (prefix) prefix[k + q] = s;
+      s = __fadd_rn(s, v[q]);
+    }
+  }
+  for (; k < n; k++) {
+    if (prefix) prefix[k] = s;
+    s = __fadd_rn(s, p[k]);
+  }
+  return s;
+}
 
 template <typename LT>
 __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SampleArgs a) {
-  extern __shared__ __align__(16) float tbuf[];  // this CTA's slice of y, then e, then t
+  extern __shared__ __align__(16) float tbuf[];  // this CTA's slice and the head of the next: y, then e, then (k > 0) t
   __shared__ float s_red[32];
   __shared__ unsigned long long s_red64[32];
   __shared__ float s_cmax[SMP_MAX_CLUSTER];
   __shared__ unsigned long long s_key[2][SMP_MAX_CLUSTER];
-  __shared__ float s_bcast[2];
-  __shared__ float s_part[256];
+  __shared__ float s_bcast;
+  __shared__ float s_part[2][256];
   __shared__ float s_out[SMP_MAXK];
   __shared__ int s_idx[SMP_MAXK];
   __shared__ float s_tot[SMP_MAX_BLOCKS], s_base[SMP_MAX_BLOCKS];
+  __shared__ float s_blk[256];
   __shared__ int s_count;
   __shared__ float* s_slices[SMP_MAX_CLUSTER];
   cg::cluster_group cluster = cg::this_cluster();
@@ -69,15 +125,19 @@ __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SampleArgs
   const int b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int V = a.V, per = a.per;
   const int j0 = cr * per, j1 = min(V, j0 + per), nloc = max(j1 - j0, 0);
+  const int next = max(min(V, j0 + a.ext) - j0, 0);  // elements in local memory, the next slice's head included
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   pdl_launch();
   pdl_wait();
   if (tid < cs) s_slices[tid] = cluster.map_shared_rank(tbuf, tid);
   if (tid == 0) s_count = 0;
   const float log2e = 1.4426950408889634f;  // (float)(1 / Math.log(2))
+  const SliceView row = {s_slices, tbuf, per, next, j0};
 
   // ---- y = (logit - penalty) * (1 / temperature), NaN -> -inf; maximum over the row
   float lmax = -INFINITY;
-  for (int i = tid; i < nloc; i += SMP_THREADS) {
+#pragma unroll 4
+  for (int i = tid; i < next; i += SMP_THREADS) {
     float x = logit_f32(reinterpret_cast<const LT*>(a.logits)[(size_t)b * V + j0 + i]);
     if (a.counter != nullptr) {
       const int c = a.counter[(size_t)b * V + j0 + i];
@@ -86,70 +146,72 @@ __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SampleArgs
     }
     if (x != x) x = -INFINITY;
     x = __fmul_rn(x, a.inv_temp);
-    tbuf[i] = x;
+    tbuf[smp_slot(i)] = x;
     lmax = fmaxf(lmax, x);
   }
   lmax = warp_max(lmax);
   if (lane == 0) s_red[warp] = lmax;
   __syncthreads();
-  if (tid == 0) {
-    float m = s_red[0];
-    for (int w = 1; w < SMP_THREADS / 32; w++) m = fmaxf(m, s_red[w]);
-    for (int c = 0; c < cs; c++) *cluster.map_shared_rank(&s_cmax[cr], c) = m;
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // the peers run: their shared memory may be written
+  if (warp == 0) {
+    const float m = warp_max(s_red[lane]);
+    if (lane < cs) *cluster.map_shared_rank(&s_cmax[cr], lane) = m;
   }
   cluster.sync();
   float M = s_cmax[0];
   for (int c = 1; c < cs; c++) M = fmaxf(M, s_cmax[c]);
 
   // ---- e = exp2((y - M) / ln 2) with the polynomial exp2 (Tensor.exp, jsgrad/tensor.ts:2872-2875)
-  for (int i = tid; i < nloc; i += SMP_THREADS) tbuf[i] = jg_xexp2_f32(__fmul_rn(__fsub_rn(tbuf[i], M), log2e));
-  cluster.sync();
+#pragma unroll 4
+  for (int i = tid; i < next; i += SMP_THREADS) tbuf[smp_slot(i)] = jg_xexp2_f32(__fmul_rn(__fsub_rn(tbuf[smp_slot(i)], M), log2e));
+  __syncthreads();
 
-  // Sum over the whole row in the reference's order; computed by CTA 0, handed to every CTA.  All CTAs call it.
+  // Sum over the whole row in the reference's order.  Every CTA adds up the chunks that begin in its slice and hands the
+  // sums to all CTAs, each of which adds them up.  All CTAs call it; `slot` 0 or 1.
   auto row_sum = [&](int slot) -> float {
-    if (cr == 0) {
-      if (a.div == 0) {
-        if (tid == 0) {
-          SliceCursor c(s_slices, per, 0);
-          float s = 0.f;
-          for (int j = 0; j < V; j++) { s = __fadd_rn(s, c.load()); c.next(); }
-          s_part[0] = s;
-        }
-      } else if (tid < a.div) {
-        SliceCursor c(s_slices, per, tid * a.len);
-        float s = 0.f;
-        for (int j = 0; j < a.len; j++) { s = __fadd_rn(s, c.load()); c.next(); }
-        s_part[tid] = s;
+    if (a.div == 0) {  // one chain: CTA 0 walks all slices
+      cluster.sync();
+      if (cr == 0 && tid == 0) {
+        const float s = row.add_up(0.f, 0, V, 1.0f);
+        for (int c = 0; c < cs; c++) *cluster.map_shared_rank(&s_part[slot][0], c) = s;
       }
-      __syncthreads();
-      if (tid == 0) {
-        float total = s_part[0];
-        if (a.div != 0) {
-          total = 0.f;
-          for (int c = 0; c < a.div; c++) total = __fadd_rn(total, s_part[c]);
-        }
-        for (int c = 0; c < cs; c++) *cluster.map_shared_rank(&s_bcast[slot], c) = total;
-      }
+      cluster.sync();
+      return s_part[slot][0];
+    }
+    const int c0 = (j0 + a.len - 1) / a.len, c1 = min((j1 + a.len - 1) / a.len, a.div);
+    if (a.len > a.ext - per) cluster.sync();  // a chunk may reach into the next slice's own memory
+    if (tid < c1 - c0) {
+      const float s = row.add_up(0.f, (c0 + tid) * a.len, a.len, 1.0f);
+      for (int c = 0; c < cs; c++) *cluster.map_shared_rank(&s_part[slot][c0 + tid], c) = s;
     }
     cluster.sync();
-    return s_bcast[slot];
+    if (tid == 0) s_bcast = chain_sum(0.f, s_part[slot], a.div, nullptr);
+    __syncthreads();
+    return s_bcast;
   };
 
   const float rinv = __fdiv_rn(1.0f, row_sum(0));
-  for (int i = tid; i < nloc; i += SMP_THREADS) tbuf[i] = __fmul_rn(tbuf[i], rinv);  // t = e * (1 / sum)
-  __syncthreads();
 
   int token = 0;
   if (a.k > 0) {
+    for (int i = tid; i < next; i += SMP_THREADS) tbuf[smp_slot(i)] = __fmul_rn(tbuf[smp_slot(i)], rinv);  // t = e * (1 / sum)
+    __syncthreads();
     // ---- k rounds: the largest probability and, among equals, its lowest index (the reference's
     //      t.eq(max) * arange(n-1 .. 0) trick); the winner is zeroed.  Probabilities are >= +0, so their bit patterns
-    //      order like the values: the key (bits << 32 | ~index) finds both with one unsigned maximum.
-    for (int it = 0; it < a.k; it++) {
+    //      order like the values: the key (bits << 32 | ~index) finds both with one unsigned maximum.  A thread keeps the
+    //      best key of its elements and looks them over again only when it was its own that won.
+    auto scan = [&]() {
       unsigned long long best = 0ull;
+#pragma unroll 4
       for (int i = tid; i < nloc; i += SMP_THREADS) {
-        const unsigned long long key = ((unsigned long long)__float_as_uint(tbuf[i]) << 32) | (unsigned long long)(0xFFFFFFFFu - (uint32_t)(j0 + i));
+        const unsigned long long key = ((unsigned long long)__float_as_uint(tbuf[smp_slot(i)]) << 32) | (unsigned long long)(0xFFFFFFFFu - (uint32_t)(j0 + i));
         best = key > best ? key : best;
       }
+      return best;
+    };
+    unsigned long long mine = scan();
+    for (int it = 0; it < a.k; it++) {
+      unsigned long long best = mine;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
@@ -157,23 +219,29 @@ __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SampleArgs
       }
       if (lane == 0) s_red64[warp] = best;
       __syncthreads();
-      if (tid == 0) {
-        unsigned long long m = s_red64[0];
-        for (int w = 1; w < SMP_THREADS / 32; w++) m = s_red64[w] > m ? s_red64[w] : m;
-        for (int c = 0; c < cs; c++) *cluster.map_shared_rank(&s_key[it & 1][cr], c) = m;
+      if (warp == 0) {
+        best = s_red64[lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
+          best = other > best ? other : best;
+        }
+        if (lane < cs) *cluster.map_shared_rank(&s_key[it & 1][cr], lane) = best;
       }
       cluster.sync();
       unsigned long long win = s_key[it & 1][0];
       for (int c = 1; c < cs; c++) win = s_key[it & 1][c] > win ? s_key[it & 1][c] : win;
-      const int idx = (int)(0xFFFFFFFFu - (uint32_t)(win & 0xFFFFFFFFull));
+      const int idx = (int)(0xFFFFFFFFu - (uint32_t)(win & 0xFFFFFFFFull)), i = idx - j0;
       if (tid == 0) {
         s_out[it] = __uint_as_float((uint32_t)(win >> 32));
         s_idx[it] = idx;
-        if (idx >= j0 && idx < j1) tbuf[idx - j0] = 0.f;
       }
-      __syncthreads();
+      if (i >= 0 && i < next && i % SMP_THREADS == tid) {
+        tbuf[smp_slot(i)] = 0.f;
+        mine = scan();
+      }
     }
-    cluster.sync();  // every removal is visible to the CTA that adds up what is left
+    __syncthreads();
     const float rest = row_sum(1);
     if (cr == 0 && tid == 0) {
       // approximate top-p: tail[i] = out[k-1] + ... + out[i] (added in that order) + rest; entry i survives while
@@ -198,53 +266,49 @@ __global__ void __launch_bounds__(SMP_THREADS, 1) sample_kernel(const SampleArgs
       token = cnt < k ? s_idx[cnt] : 0;  // an index past the end gathers nothing
     }
   } else {
-    // ---- draw from the whole distribution: cumulative sums in blocks of 256 behind a front pad, block totals added
-    //      on top, everything scaled by 1 / last, entries not above u counted
-    const int np = (V + 255) / 256 * 256, pad = np - V, nb = np / 256;
+    // ---- draw from the whole distribution: cumulative sums in blocks of 256 behind a front pad (one block up to 512
+    //      elements), block totals added on top, everything scaled by 1 / last, entries not above u counted.  Rounded sums
+    //      of terms >= 0 never decrease, and the value at a block's end is the base of the next, so the count is all blocks
+    //      whose end is not above u and what the next block holds: only that one is walked entry by entry.  (Where an entry is NaN the
+    //      normaliser is, and no comparison holds.)
     const bool blocked = V > 512;
+    const int np = (V + 255) / 256 * 256, pad = blocked ? np - V : 0, size = blocked ? 256 : V, nb = blocked ? np / 256 : 1;
+    const int b0 = cr == 0 ? 0 : (j0 + pad + size - 1) / size, b1 = min((j1 + pad + size - 1) / size, nb);
+    if (size > a.ext - per) cluster.sync();
+    for (int blk = b0 + tid; blk < b1; blk += SMP_THREADS) {
+      const int first = max(blk * size - pad, 0), n = (blk + 1) * size - pad - first;
+      *cluster.map_shared_rank(&s_tot[blk], 0) = row.add_up(0.f, first, n, rinv);  // t = e * (1 / sum)
+    }
+    cluster.sync();
     if (cr == 0) {
-      if (blocked) {
-        for (int blk = tid; blk < nb; blk += SMP_THREADS) {
-          const int first = blk * 256 - pad;  // may be negative in block 0: the pad contributes zeros
-          SliceCursor c(s_slices, per, max(first, 0));
-          float s = 0.f;
-          for (int j = 0; j < 256; j++) {
-            if (first + j >= 0) { s = __fadd_rn(s, c.load()); c.store(s); c.next(); }
-          }
-          s_tot[blk] = s;
-        }
-        __syncthreads();
-        if (tid == 0) {
-          float run = 0.f;
-          for (int blk = 0; blk < nb; blk++) { s_base[blk] = run; run = __fadd_rn(run, s_tot[blk]); }
-        }
-      } else if (tid == 0) {
-        SliceCursor c(s_slices, per, 0);
-        float s = 0.f;
-        for (int j = 0; j < V; j++) { s = __fadd_rn(s, c.load()); c.store(s); c.next(); }
-      }
+      if (tid == 0) s_bcast = chain_sum(0.f, s_tot, nb, s_base);
       __syncthreads();
-      if (tid == 0) {
-        SliceCursor c(s_slices, per, V - 1);
-        const float last = blocked ? __fadd_rn(c.load(), s_base[nb - 1]) : c.load();
-        const float r = __fdiv_rn(1.0f, last);
-        for (int q = 0; q < cs; q++) *cluster.map_shared_rank(&s_bcast[1], q) = r;
+      const float r = __fdiv_rn(1.0f, s_bcast), u = a.u[b];
+      for (int blk = tid; blk < nb; blk += SMP_THREADS)
+        if (u >= __fmul_rn(__fadd_rn(s_tot[blk], s_base[blk]), r)) atomicAdd(&s_count, 1);
+      __syncthreads();
+      const int full = s_count;
+      if (full == nb) token = V;
+      else {
+        const int first = max(full * size - pad, 0), n = (full + 1) * size - pad - first;
+        float s = 0.f;
+        int cnt = 0;
+        for (int k0 = 0; k0 < n; k0 += 256) {
+          __syncthreads();
+          if (tid < 256 && k0 + tid < n) s_blk[tid] = __fmul_rn(row.load(first + k0 + tid), rinv);
+          __syncthreads();
+          if (tid == 0) {
+            const int m = min(256, n - k0);
+#pragma unroll 16
+            for (int k = 0; k < m; k++) {
+              s = __fadd_rn(s, s_blk[k]);
+              cnt += (u >= __fmul_rn(blocked ? __fadd_rn(s, s_base[full]) : s, r)) ? 1 : 0;
+            }
+          }
+        }
+        token = first + cnt;
       }
     }
-    cluster.sync();
-    const float r = s_bcast[1];
-    const float u = a.u[b];
-    const float* base0 = cluster.map_shared_rank(s_base, 0);
-    int cnt = 0;
-    for (int i = tid; i < nloc; i += SMP_THREADS) {
-      const float cw = blocked ? __fadd_rn(tbuf[i], base0[(j0 + i + pad) >> 8]) : tbuf[i];
-      cnt += (u >= __fmul_rn(cw, r)) ? 1 : 0;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    if (lane == 0 && cnt != 0) atomicAdd(cluster.map_shared_rank(&s_count, 0), cnt);
-    cluster.sync();
-    if (cr == 0 && tid == 0) token = s_count;
   }
   if (cr == 0 && tid == 0) {
     a.tokens[b] = token;
@@ -283,10 +347,13 @@ static int run_sample(jg_dev* dev, uint64_t tokens_out, uint64_t logits, uint64_
   int cs = SMP_MAX_CLUSTER;
   while (cs > 1 && V / cs < 2048) cs >>= 1;
   a.per = (V + cs - 1) / cs;
-  const size_t smem = (size_t)a.per * sizeof(float);
+  // the head of the next slice is kept where a chunk is short enough for it (a vocabulary with a divisor near 256); longer
+  // chunks, found with odd vocabularies, read the rest through distributed shared memory
+  a.ext = cs > 1 ? a.per + (a.len > 256 && a.len <= 2048 ? a.len : 256) : a.per;
+  const size_t smem = (size_t)(smp_slot(a.ext) + 1) * sizeof(float);
   const size_t limit = (size_t)dev->prop.sharedMemPerBlockOptin - 40 * 1024;
   if (smem > limit) {
-    jg_set_error("sample: %d values per CTA need %zu B of shared memory (limit %zu)", a.per, smem, limit);
+    jg_set_error("sample: %d values per CTA need %zu B of shared memory (limit %zu)", a.ext, smem, limit);
     return JG_ENOTSUP;
   }
   static size_t smem_set[8] = {0, 0, 0, 0, 0, 0, 0, 0};

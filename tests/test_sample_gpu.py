@@ -69,3 +69,27 @@ def test_sample_wrapper_and_argument_checks(dev):
         sample(lt, 0.9, V + 1, 0.5, 0.0, 0.0)
     with pytest.raises(ffi.JgError):
         dev.call("jg_sample", lt.ptr, lt.ptr, lt.ptr, 0, 1, V, 0.9, 600, 0.5, 0.0, 0.0)  # k beyond the kernel's table
+
+
+@pytest.mark.parametrize("V", [1, 300, 513, 4099, 40007, 40009 * 8, 128256])
+@pytest.mark.parametrize("k", [0, 30])
+def test_rows_at_the_edges_of_slices_and_chains(dev, V, k):
+    """Vocabularies without a divisor for the chunked sums (one chain over all slices), with chunks longer than what a CTA
+    keeps of its neighbour's slice, with one block or a padded first one; draws at both ends of the distribution; rows with
+    infinities and NaN."""
+    k = min(k, V)
+    rng = np.random.default_rng(V + k)
+    lg = _logits(rng, 5, V, 3.0)
+    lg[1, V // 2:] = -np.inf
+    lg[2, V // 3] = np.nan
+    lg[3, :] = -np.inf
+    lg[4, V - 1] = np.inf
+    lt = Tensor(lg, device=dev)
+    out = Tensor.empty((5,), "int32", dev)
+    for u0 in (0.0, 0.37, 0.99999994):
+        u = np.full(5, u0, np.float32)
+        dev.call("jg_sample", out.ptr, lt.ptr, Tensor(u, device=dev).ptr, 0, 5, V, 0.95, k, 0.9, 0.0, 0.0)
+        want = [O.sample(lg[r].astype(np.float32), 0.95, k, 0.9, 0.0, 0.0, u0) for r in range(5)]
+        # without a finite maximum every probability is NaN: the draw then gives 0, the rounds of the top k are not defined
+        rows = [r for r in range(5) if k == 0 or np.isfinite(np.where(np.isnan(lg[r]), -np.inf, lg[r]).max())]
+        assert [out.numpy()[r] for r in rows] == [want[r] for r in rows], (V, k, u0)
