@@ -144,26 +144,30 @@ class TransformerBlock:
         h = self.attention.call(self.attention_norm.call(x), pos, freqs_cis, mask, residual=x)
         return self.feed_forward.call(self.ffn_norm.call(h), residual=h)
 
-    def call_fused(self, ws: "_Workspace", pos: Tensor, freqs_cis: Tensor, tp=None) -> None:
+    def call_fused(self, ws: "_Workspace", pos: Tensor, freqs_cis: Tensor, tp=None, fp16=None) -> None:
         """Same block on the workspace `ws` (h is updated in place) with the norms and elementwise ops folded into
-        the projection kernels."""
+        the projection kernels.  `fp16`: dequantises matrices (Transformer._fp16_weights), for NF4 weights."""
         a, f, dev, B = self.attention, self.feed_forward, ws.h.dev, ws.B
         d = ws.h.shape[-1]
         wqkv = a._wqkv
+        nf4 = getattr(wqkv, "nf4_block", 0)
         int8 = wqkv.scale_ptr != 0
         # tensor parallelism, 1-2 rows: the row-parallel projections push their partial sums and the norm + projection
         # that follows gathers them (and writes the new residual stream into the workspace's other h buffer)
         split = tp is not None and B <= tp.split_rows(int8)
         # from 3 rows on (fp16 weights) normalise into ws.xn and project on the tensor cores; the fused-norm kernels
         # stream through the CUDA cores and only keep up with the weights for 1-2 rows (int8 weights: never)
-        big = _norm_first(B, int8, d) and not split
+        big = nf4 or (_norm_first(B, int8, d) and not split)
         if split and ws.pending:  # the previous block's w2 left its sum on the wire
             h_in, h_out = ws.flip()
             ffi.call("jg_tp_norm_linear", tp.handle, ws.qkv.ptr, h_out.ptr, h_in.ptr, self.attention_norm.weight.ptr,
                      self.attention_norm.eps, wqkv.weight.ptr, wqkv.scale_ptr, B, wqkv.out_features, d)
         elif big:
             self.attention_norm.call(ws.h, out=ws.xn)
-            dev.call("jg_linear", ws.qkv.ptr, ws.xn.ptr, wqkv.weight.ptr, wqkv.scale_ptr, 0, B, wqkv.out_features, d)
+            if nf4:
+                wqkv.call(ws.xn, out=ws.qkv) if wqkv.direct(B) else self._linear(ws.qkv, ws.xn, wqkv, fp16(wqkv)[0], B)
+            else:
+                dev.call("jg_linear", ws.qkv.ptr, ws.xn.ptr, wqkv.weight.ptr, wqkv.scale_ptr, 0, B, wqkv.out_features, d)
         else:
             dev.call("jg_norm_linear", ws.qkv.ptr, ws.h.ptr, self.attention_norm.weight.ptr, self.attention_norm.eps,
                      wqkv.weight.ptr, wqkv.scale_ptr, B, wqkv.out_features, d)
@@ -178,11 +182,18 @@ class TransformerBlock:
         if not a._kv.fused_attention:
             apply_rotary_emb_kvwrite(ws.qkv, freqs_cis, pos, a._kv, a._layer, a.n_heads)
             dev.call("jg_attn_decode", a._kv.handle, a._layer, ws.attn.ptr, ws.qkv.ptr, pos.ptr, B, a.n_heads)
-        self._row_parallel(a.wo, ws.attn, ws, tp, split=split)
+        self._row_parallel(a.wo, ws.attn, ws, tp, fp16(a.wo)[0] if nf4 and not a.wo.direct(B) else None, split=split)
         if split:
             h_in, h_out = ws.flip()
             ffi.call("jg_tp_norm_swiglu", tp.handle, ws.ffn.ptr, h_out.ptr, h_in.ptr, self.ffn_norm.weight.ptr, self.ffn_norm.eps,
                      f.w1.weight.ptr, f.w1.scale_ptr, f.w3.weight.ptr, f.w3.scale_ptr, B, f.w1.out_features, d)
+        elif nf4 and f.w1.direct(B):
+            self.ffn_norm.call(ws.h, out=ws.xn)
+            dev.call("jg_swiglu_nf4", ws.ffn.ptr, ws.xn.ptr, f.w1.weight.ptr, f.w1.scale.ptr, f.w3.weight.ptr, f.w3.scale.ptr, B, f.w1.out_features, d, nf4)
+        elif nf4:
+            self.ffn_norm.call(ws.h, out=ws.xn)
+            (w1, _), (w3, _) = fp16(f.w1, f.w3)
+            dev.call("jg_norm_swiglu", ws.ffn.ptr, ws.xn.ptr, 0, self.ffn_norm.eps, w1, 0, w3, 0, B, f.w1.out_features, d)
         elif big:
             self.ffn_norm.call(ws.h, out=ws.xn)
             dev.call("jg_norm_swiglu", ws.ffn.ptr, ws.xn.ptr, 0, self.ffn_norm.eps, f.w1.weight.ptr,
@@ -190,7 +201,11 @@ class TransformerBlock:
         else:
             dev.call("jg_norm_swiglu", ws.ffn.ptr, ws.h.ptr, self.ffn_norm.weight.ptr, self.ffn_norm.eps, f.w1.weight.ptr,
                      f.w1.scale_ptr, f.w3.weight.ptr, f.w3.scale_ptr, B, f.w1.out_features, d)
-        self._row_parallel(f.w2, ws.ffn, ws, tp, split=split)
+        self._row_parallel(f.w2, ws.ffn, ws, tp, fp16(f.w2)[0] if nf4 and not f.w2.direct(B) else None, split=split)
+
+    @staticmethod
+    def _linear(y: Tensor, x: Tensor, lin, w: tuple, M: int) -> None:
+        y.dev.call("jg_linear", y.ptr, x.ptr, *w, 0, M, lin.out_features, lin.in_features)
 
     @staticmethod
     def _row_parallel(lin, x: Tensor, ws: "_Workspace", tp, w=None, split: bool = False) -> None:
@@ -203,6 +218,9 @@ class TransformerBlock:
         if split:
             tp.linear_push(x, lin, ws.B)
             ws.pending = True
+            return
+        if w is None and getattr(lin, "nf4_block", 0):
+            lin.call(x, residual=ws.h, out=ws.h)
             return
         if tp is None:
             dev.call("jg_linear", ws.h.ptr, x.ptr, wp, sp, ws.h.ptr, ws.B, lin.out_features, lin.in_features)
@@ -428,7 +446,7 @@ class Transformer(Decoder):
         self.tok_embeddings.call(ws.tokens, out=ws.h)
         if self.fused:
             for layer in self.layers:
-                layer.call_fused(ws, ws.pos, self.freqs_cis, self._tp)
+                layer.call_fused(ws, ws.pos, self.freqs_cis, self._tp, self._fp16_weights)
             out = self.output
             if ws.pending:  # the last block's w2 pushed its sum: the output layer's prologue completes it
                 h_in, h_out = ws.flip()
@@ -501,7 +519,8 @@ class Transformer(Decoder):
 
     def _fp16_weights(self, *lins):
         """(pointer, 0) per projection: the weights themselves when fp16, else their dequantised copy in the scratch."""
-        if lins[0].scale_ptr == 0:
+        nf4 = getattr(lins[0], "nf4_block", 0)
+        if lins[0].scale_ptr == 0 and not nf4:
             return [(l.weight.ptr, 0) for l in lins]
         need = sum(l.out_features * l.in_features for l in lins)
         if getattr(self, "_dq_scratch", None) is None or self._dq_scratch.numel() < need:
@@ -509,7 +528,10 @@ class Transformer(Decoder):
         out, off = [], 0
         for l in lins:
             ptr = self._dq_scratch.ptr + 2 * off
-            self.dev.call("jg_dequant_i8_f16", ptr, l.weight.ptr, l.scale_ptr, l.out_features, l.in_features)
+            if nf4:
+                l.dequantise(ptr)
+            else:
+                self.dev.call("jg_dequant_i8_f16", ptr, l.weight.ptr, l.scale_ptr, l.out_features, l.in_features)
             out.append((ptr, 0))
             off += l.out_features * l.in_features
         return out
@@ -530,7 +552,8 @@ class Transformer(Decoder):
         # the int8 tiles itself (every 256-row tile of activations converts the weight tiles again); beyond, and with
         # JG_W8_TC=0, it is given dequantised fp16 copies, made once per chunk
         tc_rows = 0 if os.environ.get("JG_W8_TC", "1") == "0" else int(os.environ.get("JG_W8_TC_ROWS", "768"))
-        dq = R > 64 and self.output.scale_ptr != 0 and R > tc_rows
+        nf4 = getattr(self.layers[0].attention.wo, "nf4_block", 0)
+        dq = bool(nf4) or (R > 64 and self.output.scale_ptr != 0 and R > tc_rows)
 
         def weights(*lins):
             return self._fp16_weights(*lins) if dq else [(l.weight.ptr, l.scale_ptr) for l in lins]

@@ -57,10 +57,8 @@ class Llama3(Driver):
     def __post_init__(self):
         if self.quantize not in ("float16", "int8", "nf4", None):
             raise ValueError(f"quantize={self.quantize!r}: expected 'float16', 'int8' or 'nf4'")
-        if self.quantize == "nf4":
-            if self.tp is not None:
-                raise NotImplementedError("NF4 weights under tensor parallelism")
-            self.fused = False  # NF4 layers dequantise per call: the per-op block path
+        if self.quantize == "nf4" and self.tp is not None:
+            raise NotImplementedError("NF4 weights under tensor parallelism")
         p = dict(MODEL_PARAMS[self.size]["args"])
         p.update(self.args)
         if self.n_layers is not None:

@@ -97,8 +97,8 @@ def NF4Linear(block_size: int):
     """NF4Linear(block_size) -> layer class (jsgrad/models/llama3.ts:79-117): `weight` holds two 4-bit codes per byte
     (element 2i in the high nibble), `scale` one fp16 per `block_size` consecutive elements of the flattened
     [out, in] matrix; call(x) = x.linear(half(CODE[code] * scale).reshape(out, in).T).  On this device the packed form
-    is what stays resident; a call dequantises the matrix into a scratch shared by all NF4 layers of the device
-    (jg_dequant_nf4_f16) and runs the fp16 projection on it."""
+    is what stays resident; calls of up to 8 rows project straight from it (jg_linear_nf4), larger ones dequantise the
+    matrix into a scratch shared by all NF4 layers of the device (jg_dequant_nf4_f16) and run the fp16 projection on it."""
     scratch: dict[str, Tensor] = {}
 
     class _NF4Linear:
@@ -124,21 +124,32 @@ def NF4Linear(block_size: int):
             return {"weight": self.weight.view_rows(r0 * k // 2, r1 * k // 2),
                     "scale": self.scale.view_rows(r0 * k // block_size, r1 * k // block_size)}
 
+        def direct(self, M: int) -> bool:
+            """Whether M rows are projected straight from the packed matrix: one tile of the kernel's columns, whole 128-wide
+            k blocks, a scale per 32 codes or more."""
+            return M <= 8 and self.in_features % 128 == 0 and block_size >= 32 and block_size & (block_size - 1) == 0
+
+        def dequantise(self, ptr: int) -> None:
+            """fp16 [out, in] at `ptr`."""
+            self.weight.dev.call("jg_dequant_nf4_f16", ptr, self.weight.ptr, self.scale.ptr, self.out_features * self.in_features, block_size)
+
         def dequantised(self) -> Tensor:
             """fp16 [out, in] in the shared scratch (valid until the next NF4 layer of this device is called)."""
             dev, n = self.weight.dev, self.out_features * self.in_features
             t = scratch.get(dev.device)
             if t is None or t.numel() < n:
                 t = scratch[dev.device] = Tensor.empty((n,), "float16", dev)
-            dev.call("jg_dequant_nf4_f16", t.ptr, self.weight.ptr, self.scale.ptr, n, block_size)
+            self.dequantise(t.ptr)
             return t
 
         def call(self, x: Tensor, residual: Tensor | None = None, out: Tensor | None = None) -> Tensor:
             M = _rows(x)
             y = out if out is not None else Tensor.empty(x.shape[:-1] + (self.out_features,), "float16", x.dev)
-            w = self.dequantised()
-            x.dev.call("jg_linear", y.ptr, x.ptr, w.ptr, 0, residual.ptr if residual is not None else 0,
-                       M, self.out_features, self.in_features)
+            res = residual.ptr if residual is not None else 0
+            if self.direct(M):
+                x.dev.call("jg_linear_nf4", y.ptr, x.ptr, self.weight.ptr, self.scale.ptr, res, M, self.out_features, self.in_features, block_size)
+                return y
+            x.dev.call("jg_linear", y.ptr, x.ptr, self.dequantised().ptr, 0, res, M, self.out_features, self.in_features)
             return y
 
         __call__ = call

@@ -79,6 +79,8 @@ export const SYMBOLS = {
   jg_pos_advance: fn([ptr, u64, i32]),
   jg_dequant_i8_f16: fn([ptr, u64, u64, u64, 'i64', 'i64']),
   jg_dequant_nf4_f16: fn([ptr, u64, u64, u64, 'i64', i32]),
+  jg_linear_nf4: fn([ptr, u64, u64, u64, u64, u64, i32, i32, i32, i32]),
+  jg_swiglu_nf4: fn([ptr, u64, u64, u64, u64, u64, u64, i32, i32, i32, i32]),
   jg_step_create: fn([ptr, ptr, buf, buf]),
   jg_step_destroy: fn([ptr]),
   jg_step_run: fn([ptr, u64, u64, u64, u64, u64, u64, u64, u64, i32, i32, i32]),

@@ -379,8 +379,17 @@ int jg_dequant_i8_f16(jg_dev* dev, uint64_t dst, uint64_t w, uint64_t scale, int
 /* NF4Linear's dequantised matrix (jsgrad/models/llama3.ts:79-94): element i of the flattened [out][in] matrix is
  * half(CODE[code_i] * scale[i / block]); byte j of `w` holds code_2j in its high nibble and code_2j+1 in its low one;
  * scale: fp16 [n / block].  dst: fp16 [n].  The fp16 projection entry points then run on the copy, which is how this
- * device serves NF4 weights (the packed form stays the resident one; the copy is a per-call scratch). */
+ * device serves NF4 weights to calls of more than 8 rows (the packed form stays the resident one; the copy is a scratch). */
 int jg_dequant_nf4_f16(jg_dev* dev, uint64_t dst, uint64_t w, uint64_t scale, int64_t n, int32_t block);
+
+/* jg_linear and the gate / up half of the feed-forward straight from NF4 weights: x fp16 [M][K], M <= 8, K a multiple of
+ * 128 and of `block`, a power of two from 32 on (JG_ENOTSUP otherwise); every weight is half(CODE * scale) as above.
+ *   linear:  y = half(x W^T), or residual + that (residual may be y)
+ *   swiglu:  y = silu(half(x Wg^T)) * half(x Wu^T) */
+int jg_linear_nf4(jg_dev* dev, uint64_t y, uint64_t x, uint64_t w, uint64_t scale, uint64_t residual, int32_t M, int32_t N, int32_t K,
+                  int32_t block);
+int jg_swiglu_nf4(jg_dev* dev, uint64_t y, uint64_t x, uint64_t w_gate, uint64_t s_gate, uint64_t w_up, uint64_t s_up, int32_t M, int32_t N,
+                  int32_t K, int32_t block);
 
 /* ---- Models given as a list of layers (denograd_b200/hybrid.py): recurrent mixers and latent attention with a norm before
  *      and after every sublayer.  They have no counterpart in the reference, whose one decoder is the Llama block above.

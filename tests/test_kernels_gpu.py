@@ -541,3 +541,44 @@ def test_int8_dequantised_copy_is_bit_exact(dev):
     with pytest.raises(ffi.JgError):
         dev.call("jg_dequant_i8_f16", dq.ptr, wt.ptr, st.ptr, N, K + 8)
     dev.synchronize()
+
+
+@pytest.mark.parametrize("M", [1, 2, 7, 8])
+@pytest.mark.parametrize("N,K,block", [(16, 128, 64), (40, 256, 32), (2368 * 16 + 3, 128, 128), (1000, 1408, 64), (256, 4096, 64), (96, 14336, 64)])
+def test_projections_from_nf4_weights(dev, M, N, K, block):
+    """jg_linear_nf4 / jg_swiglu_nf4 against the same products of the dequantised matrix in 64 bits.  Tolerance: the fp32 sum
+    of K exact products (relative to the sum of their magnitudes) and one fp16 rounding per output and elementwise op."""
+    rng = np.random.default_rng(M * 1000 + N + K)
+    code = np.array([-1.0, -0.6961928009986877, -0.5250730514526367, -0.39491748809814453, -0.28444138169288635, -0.18477343022823334,
+                     -0.09105003625154495, 0.0, 0.07958029955625534, 0.16093020141124725, 0.24611230194568634, 0.33791524171829224,
+                     0.44070982933044434, 0.5626170039176941, 0.7229568362236023, 1.0]).astype(np.float16)
+    x = rng.standard_normal((M, K)).astype(np.float16)
+    res = rng.standard_normal((M, N)).astype(np.float16)
+    ws, dw = [], []
+    for _ in range(2):
+        c = rng.integers(0, 16, N * K).astype(np.uint8)
+        s = (0.02 + 0.05 * rng.random(N * K // block)).astype(np.float16)
+        ws.append((Tensor(c[0::2] * 16 + c[1::2], device=dev), Tensor(s, device=dev)))
+        dw.append((code[c].reshape(-1, block) * s[:, None]).astype(np.float16).reshape(N, K).astype(np.float64))
+    xt, rt, y = Tensor(x, device=dev), Tensor(res, device=dev), Tensor.zeros((M, N), "float16", dev)
+    sums = [x.astype(np.float64) @ w.T for w in dw]
+    mags = [np.abs(x.astype(np.float64)) @ np.abs(w).T for w in dw]
+    ulp = 2.0 ** -11
+    for residual in (None, rt):
+        dev.call("jg_linear_nf4", y.ptr, xt.ptr, ws[0][0].ptr, ws[0][1].ptr, residual.ptr if residual else 0, M, N, K, block)
+        want = sums[0] + (res if residual else 0.0)
+        err = np.abs(y.numpy().astype(np.float64) - want)
+        assert (err <= 2.0 ** -20 * mags[0] + ulp * (np.abs(sums[0]) + np.abs(want)) * 1.01 + 1e-7).all()
+    dev.call("jg_swiglu_nf4", y.ptr, xt.ptr, ws[0][0].ptr, ws[0][1].ptr, ws[1][0].ptr, ws[1][1].ptr, M, N, K, block)
+    g, u = sums
+    want = g / (1 + np.exp(-g)) * u
+    err = np.abs(y.numpy().astype(np.float64) - want)
+    assert (err <= (8 * ulp) * np.abs(want) + 1.2 * np.abs(u) * (2.0 ** -20 * mags[0] + ulp * np.abs(g)) + np.abs(g) * 2.0 ** -20 * mags[1] + 1e-4).all()
+
+
+def test_nf4_shapes_that_need_the_dequantised_copy_are_refused(dev):
+    x = Tensor.zeros((9, 256), "float16", dev)
+    w, s = Tensor.zeros((64 * 128,), "uint8", dev), Tensor.zeros((64 * 256 // 64,), "float16", dev)
+    for M, K, block in ((9, 256, 64), (1, 192, 64), (1, 256, 16), (1, 256, 96)):
+        with pytest.raises(ffi.JgError):
+            dev.call("jg_linear_nf4", x.ptr, x.ptr, w.ptr, s.ptr, 0, M, 64, K, block)
