@@ -67,3 +67,11 @@ int jg_tensor_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t co
   *out = s.m;
   return JG_OK;
 }
+
+int jg_tc_error_word(jg_dev* dev) {
+  if (dev->err_word != nullptr) return JG_OK;
+  JG_REQUIRE(!dev->capturing, "first tensor-core launch on a device must not be inside a graph capture");
+  JG_CUDA(cudaMalloc(&dev->err_word, sizeof(int)));
+  JG_CUDA(cudaMemsetAsync(dev->err_word, 0, sizeof(int), dev->stream));
+  return JG_OK;
+}
