@@ -23,6 +23,8 @@ struct jg_dev {
   bool pdl_cluster;  // ... also the thread-block-cluster launches of the gathering projections (JG_PDL_CLUSTER=1; default off)
   bool pdl_attn;     // ... also the decode-attention cluster launches (JG_PDL_ATTN=1; default off)
   int* err_word;    // device word written by kernels whose bounded waits gave up (0 = fine); allocated on first use
+  float* pair_slots;    // gemm_pair.cuh: accumulators of tiles that several CTA pairs share, and their flags; allocated on first use
+  uint32_t* pair_flags;
   bool tc_pending;  // such kernels were launched since the word was last checked
   bool peer_pending;  // peer-memory reductions (comm.cu) were launched since their error word was last checked
   // Device ranges written by the library's own launches since the stream was last synchronised (the latest
@@ -191,7 +193,7 @@ __device__ __forceinline__ float warp_max(float v) {
 __device__ __forceinline__ __half hmul1(__half a, __half b) { return __hmul_rn(a, b); }
 __device__ __forceinline__ __half hadd1(__half a, __half b) { return __hadd_rn(a, b); }
 __device__ __forceinline__ __half hsub1(__half a, __half b) { return __hsub_rn(a, b); }
-__device__ __forceinline__ __half hrecip1(__half a) { return __float2half_rn(__fdiv_rn(1.0f, __half2float(a))); }
+__device__ __forceinline__ __half hrecip1(__half a) { return __float2half_rn(__frcp_rn(__half2float(a))); }
 
 // Order-preserving map of fp16 bits to uint16 (larger value -> larger key); NaNs are not expected.
 __device__ __forceinline__ uint32_t half_order_key(__half h) {

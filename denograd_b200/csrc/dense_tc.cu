@@ -10,7 +10,7 @@
 #include <stdlib.h>
 
 #include "dense.cuh"
-#include "tcgen05.cuh"
+#include "gemm_pair.cuh"
 
 constexpr int DT_BM = 128, DT_BK = 64;
 
@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(DtCfg<TN, GLU, HALF>::THREADS, HALF ? 2 : 1)
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], acc_bar;
   __shared__ uint32_t s_tmem;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int tok0 = blockIdx.x * TN, feat0 = blockIdx.y * DT_BM;
   const int ks = gridDim.z, rank = blockIdx.z;
   const int n_kb = (a.K + DT_BK - 1) / DT_BK;
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(DtCfg<TN, GLU, HALF>::THREADS, HALF ? 2 : 1)
   const uint32_t tmem_base = s_tmem;
   bool acc_ok = false;
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0) {
     const int pre = nk < STAGES ? nk : STAGES;
     if (a.w_late) pdl_wait();
     auto load_w = [&](int i, int s) {
@@ -80,17 +80,21 @@ __global__ void __launch_bounds__(DtCfg<TN, GLU, HALF>::THREADS, HALF ? 2 : 1)
       tma_load_2d(st, &tm_w0, (kb0 + i) * DT_BK, feat0, &full_bar[s]);
       if (NW == 2) tma_load_2d(st + A_BYTES, &tm_w1, (kb0 + i) * DT_BK, feat0, &full_bar[s]);
     };
-    for (int i = 0; i < pre; i++) load_w(i, i);
+    if (elect_one())
+      for (int i = 0; i < pre; i++) load_w(i, i);
     pdl_wait();  // the rows come from the previous kernel
-    for (int i = 0; i < pre; i++)
-      tma_load_2d(tiles + (size_t)i * STAGE_BYTES + NW * A_BYTES, &tm_x, (kb0 + i) * DT_BK, tok0, &full_bar[i]);
+    if (elect_one())
+      for (int i = 0; i < pre; i++)
+        tma_load_2d(tiles + (size_t)i * STAGE_BYTES + NW * A_BYTES, &tm_x, (kb0 + i) * DT_BK, tok0, &full_bar[i]);
     for (int i = pre; i < nk; i++) {
       const int s = i % STAGES;
       if (!mbar_wait(&empty_bar[s], ((i / STAGES) - 1) & 1)) { atomicCAS(a.err, 0, 1); break; }
-      load_w(i, s);
-      tma_load_2d(tiles + (size_t)s * STAGE_BYTES + NW * A_BYTES, &tm_x, (kb0 + i) * DT_BK, tok0, &full_bar[s]);
+      if (elect_one()) {
+        load_w(i, s);
+        tma_load_2d(tiles + (size_t)s * STAGE_BYTES + NW * A_BYTES, &tm_x, (kb0 + i) * DT_BK, tok0, &full_bar[s]);
+      }
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1) {
     // instruction descriptor: fp32 accumulator, bf16 x bf16, both operands K-major
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(DT_BM >> 4) << 24);
     bool ok = true;
@@ -101,15 +105,18 @@ __global__ void __launch_bounds__(DtCfg<TN, GLU, HALF>::THREADS, HALF ? 2 : 1)
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       unsigned char* st = tiles + (size_t)s * STAGE_BYTES;
       const uint64_t bdesc = umma_desc(st + NW * A_BYTES);
+      if (elect_one()) {
 #pragma unroll
-      for (int w = 0; w < NW; w++) {
-        const uint64_t adesc = umma_desc(st + w * A_BYTES);
+        for (int w = 0; w < NW; w++) {
+          const uint64_t adesc = umma_desc(st + w * A_BYTES);
 #pragma unroll
-        for (int k = 0; k < DT_BK / 16; k++) umma_f16(tmem_base + w * TN, adesc + 2 * k, bdesc + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < DT_BK / 16; k++)
+            umma_f16(tmem_base + w * TN, adesc + 2 * k, bdesc + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
+        }
+        umma_commit(&empty_bar[s]);
       }
-      umma_commit(&empty_bar[s]);
     }
-    if (ok) umma_commit(&acc_bar);
+    if (ok && elect_one()) umma_commit(&acc_bar);
   } else if (warp >= 2) {
     pdl_wait();
     if (!GLU && a.out.act == JG_ACT_GELU_SIDE && rank == 0)  // the tile's rows of the token table, on their way while the product runs
@@ -248,6 +255,39 @@ static int launch_dt(jg_dev* dev, const DenseCall& c, const DtArgs& a) {
   return jg_after_launch(dev, "dense_tc");
 }
 
+// What the paired kernel (gemm_pair.cuh) does with an accumulator: the epilogue above.
+template <bool GLU_>
+struct DensePairEpi {
+  static constexpr bool GLU = GLU_, BF16 = true;
+  struct Args {
+    bf16* y;
+    float* y32;
+    const float *b0, *b1;
+    int ldy;
+    float limit;
+    DenseOut out;
+  };
+  struct Extra {};
+  static __device__ __forceinline__ void fetch(const Args&, const PairPlan&, int, int, int, Extra&) {}
+  static __device__ __forceinline__ void store(const Args& e, const PairPlan&, int feat, int tok, int n, const float (&r)[16], const Extra&) {
+    const float bias = e.b0 ? e.b0[feat] : 0.f;
+    const size_t o = (size_t)tok * e.ldy + feat;
+    const bool second = feat >= e.out.split;
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+      if (j >= n) break;
+      const float v = dense_act(e.out, feat, r[j] + bias, dense_side<bf16>(e.out, tok + j, feat));
+      if (second) e.out.y2[(size_t)(tok + j) * e.out.ld2 + feat - e.out.split] = v;
+      else if (e.y32) e.y32[o + (size_t)j * e.ldy] = v;
+      else e.y[o + (size_t)j * e.ldy] = __float2bfloat16_rn(v);
+    }
+  }
+  static __device__ __forceinline__ void glu(const Args& e, const PairPlan&, int feat, int tok, float gate, float up) {
+    const float b0 = e.b0 ? e.b0[feat] : 0.f, b1 = e.b1 ? e.b1[feat] : 0.f;
+    e.y[(size_t)tok * e.ldy + feat] = __float2bfloat16_rn(clamped_glu(gate + b0, up + b1, e.limit));
+  }
+};
+
 int jg_dense_tc(jg_dev* dev, const DenseCall& c) {
   JG_REQUIRE(((uintptr_t)c.x % 16) == 0 && c.ldx % 8 == 0 && c.ldw % 8 == 0, "dense: operands must be 16-byte aligned with row strides of a multiple of 8");
   const int erc = jg_tc_error_word(dev);
@@ -257,12 +297,17 @@ int jg_dense_tc(jg_dev* dev, const DenseCall& c) {
   else a.y = (bf16*)c.y;
   a.b0 = c.bias[0]; a.b1 = c.bias[1]; a.err = dev->err_word; a.M = c.M; a.N = c.N; a.K = c.K; a.ldy = c.ldy; a.limit = c.limit; a.out = c.out;
   a.w_late = jg_is_fresh(dev, c.w[0]) || jg_is_fresh(dev, c.w[1]);
+  // more than 128 rows: pairs of CTAs (gemm_pair.cuh), but for few features or a short K, where tiles of theirs are too few or over
+  // too soon (prompts of 1999 tokens at 8B sizes, a 128 x 256 tile per CTA / pairs: Matulorn 42.5 / 38.7 ms, Rigazen 40.2 / 34.3)
+  if (c.M > 128 && c.epilogue == JG_DENSE_GLU)
+    return launch_pair<DensePairEpi<true>>(dev, "dense_pair", c.x, c.ldx, c.w[0], c.w[1], c.ldw, c.M, c.N, c.K, true, a.w_late, {a.y, a.y32, a.b0, a.b1, a.ldy, a.limit, a.out});
+  if (c.M > 128 && c.N > 512 && c.K > 512)
+    return launch_pair<DensePairEpi<false>>(dev, "dense_pair", c.x, c.ldx, c.w[0], c.w[0], c.ldw, c.M, c.N, c.K, true, a.w_late, {a.y, a.y32, a.b0, a.b1, a.ldy, a.limit, a.out});
   if (c.epilogue == JG_DENSE_GLU) {
     if (c.M <= 16) return launch_dt<16, true, false>(dev, c, a);
     if (c.M <= 32) return launch_dt<32, true, false>(dev, c, a);
     if (c.M <= 64) return launch_dt<64, true, false>(dev, c, a);
-    if (c.M <= 128) return launch_dt<128, true, false>(dev, c, a);
-    return launch_dt<256, true, false>(dev, c, a);
+    return launch_dt<128, true, false>(dev, c, a);
   }
   if (c.M <= 16) return launch_dt<16, false, true>(dev, c, a);
   if (c.M <= 32) return launch_dt<32, false, true>(dev, c, a);

@@ -87,11 +87,13 @@ JG_API int jg_device_close(jg_dev* dev) {
   cudaEventDestroy(dev->t0);
   cudaEventDestroy(dev->t1);
   cudaFreeHost(dev->pinned_stage);
+  if (dev->pair_slots) cudaFree(dev->pair_slots);  // the flags lie behind the slots
   cudaStreamDestroy(dev->stream);
   delete dev;
   return JG_OK;
 }
 
+void jg_pair_reset(jg_dev* dev);            // tensor_map.cu: flags that a launch which gave up left behind
 int jg_peer_error(jg_dev* dev, int* code);  // comm.cu
 int jg_peer_run_boundary(jg_dev* dev);      // comm.cu: fold the exchange ordinals into the device-resident base
 
@@ -114,6 +116,7 @@ int jg_check_device_errors(jg_dev* dev) {
   JG_CUDA(cudaMemcpy(&code, dev->err_word, sizeof(int), cudaMemcpyDeviceToHost));
   if (code != 0) {
     cudaMemset(dev->err_word, 0, sizeof(int));
+    jg_pair_reset(dev);
     jg_set_error("a device-side wait gave up (code %d: 1 = TMA producer, 2 = MMA issuer, 3 = epilogue of a tensor-core "
                  "projection, 4 = grid barrier of the single-kernel decode step); results since the last synchronisation "
                  "are invalid", code);

@@ -100,7 +100,7 @@ __device__ __forceinline__ void flash_tc(P& p, int* err) {
   __shared__ __align__(8) uint64_t k_full[FT_ST], k_empty[FT_ST], v_full[FT_ST], v_empty[FT_ST], s_full[2], s_used[2], o_full[2], q_full, v_part;
   __shared__ uint32_t s_tmem;
   __shared__ float s_m[2][FT_ROWS], s_l[2][FT_ROWS];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = uniform_warp();
   pdl_launch();
   if (tid == 0) {
     for (int i = 0; i < FT_ST; i++) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
@@ -157,76 +157,81 @@ __device__ __forceinline__ void flash_tc(P& p, int* err) {
     }
     if (!ok && lane == 0) atomicCAS(err, 0, 1);
   } else if (warp == 9) {
-    if (lane == 0) {
-      // ---- MMA issuer
-      constexpr uint32_t F = P::BF16 ? (1u << 7) | (1u << 10) : 0u;
-      constexpr uint32_t id_s = (1u << 4) | F | ((uint32_t)(FT_KV >> 3) << 17) | ((uint32_t)(FT_ROWS >> 4) << 24);
-      constexpr uint32_t id_o = (1u << 4) | F | (1u << 16) | ((uint32_t)(P::DV >> 3) << 17) | ((uint32_t)(FT_ROWS >> 4) << 24);
-      int made[2] = {0, 0};  // score tiles issued per stream
-      bool ok = mbar_wait(&q_full, 0);
-      auto qk = [&](int q, int slot) {
-        const uint64_t a = umma_desc(sQ + (SPLIT ? 0 : (size_t)q * Cfg::Q_BYTES)), b = umma_desc(sK + (size_t)slot * Cfg::K_BYTES);
+    // ---- MMA issuer
+    constexpr uint32_t F = P::BF16 ? (1u << 7) | (1u << 10) : 0u;
+    constexpr uint32_t id_s = (1u << 4) | F | ((uint32_t)(FT_KV >> 3) << 17) | ((uint32_t)(FT_ROWS >> 4) << 24);
+    constexpr uint32_t id_o = (1u << 4) | F | (1u << 16) | ((uint32_t)(P::DV >> 3) << 17) | ((uint32_t)(FT_ROWS >> 4) << 24);
+    int made[2] = {0, 0};  // score tiles issued per stream
+    bool ok = mbar_wait(&q_full, 0);
+    auto qk = [&](int q, int slot) {
+      const uint64_t a = umma_desc(sQ + (SPLIT ? 0 : (size_t)q * Cfg::Q_BYTES)), b = umma_desc(sK + (size_t)slot * Cfg::K_BYTES);
+      if (elect_one()) {
 #pragma unroll
         for (int c = 0; c < KB; c++)
 #pragma unroll
           for (int k = 0; k < 4; k++)
             umma_f16(tmem + q * 128, a + c * (Q_BLOCK >> 4) + 2 * k, b + c * (K_BLOCK >> 4) + 2 * k, id_s, (c > 0 || k > 0) ? 1u : 0u);
         umma_commit(&s_full[q]);
-        made[q]++;
-      };
-      auto used = [&](int q) {  // the last score tile of the stream has been read (pass 1) or replaced by weights (pass 2)
-        const bool r = mbar_wait(&s_used[q], (made[q] - 1) & 1);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        return r;
-      };
-      auto keys = [&](int i) {
-        const bool r = mbar_wait(&k_full[i % FT_ST], (i / FT_ST) & 1);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        return r;
-      };
-      for (int j = 0; j < n && ok; j++) {  // pass 1
-        ok = keys(j);
-        for (int q = SPLIT ? j & 1 : 0; q < (SPLIT ? (j & 1) + 1 : 2) && ok; q++) {
-          if (made[q] > 0) ok = used(q);
-          if (ok) qk(q, j % FT_ST);
-        }
-        if (ok) umma_commit(&k_empty[j % FT_ST]);
       }
-      auto pv = [&](int q, int slot, bool first) {
-        const uint64_t b = umma_desc_mn(sV + (size_t)slot * Cfg::V_BYTES, K_BLOCK);
+      made[q]++;
+    };
+    auto commit = [&](uint64_t* bar) {
+      if (elect_one()) umma_commit(bar);
+    };
+    auto used = [&](int q) {  // the last score tile of the stream has been read (pass 1) or replaced by weights (pass 2)
+      const bool r = mbar_wait(&s_used[q], (made[q] - 1) & 1);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      return r;
+    };
+    auto keys = [&](int i) {
+      const bool r = mbar_wait(&k_full[i % FT_ST], (i / FT_ST) & 1);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      return r;
+    };
+    for (int j = 0; j < n && ok; j++) {  // pass 1
+      ok = keys(j);
+      for (int q = SPLIT ? j & 1 : 0; q < (SPLIT ? (j & 1) + 1 : 2) && ok; q++) {
+        if (made[q] > 0) ok = used(q);
+        if (ok) qk(q, j % FT_ST);
+      }
+      if (ok) commit(&k_empty[j % FT_ST]);
+    }
+    auto pv = [&](int q, int slot, bool first) {
+      const uint64_t b = umma_desc_mn(sV + (size_t)slot * Cfg::V_BYTES, K_BLOCK);
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < FT_KV / 16; k++)  // 16 rows of values = 2048 bytes further
           umma_f16_ts(tmem + 256 + q * 128, tmem + q * 128 + k * 8, b + k * 128, id_o, (!first || k > 0) ? 1u : 0u);
-      };
-      const int ahead = SPLIT ? 2 : 1;  // tiles whose scores are made before the first product with values
-      for (int j = 0; j < ahead && j < n && ok; j++) {
-        ok = keys(n + j);
-        for (int q = SPLIT ? j : 0; q < (SPLIT ? j + 1 : 2) && ok; q++) {
-          ok = made[q] == 0 || used(q);
-          if (ok) qk(q, (n + j) % FT_ST);
-        }
-        if (ok) umma_commit(&k_empty[(n + j) % FT_ST]);
       }
-      for (int j = 0; j < n && ok; j++) {  // pass 2
-        ok = mbar_wait(&v_full[j % FT_ST], (j / FT_ST) & 1);
-        const bool more = j + ahead < n;
-        bool have = false;
-        for (int q = SPLIT ? j & 1 : 0; q < (SPLIT ? (j & 1) + 1 : 2) && ok; q++) {
-          ok = used(q);
-          if (!ok) break;
-          pv(q, j % FT_ST, SPLIT ? j < 2 : j == 0);
-          if (j + ahead >= n) umma_commit(&o_full[q]);
-          if (more) {
-            if (!have) { ok = keys(n + j + ahead); have = true; }
-            if (ok) qk(q, (n + j + ahead) % FT_ST);
-          }
-        }
-        if (!ok) break;
-        umma_commit(&v_empty[j % FT_ST]);
-        if (more) umma_commit(&k_empty[(n + j + ahead) % FT_ST]);
+    };
+    const int ahead = SPLIT ? 2 : 1;  // tiles whose scores are made before the first product with values
+    for (int j = 0; j < ahead && j < n && ok; j++) {
+      ok = keys(n + j);
+      for (int q = SPLIT ? j : 0; q < (SPLIT ? j + 1 : 2) && ok; q++) {
+        ok = made[q] == 0 || used(q);
+        if (ok) qk(q, (n + j) % FT_ST);
       }
-      if (!ok) atomicCAS(err, 0, 2);
+      if (ok) commit(&k_empty[(n + j) % FT_ST]);
     }
+    for (int j = 0; j < n && ok; j++) {  // pass 2
+      ok = mbar_wait(&v_full[j % FT_ST], (j / FT_ST) & 1);
+      const bool more = j + ahead < n;
+      bool have = false;
+      for (int q = SPLIT ? j & 1 : 0; q < (SPLIT ? (j & 1) + 1 : 2) && ok; q++) {
+        ok = used(q);
+        if (!ok) break;
+        pv(q, j % FT_ST, SPLIT ? j < 2 : j == 0);
+        if (j + ahead >= n) commit(&o_full[q]);
+        if (more) {
+          if (!have) { ok = keys(n + j + ahead); have = true; }
+          if (ok) qk(q, (n + j + ahead) % FT_ST);
+        }
+      }
+      if (!ok) break;
+      commit(&v_empty[j % FT_ST]);
+      if (more) commit(&k_empty[(n + j + ahead) % FT_ST]);
+    }
+    if (!ok && lane == 0) atomicCAS(err, 0, 2);
   } else {
     // ---- softmax: thread = row
     const int q = warp >> 2, r = tid & 127, mine = count(q);

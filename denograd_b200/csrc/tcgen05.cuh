@@ -14,6 +14,18 @@ constexpr uint32_t TC_SPIN_LIMIT = 1u << 24;
 #ifdef __CUDACC__
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// The warp's index, known to the compiler as the same in all lanes.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+// One lane of a converged warp.  The roles that issue tcgen05.mma, tcgen05.commit and TMA run their loops with all lanes and
+// put only these instructions behind it: their operands then stay in uniform registers.  Loops behind `lane == 0` had them
+// moved there lane by lane, some 84 cycles for each MMA and 264 for a stage's wait and commit (600 per 64-wide k-block of
+// 256 x 128 as of 256 x 256, where the MMAs themselves take 256 and 512).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok)::"memory");
+  return ok != 0;
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }

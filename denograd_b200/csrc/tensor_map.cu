@@ -1,14 +1,14 @@
 // Encoded TMA tensor maps of the tensor-core projections, kept per operand (declared in tcgen05.cuh).
-#include "tcgen05.cuh"
+#include <mutex>
+
+#include "gemm_pair.cuh"
 
 typedef CUresult (*encode_tiled_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                     const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                     CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 static encode_tiled_fn g_encode = nullptr;
 
-// `bytes` = element size: 2 for fp16 operands (128-byte swizzle, the layout the MMA descriptors name), 1 for int8
-// weight tiles, which land unswizzled (64-byte rows) for the converting warps
-static int make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, const char* what, int bytes, bool bf16) {
+static int find_encoder() {
   if (!g_encode) {
     void* fn = nullptr;
     cudaDriverEntryPointQueryResult qres;
@@ -19,6 +19,13 @@ static int make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t co
     }
     g_encode = (encode_tiled_fn)fn;
   }
+  return JG_OK;
+}
+// `bytes` = element size: 2 for fp16 operands (128-byte swizzle, the layout the MMA descriptors name), 1 for int8
+// weight tiles, which land unswizzled (64-byte rows) for the converting warps
+static int make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, const char* what, int bytes, bool bf16) {
+  const int rc = find_encoder();
+  if (rc) return rc;
   const cuuint64_t dims[2] = {cols, rows};           // innermost first
   const cuuint64_t strides[1] = {ld * (cuuint64_t)bytes};  // bytes between rows
   const cuuint32_t box[2] = {64, box_rows};
@@ -68,10 +75,37 @@ int jg_tensor_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t co
   return JG_OK;
 }
 
+bool jg_tensor_map_two(CUtensorMap* out, const void* lo, const void* hi, uint64_t rows, uint64_t cols, uint64_t ld, bool bf16) {
+  const uint64_t apart = (uint64_t)(uintptr_t)hi - (uint64_t)(uintptr_t)lo;
+  if (lo >= hi || apart % 16 != 0 || apart >= (1ull << 40) || rows % 16 != 0 || find_encoder() != JG_OK) return false;
+  const cuuint64_t dims[4] = {cols, 16, 2, rows / 16}, strides[3] = {2 * ld, apart, 32 * ld};
+  const cuuint32_t box[4] = {64, 16, 2, 4}, estr[4] = {1, 1, 1, 1};
+  return g_encode(out, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(lo), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 int jg_tc_error_word(jg_dev* dev) {
   if (dev->err_word != nullptr) return JG_OK;
   JG_REQUIRE(!dev->capturing, "first tensor-core launch on a device must not be inside a graph capture");
   JG_CUDA(cudaMalloc(&dev->err_word, sizeof(int)));
   JG_CUDA(cudaMemsetAsync(dev->err_word, 0, sizeof(int), dev->stream));
   return JG_OK;
+}
+
+static size_t pair_flag_bytes(const jg_dev* dev) { return (size_t)(dev->sm_count / 2) * 2 * GP_EPI_WARPS * sizeof(uint32_t); }
+bool jg_pair_workspace(jg_dev* dev) {
+  static std::mutex m;
+  std::lock_guard<std::mutex> lock(m);
+  if (dev->pair_slots != nullptr) return true;
+  if (dev->capturing) return false;
+  const size_t slots = (size_t)(dev->sm_count / 2) * 2 * GP_SLOT * sizeof(float);
+  void* p = nullptr;
+  if (cudaMalloc(&p, slots + pair_flag_bytes(dev)) != cudaSuccess) { cudaGetLastError(); return false; }
+  if (cudaMemsetAsync((char*)p + slots, 0, pair_flag_bytes(dev), dev->stream) != cudaSuccess) { cudaGetLastError(); cudaFree(p); return false; }
+  dev->pair_flags = (uint32_t*)((char*)p + slots);
+  dev->pair_slots = (float*)p;
+  return true;
+}
+void jg_pair_reset(jg_dev* dev) {
+  if (dev->pair_flags != nullptr) cudaMemset(dev->pair_flags, 0, pair_flag_bytes(dev));
 }

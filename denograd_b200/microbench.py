@@ -1,5 +1,5 @@
 """Per-kernel timings through the C ABI, for choosing the library's environment knobs on a given machine
-(`JG_TC_SPLITK`, `JG_TC_PAIR`, `JG_ATTN_CLUSTER`, `JG_ATTN_STAGES`, ...: they are read once per process, so run one
+(`JG_TC_SPLITK`, `JG_ATTN_CLUSTER`, `JG_ATTN_STAGES`, ...: they are read once per process, so run one
 process per setting) and for checking a kernel in isolation:
 
     python -m denograd_b200.microbench projections --rows 512          # the four projections of a layer
