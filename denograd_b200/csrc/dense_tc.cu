@@ -226,7 +226,7 @@ static int launch_dt(jg_dev* dev, const DenseCall& c, const DtArgs& a) {
       if (s == 1 || t < best) { best = t; ks = s; }
     }
   } else {
-    while (ks < (HALF && tiles > 8 ? 4 : 8) && ks < Cfg::MAX_KS && tiles * ks * 3 < dev->sm_count * 2 * (HALF ? 2 : 1) && n_kb / (ks + 1) >= 8) ks++;
+    while (ks < (tiles > 8 ? 4 : 8) && ks < Cfg::MAX_KS && tiles * ks * 3 < dev->sm_count * 2 * (HALF ? 2 : 1) && n_kb / (ks + 1) >= 8) ks++;
   }
   dev->tc_pending = true;
   cudaLaunchConfig_t cfg = {};
@@ -258,33 +258,32 @@ static int launch_dt(jg_dev* dev, const DenseCall& c, const DtArgs& a) {
 // What the paired kernel (gemm_pair.cuh) does with an accumulator: the epilogue above.
 template <bool GLU_>
 struct DensePairEpi {
-  static constexpr bool GLU = GLU_, BF16 = true;
+  static constexpr bool GLU = GLU_, BF16 = true, RESIDUAL = false;
   struct Args {
     bf16* y;
     float* y32;
     const float *b0, *b1;
-    int ldy;
+    int ldy, aligned;  // aligned: rows of results start on 16 bytes
     float limit;
     DenseOut out;
   };
-  struct Extra {};
-  static __device__ __forceinline__ void fetch(const Args&, const PairPlan&, int, int, int, Extra&) {}
-  static __device__ __forceinline__ void store(const Args& e, const PairPlan&, int feat, int tok, int n, const float (&r)[16], const Extra&) {
-    const float bias = e.b0 ? e.b0[feat] : 0.f;
-    const size_t o = (size_t)tok * e.ldy + feat;
-    const bool second = feat >= e.out.split;
-#pragma unroll
-    for (int j = 0; j < 16; j++) {
-      if (j >= n) break;
-      const float v = dense_act(e.out, feat, r[j] + bias, dense_side<bf16>(e.out, tok + j, feat));
-      if (second) e.out.y2[(size_t)(tok + j) * e.out.ld2 + feat - e.out.split] = v;
-      else if (e.y32) e.y32[o + (size_t)j * e.ldy] = v;
-      else e.y[o + (size_t)j * e.ldy] = __float2bfloat16_rn(v);
-    }
+  static __device__ __forceinline__ bool wide(const Args& e, const PairPlan& a, int feat) { return e.aligned && feat + (GLU ? 16 : 32) <= min(a.N, e.out.split); }
+  static __device__ __forceinline__ bool f32(const Args& e) { return e.y32 != nullptr; }
+  static __device__ __forceinline__ float* out32(const Args& e, const PairPlan&, int tok, int feat) { return e.y32 + (size_t)tok * e.ldy + feat; }
+  static __device__ __forceinline__ bf16* out(const Args& e, const PairPlan&, int tok, int feat) { return e.y + (size_t)tok * e.ldy + feat; }
+  static __device__ __forceinline__ const bf16* residual(const Args&, const PairPlan&, int, int) { return nullptr; }
+  static __device__ __forceinline__ float value(const Args& e, const PairPlan& a, int feat, int tok, float r) {
+    return dense_act(e.out, feat, r + (e.b0 ? e.b0[feat] : 0.f), dense_side<bf16>(e.out, min(tok, a.M - 1), feat));
   }
-  static __device__ __forceinline__ void glu(const Args& e, const PairPlan&, int feat, int tok, float gate, float up) {
-    const float b0 = e.b0 ? e.b0[feat] : 0.f, b1 = e.b1 ? e.b1[feat] : 0.f;
-    e.y[(size_t)tok * e.ldy + feat] = __float2bfloat16_rn(clamped_glu(gate + b0, up + b1, e.limit));
+  static __device__ __forceinline__ uint16_t round(float v) { return __bfloat16_as_ushort(__float2bfloat16_rn(v)); }
+  static __device__ __forceinline__ uint32_t add(uint32_t v, uint32_t) { return v; }
+  static __device__ __forceinline__ uint16_t glu(const Args& e, int feat, float gate, float up) {
+    return round(clamped_glu(gate + (e.b0 ? e.b0[feat] : 0.f), up + (e.b1 ? e.b1[feat] : 0.f), e.limit));
+  }
+  static __device__ __forceinline__ void store(const Args& e, const PairPlan& a, int feat, int tok, float v) {
+    if (feat >= e.out.split) e.out.y2[(size_t)tok * e.out.ld2 + feat - e.out.split] = v;
+    else if (e.y32) *out32(e, a, tok, feat) = v;
+    else *out(e, a, tok, feat) = __float2bfloat16_rn(v);
   }
 };
 
@@ -297,17 +296,16 @@ int jg_dense_tc(jg_dev* dev, const DenseCall& c) {
   else a.y = (bf16*)c.y;
   a.b0 = c.bias[0]; a.b1 = c.bias[1]; a.err = dev->err_word; a.M = c.M; a.N = c.N; a.K = c.K; a.ldy = c.ldy; a.limit = c.limit; a.out = c.out;
   a.w_late = jg_is_fresh(dev, c.w[0]) || jg_is_fresh(dev, c.w[1]);
-  // more than 128 rows: pairs of CTAs (gemm_pair.cuh), but for few features or a short K, where tiles of theirs are too few or over
+  const int aligned = (uintptr_t)c.y % 16 == 0 && c.ldy % (c.out_f32 ? 4 : 8) == 0;
+  // more than 64 rows, GLU more than 32: pairs of CTAs (gemm_pair.cuh; both sides measured in gemm_tc.cu), but for few features or a short K, where tiles of theirs are too few or over
   // too soon (prompts of 1999 tokens at 8B sizes, a 128 x 256 tile per CTA / pairs: Matulorn 42.5 / 38.7 ms, Rigazen 40.2 / 34.3)
-  if (c.M > 128 && c.epilogue == JG_DENSE_GLU)
-    return launch_pair<DensePairEpi<true>>(dev, "dense_pair", c.x, c.ldx, c.w[0], c.w[1], c.ldw, c.M, c.N, c.K, true, a.w_late, {a.y, a.y32, a.b0, a.b1, a.ldy, a.limit, a.out});
-  if (c.M > 128 && c.N > 512 && c.K > 512)
-    return launch_pair<DensePairEpi<false>>(dev, "dense_pair", c.x, c.ldx, c.w[0], c.w[0], c.ldw, c.M, c.N, c.K, true, a.w_late, {a.y, a.y32, a.b0, a.b1, a.ldy, a.limit, a.out});
+  if (c.M > 32 && c.epilogue == JG_DENSE_GLU)
+    return launch_pair<DensePairEpi<true>>(dev, "dense_pair", c.x, c.ldx, c.w[0], c.w[1], c.ldw, c.M, c.N, c.K, true, a.w_late, {a.y, a.y32, a.b0, a.b1, a.ldy, aligned, a.limit, a.out});
+  if (c.M > 64 && c.N > 512 && c.K > 512)
+    return launch_pair<DensePairEpi<false>>(dev, "dense_pair", c.x, c.ldx, c.w[0], c.w[0], c.ldw, c.M, c.N, c.K, true, a.w_late, {a.y, a.y32, a.b0, a.b1, a.ldy, aligned, a.limit, a.out});
   if (c.epilogue == JG_DENSE_GLU) {
     if (c.M <= 16) return launch_dt<16, true, false>(dev, c, a);
-    if (c.M <= 32) return launch_dt<32, true, false>(dev, c, a);
-    if (c.M <= 64) return launch_dt<64, true, false>(dev, c, a);
-    return launch_dt<128, true, false>(dev, c, a);
+    return launch_dt<32, true, false>(dev, c, a);
   }
   if (c.M <= 16) return launch_dt<16, false, true>(dev, c, a);
   if (c.M <= 32) return launch_dt<32, false, true>(dev, c, a);

@@ -114,10 +114,66 @@ struct PairWork {
   }
 };
 
-// Epi: GLU (two interleaved matrices), BF16, Args, Extra, and
-//   fetch(args, plan, feat, tok, n, extra)    what the store adds to tokens tok ... tok + n - 1, requested ahead
-//   store(args, plan, feat, tok, n, r, extra) r[j] = accumulator of token tok + j, j < n <= 16, one feature per lane
-//   glu(args, plan, feat, tok, gate, up)      one value (GLU)
+// Between lanes = features and lanes = tokens, so that a lane stores 16 bytes of a row.  A lane has the values of its feature for
+// 16 tokens (pairs of 16-bit values, or 32-bit ones) and ends up with those of 8 features (lane & ~7 ...) for tokens lane & 7 and
+// 8 + (lane & 7); of 4 features for tokens 4 m + (lane & 3).  Stores of 2 bytes per lane took 7.5 cycles an instruction: 7600
+// cycles for a 256 x 256 tile at the end of a launch.
+__device__ __forceinline__ uint32_t swap_lanes(uint32_t send, int bit) { return __shfl_xor_sync(0xffffffffu, send, bit); }
+template <int NP>  // NP packed pairs: 8 (16 tokens) or 4 (8 tokens)
+__device__ __forceinline__ void transpose_16bit(const uint32_t (&p)[NP], uint32_t (&o)[NP / 4][4], int lane) {
+  const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4;
+  uint32_t q[NP], m[NP / 2][2];
+#pragma unroll
+  for (int i = 0; i < NP; i += 2) {  // two features of token 2 i + (lane & 1)
+    const uint32_t got = swap_lanes(b0 ? __byte_perm(p[i], p[i + 1], 0x5410) : __byte_perm(p[i], p[i + 1], 0x7632), 1);
+    q[i] = b0 ? __byte_perm(got, p[i], 0x7610) : __byte_perm(p[i], got, 0x5410);
+    q[i + 1] = b0 ? __byte_perm(got, p[i + 1], 0x7632) : __byte_perm(p[i + 1], got, 0x7610);
+  }
+#pragma unroll
+  for (int i = 0; i < NP; i += 2) {  // four
+    const uint32_t got = swap_lanes(b1 ? q[i] : q[i + 1], 2);
+    m[i / 2][0] = b1 ? got : q[i];
+    m[i / 2][1] = b1 ? q[i + 1] : got;
+  }
+#pragma unroll
+  for (int i = 0; i < NP / 2; i += 2)  // eight
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const uint32_t got = swap_lanes(b2 ? m[i][k] : m[i + 1][k], 4);
+      o[i / 2][k] = b2 ? got : m[i][k];
+      o[i / 2][2 + k] = b2 ? m[i + 1][k] : got;
+    }
+}
+__device__ __forceinline__ void transpose_32bit(const float (&r)[16], float4 (&o)[4], int lane) {
+  const bool b0 = lane & 1, b1 = lane & 2;
+  float q[8][2];
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const float got = __shfl_xor_sync(0xffffffffu, b0 ? r[2 * i] : r[2 * i + 1], 1);
+    q[i][0] = b0 ? got : r[2 * i];
+    q[i][1] = b0 ? r[2 * i + 1] : got;
+  }
+#pragma unroll
+  for (int m = 0; m < 4; m++) {
+    float w[4];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const float got = __shfl_xor_sync(0xffffffffu, b1 ? q[2 * m][k] : q[2 * m + 1][k], 2);
+      w[k] = b1 ? got : q[2 * m][k];
+      w[2 + k] = b1 ? q[2 * m + 1][k] : got;
+    }
+    o[m] = make_float4(w[0], w[1], w[2], w[3]);
+  }
+}
+
+// Epi: GLU (two interleaved matrices), BF16, RESIDUAL, Args, and
+//   wide(args, plan, feat)                whether the 32 (GLU: 16) features from feat on are stored in 16-byte pieces of rows
+//   f32(args)                             results in 32 bits
+//   out32, out, residual(args, plan, tok, feat)   where they, 16-bit ones and what is added to these are
+//   value(args, plan, feat, tok, r)       what a 32-bit accumulator becomes ahead of the last rounding
+//   round(v) / add(x, residual)           its 16 bits / two of them plus two of the residual
+//   glu(args, feat, gate, up)             the 16 bits of a result (GLU)
+//   store(args, plan, feat, tok, v)       one value, where the features are not wide
 template <class Epi>
 __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,
                                                                   const __grid_constant__ CUtensorMap tm_x, const PairPlan a, const typename Epi::Args ea) {
@@ -232,57 +288,100 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
         if (__any_sync(0xffffffffu, v == 0)) { if (lane == 0) atomicCAS(a.err, 0, 3); break; }
       }
       const int feat0 = ((w.tile / a.tok_tiles) * 2 + (int)rank) * FEATS, tok0 = (w.tile % a.tok_tiles) * a.tn;
-      float* mine = a.slots + ((size_t)share * 2 + rank) * GP_SLOT + row;
-      const float* theirs = mine + 2 * GP_SLOT;  // the next share's
+      float4* mine = reinterpret_cast<float4*>(a.slots + ((size_t)share * 2 + rank) * GP_SLOT);
+      const float4* theirs = mine + 2 * GP_SLOT / 4;  // the next share's
       auto release = [&] {  // this warp's columns are read: the MMAs may have this half of tensor memory again
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(&acc_empty[buf]), 0));
       };
       if (part * 16 >= a.tn) release();
+      const int fw = feat0 + q * (Epi::GLU ? 16 : 32), feat = fw + (Epi::GLU ? lane & 15 : lane);  // the warp's features, the lane's
+      const bool wide = Epi::wide(ea, a, fw);
 #pragma unroll 1
       for (int c0 = part * 16; c0 < a.tn; c0 += GP_PARTS * 16) {
+        const int tok = tok0 + c0, wt = tok + (lane & 7), wf = fw + (lane & 24);
         // what the columns are added to is on its way while the accumulators come from tensor memory
-        const int feat = feat0 + (Epi::GLU ? q * 16 + (lane & 15) : row), n = min(16, a.M - tok0 - c0);
-        typename Epi::Extra extra;
-        if (!Epi::GLU && w.k0 == 0 && feat < a.N) Epi::fetch(ea, a, feat, tok0 + c0, n, extra);
-        float r[16], v[2][16];
+        uint4 res[2] = {};
+        if (Epi::RESIDUAL && wide && w.k0 == 0) {
+#pragma unroll
+          for (int i = 0; i < 2; i++)
+            if (wt + 8 * i < a.M) res[i] = *reinterpret_cast<const uint4*>(Epi::residual(ea, a, wt + 8 * i, wf));
+        }
+        float r[16];
+        float4 v[2][4];
+        const int at = c0 * 32 + row;  // [four columns][row] of a slot
 #pragma unroll
         for (int p = 0; p < 2; p++)
           if (p < parts) {
 #pragma unroll
-            for (int j = 0; j < 16; j++) v[p][j] = __ldcg(theirs + (size_t)p * 2 * GP_SLOT + (c0 + j) * 128);
+            for (int j = 0; j < 4; j++) v[p][j] = __ldcg(theirs + (size_t)p * (2 * GP_SLOT / 4) + at + j * 128);
           }
         tmem_ld16(t_lane + c0, r);
         if (c0 + GP_PARTS * 16 >= a.tn) release();
         if (w.k0 > 0) {
 #pragma unroll
-          for (int j = 0; j < 16; j++) __stcg(mine + (c0 + j) * 128, r[j]);
+          for (int j = 0; j < 4; j++) __stcg(mine + at + j * 128, make_float4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]));
           continue;
         }
+        auto plus = [&](const float4 (&x)[4]) {
 #pragma unroll
-        for (int p = 0; p < 2; p++)  // in order of k
-          if (p < parts) {
-#pragma unroll
-            for (int j = 0; j < 16; j++) r[j] = __fadd_rn(r[j], v[p][j]);
-          }
+          for (int j = 0; j < 4; j++) { r[4 * j] += x[j].x; r[4 * j + 1] += x[j].y; r[4 * j + 2] += x[j].z; r[4 * j + 3] += x[j].w; }
+        };
+        if (parts > 0) plus(v[0]);  // in order of k
+        if (parts > 1) plus(v[1]);
         for (int p = 2; p < parts; p++) {
 #pragma unroll
-          for (int j = 0; j < 16; j++) v[0][j] = __ldcg(theirs + (size_t)p * 2 * GP_SLOT + (c0 + j) * 128);
-#pragma unroll
-          for (int j = 0; j < 16; j++) r[j] = __fadd_rn(r[j], v[0][j]);
+          for (int j = 0; j < 4; j++) v[0][j] = __ldcg(theirs + (size_t)p * (2 * GP_SLOT / 4) + at + j * 128);
+          plus(v[0]);
         }
-        if (tok0 + c0 >= a.M) continue;
-        if (Epi::GLU) {
+        if (tok >= a.M) continue;
+        if constexpr (Epi::GLU) {
+          // lanes l and l + 16 have gate and up of a feature: the lower ones finish even columns, the upper ones odd ones
+          uint16_t y[8];
 #pragma unroll
-          for (int j = 0; j < 16; j += 2) {  // the lower lanes finish column j, the upper ones column j + 1
-            const float other = __shfl_xor_sync(0xffffffffu, lane < 16 ? r[j + 1] : r[j], 16);
-            const int tok = tok0 + c0 + j + (lane >> 4);
-            const float first = lane < 16 ? r[j] : other, second = lane < 16 ? other : r[j + 1];
-            if (tok < a.M && feat < a.N) Epi::glu(ea, a, feat, tok, a.glu_swap ? second : first, a.glu_swap ? first : second);
+          for (int j = 0; j < 8; j++) {
+            const float other = __shfl_xor_sync(0xffffffffu, lane < 16 ? r[2 * j + 1] : r[2 * j], 16);
+            const float first = lane < 16 ? r[2 * j] : other, second = lane < 16 ? other : r[2 * j + 1];
+            y[j] = Epi::glu(ea, min(feat, a.N - 1), a.glu_swap ? second : first, a.glu_swap ? first : second);
+          }
+          const int half = lane >> 4;
+          if (wide) {
+            uint32_t p[4], o[1][4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) p[j] = (uint32_t)y[2 * j] | ((uint32_t)y[2 * j + 1] << 16);
+            transpose_16bit<4>(p, o, lane);
+            const int t = tok + 2 * (lane & 7) + half;
+            if (t < a.M) *reinterpret_cast<uint4*>(Epi::out(ea, a, t, fw + (lane & 8))) = make_uint4(o[0][0], o[0][1], o[0][2], o[0][3]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+              if (feat < a.N && tok + 2 * j + half < a.M) *reinterpret_cast<uint16_t*>(Epi::out(ea, a, tok + 2 * j + half, feat)) = y[j];
+          }
+        } else if (wide) {
+#pragma unroll
+          for (int j = 0; j < 16; j++) r[j] = Epi::value(ea, a, feat, tok + j, r[j]);
+          if (Epi::f32(ea)) {
+            float4 o[4];
+            transpose_32bit(r, o, lane);
+#pragma unroll
+            for (int m = 0; m < 4; m++)
+              if (tok + 4 * m + (lane & 3) < a.M) *reinterpret_cast<float4*>(Epi::out32(ea, a, tok + 4 * m + (lane & 3), fw + (lane & 28))) = o[m];
+          } else {
+            uint32_t p[8], o[2][4];
+#pragma unroll
+            for (int j = 0; j < 8; j++) p[j] = (uint32_t)Epi::round(r[2 * j]) | ((uint32_t)Epi::round(r[2 * j + 1]) << 16);
+            transpose_16bit<8>(p, o, lane);
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+              if (Epi::RESIDUAL) { o[i][0] = Epi::add(o[i][0], res[i].x); o[i][1] = Epi::add(o[i][1], res[i].y); o[i][2] = Epi::add(o[i][2], res[i].z); o[i][3] = Epi::add(o[i][3], res[i].w); }
+              if (wt + 8 * i < a.M) *reinterpret_cast<uint4*>(Epi::out(ea, a, wt + 8 * i, wf)) = make_uint4(o[i][0], o[i][1], o[i][2], o[i][3]);
+            }
           }
         } else if (feat < a.N) {
-          Epi::store(ea, a, feat, tok0 + c0, n, r, extra);
+#pragma unroll
+          for (int j = 0; j < 16; j++)
+            if (tok + j < a.M) Epi::store(ea, a, feat, tok + j, Epi::value(ea, a, feat, tok + j, r[j]));
         }
       }
       if (w.k0 > 0) {
@@ -304,23 +403,27 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
   }
 }
 
-// Tiles and shares with the smallest estimate, in SM cycles.  Measured at 8B shapes, 200 to 2048 rows: a k-block takes 330
-// (128 rows to a tile), 410 (192) and 530 (256); a tile's stores 4000 + 30 per row; a second share 3000 + 28 per row, each
-// further one half of that.  Cutting whole rounds and their remainder into equal shares gained nothing at 1024 rows and more,
-// where the power limit decides (gate and up, 1024 rows: 174 us in whole tiles, 178 in equal shares).
+// Tiles and shares with the smallest estimate, in SM cycles.  Measured at 1B and 8B shapes, 45 to 2048 rows: a k-block takes 300
+// (up to 96 rows to a tile), 330 (128), 410 (192) and 530 (256), or as long as its weights need from HBM (9.6 for each pair that
+// fetches other weights); a launch and its last tile's stores 4000 + 60 per row; a second share 5000 + 16 per row, each further
+// one 400 + 8 per row.  us, 8B shapes, 200 rows, the plans taken / whole 256-row tiles: qkv 17.7 / 26.0, wo 16.2 / 27.5, gate and
+// up 56.8 / 59.7, down 35.7 / 82.0.  Cutting whole rounds and their remainder into equal shares gained nothing at 1024 rows and
+// more, where the power limit decides (gate and up, 1024 rows: 174 us in whole tiles, 178 in equal shares).
 static inline void pair_plan(PairPlan& a, int feat_tiles, int P, bool shares) {
   float best = 0.f;
-  for (int tn = 256; tn >= 64; tn -= 32) {
+  for (int tn = 256; tn >= 32; tn -= 32) {
     const int tok = (a.M + tn - 1) / tn, T = tok * feat_tiles, waves = (T + P - 1) / P;
-    const float kb = fmaxf(130.f + 1.57f * (float)tn, 300.f);
     for (int s = 1; s == 1 || (shares && s <= 4 && s * T <= P && a.n_kb >= 8 * s); s++) {
+      const int pairs = s == 1 ? (T < P ? T : P) : s * T;
+      const float kb = fmaxf(fmaxf(130.f + 1.57f * (float)tn, 300.f), 9.6f * (float)pairs / (float)tok);
       // the others' accumulators are written while the first share is still at work
-      const int ahead = (int)(12.f * (float)tn / kb), head = s == 1 ? a.n_kb : (a.n_kb + (s - 1) * ahead) / s;
+      const int ahead = (int)(8.f * (float)tn / kb), head = s == 1 ? a.n_kb : (a.n_kb + (s - 1) * ahead) / s;
       if (s > 1 && a.n_kb - head < 2 * (s - 1)) break;
-      const float t = (float)(waves * head) * kb + 4000.f + 30.f * (float)tn + (s == 1 ? 0.f : (3000.f + 28.f * (float)tn) * (0.5f * (float)s));
+      float t = (float)(waves * head) * kb + 4000.f + 60.f * (float)tn;
+      if (s > 1) t += 5000.f + 16.f * (float)tn + (float)(s - 2) * (400.f + 8.f * (float)tn);
       if (best != 0.f && t >= best) continue;
       best = t;
-      a.tn = tn; a.tok_tiles = tok; a.tiles = T; a.pairs = s == 1 ? (T < P ? T : P) : s * T; a.split = s; a.head = head;
+      a.tn = tn; a.tok_tiles = tok; a.tiles = T; a.pairs = pairs; a.split = s; a.head = head;
     }
   }
 }

@@ -295,33 +295,32 @@ __global__ void __launch_bounds__(TcCfg<TN, EPI, W8, HALF>::THREADS, HALF ? 2 : 
 // What the paired kernel (gemm_pair.cuh) does with an accumulator: the same roundings as above.
 template <int EPI>
 struct TcPairEpi {
-  static constexpr bool GLU = EPI == TC_SWIGLU, BF16 = false;
+  static constexpr bool GLU = EPI == TC_SWIGLU, BF16 = false, RESIDUAL = EPI == TC_RESIDUAL;
   struct Args {
     __half* y;
     float* y32;
     const __half* residual;
+    int aligned;  // results (and residual) start on 16 bytes
   };
-  struct Extra { __half residual[16]; };
-  // all loads ahead of the stores: Y may alias the residual
-  static __device__ __forceinline__ void fetch(const Args& e, const PairPlan& a, int feat, int tok, int n, Extra& x) {
-    if (EPI != TC_RESIDUAL) return;
-    const __half* p = e.residual + (size_t)tok * a.N + feat;
-#pragma unroll
-    for (int j = 0; j < 16; j++) x.residual[j] = j < n ? p[(size_t)j * a.N] : __float2half_rn(0.f);
+  static __device__ __forceinline__ bool wide(const Args& e, const PairPlan& a, int feat) { return e.aligned && feat + 32 <= a.N; }
+  static __device__ __forceinline__ bool f32(const Args&) { return EPI == TC_PARTIAL; }
+  static __device__ __forceinline__ float* out32(const Args& e, const PairPlan& a, int tok, int feat) { return e.y32 + (size_t)tok * a.N + feat; }
+  static __device__ __forceinline__ __half* out(const Args& e, const PairPlan& a, int tok, int feat) { return e.y + (size_t)tok * a.N + feat; }
+  static __device__ __forceinline__ const __half* residual(const Args& e, const PairPlan& a, int tok, int feat) { return e.residual + (size_t)tok * a.N + feat; }
+  static __device__ __forceinline__ float value(const Args&, const PairPlan&, int, int, float r) { return r; }
+  static __device__ __forceinline__ uint16_t round(float v) { return __half_as_ushort(__float2half_rn(v)); }
+  static __device__ __forceinline__ uint32_t add(uint32_t v, uint32_t res) {
+    const __half2 h = __hadd2_rn(*reinterpret_cast<const __half2*>(&res), *reinterpret_cast<const __half2*>(&v));
+    return *reinterpret_cast<const uint32_t*>(&h);
   }
-  static __device__ __forceinline__ void store(const Args& e, const PairPlan& a, int feat, int tok, int n, const float (&r)[16], const Extra& x) {
-    const size_t o = (size_t)tok * a.N + feat;
-#pragma unroll
-    for (int j = 0; j < 16; j++) {
-      if (j >= n) break;
-      if (EPI == TC_PARTIAL) { e.y32[o + (size_t)j * a.N] = r[j]; continue; }
-      __half v = __float2half_rn(r[j]);
-      if (EPI == TC_RESIDUAL) v = hadd1(x.residual[j], v);
-      e.y[o + (size_t)j * a.N] = v;
-    }
+  static __device__ __forceinline__ uint16_t glu(const Args&, int, float gate, float up) {
+    return __half_as_ushort(jg_silu_mul(__float2half_rn(gate), __float2half_rn(up)));
   }
-  static __device__ __forceinline__ void glu(const Args& e, const PairPlan& a, int feat, int tok, float gate, float up) {
-    e.y[(size_t)tok * a.N + feat] = jg_silu_mul(__float2half_rn(gate), __float2half_rn(up));
+  static __device__ __forceinline__ void store(const Args& e, const PairPlan& a, int feat, int tok, float v) {
+    if (EPI == TC_PARTIAL) { *out32(e, a, tok, feat) = v; return; }
+    __half h = __float2half_rn(v);
+    if (EPI == TC_RESIDUAL) h = hadd1(*residual(e, a, tok, feat), h);
+    *out(e, a, tok, feat) = h;
   }
 };
 
@@ -366,8 +365,9 @@ static int launch_tc(jg_dev* dev, const void* x, const void* w0, const void* w1,
     }
   } else {
     // half-size rings (two CTAs per SM): CTAs for four thirds of the SMs, but no more than four to a tile — beyond
-    // that the cluster reduction costs more than the shorter streams save (wo at 32 rows: 18.5 us split in 4, 20.5 in 7)
-    while (ks < (HALF ? 4 : 8) && ks < Cfg::MAX_KS && tiles * ks * 3 < dev->sm_count * 2 * (HALF ? 2 : 1) && n_kb / (ks + 1) >= 8) ks++;
+    // that the cluster reduction costs more than the shorter streams save (wo at 32 rows: 18.5 us split in 4, 20.5 in 7;
+    // 1B down projection, 45 rows, full rings: 23 us split in 7)
+    while (ks < (tiles > 8 ? 4 : 8) && ks < Cfg::MAX_KS && tiles * ks * 3 < dev->sm_count * 2 * (HALF ? 2 : 1) && n_kb / (ks + 1) >= 8) ks++;
   }
   if (ks_env >= 1 && ks_env <= 8 && ks_env <= Cfg::MAX_KS && n_kb / ks_env >= 1) ks = ks_env;
   dev->tc_pending = true;
@@ -399,10 +399,12 @@ static int launch_tc(jg_dev* dev, const void* x, const void* w0, const void* w1,
 
 template <int EPI>
 static int launch_tc_rows(jg_dev* dev, const void* x, const void* w0, const void* w1, const TcArgs& a) {
-  // more than 128 rows: pairs of CTAs (8B shapes, us per launch, one 128 x 256 tile per CTA / pairs: 512 rows qkv 37 / 24, wo 35 / 22,
-  // gate and up 140 / 105, down 70 / 59; 2048 rows gate and up 431 / 365)
-  if (a.s0 == nullptr && a.M > 128)
-    return launch_pair<TcPairEpi<EPI>>(dev, "gemm_pair", x, a.K, w0, w1, a.K, a.M, a.N, a.K, false, a.w_late, {a.y, a.y32, a.residual});
+  // more than 64 rows, gate and up more than 32: pairs of CTAs.  us per launch, one tile per CTA / pairs: 8B shapes, 45 rows qkv 19 / 15,
+  // wo 12 / 13, gate and up 45 / 44, down 25 / 28; 100 rows 23 / 17, 16 / 15, 48 / 48, 29 / 31; 512 rows 37 / 24, 35 / 19, 140 / 102,
+  // 70 / 54; 1B shapes, 45 rows 8 / 9, 9 / 10, 22 / 16, 15 / 15; 100 rows 11 / 10, 11 / 10, 25 / 18, 17 / 16
+  if (a.s0 == nullptr && a.M > (EPI == TC_SWIGLU ? 32 : 64))
+    return launch_pair<TcPairEpi<EPI>>(dev, "gemm_pair", x, a.K, w0, w1, a.K, a.M, a.N, a.K, false, a.w_late, 
+                                        {a.y, a.y32, a.residual, (uintptr_t)a.y % 16 == 0 && (uintptr_t)a.residual % 16 == 0});
   if (a.s0 != nullptr) {  // int8 weights: used from 20 rows on (fewer go to the mma.sync kernel)
     if (a.M <= 32) return launch_tc<32, EPI, true>(dev, x, w0, w1, a);
     if (a.M <= 128) return launch_tc<128, EPI, true>(dev, x, w0, w1, a);
@@ -421,8 +423,7 @@ static int launch_tc_rows(jg_dev* dev, const void* x, const void* w0, const void
   }
   if (a.M <= 16) return launch_tc<16, EPI>(dev, x, w0, w1, a);
   if (a.M <= 32) return launch_tc<32, EPI>(dev, x, w0, w1, a);
-  if (a.M <= 64) return launch_tc<64, EPI>(dev, x, w0, w1, a);
-  return launch_tc<128, EPI>(dev, x, w0, w1, a);
+  return launch_tc<64, EPI>(dev, x, w0, w1, a);
 }
 
 // Whether jg_gemm_tc takes this shape: fp16 weights, whole 128-row weight tiles and 64-wide k-blocks.
