@@ -343,17 +343,27 @@ __global__ void glu_f32_kernel(float* __restrict__ y, const float* __restrict__ 
   }
 }
 
-// (value, lowest index) keys of fp32 rows; one CTA per row
-__global__ void __launch_bounds__(256) key_f32_kernel(unsigned long long* __restrict__ key, const float* __restrict__ x, int n, int ld) {
-  __shared__ unsigned long long red[8];
+// (value, lowest index) keys of fp32 rows; one CTA per row, which has to have many loads in flight (eight rows of 128256, 256
+// threads with a value at a time: 48 us)
+constexpr int KEY_THREADS = 1024;
+__global__ void __launch_bounds__(KEY_THREADS) key_f32_kernel(unsigned long long* __restrict__ key, const float* __restrict__ x, int n, int ld) {
+  __shared__ unsigned long long red[KEY_THREADS / 32];
   pdl_launch();
   pdl_wait();
   const float* xr = x + (size_t)blockIdx.x * ld;
   unsigned long long b = 0ull;
-  for (int i = threadIdx.x; i < n; i += 256) {
-    const unsigned long long k = argmax_key_f32(xr[i], (uint32_t)i);
+  auto take = [&](float v, int i) {
+    const unsigned long long k = argmax_key_f32(v, (uint32_t)i);
     b = k > b ? k : b;
+  };
+  const int n4 = reinterpret_cast<uintptr_t>(xr) % 16 == 0 ? n / 4 : 0;
+#pragma unroll 8
+  for (int i = threadIdx.x; i < n4; i += KEY_THREADS) {
+    const float4 v = reinterpret_cast<const float4*>(xr)[i];
+    take(v.x, 4 * i); take(v.y, 4 * i + 1); take(v.z, 4 * i + 2); take(v.w, 4 * i + 3);
   }
+#pragma unroll 4
+  for (int i = 4 * n4 + threadIdx.x; i < n; i += KEY_THREADS) take(xr[i], i);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const unsigned long long other = __shfl_xor_sync(0xffffffffu, b, o);
@@ -362,7 +372,7 @@ __global__ void __launch_bounds__(256) key_f32_kernel(unsigned long long* __rest
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = b;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int i = 1; i < 8; i++) b = red[i] > b ? red[i] : b;
+    for (int i = 1; i < KEY_THREADS / 32; i++) b = red[i] > b ? red[i] : b;
     key[blockIdx.x] = b;
   }
 }
@@ -465,7 +475,7 @@ int jg_dense_call(jg_dev* dev, const DenseCall& c) {
     rc = f32_gemm(dev, c, c.w[0], c.bias[0], (float*)c.y, c.ldy);
   }
   if (rc || c.epilogue != JG_DENSE_LOGITS) return rc;
-  return jg_launch(dev, "key_f32", key_f32_kernel, dim3((unsigned)c.M), dim3(256), 0, c.key, (const float*)c.y, c.N, c.ldy);
+  return jg_launch(dev, "key_f32", key_f32_kernel, dim3((unsigned)c.M), dim3(KEY_THREADS), 0, c.key, (const float*)c.y, c.N, c.ldy);
 }
 
 static int check_batch(const char* name, const jg_batch* b) {
