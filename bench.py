@@ -437,7 +437,7 @@ def prefill_leg(rig: Rig, llm, B: int, P: int, int8: bool, reps: int = 3) -> dic
     return {"tok_s": B * P / pf, "ms": pf * 1e3, "prompt_tokens": P, "batch": B, "tflops_per_gpu": fl / pf / 1e12,
             "frac_of_measured_bf16_peak": fl / pf / 1e12 / tf,
             "flops": "layers on all rows + output matrix on the last row + causal attention",
-            "how": ("Transformer.forward over the whole prompt in chunks of up to 2048 rows: tcgen05/TMA projections"
+            "how": ("Transformer.forward over the whole prompt in chunks of up to 4096 rows: tcgen05/TMA projections"
                     + (" over int8 weights" if int8 else "") + ", tensor-core causal attention")}
 
 

@@ -326,8 +326,8 @@ export class CudaTransformer {
       this.decode_step(wsb)
       return await this.pick(wsb, temperature, top_k, top_p, alpha_f, alpha_p)
     }
-    // several positions: chunks of up to 2048 rows, position-major (row = s * bsz + b)
-    const per = Math.max(1, Math.trunc(2048 / bsz))
+    // several positions: chunks of up to 4096 rows, position-major (row = s * bsz + b)
+    const per = Math.max(1, Math.trunc(4096 / bsz))
     for (let s0 = 0; s0 < seqlen; s0 += per) {
       const sc = Math.min(per, seqlen - s0), R = bsz * sc, ws = this.workspace(R, false), dev = this.dev
       const flat: number[] = [], pos: number[] = [], seq: number[] = []
