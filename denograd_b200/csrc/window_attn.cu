@@ -6,7 +6,8 @@
 //                   warp runs through its own tiles of 16 positions.  One token: it writes the cache row itself
 //   window_split    the same for one head on the CUDA cores (fp32, and sizes the other does not take)
 //   window_combine  context slices -> output
-//   window_chunk    bf16 prompt portions: 64 or 128 queries of a head against tiles of 64 keys, one pass
+//   window_flash    longer bf16 portions, heads of 64 or 128: flash_tc.cuh (tcgen05) over the paged ring
+//   window_chunk    other bf16 prompt portions: 64 or 128 queries of a head against tiles of 64 keys, one pass
 //
 // What a row sees is two runs of positions, the kept first ones and the window; both are numbered through (`Seen`), so tiles and
 // slices go over one index.  Scores, softmax statistics and weights are fp32; on the tensor cores the weights meet the
@@ -14,6 +15,7 @@
 #include <math.h>
 #include <stddef.h>
 
+#include "flash_tc.cuh"
 #include "mma.cuh"
 
 template <typename T>
@@ -592,8 +594,94 @@ __global__ void __launch_bounds__(32 * NW, VT <= 16 ? (NW == 8 ? 2 : 3) : 1) win
   }
 }
 
+// ------------------------------------------------------------------------------------------------ long prompt portions
+// 128-row tiles: the heads of a kv head times consecutive tokens.  Key tiles are runs of 128 positions from a multiple of 128 on, those
+// with kept tokens first and then the window's; a tile's other positions are masked (their places in the ring hold some
+// token's keys and values, all of them written), and values past the last token are zeroed.
+template <int D, bool SPLIT>
+struct WindowPolicy {
+  static constexpr int DK = D, DV = D;
+  static constexpr bool BF16 = true;
+  const WinArgs<bf16>& a;
+  const CUtensorMap* map;
+  int tiles, b, kv, per, pt, s0, p_lo, kept, first, written, q_pos, q_from;
+  uint32_t seen[4];
+  bool valid;
+  const int32_t* bt;
+  float scale2;
+  __device__ WindowPolicy(const WinArgs<bf16>& a_, const CUtensorMap* m) : a(a_), map(m) {}
+  __device__ __forceinline__ bool begin() {
+    per = a.H / a.G;
+    pt = FT_ROWS / per;
+    const int n = pt * (SPLIT ? 1 : 2), qt = (int)gridDim.x - 1 - (int)blockIdx.x;  // long rows first
+    kv = blockIdx.y;
+    b = blockIdx.z;
+    s0 = qt * n;
+    const int p0 = a.pos[b], last = p0 + min(s0 + n, a.Sc) - 1;
+    if (p0 < 0 || last >= a.rot_rows) return false;
+    p_lo = p0 + s0;
+    written = min(p0 + a.Sc, a.rot_rows);
+    first = (a.window > 0 ? max(0, p_lo - a.window + 1) : 0) / FT_KV;  // the window's first tile
+    kept = min((a.keep + FT_KV - 1) / FT_KV, first);                   // tiles ahead of it
+    tiles = kept + last / FT_KV + 1 - first;
+    bt = a.bt + (size_t)a.seq[b] * a.pps;
+    scale2 = a.scale * LOG2E;
+    return true;
+  }
+  __device__ __forceinline__ int start(int j) const { return (j < kept ? j : first + j - kept) * FT_KV; }
+  __device__ __forceinline__ int token(int stream, int r) const { return s0 + stream * pt + r / per; }
+  template <typename F>
+  __device__ __forceinline__ void q_row(int stream, int r, F dst) const {
+    const bf16* q = a.qs + (((size_t)min(token(stream, r), a.Sc - 1) * a.B + b) * a.H + kv * per + r % per) * a.dk8;
+#pragma unroll
+    for (int c = 0; c < D / 8; c++) dst(c, ld_128(q + c * 8));
+  }
+  __device__ __forceinline__ void rows(int stream, int r) {
+    const int s = token(stream, r);
+    valid = s < a.Sc;
+    q_pos = p_lo - s0 + min(s, a.Sc - 1);
+    q_from = a.window > 0 ? max(0, q_pos - a.window + 1) : 0;
+  }
+  static __device__ __forceinline__ uint32_t below(int n) { return n <= 0 ? 0u : n >= 32 ? ~0u : (1u << n) - 1u; }
+  __device__ __forceinline__ bool all(int j) {  // and the tile's columns that the row sees, as bits (comparisons per column spilt registers)
+    const int from = start(j);
+#pragma unroll
+    for (int w = 0; w < 4; w++) {
+      const int at = from + 32 * w;
+      seen[w] = below(q_pos + 1 - at) & (~below(q_from - at) | below(a.keep - at));
+    }
+    return (seen[0] & seen[1] & seen[2] & seen[3]) == ~0u;
+  }
+  __device__ __forceinline__ bool sees(int, int c) const { return seen[c >> 5] >> (c & 31) & 1u; }
+  __device__ __forceinline__ float extra2() const { return -INFINITY; }
+  __device__ __forceinline__ int dead(int j) const { return min(FT_KV, written - start(j)); }
+  __device__ __forceinline__ void load(int col, int j, unsigned char* dst, uint64_t* bar, int lane) const {
+    constexpr int KB = D / 64;
+    const int n = min(a.page, FT_KV), run = lane / KB, block = lane % KB;
+    if (run * n >= FT_KV) return;
+    const uint32_t row = a.row_number(bt, min(start(j) + run * n, (written - 1) / n * n));  // past the end: some page, masked
+    tma_load_2d(dst + block * (FT_KV * 128) + run * n * 128, map, col + block * 64, (int)row, bar);
+  }
+  __device__ __forceinline__ void load_k(int j, unsigned char* dst, uint64_t* bar, int lane) const { load(kv * D, j, dst, bar, lane); }
+  __device__ __forceinline__ void load_v(int j, unsigned char* dst, uint64_t* bar, int lane) const { load((a.G + kv) * D, j, dst, bar, lane); }
+  __device__ __forceinline__ void store(int stream, int r, const float* o, int c) const {
+    if (!valid) return;
+    bf16* out = a.out + ((size_t)token(stream, r) * a.B + b) * a.ldo + (size_t)(kv * per + r % per) * D + c;
+    const float f = a.out_scale;
+#pragma unroll
+    for (int k = 0; k < 32; k += 8)
+      *reinterpret_cast<uint4*>(out + k) = make_uint4(pack_bf16(o[k] * f, o[k + 1] * f), pack_bf16(o[k + 2] * f, o[k + 3] * f), pack_bf16(o[k + 4] * f, o[k + 5] * f),
+                                                      pack_bf16(o[k + 6] * f, o[k + 7] * f));
+  }
+};
+template <int D, bool SPLIT>
+__global__ void __launch_bounds__(FT_THREADS, 1) window_flash_kernel(const __grid_constant__ CUtensorMap map, const WinArgs<bf16> a, int* err) {
+  WindowPolicy<D, SPLIT> p(a, &map);
+  flash_tc<WindowPolicy<D, SPLIT>, SPLIT>(p, err);
+}
+
 // ------------------------------------------------------------------------------------------------ host side
-constexpr int WINDOW_MIN_CHUNK = 16, WINDOW_MAX_PARTS = 32 * 160;
+constexpr int WINDOW_MIN_CHUNK = 16, WINDOW_MIN_FLASH = 256, WINDOW_MAX_PARTS = 32 * 160;
 static bool on_tensor_cores(const jg_window_desc* d) { return d->dtype == JG_BF16 && d->dim <= 256 && d->vdim <= 256; }
 static bool in_chunks(const jg_window_desc* d, int Sc) { return on_tensor_cores(d) && Sc >= WINDOW_MIN_CHUNK; }
 static int heads_per_cta(const jg_window_desc* d) { return on_tensor_cores(d) ? (d->heads / d->kv_heads < 16 ? d->heads / d->kv_heads : 16) : 1; }
@@ -648,10 +736,44 @@ static int launch_wx_rows(jg_dev* dev, const WinArgs<bf16>& a, int qkp) {
   return launch_wx<VT, 4>(dev, a, qkp);
 }
 
+// Portions that window_flash takes: equal heads of 64 or 128 whose number per kv head divides a tile, pages that a tile's runs fit, results
+// in 16-byte pieces, and tokens enough (us, cache writes included, window_flash / window_chunk; 32 heads on 8: 128 tokens 15.7 / 15.7, 256
+// 19.7 / 22.0, 512 25.9 / 34.2, 1024 59 / 85, 1999 135 / 252; 16 on 4, eight sequences of 128 21.5 / 21.1, of 256 41.9 / 40.2).
+static bool flash_fits(const WinArgs<bf16>& a) {
+  const int per = a.H / a.G;
+  return a.Sc >= WINDOW_MIN_FLASH && a.dim == a.vd && (a.dim == 64 || a.dim == 128) && per <= FT_ROWS && FT_ROWS % per == 0 && a.page >= 8 && a.ldo % 8 == 0 &&
+         (uintptr_t)a.out % 16 == 0 && a.G <= 65535 && a.B <= 65535;
+}
+template <int D, bool SPLIT>
+static int launch_flash(jg_dev* dev, const WinArgs<bf16>& a, const CUtensorMap& map) {
+  auto kern = window_flash_kernel<D, SPLIT>;
+  const size_t smem = FtCfg<D, D, SPLIT>::SMEM;
+  static bool set[8] = {};
+  if (!set[dev->ordinal & 7]) {
+    JG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    set[dev->ordinal & 7] = true;
+  }
+  const int n = FT_ROWS / (a.H / a.G) * (SPLIT ? 1 : 2);
+  dev->tc_pending = true;
+  return jg_launch(dev, "window_flash", kern, dim3((unsigned)((a.Sc + n - 1) / n), (unsigned)a.G, (unsigned)a.B), dim3(FT_THREADS), smem, map, a, dev->err_word);
+}
+template <int D>
+static int run_flash(jg_dev* dev, const WinArgs<bf16>& a) {
+  int rc = jg_tc_error_word(dev);
+  if (rc) return rc;
+  CUtensorMap map;  // as many rows as any GPU holds: the block table says which there are
+  rc = jg_tensor_map(&map, a.pool, (1ull << 38) / (2ull * a.row_size()), a.row_size(), a.row_size(), a.page < FT_KV ? a.page : FT_KV, "cached keys and values", 2, true);
+  if (rc) return rc;
+  const int n = FT_ROWS / (a.H / a.G) * 2;
+  // pairs of query tiles where they give every SM a CTA; below that the key tiles of single ones are split between the streams
+  return (long long)((a.Sc + n - 1) / n) * a.G * a.B >= dev->sm_count ? launch_flash<D, false>(dev, a, map) : launch_flash<D, true>(dev, a, map);
+}
+
 static int run_chunks(jg_dev*, const WinArgs<float>&) { return JG_ENOTSUP; }
 static int run_chunks(jg_dev* dev, const WinArgs<bf16>& a) {
   int rc = jg_launch(dev, "window_write", window_write_kernel<bf16>, dim3((unsigned)(a.B * a.Sc)), dim3(256), 0, a, 1);
   if (rc) return rc;
+  if (flash_fits(a) && (dev->err_word != nullptr || !dev->capturing)) return a.dim == 64 ? run_flash<64>(dev, a) : run_flash<128>(dev, a);
   const int qkp = (a.dim + 15) & ~15;
   if (a.vd <= 64) return launch_wx_rows<8>(dev, a, qkp);
   if (a.vd <= 128) return launch_wx_rows<16>(dev, a, qkp);

@@ -77,3 +77,16 @@ def test_bf16_epilogues(dev, M, N, K, glu):
         got[:M, split:N] = y2.numpy()[:M, :N - split]
         assert (y2.numpy()[M:] == 0).all()
     assert (np.abs(got[:M, :N] - a) <= off).all() and (got[M:] == 0).all() and (got[:, N:] == 0).all()
+
+
+def test_silu_of_every_gate(dev):
+    """Both forms of the fp16 exponential: every 16-bit gate, bit for bit."""
+    g = np.arange(1 << 16, dtype=np.uint32).astype(np.uint16).view(np.float16)
+    g = g[np.isfinite(g)]
+    for up in (1.0, -0.37):
+        u = np.full(g.shape, up, np.float16)
+        y, gt, ut = Tensor.zeros(g.shape, "float16", dev), Tensor(g, device=dev), Tensor(u, device=dev)
+        dev.call("jg_swiglu", y.ptr, gt.ptr, ut.ptr, g.size)
+        want = O.swiglu(g[None], u[None])[0]
+        got = y.numpy()
+        assert ((got.view(np.uint16) == want.view(np.uint16)) | (np.isnan(got) & np.isnan(want))).all()
