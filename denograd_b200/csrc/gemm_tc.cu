@@ -129,7 +129,9 @@ __global__ void __launch_bounds__(TcCfg<TN, EPI, W8, HALF>::THREADS, HALF ? 2 : 
   const uint32_t tmem_base = s_tmem;
   bool acc_ok = false;
 
-  if (warp == 0) {
+  // int8 weights keep the issue loops of one lane: with all lanes in them, passes of 100 rows were seen to stop
+  auto leader = [] { if constexpr (W8) return true; else return elect_one(); };
+  if (warp == 0 && (!W8 || lane == 0)) {
     // ---- producer.  Weights do not depend on the preceding kernel: the first tiles are requested before the wait.
     const int pre = nk < STAGES ? nk : STAGES;
     if (a.w_late) pdl_wait();
@@ -148,10 +150,10 @@ __global__ void __launch_bounds__(TcCfg<TN, EPI, W8, HALF>::THREADS, HALF ? 2 : 
         if (NW == 2) tma_load_2d(st + A_BYTES, &tm_w1, (kb0 + i) * TC_BK, feat0, &full_bar[s]);
       }
     };
-    if (elect_one())
+    if (leader())
       for (int i = 0; i < pre; i++) load_w(i, i);
     pdl_wait();  // X comes from the previous kernel
-    if (elect_one())
+    if (leader())
       for (int i = 0; i < pre; i++)
         tma_load_2d(tiles + (size_t)i * STAGE_BYTES + NW * A_BYTES, &tm_x, (kb0 + i) * TC_BK, tok0, &full_bar[i]);
     for (int i = pre; i < nk; i++) {
@@ -159,12 +161,12 @@ __global__ void __launch_bounds__(TcCfg<TN, EPI, W8, HALF>::THREADS, HALF ? 2 : 
       // the MMAs of the stage's previous use are done: its A and B tiles are free, and so is its raw tile (converted
       // before those MMAs could start)
       if (!mbar_wait(&empty_bar[s], ((i / STAGES) - 1) & 1)) { atomicCAS(a.err, 0, 1); break; }
-      if (elect_one()) {
+      if (leader()) {
         load_w(i, s);
         tma_load_2d(tiles + (size_t)s * STAGE_BYTES + NW * A_BYTES, &tm_x, (kb0 + i) * TC_BK, tok0, &full_bar[s]);
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == 1 && (!W8 || lane == 0)) {
     // ---- MMA issuer: 4 x (128 x TN x 16) per stage and matrix, accumulating in tensor memory
     const uint32_t idesc = (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);  // f32 acc, f16 x f16, K-major both
     bool ok = true;
@@ -178,7 +180,7 @@ __global__ void __launch_bounds__(TcCfg<TN, EPI, W8, HALF>::THREADS, HALF ? 2 : 
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       unsigned char* st = tiles + (size_t)s * STAGE_BYTES;
       const uint64_t bdesc = umma_desc(st + NW * A_BYTES);
-      if (elect_one()) {
+      if (leader()) {
 #pragma unroll
         for (int w = 0; w < NW; w++) {
           const uint64_t adesc = umma_desc(st + w * A_BYTES);
@@ -189,7 +191,7 @@ __global__ void __launch_bounds__(TcCfg<TN, EPI, W8, HALF>::THREADS, HALF ? 2 : 
         umma_commit(&empty_bar[s]);  // arrives when the MMAs above have finished reading the stage
       }
     }
-    if (ok && elect_one()) umma_commit(&acc_bar);  // ... and when the whole accumulation is complete
+    if (ok && leader()) umma_commit(&acc_bar);  // ... and when the whole accumulation is complete
   } else if (warp >= 2) {
     if (W8 && warp - 2 < Cfg::CONV_WARPS) {
       // ---- converter: this thread's weight row of every stage, int8 -> half(q) * scale -> swizzled fp16 tile
