@@ -60,14 +60,22 @@ struct TcCfg {
   static constexpr uint32_t A_BYTES = TC_BM * TC_BK * 2;  // 16 KB
   static constexpr uint32_t B_BYTES = TN * TC_BK * 2;
   static constexpr uint32_t STAGE_BYTES = NW * (A_BYTES + RAW_BYTES) + B_BYTES;  // [A0 | A1 | B | raw0 | raw1]
+  // HALF: a ring of half the shared memory, so that two CTAs share an SM (few activation rows only)
+  static constexpr int STAGES_FIT = ((HALF ? 110 : 225) * 1024) / STAGE_BYTES;
+  static constexpr int STAGES = STAGES_FIT > 10 ? 10 : STAGES_FIT;
   // int8: every epilogue warp converts during the main loop, in CONV_SPLIT groups (EPW / NW: 1, 2 or 4) of four warps per
   // matrix (one thread per weight row); group g takes the k-blocks g, g + CONV_SPLIT, ..., so that many k-blocks are being
   // converted at once and a group's fixed costs (barrier wait, proxy fence, arrival) hide behind the other groups' work
   static constexpr int CONV_SPLIT = W8 ? (EPW / NW >= 1 ? EPW / NW : 1) : 1;
   static constexpr int CONV_WARPS = W8 ? 4 * NW * CONV_SPLIT : 0;
-  // HALF: a ring of half the shared memory, so that two CTAs share an SM (few activation rows only)
-  static constexpr int STAGES_FIT = ((HALF ? 110 : 225) * 1024) / STAGE_BYTES;
-  static constexpr int STAGES = STAGES_FIT > 10 ? 10 : STAGES_FIT;
+  // A wait by parity tells a phase from its neighbours only, so a group may be at most one use of a stage ahead of the
+  // loads.  Where STAGES is a multiple of the groups, the group that converts a use of a stage converted the use before, and
+  // is never further ahead.  In rings of 5 stages and 4 groups, or 3 and 2 (33 to 128 rows), that was another group: one whose
+  // block landed early went through the wait for use u + 1 while use u was still on its way (its phase open, the one before
+  // of the same parity), converted stale bytes and arrived for them, and the sums were wrong or the ring stopped.  There a
+  // group first waits for the MMAs on the previous use, which come behind its conversion; the producer waits for the same
+  // before it requests the tile, so this costs no time.
+  static constexpr bool CONV_WAIT_EMPTY = W8 && STAGES % CONV_SPLIT != 0;
   static constexpr uint32_t TMEM_COLS = NCOL <= 32 ? 32 : (NCOL <= 64 ? 64 : (NCOL <= 128 ? 128 : (NCOL <= 256 ? 256 : 512)));
   static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + 1024;
   // split-K peers park their accumulators ([column][128 lanes] fp32 each) in rank 0's pipeline buffers
@@ -129,7 +137,7 @@ __global__ void __launch_bounds__(TcCfg<TN, EPI, W8, HALF>::THREADS, HALF ? 2 : 
   const uint32_t tmem_base = s_tmem;
   bool acc_ok = false;
 
-  // int8 weights keep the issue loops of one lane: with all lanes in them, passes of 100 rows were seen to stop
+  // int8 weights keep the issue loops of one lane
   auto leader = [] { if constexpr (W8) return true; else return elect_one(); };
   if (warp == 0 && (!W8 || lane == 0)) {
     // ---- producer.  Weights do not depend on the preceding kernel: the first tiles are requested before the wait.
@@ -202,6 +210,7 @@ __global__ void __launch_bounds__(TcCfg<TN, EPI, W8, HALF>::THREADS, HALF ? 2 : 
       const uint32_t row_off = (uint32_t)(r >> 3) * 1024u + (uint32_t)(r & 7) * 128u;
       for (int i = group; i < nk; i += CS) {
         const int s = i % STAGES;
+        if (Cfg::CONV_WAIT_EMPTY && i >= STAGES && !mbar_wait(&empty_bar[s], ((i / STAGES) - 1) & 1)) { atomicCAS(a.err, 0, 1); break; }
         if (!mbar_wait(&raw_full[s], (i / STAGES) & 1)) { atomicCAS(a.err, 0, 1); break; }
         unsigned char* st = tiles + (size_t)s * STAGE_BYTES;
         const uint4* src = reinterpret_cast<const uint4*>(st + RAW_OFF + w * RAW_BYTES + r * TC_BK);
