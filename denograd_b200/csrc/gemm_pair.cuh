@@ -73,7 +73,6 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
 }
 // mbar_wait for arrivals of the other CTA's threads
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity) {
-  const uint32_t addr = smem_u32(bar);
   for (uint32_t i = 0; i < TC_SPIN_LIMIT; i++) {
     uint32_t ok;
     asm volatile(
@@ -81,9 +80,9 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
         "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(addr), "r"(parity)
+        : "r"(smem_u32(bar)), "r"(parity)
         : "memory");
-    if (ok) return true;
+    if (__all_sync(0xffffffffu, ok != 0)) return true;
   }
   return false;
 }

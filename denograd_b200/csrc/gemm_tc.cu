@@ -138,6 +138,7 @@ __global__ void __launch_bounds__(TcCfg<TN, EPI, W8, HALF>::THREADS, HALF ? 2 : 
   bool acc_ok = false;
 
   // int8 weights keep the issue loops of one lane
+  auto wait = [](uint64_t* bar, uint32_t parity) { return W8 ? mbar_wait_lane(bar, parity) : mbar_wait(bar, parity); };
   auto leader = [] { if constexpr (W8) return true; else return elect_one(); };
   if (warp == 0 && (!W8 || lane == 0)) {
     // ---- producer.  Weights do not depend on the preceding kernel: the first tiles are requested before the wait.
@@ -168,7 +169,7 @@ __global__ void __launch_bounds__(TcCfg<TN, EPI, W8, HALF>::THREADS, HALF ? 2 : 
       const int s = i % STAGES;
       // the MMAs of the stage's previous use are done: its A and B tiles are free, and so is its raw tile (converted
       // before those MMAs could start)
-      if (!mbar_wait(&empty_bar[s], ((i / STAGES) - 1) & 1)) { atomicCAS(a.err, 0, 1); break; }
+      if (!wait(&empty_bar[s], ((i / STAGES) - 1) & 1)) { atomicCAS(a.err, 0, 1); break; }
       if (leader()) {
         load_w(i, s);
         tma_load_2d(tiles + (size_t)s * STAGE_BYTES + NW * A_BYTES, &tm_x, (kb0 + i) * TC_BK, tok0, &full_bar[s]);
@@ -183,8 +184,8 @@ __global__ void __launch_bounds__(TcCfg<TN, EPI, W8, HALF>::THREADS, HALF ? 2 : 
     pdl_wait();
     for (int i = 0; i < nk; i++) {
       const int s = i % STAGES;
-      if (!mbar_wait(&full_bar[s], (i / STAGES) & 1)) { atomicCAS(a.err, 0, 2); ok = false; break; }
-      if (W8 && !mbar_wait(&a_full[s], (i / STAGES) & 1)) { atomicCAS(a.err, 0, 2); ok = false; break; }
+      if (!wait(&full_bar[s], (i / STAGES) & 1)) { atomicCAS(a.err, 0, 2); ok = false; break; }
+      if (W8 && !wait(&a_full[s], (i / STAGES) & 1)) { atomicCAS(a.err, 0, 2); ok = false; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       unsigned char* st = tiles + (size_t)s * STAGE_BYTES;
       const uint64_t bdesc = umma_desc(st + NW * A_BYTES);

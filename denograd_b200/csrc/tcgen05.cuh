@@ -32,20 +32,29 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
-// Bounded wait for the phase with the given parity; false = gave up.
+__device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// Bounded wait of a converged warp for the phase with the given parity; false = gave up.  The lanes poll together and leave
+// together: a verdict of each lane's own would let some go on to elect.sync, __syncwarp or a tcgen05 .aligned instruction
+// that waits for all of them.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  const uint32_t addr = smem_u32(bar);
-  for (uint32_t i = 0; i < TC_SPIN_LIMIT; i++) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
+  for (uint32_t i = 0; i < TC_SPIN_LIMIT; i++)
+    if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+  return false;
+}
+// The same for a loop that one lane runs.
+__device__ __forceinline__ bool mbar_wait_lane(uint64_t* bar, uint32_t parity) {
+  for (uint32_t i = 0; i < TC_SPIN_LIMIT; i++)
+    if (mbar_try(bar, parity)) return true;
   return false;
 }
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
