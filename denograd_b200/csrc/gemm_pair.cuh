@@ -284,6 +284,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
         const uint32_t* f = a.flags + ((size_t)(share + 1 + min(lane, parts - 1)) * 2 + rank) * GP_EPI_WARPS + ew;
         uint32_t v = 0;
         for (uint32_t i = 0; i < TC_SPIN_LIMIT && v == 0; i++) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
+        __syncwarp();  // each flag was acquired by one lane, and all lanes read what stands behind it (a vote orders no memory)
         if (__any_sync(0xffffffffu, v == 0)) { if (lane == 0) atomicCAS(a.err, 0, 3); break; }
       }
       const int feat0 = ((w.tile / a.tok_tiles) * 2 + (int)rank) * FEATS, tok0 = (w.tile % a.tok_tiles) * a.tn;
