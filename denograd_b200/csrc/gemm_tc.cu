@@ -7,7 +7,7 @@
 // B = TN activation rows x 64 k (TN = 16 ... 256), D[128 lanes = weight rows][TN columns = activation rows] in fp32.
 // With few activation rows the kernel is a weight stream: every weight byte crosses HBM once, the pipeline is as deep
 // as shared memory allows, and the first weight tiles are requested before the kernel waits for its predecessor.
-// Warp roles: warp 0 issues the TMA loads (one lane), warp 1 owns tensor memory and issues the MMAs (one lane),
+// Warp roles: warp 0 issues the TMA loads, warp 1 owns tensor memory and issues the MMAs,
 // warps 2-9 read the accumulator back (tcgen05.ld; a warp may touch the 32-lane quarter given by its id modulo 4, so
 // two warps share a quarter and split its columns) and apply the epilogue.
 //
@@ -137,10 +137,13 @@ __global__ void __launch_bounds__(TcCfg<TN, EPI, W8, HALF>::THREADS, HALF ? 2 : 
   const uint32_t tmem_base = s_tmem;
   bool acc_ok = false;
 
-  // int8 weights keep the issue loops of one lane
-  auto wait = [](uint64_t* bar, uint32_t parity) { return W8 ? mbar_wait_lane(bar, parity) : mbar_wait(bar, parity); };
-  auto leader = [] { if constexpr (W8) return true; else return elect_one(); };
-  if (warp == 0 && (!W8 || lane == 0)) {
+  // All lanes run the loops of warps 0 and 1 (see elect_one) but in int8 tiles of 256 rows, where 16 converting warps want the issue
+  // slots that 31 more polling lanes take: us, 8B shapes, loops of one lane / of all: 100 rows qkv 33.4 / 28.7, wo 17.2 / 15.5,
+  // gate and up 61.0 / 58.6, down 36.4 / 31.1; 300 rows 33.2 / 37.2, 24.8 / 25.5, 169.1 / 170.6, 61.4 / 67.0
+  constexpr bool ONE_LANE = W8 && TN > 128;
+  auto wait = [](uint64_t* bar, uint32_t parity) { return ONE_LANE ? mbar_wait_lane(bar, parity) : mbar_wait(bar, parity); };
+  auto leader = [] { return ONE_LANE || elect_one(); };
+  if (warp == 0 && (!ONE_LANE || lane == 0)) {
     // ---- producer.  Weights do not depend on the preceding kernel: the first tiles are requested before the wait.
     const int pre = nk < STAGES ? nk : STAGES;
     if (a.w_late) pdl_wait();
@@ -175,7 +178,7 @@ __global__ void __launch_bounds__(TcCfg<TN, EPI, W8, HALF>::THREADS, HALF ? 2 : 
         tma_load_2d(tiles + (size_t)s * STAGE_BYTES + NW * A_BYTES, &tm_x, (kb0 + i) * TC_BK, tok0, &full_bar[s]);
       }
     }
-  } else if (warp == 1 && (!W8 || lane == 0)) {
+  } else if (warp == 1 && (!ONE_LANE || lane == 0)) {
     // ---- MMA issuer: 4 x (128 x TN x 16) per stage and matrix, accumulating in tensor memory
     const uint32_t idesc = (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);  // f32 acc, f16 x f16, K-major both
     bool ok = true;
