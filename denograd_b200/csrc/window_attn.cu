@@ -736,12 +736,13 @@ static int launch_wx_rows(jg_dev* dev, const WinArgs<bf16>& a, int qkp) {
   return launch_wx<VT, 4>(dev, a, qkp);
 }
 
-// Portions that window_flash takes: equal heads of 64 or 128 whose number per kv head divides a tile, pages that a tile's runs fit, results
-// in 16-byte pieces, and tokens enough (us, cache writes included, window_flash / window_chunk; 32 heads on 8: 128 tokens 15.7 / 15.7, 256
+// Portions that window_flash takes: a positive scale (it masks and takes the maximum ahead of scaling: with 0 a masked score would be NaN,
+// below 0 it would win), equal heads of 64 or 128 whose number per kv head divides a tile, pages that a tile's runs fit, results in
+// 16-byte pieces, and tokens enough (us, cache writes included, window_flash / window_chunk; 32 heads on 8: 128 tokens 15.7 / 15.7, 256
 // 19.7 / 22.0, 512 25.9 / 34.2, 1024 59 / 85, 1999 135 / 252; 16 on 4, eight sequences of 128 21.5 / 21.1, of 256 41.9 / 40.2).
 static bool flash_fits(const WinArgs<bf16>& a) {
   const int per = a.H / a.G;
-  return a.Sc >= WINDOW_MIN_FLASH && a.dim == a.vd && (a.dim == 64 || a.dim == 128) && per <= FT_ROWS && FT_ROWS % per == 0 && a.page >= 8 && a.ldo % 8 == 0 &&
+  return a.scale > 0.f && a.Sc >= WINDOW_MIN_FLASH && a.dim == a.vd && (a.dim == 64 || a.dim == 128) && per <= FT_ROWS && FT_ROWS % per == 0 && a.page >= 8 && a.ldo % 8 == 0 &&
          (uintptr_t)a.out % 16 == 0 && a.G <= 65535 && a.B <= 65535;
 }
 template <int D, bool SPLIT>

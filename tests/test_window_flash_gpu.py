@@ -9,9 +9,9 @@ from tests.test_rigazen_gpu import build, check, config, parallel, run, tokens, 
 pytestmark = pytest.mark.gpu
 
 
-def branch(heads, kv_heads, dim, size, keep):
+def branch(heads, kv_heads, dim, size, keep, scale=None):
     return parallel(window(dim=dim, heads=heads, kv_heads=kv_heads, mask={"keep_first": keep, "size": size}, rot={"base": 2000.0, "dims": dim // 2},
-                           scale=dim ** -0.5, vdim=dim), right_scale=0.4)
+                           scale=dim ** -0.5 if scale is None else scale, vdim=dim), right_scale=0.4)
 
 
 @pytest.mark.parametrize("heads,kv_heads,dim", [(4, 1, 128), (2, 2, 64), (8, 1, 64), (6, 3, 128)])
@@ -34,3 +34,13 @@ def test_two_sequences_at_once():
     got = m.last_logits(2)
     for b in range(2):
         check(got[b:b + 1], O.forward(params, cfg, rows[b].tolist())[-1:], "bfloat16")
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.11])
+def test_scales_that_are_not_positive(scale):
+    cfg = config(branch(4, 1, 128, 150, 70, scale), width=64)
+    params, toks = O.random_params(cfg, seed=6), tokens(cfg, 300)
+    want = O.forward(params, cfg, toks)
+    m = build(cfg, params, "bfloat16", max_context=320, max_rows=300)
+    for cuts in ([300], [255, 45], [43, 257]):
+        check(run(m, toks, cuts), want, "bfloat16", (scale, cuts))
