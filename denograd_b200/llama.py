@@ -382,6 +382,7 @@ class Transformer(Decoder):
             layer.attention._kv, layer.attention._layer = self._kv, i
         self._ws: dict[int, _Workspace] = {}
         self._init_decoder(dev, jit)
+        self._dq_scratch: Tensor | None = None  # fp16 copies of quantised matrices (_fp16_weights)
         self._step_plan = None  # None: not tried yet, False: this model keeps the launch-per-op step
 
     def new_cache(self) -> None:
@@ -523,9 +524,9 @@ class Transformer(Decoder):
         nf4 = getattr(lins[0], "nf4_block", 0)
         if lins[0].scale_ptr == 0 and not nf4:
             return [(l.weight.ptr, 0) for l in lins]
-        need = sum(l.out_features * l.in_features for l in lins)
-        if getattr(self, "_dq_scratch", None) is None or self._dq_scratch.numel() < need:
-            self._dq_scratch = Tensor.empty((need,), "float16", self.dev)
+        if self._dq_scratch is None:  # once, for the largest call of any layer: a captured step keeps its address
+            size = [[l.out_features * l.in_features for l in (y.attention._wqkv, y.attention.wo, y.feed_forward.w1, y.feed_forward.w2)] for y in self.layers]
+            self._dq_scratch = Tensor.empty((max(max(qkv, wo, 2 * w1, w2) for qkv, wo, w1, w2 in size),), "float16", self.dev)
         out, off = [], 0
         for l in lins:
             ptr = self._dq_scratch.ptr + 2 * off
