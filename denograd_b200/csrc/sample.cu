@@ -350,15 +350,16 @@ static int run_sample(jg_dev* dev, uint64_t tokens_out, uint64_t logits, uint64_
   // the head of the next slice is kept where a chunk is short enough for it (a vocabulary with a divisor near 256); longer
   // chunks, found with odd vocabularies, read the rest through distributed shared memory
   a.ext = cs > 1 ? a.per + (a.len > 256 && a.len <= 2048 ? a.len : 256) : a.per;
-  const size_t smem = (size_t)(smp_slot(a.ext) + 1) * sizeof(float);
-  const size_t limit = (size_t)dev->prop.sharedMemPerBlockOptin - 40 * 1024;
-  if (smem > limit) {
-    jg_set_error("sample: %d values per CTA need %zu B of shared memory (limit %zu)", a.ext, smem, limit);
+  // a slice takes as much as it ever did (its values, 40 KB left over); its padding and the neighbour's head come out of those 40 KB,
+  // of which the static tables take 25
+  const size_t optin = dev->prop.sharedMemPerBlockOptin, limit = optin - 28 * 1024, smem = (size_t)(smp_slot(a.ext) + 1) * sizeof(float);
+  if ((size_t)a.per * sizeof(float) > optin - 40 * 1024 || smem > limit) {
+    jg_set_error("sample: %d values per CTA need %zu B of shared memory (limit %zu)", a.per, smem, limit);
     return JG_ENOTSUP;
   }
   static size_t smem_set[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   const int slot = dev->ordinal & 7;
-  if (smem > 48 * 1024 - 40 * 1024 && smem > smem_set[slot]) {
+  if (smem > 8 * 1024 && smem > smem_set[slot]) {
     JG_CUDA(cudaFuncSetAttribute(sample_kernel<LT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
     smem_set[slot] = limit;
   }

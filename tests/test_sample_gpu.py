@@ -93,3 +93,17 @@ def test_rows_at_the_edges_of_slices_and_chains(dev, V, k):
         # without a finite maximum every probability is NaN: the draw then gives 0, the rounds of the top k are not defined
         rows = [r for r in range(5) if k == 0 or np.isfinite(np.where(np.isnan(lg[r]), -np.inf, lg[r]).max())]
         assert [out.numpy()[r] for r in rows] == [want[r] for r in rows], (V, k, u0)
+
+
+@pytest.mark.parametrize("V", [370001, 380000, 382976])
+@pytest.mark.parametrize("k", [0, 30])
+def test_the_largest_vocabularies(dev, V, k):
+    """Slices that leave room for no more than their padding and the head of the next one; one value more per slice is refused."""
+    rng = np.random.default_rng(V + k)
+    lg = _logits(rng, 2, V, 3.0)
+    lt, out = Tensor(lg, device=dev), Tensor.empty((2,), "int32", dev)
+    for u0 in (0.0, 0.61, 0.99999994):
+        dev.call("jg_sample", out.ptr, lt.ptr, Tensor(np.full(2, u0, np.float32), device=dev).ptr, 0, 2, V, 0.95, k, 0.9, 0.0, 0.0)
+        assert out.numpy().tolist() == [O.sample(r.astype(np.float32), 0.95, k, 0.9, 0.0, 0.0, u0) for r in lg], (V, k, u0)
+    with pytest.raises(ffi.JgError):
+        dev.call("jg_sample", out.ptr, lt.ptr, lt.ptr, 0, 2, 382977, 0.95, k, 0.9, 0.0, 0.0)
