@@ -282,6 +282,17 @@ class _Workspace:
         arr = np.ctypeslib.as_array((C.c_int32 * (3 * B)).from_address(self._pinned.value))
         self.h_tokens, self.h_pos, self.h_next = arr[:B], arr[B:2 * B], arr[2 * B:]
 
+    def first_rows(self, n: int, tp=None) -> "_Workspace":
+        """The buffers of the first n rows, as a chunk of n rows uses them."""
+        v = object.__new__(_Workspace)
+        v.B, v._dev, v._pinned, v.cur, v.pending, v.hist, v.logits = n, self._dev, None, 0, False, None, None
+        v._h = [t.view_rows(0, n) for t in self._h]
+        for name in ("tokens", "pos", "seq", "xn", "qkv", "attn", "ffn", "key", "next_tokens"):
+            setattr(v, name, getattr(self, name).view_rows(0, n))
+        dim = self.xn.shape[1]
+        v.part32 = (tp.partial_tensor(n, dim) if tp is not None else None) or self.part32.view_rows(0, n)
+        return v
+
     @property
     def h(self) -> Tensor:
         return self._h[self.cur]
@@ -381,6 +392,8 @@ class Transformer(Decoder):
         for i, layer in enumerate(self.layers):
             layer.attention._kv, layer.attention._layer = self._kv, i
         self._ws: dict[int, _Workspace] = {}
+        self._chunk_ws: _Workspace | None = None    # buffers of the chunks with most rows so far
+        self._chunk_view: _Workspace | None = None  # their first rows, as the last chunk had them
         self._init_decoder(dev, jit)
         self._dq_scratch: Tensor | None = None  # fp16 copies of quantised matrices (_fp16_weights)
         self._step_plan = None  # None: not tried yet, False: this model keeps the launch-per-op step
@@ -400,15 +413,27 @@ class Transformer(Decoder):
 
     # ------------------------------------------------------------------------------------------ internals
     def _workspace(self, B: int, rows: bool = False) -> _Workspace:
-        """Workspace for B activation rows; `rows` marks a multi-position chunk (more rows than sequences allowed)."""
+        """Workspace for B activation rows; `rows` marks a multi-position chunk (more rows than sequences allowed).  Chunks
+        beyond the batch limit share one set of buffers, which grows by powers of two, and carry no logits: a set for each row
+        count (8B: 82 KB a row) would fill the device with the lengths of the prompts a server has seen."""
         if B > self.max_batch and not rows:
             raise ValueError(f"batch {B} exceeds max_batch {self.max_batch}")
-        key = B if (not rows or B <= self.max_batch) else -B  # chunks beyond the batch limit carry no logits buffer
-        if key not in self._ws:
-            qkv_dim = (self.n_heads + 2 * self.n_kv_heads) * self.head_dim
-            self._ws[key] = _Workspace(self.dev, B, self.dim, qkv_dim, self.n_heads * self.head_dim, self.hidden_dim,
-                                       self.vocab_local if key > 0 else 0, tp=self._tp)
-        return self._ws[key]
+        qkv_dim = (self.n_heads + 2 * self.n_kv_heads) * self.head_dim
+
+        def make(n: int, vocab: int) -> _Workspace:
+            return _Workspace(self.dev, n, self.dim, qkv_dim, self.n_heads * self.head_dim, self.hidden_dim, vocab, tp=self._tp)
+
+        if B <= self.max_batch:
+            if B not in self._ws:
+                self._ws[B] = make(B, self.vocab_local)
+            return self._ws[B]
+        if self._chunk_view is None or self._chunk_view.B != B:
+            self._chunk_view = None
+            if self._chunk_ws is None or self._chunk_ws.B < B:
+                self._chunk_ws = None  # given back first
+                self._chunk_ws = make(1 << (B - 1).bit_length(), 0)
+            self._chunk_view = self._chunk_ws.first_rows(B, self._tp)
+        return self._chunk_view
 
     def _single_kernel_step(self, B: int):
         """The step plan (jg_step_create) when this model and batch can run the decode step as one persistent kernel:

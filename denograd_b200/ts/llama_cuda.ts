@@ -193,7 +193,7 @@ export class CudaTransformerBlock {
    *  position-major; every row attends to the cache up to its own position, which is what the reference's additive
    *  causal mask (:208) computes. */
   prefill_chunk = (dev: CUDA, ws: Workspace, kv: KVCache, freqs_cis: Dev, freqs_rows: number, dim: number, batch: number, positions: number) => {
-    const a = this.attention, f = this.feed_forward, R = ws.B
+    const a = this.attention, f = this.feed_forward, R = batch * positions
     cu(dev, 'jg_rmsnorm', ws.xn, ws.h, this.attention_norm, R, dim, this.attention_norm.eps)
     cu(dev, 'jg_linear', ws.qkv, ws.xn, a.wqkv, a.wqkv.scale_ptr, 0, R, a.wqkv.out_features, dim)
     cu(dev, 'jg_rope_kvwrite_rows', kv.handle, a.layer, ws.qkv, freqs_cis, freqs_rows, ws.pos, ws.seq, R, a.n_heads)
@@ -243,6 +243,7 @@ export class CudaTransformer {
   kv!: KVCache
   private step_plan?: StepPlan
   private ws = new Map<number, Workspace>()
+  private chunk_ws?: Workspace
   private step_graph = new Map<number, CUDAGraph>()
   private calls = new Map<number, number>()
   constructor(public dim: number, public hidden_dim: number, public n_heads: number, n_layers: number, norm_eps: number, public vocab_size: number, linear: typeof CudaLinear = CudaLinear, embedding: typeof CudaEmbedding = CudaEmbedding, public n_kv_heads?: number, public rope_theta = 10000, public max_context = 1024, public jit = true, feed_forward: typeof CudaFeedForward = CudaFeedForward, public max_batch = 1) {
@@ -265,13 +266,18 @@ export class CudaTransformer {
     this.kv = new KVCache(this.dev, this.layers.length, this.n_heads, this.n_kv_heads ?? this.n_heads, this.head_dim, this.max_context, this.max_batch)
   }
 
-  private workspace = (B: number, logits = true) => {
-    const key = logits ? B : -B
-    if (!this.ws.has(key)) {
-      const kvh = this.n_kv_heads ?? this.n_heads
-      this.ws.set(key, new Workspace(B, this.dim, (this.n_heads + 2 * kvh) * this.head_dim, this.n_heads * this.head_dim, this.hidden_dim, logits ? this.vocab_size : 0, this.dev.device))
-    }
-    return this.ws.get(key)!
+  private make_workspace = (B: number, vocab: number) => {
+    const kvh = this.n_kv_heads ?? this.n_heads
+    return new Workspace(B, this.dim, (this.n_heads + 2 * kvh) * this.head_dim, this.n_heads * this.head_dim, this.hidden_dim, vocab, this.dev.device)
+  }
+  private workspace = (B: number) => {
+    if (!this.ws.has(B)) this.ws.set(B, this.make_workspace(B, this.vocab_size))
+    return this.ws.get(B)!
+  }
+  /** Buffers of prompt chunks: one set of at least R rows, which grows by powers of two. */
+  private chunk_workspace = (R: number) => {
+    if (this.chunk_ws === undefined || this.chunk_ws.B < R) this.chunk_ws = this.make_workspace(2 ** Math.ceil(Math.log2(R)), 0)
+    return this.chunk_ws
   }
 
   /** The plan of the single-kernel step when this model and row count can take it: fp16 weights, 1-2 rows. */
@@ -329,9 +335,10 @@ export class CudaTransformer {
     // several positions: chunks of up to 4096 rows, position-major (row = s * bsz + b)
     const per = Math.max(1, Math.trunc(4096 / bsz))
     for (let s0 = 0; s0 < seqlen; s0 += per) {
-      const sc = Math.min(per, seqlen - s0), R = bsz * sc, ws = this.workspace(R, false), dev = this.dev
+      const sc = Math.min(per, seqlen - s0), R = bsz * sc, ws = this.chunk_workspace(R), dev = this.dev
       const flat: number[] = [], pos: number[] = [], seq: number[] = []
       for (let s = 0; s < sc; s++) for (let b = 0; b < bsz; b++) flat.push(toks[b][s0 + s]), pos.push(start_pos + s0 + s), seq.push(b)
+      while (flat.length < ws.B) flat.push(0), pos.push(0), seq.push(0) // rows that this chunk does not have
       await ws.tokens.t.assign(new Tensor(flat, { dtype: dtypes.int32, device: dev.device })).realize()
       await ws.pos.t.assign(new Tensor(pos, { dtype: dtypes.int32, device: dev.device })).realize()
       await ws.seq.t.assign(new Tensor(seq, { dtype: dtypes.int32, device: dev.device })).realize()
