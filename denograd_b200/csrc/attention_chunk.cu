@@ -157,8 +157,7 @@ JG_API int jg_attn_chunk(jg_dev* dev, jg_kvcache* kv, int32_t layer, uint64_t ou
   a.scale = (float)(1.0 / (double)(float)sqrt((double)hd));  // as the reference folds it (jsgrad/tensor.ts:3923)
   CUtensorMap mk, mv;
   const uint64_t rows = (uint64_t)kv->d.n_pages * G * kv->d.page_size;
-  int rc = jg_tc_error_word(dev);
-  if (!rc) rc = jg_tensor_map(&mk, a.k_layer, rows, hd, hd, a.page, "cached keys");
+  int rc = jg_tensor_map(&mk, a.k_layer, rows, hd, hd, a.page, "cached keys");
   if (!rc) rc = jg_tensor_map(&mv, a.v_layer, rows, hd, hd, a.page, "cached values");
   if (rc) return rc;
   a.err = dev->err_word;

@@ -22,7 +22,8 @@ struct jg_dev {
   bool pdl;  // launch kernels with programmatic stream serialization (JG_PDL=0 turns it off)
   bool pdl_cluster;  // ... also the thread-block-cluster launches of the gathering projections (JG_PDL_CLUSTER=1; default off)
   bool pdl_attn;     // ... also the decode-attention cluster launches (JG_PDL_ATTN=1; default off)
-  int* err_word;    // device word written by kernels whose bounded waits gave up (0 = fine); allocated on first use
+  int* err_word;    // page-locked word written by kernels whose bounded waits gave up (0 = fine): there from the start, so that no
+                    // launch is the one that has to allocate it, and read without a copy
   float* pair_slots;    // gemm_pair.cuh: accumulators of tiles that several CTA pairs share, and their flags; allocated on first use
   uint32_t* pair_flags;
   bool tc_pending;  // such kernels were launched since the word was last checked

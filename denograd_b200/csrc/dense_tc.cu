@@ -289,8 +289,6 @@ struct DensePairEpi {
 
 int jg_dense_tc(jg_dev* dev, const DenseCall& c) {
   JG_REQUIRE(((uintptr_t)c.x % 16) == 0 && c.ldx % 8 == 0 && c.ldw % 8 == 0, "dense: operands must be 16-byte aligned with row strides of a multiple of 8");
-  const int erc = jg_tc_error_word(dev);
-  if (erc) return erc;
   DtArgs a = {};
   if (c.out_f32) a.y32 = (float*)c.y;
   else a.y = (bf16*)c.y;

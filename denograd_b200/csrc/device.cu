@@ -77,6 +77,8 @@ JG_API int jg_device_open(int32_t ordinal, jg_dev** out) {
   JG_CUDA(cudaEventCreate(&d->t1));
   d->pinned_stage_bytes = 1 << 16;
   JG_CUDA(cudaHostAlloc(&d->pinned_stage, d->pinned_stage_bytes, cudaHostAllocDefault));
+  JG_CUDA(cudaHostAlloc((void**)&d->err_word, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+  *d->err_word = 0;
   *out = d;
   return JG_OK;
 }
@@ -87,6 +89,7 @@ JG_API int jg_device_close(jg_dev* dev) {
   cudaEventDestroy(dev->t0);
   cudaEventDestroy(dev->t1);
   cudaFreeHost(dev->pinned_stage);
+  cudaFreeHost(dev->err_word);
   if (dev->pair_slots) cudaFree(dev->pair_slots);  // the flags lie behind the slots
   cudaStreamDestroy(dev->stream);
   delete dev;
@@ -110,12 +113,11 @@ int jg_check_device_errors(jg_dev* dev) {
       return JG_ETIMEDOUT;
     }
   }
-  if (!dev->tc_pending || dev->err_word == nullptr) return JG_OK;
+  if (!dev->tc_pending) return JG_OK;
   dev->tc_pending = false;
-  int code = 0;
-  JG_CUDA(cudaMemcpy(&code, dev->err_word, sizeof(int), cudaMemcpyDeviceToHost));
+  const int code = *(volatile int*)dev->err_word;
   if (code != 0) {
-    cudaMemset(dev->err_word, 0, sizeof(int));
+    *(volatile int*)dev->err_word = 0;
     jg_pair_reset(dev);
     jg_set_error("a device-side wait gave up (code %d: 1 = TMA producer, 2 = MMA issuer, 3 = epilogue of a tensor-core "
                  "projection, 4 = grid barrier of the single-kernel decode step); results since the last synchronisation "

@@ -453,8 +453,6 @@ int jg_gemm_tc(jg_dev* dev, int epi, const void* x, const void* w0, const void* 
     return JG_ENOTSUP;
   }
   JG_REQUIRE(((uintptr_t)x % 16) == 0 && ((uintptr_t)w0 % 16) == 0, "projection: operands must be 16-byte aligned for TMA");
-  const int erc = jg_tc_error_word(dev);
-  if (erc) return erc;
   TcArgs a = {};
   a.y = (__half*)y; a.y32 = (float*)y; a.residual = (const __half*)residual; a.err = dev->err_word; a.M = M; a.N = N; a.K = K;
   a.w_late = jg_is_fresh(dev, w0) || jg_is_fresh(dev, w1) || jg_is_fresh(dev, s0) || jg_is_fresh(dev, s1);

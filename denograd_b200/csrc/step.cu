@@ -1094,10 +1094,6 @@ JG_API int jg_step_create(jg_dev* dev, jg_kvcache* kv, const jg_step_desc* desc,
     return jg_cuda_fail(e, "step_create", __FILE__, __LINE__);
   }
   a.layers = s->d_layers;
-  if (dev->err_word == nullptr) {
-    JG_CUDA(cudaMalloc(&dev->err_word, sizeof(int)));
-    JG_CUDA(cudaMemset(dev->err_word, 0, sizeof(int)));
-  }
   a.err = dev->err_word;
   *out = s;
   return JG_OK;

@@ -117,6 +117,3 @@ __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
 // copy, because the next call may reuse the slot this one came from.
 int jg_tensor_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows,
                   const char* what, int bytes = 2, bool bf16 = false);
-
-// Makes sure that the device's error word for bounded waits exists.
-int jg_tc_error_word(jg_dev* dev);

@@ -84,14 +84,6 @@ bool jg_tensor_map_two(CUtensorMap* out, const void* lo, const void* hi, uint64_
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-int jg_tc_error_word(jg_dev* dev) {
-  if (dev->err_word != nullptr) return JG_OK;
-  JG_REQUIRE(!dev->capturing, "first tensor-core launch on a device must not be inside a graph capture");
-  JG_CUDA(cudaMalloc(&dev->err_word, sizeof(int)));
-  JG_CUDA(cudaMemsetAsync(dev->err_word, 0, sizeof(int), dev->stream));
-  return JG_OK;
-}
-
 static size_t pair_flag_bytes(const jg_dev* dev) { return (size_t)(dev->sm_count / 2) * 2 * GP_EPI_WARPS * sizeof(uint32_t); }
 bool jg_pair_workspace(jg_dev* dev) {
   static std::mutex m;

@@ -760,10 +760,8 @@ static int launch_flash(jg_dev* dev, const WinArgs<bf16>& a, const CUtensorMap& 
 }
 template <int D>
 static int run_flash(jg_dev* dev, const WinArgs<bf16>& a) {
-  int rc = jg_tc_error_word(dev);
-  if (rc) return rc;
   CUtensorMap map;  // as many rows as any GPU holds: the block table says which there are
-  rc = jg_tensor_map(&map, a.pool, (1ull << 38) / (2ull * a.row_size()), a.row_size(), a.row_size(), a.page < FT_KV ? a.page : FT_KV, "cached keys and values", 2, true);
+  const int rc = jg_tensor_map(&map, a.pool, (1ull << 38) / (2ull * a.row_size()), a.row_size(), a.row_size(), a.page < FT_KV ? a.page : FT_KV, "cached keys and values", 2, true);
   if (rc) return rc;
   const int n = FT_ROWS / (a.H / a.G) * 2;
   // pairs of query tiles where they give every SM a CTA; below that the key tiles of single ones are split between the streams
@@ -774,7 +772,7 @@ static int run_chunks(jg_dev*, const WinArgs<float>&) { return JG_ENOTSUP; }
 static int run_chunks(jg_dev* dev, const WinArgs<bf16>& a) {
   int rc = jg_launch(dev, "window_write", window_write_kernel<bf16>, dim3((unsigned)(a.B * a.Sc)), dim3(256), 0, a, 1);
   if (rc) return rc;
-  if (flash_fits(a) && (dev->err_word != nullptr || !dev->capturing)) return a.dim == 64 ? run_flash<64>(dev, a) : run_flash<128>(dev, a);
+  if (flash_fits(a)) return a.dim == 64 ? run_flash<64>(dev, a) : run_flash<128>(dev, a);
   const int qkp = (a.dim + 15) & ~15;
   if (a.vd <= 64) return launch_wx_rows<8>(dev, a, qkp);
   if (a.vd <= 128) return launch_wx_rows<16>(dev, a, qkp);
