@@ -26,7 +26,8 @@ struct jg_dev {
                     // launch is the one that has to allocate it, and read without a copy
   float* pair_slots;    // gemm_pair.cuh: accumulators of tiles that several CTA pairs share, and their flags; allocated on first use
   uint32_t* pair_flags;
-  bool tc_pending;  // such kernels were launched since the word was last checked
+  bool tc_pending;  // such kernels were launched, or replayed from a graph, since the word was last checked
+  bool tc_before_capture;  // tc_pending as it was when the capture in progress began
   bool peer_pending;  // peer-memory reductions (comm.cu) were launched since their error word was last checked
   // Device ranges written by the library's own launches since the stream was last synchronised (the latest
   // JG_FRESH_RING of them).  The tensor-core projection kernels load weight tiles before they wait for their
@@ -41,6 +42,7 @@ struct jg_graph {
   cudaGraph_t graph;
   cudaGraphExec_t exec;
   uint64_t n_kernels;
+  bool tc;  // holds kernels with bounded waits
 };
 
 void jg_set_error(const char* fmt, ...);

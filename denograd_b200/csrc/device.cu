@@ -296,6 +296,8 @@ JG_API int jg_graph_begin(jg_dev* dev) {
   dev->capturing = true;
   g_jg_capturing++;
   dev->capture_launches = 0;
+  dev->tc_before_capture = dev->tc_pending;
+  dev->tc_pending = false;
   return JG_OK;
 }
 
@@ -306,6 +308,8 @@ JG_API int jg_graph_end(jg_dev* dev, jg_graph** out) {
   int prc = jg_peer_run_boundary(dev);  // last captured launch: a replay moves the exchange base on by what it holds
   dev->capturing = false;
   g_jg_capturing--;
+  const bool tc = dev->tc_pending;
+  dev->tc_pending = tc || dev->tc_before_capture;
   cudaGraph_t g = nullptr;
   JG_CUDA(cudaStreamEndCapture(dev->stream, &g));
   if (prc) { cudaGraphDestroy(g); return prc; }
@@ -319,6 +323,7 @@ JG_API int jg_graph_end(jg_dev* dev, jg_graph** out) {
   gr->graph = g;
   gr->exec = exec;
   gr->n_kernels = dev->capture_launches;
+  gr->tc = tc;
   *out = gr;
   jg_run_deferred();
   return JG_OK;
@@ -329,6 +334,7 @@ JG_API int jg_graph_launch(jg_dev* dev, jg_graph* g) {
   JG_REQUIRE(g != nullptr && g->exec != nullptr, "null graph");
   JG_REQUIRE(!dev->capturing, "graph launch during capture");
   JG_CUDA(cudaGraphLaunch(g->exec, dev->stream));
+  if (g->tc) dev->tc_pending = true;
   dev->launches += g->n_kernels;
   return JG_OK;
 }

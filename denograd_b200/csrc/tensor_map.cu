@@ -99,5 +99,5 @@ bool jg_pair_workspace(jg_dev* dev) {
   return true;
 }
 void jg_pair_reset(jg_dev* dev) {
-  if (dev->pair_flags != nullptr) cudaMemset(dev->pair_flags, 0, pair_flag_bytes(dev));
+  if (dev->pair_flags != nullptr) cudaMemsetAsync(dev->pair_flags, 0, pair_flag_bytes(dev), dev->stream);
 }
