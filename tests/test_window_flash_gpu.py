@@ -25,6 +25,18 @@ def test_long_portions(heads, kv_heads, dim, size, keep, page):
         check(run(m, toks, cuts), want, "bfloat16", (size, keep, cuts))
 
 
+# heads and tokens enough for two tiles of queries to a CTA (a pair of tiles for every SM): 601 and 472 tokens, or 601 alone
+@pytest.mark.parametrize("heads,kv_heads,dim", [(128, 16, 64), (64, 8, 128)])
+@pytest.mark.parametrize("size,keep,page", [(4096, 0, 64), (100, 5, 16), (130, 140, 8), (257, 64, 128)])
+def test_pairs_of_query_tiles(heads, kv_heads, dim, size, keep, page):
+    cfg = config(branch(heads, kv_heads, dim, size, keep), width=64)
+    params, toks = O.random_params(cfg, seed=7), tokens(cfg, 601)
+    want = O.forward(params, cfg, toks)
+    m = build(cfg, params, "bfloat16", max_context=640, page_size=page, max_rows=601)
+    for cuts in ([601], [129, 472], [20, 300, 281]):
+        check(run(m, toks, cuts), want, "bfloat16", (size, keep, cuts))
+
+
 def test_two_sequences_at_once():
     cfg = config(branch(4, 2, 128, 150, 70), width=64)
     params, rows = O.random_params(cfg, seed=4), np.stack([tokens(cfg, 620, seed=s) for s in (5, 6)])
