@@ -53,7 +53,6 @@ __global__ void __launch_bounds__(DtCfg<TN, GLU, HALF>::THREADS, HALF ? 2 : 1)
   const int ks = gridDim.z, rank = blockIdx.z;
   const int n_kb = (a.K + DT_BK - 1) / DT_BK;
   const int kb0 = (int)((long long)rank * n_kb / ks), nk = (int)((long long)(rank + 1) * n_kb / ks) - kb0;
-  pdl_launch();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -69,6 +68,7 @@ __global__ void __launch_bounds__(DtCfg<TN, GLU, HALF>::THREADS, HALF ? 2 : 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = s_tmem;
+  pdl_launch();  // only now: see tcgen05.cuh
   bool acc_ok = false;
 
   if (warp == 0) {

@@ -101,7 +101,6 @@ __device__ __forceinline__ void flash_tc(P& p, int* err) {
   __shared__ uint32_t s_tmem;
   __shared__ float s_m[2][FT_ROWS], s_l[2][FT_ROWS];
   const int tid = threadIdx.x, lane = tid & 31, warp = uniform_warp();
-  pdl_launch();
   if (tid == 0) {
     for (int i = 0; i < FT_ST; i++) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
     for (int i = 0; i < 2; i++) { mbar_init(&s_full[i], 1); mbar_init(&s_used[i], 4); mbar_init(&o_full[i], 1); }
@@ -118,6 +117,7 @@ __device__ __forceinline__ void flash_tc(P& p, int* err) {
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = s_tmem;
+  pdl_launch();  // only now: see tcgen05.cuh
   pdl_wait();
   const bool work = p.begin();  // the same for all threads
   const int n = work ? p.tiles : 0;

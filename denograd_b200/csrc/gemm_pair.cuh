@@ -185,7 +185,6 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
   const int warp = uniform_warp(), lane = threadIdx.x & 31, pair = blockIdx.x >> 1;
   uint32_t rank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-  pdl_launch();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -202,6 +201,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
   cluster_barrier();  // the peer's barriers exist before anything is signalled across
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = s_tmem;
+  pdl_launch();  // only now: see tcgen05.cuh
 
   if (warp == 0 || warp == GP_X_WARP) {
     // ---- producers of this CTA's weights and activations, a warp each.  Completions go to rank 0's barrier, armed there for both CTAs (by the weights' producer;

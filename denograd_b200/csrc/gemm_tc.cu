@@ -117,7 +117,6 @@ __global__ void __launch_bounds__(TcCfg<TN, EPI, W8, HALF>::THREADS, HALF ? 2 : 
   const int ks = gridDim.z, rank = blockIdx.z;  // the cluster is (1,1,ks): the rank in it is blockIdx.z
   const int n_kb = a.K / TC_BK;
   const int kb0 = (int)((long long)rank * n_kb / ks), nk = (int)((long long)(rank + 1) * n_kb / ks) - kb0;
-  pdl_launch();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -135,6 +134,7 @@ __global__ void __launch_bounds__(TcCfg<TN, EPI, W8, HALF>::THREADS, HALF ? 2 : 
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = s_tmem;
+  pdl_launch();  // only now: see tcgen05.cuh
   bool acc_ok = false;
 
   // All lanes run the loops of warps 0 and 1 (see elect_one) but in int8 tiles of 256 rows, where 16 converting warps want the issue

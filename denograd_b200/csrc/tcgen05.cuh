@@ -6,6 +6,10 @@
 
 #include "common.cuh"
 
+// Tensor memory.  A kernel lets its successor start (pdl_launch) only behind its own tcgen05.alloc.  That waits, without a limit, until the
+// SM has enough columns free, and a successor's CTA that shares the SM and was first to take them keeps them until the kernel it
+// waits for has ended: all 512 columns of the prompt attention beside the 32 of a half-ring projection would wait for ever.
+
 // Polls of one mbarrier phase before a wait gives up.  A try_wait that fails returns after the hardware's own
 // suspend time (up to ~1 us), so the limit is of the order of seconds; every wait starts after the kernel's dependency
 // wait, i.e. it only ever measures this kernel's own TMA / MMA progress.
