@@ -297,20 +297,22 @@ int jg_dense_tc(jg_dev* dev, const DenseCall& c) {
   const int aligned = (uintptr_t)c.y % 16 == 0 && c.ldy % (c.out_f32 ? 4 : 8) == 0;
   // more than 64 rows, GLU more than 32: pairs of CTAs (gemm_pair.cuh; both sides measured in gemm_tc.cu), but for few features or a short K, where tiles of theirs are too few or over
   // too soon (prompts of 1999 tokens at 8B sizes, a 128 x 256 tile per CTA / pairs: Matulorn 42.5 / 38.7 ms, Rigazen 40.2 / 34.3)
-  if (c.M > 32 && c.epilogue == JG_DENSE_GLU)
+  if (c.M > 32 && c.epilogue == JG_DENSE_GLU && !cta_per_tile(dev, c.M, c.N))
     return launch_pair<DensePairEpi<true>>(dev, "dense_pair", c.x, c.ldx, c.w[0], c.w[1], c.ldw, c.M, c.N, c.K, true, a.w_late, {a.y, a.y32, a.b0, a.b1, a.ldy, aligned, a.limit, a.out});
-  if (c.M > 64 && c.N > 512 && c.K > 512)
+  if (c.M > 64 && c.N > 512 && c.K > 512 && c.epilogue != JG_DENSE_GLU)
     return launch_pair<DensePairEpi<false>>(dev, "dense_pair", c.x, c.ldx, c.w[0], c.w[0], c.ldw, c.M, c.N, c.K, true, a.w_late, {a.y, a.y32, a.b0, a.b1, a.ldy, aligned, a.limit, a.out});
   if (c.epilogue == JG_DENSE_GLU) {
     if (c.M <= 16) return launch_dt<16, true, false>(dev, c, a);
-    return launch_dt<32, true, false>(dev, c, a);
+    if (c.M <= 32) return launch_dt<32, true, false>(dev, c, a);
+    if (c.M <= 64) return launch_dt<64, true, false>(dev, c, a);
+    return c.M <= 128 ? launch_dt<128, true, false>(dev, c, a) : launch_dt<256, true, false>(dev, c, a);
   }
   if (c.M <= 16) return launch_dt<16, false, true>(dev, c, a);
   if (c.M <= 32) return launch_dt<32, false, true>(dev, c, a);
   // few features: narrow tiles, two CTAs per SM and a deep split, so that there are CTAs enough; a short K: the same by tiles alone
   if (c.N <= 512) return launch_dt<32, false, true>(dev, c, a);
   if (c.M <= 64) return launch_dt<64, false, false>(dev, c, a);
-  const bool few = c.K <= 512 && (c.N + DT_BM - 1) / DT_BM * ((c.M + 255) / 256) < dev->sm_count;
+  const bool few = (c.N + DT_BM - 1) / DT_BM * ((c.M + 255) / 256) < dev->sm_count;
   if (c.M <= 128 || few) return launch_dt<128, false, false>(dev, c, a);
   return launch_dt<256, false, false>(dev, c, a);
 }

@@ -403,6 +403,14 @@ __global__ void __launch_bounds__(GP_THREADS, 1) gemm_pair_kernel(const __grid_c
   }
 }
 
+// Gate and up of up to 256 rows where a CTA to a 128-feature tile gives most of the SMs one, once: the launch is a stream of weights, and
+// pairs need a second, half empty round.  us, weights from HBM, a CTA per tile / pairs: 14336 features (112 tiles) of 4096, 33 rows
+// 44.3 / 58.4, 100 rows 48.6 / 60.1, 200 rows 61.8 / 68.3, 256 rows 65.3 / 70.0; 11008 (86 tiles) 54.4 / 45.6, 62.5 / 47.0, 58.8 / 53.2, 60.1 / 54.7.
+static inline bool cta_per_tile(const jg_dev* dev, int M, int N) {
+  const int tiles = (N + 127) / 128;
+  return M <= 256 && tiles * 3 > dev->sm_count * 2 && tiles <= dev->sm_count;
+}
+
 // Tiles and shares with the smallest estimate, in SM cycles.  Measured at 1B and 8B shapes, 45 to 2048 rows: a k-block takes 300
 // (up to 96 rows to a tile), 330 (128), 410 (192) and 530 (256), or as long as its weights need from HBM (9.6 for each pair that
 // fetches other weights); a launch and its last tile's stores 4000 + 60 per row; a second share 5000 + 16 per row, each further

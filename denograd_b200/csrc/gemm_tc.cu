@@ -417,7 +417,7 @@ static int launch_tc_rows(jg_dev* dev, const void* x, const void* w0, const void
   // more than 64 rows, gate and up more than 32: pairs of CTAs.  us per launch, one tile per CTA / pairs: 8B shapes, 45 rows qkv 19 / 15,
   // wo 12 / 13, gate and up 45 / 44, down 25 / 28; 100 rows 23 / 17, 16 / 15, 48 / 48, 29 / 31; 512 rows 37 / 24, 35 / 19, 140 / 102,
   // 70 / 54; 1B shapes, 45 rows 8 / 9, 9 / 10, 22 / 16, 15 / 15; 100 rows 11 / 10, 11 / 10, 25 / 18, 17 / 16
-  if (a.s0 == nullptr && a.M > (EPI == TC_SWIGLU ? 32 : 64))
+  if (a.s0 == nullptr && a.M > (EPI == TC_SWIGLU ? 32 : 64) && !(EPI == TC_SWIGLU && cta_per_tile(dev, a.M, a.N)))
     return launch_pair<TcPairEpi<EPI>>(dev, "gemm_pair", x, a.K, w0, w1, a.K, a.M, a.N, a.K, false, a.w_late, 
                                         {a.y, a.y32, a.residual, (uintptr_t)a.y % 16 == 0 && (uintptr_t)a.residual % 16 == 0});
   if (a.s0 != nullptr) {  // int8 weights: used from 20 rows on (fewer go to the mma.sync kernel)
@@ -438,7 +438,9 @@ static int launch_tc_rows(jg_dev* dev, const void* x, const void* w0, const void
   }
   if (a.M <= 16) return launch_tc<16, EPI>(dev, x, w0, w1, a);
   if (a.M <= 32) return launch_tc<32, EPI>(dev, x, w0, w1, a);
-  return launch_tc<64, EPI>(dev, x, w0, w1, a);
+  if (a.M <= 64) return launch_tc<64, EPI>(dev, x, w0, w1, a);
+  if constexpr (EPI == TC_SWIGLU) return a.M <= 128 ? launch_tc<128, EPI>(dev, x, w0, w1, a) : launch_tc<256, EPI>(dev, x, w0, w1, a);
+  return JG_ENOTSUP;  // taken above
 }
 
 // Whether jg_gemm_tc takes this shape: fp16 weights, whole 128-row weight tiles and 64-wide k-blocks.

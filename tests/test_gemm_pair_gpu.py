@@ -20,7 +20,8 @@ def bound(x, w):
 
 
 # one k-block; half a weight tile; few tiles in shares; whole rounds and remainders; the last activation row alone
-@pytest.mark.parametrize("M,N,K", [(65, 128, 64), (33, 384, 2048), (129, 384, 4096), (225, 256, 1024), (513, 1280, 640), (700, 4096, 576), (1999, 2304, 192), (257, 512, 14336)])
+@pytest.mark.parametrize("M,N,K", [(65, 128, 64), (33, 384, 2048), (129, 384, 4096), (225, 256, 1024), (513, 1280, 640), (700, 4096, 576), (1999, 2304, 192), (257, 512, 14336),
+                                   (33, 12672, 128), (65, 14336, 128), (256, 12672, 576), (257, 12672, 128), (200, 18944, 64), (100, 19072, 64), (100, 12544, 128)])
 def test_fp16_epilogues(dev, M, N, K):
     rng = np.random.default_rng(M + N + K)
     x, res = (rng.standard_normal(s).astype(np.float16) for s in ((M, K), (M, N)))
@@ -46,7 +47,9 @@ def test_fp16_epilogues(dev, M, N, K):
     assert (y.numpy()[M:] == 0).all()
 
 
-@pytest.mark.parametrize("M,N,K", [(33, 600, 1000), (65, 513, 520), (300, 1000, 1500), (1030, 4100, 712), (131, 1, 8)])
+# 12672 features, 99 tiles, and 18944, 148: a CTA per tile up to 256 rows; 12544, 98, and 19072, 149: pairs
+@pytest.mark.parametrize("M,N,K", [(33, 600, 1000), (65, 513, 520), (300, 1000, 1500), (1030, 4100, 712), (131, 1, 8), (64, 12665, 576), (65, 12665, 576), (129, 18944, 136), (256, 12665, 576),
+                                   (257, 12665, 136), (40, 12544, 136), (129, 19072, 136)])
 @pytest.mark.parametrize("glu", [False, True])
 def test_bf16_epilogues(dev, M, N, K, glu):
     """Any N and K: edges of the tiles in every direction, columns in 32 bits elsewhere, biases."""
