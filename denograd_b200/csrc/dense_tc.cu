@@ -295,12 +295,15 @@ int jg_dense_tc(jg_dev* dev, const DenseCall& c) {
   a.b0 = c.bias[0]; a.b1 = c.bias[1]; a.err = dev->err_word; a.M = c.M; a.N = c.N; a.K = c.K; a.ldy = c.ldy; a.limit = c.limit; a.out = c.out;
   a.w_late = jg_is_fresh(dev, c.w[0]) || jg_is_fresh(dev, c.w[1]);
   const int aligned = (uintptr_t)c.y % 16 == 0 && c.ldy % (c.out_f32 ? 4 : 8) == 0;
-  // more than 64 rows, GLU more than 32: pairs of CTAs (gemm_pair.cuh; both sides measured in gemm_tc.cu), but for few features or a short K, where tiles of theirs are too few or over
-  // too soon (prompts of 1999 tokens at 8B sizes, a 128 x 256 tile per CTA / pairs: Matulorn 42.5 / 38.7 ms, Rigazen 40.2 / 34.3)
+  // more than 64 rows, GLU more than 32 (see cta_per_tile): pairs of CTAs (gemm_pair.cuh; both sides measured in gemm_tc.cu), but for few
+  // features or a short K, where tiles of theirs are too few or over too soon (prompts of 1999 tokens at 8B sizes, a 128 x 256 tile per
+  // CTA / pairs: Matulorn 42.5 / 38.7 ms, Rigazen 40.2 / 34.3)
   if (c.M > 32 && c.epilogue == JG_DENSE_GLU && !cta_per_tile(dev, c.M, c.N))
-    return launch_pair<DensePairEpi<true>>(dev, "dense_pair", c.x, c.ldx, c.w[0], c.w[1], c.ldw, c.M, c.N, c.K, true, a.w_late, {a.y, a.y32, a.b0, a.b1, a.ldy, aligned, a.limit, a.out});
+    return launch_pair<DensePairEpi<true>>(dev, "dense_pair", c.x, c.ldx, c.w[0], c.w[1], c.ldw, c.M, c.N, c.K, true, a.w_late,
+                                           {a.y, a.y32, a.b0, a.b1, a.ldy, aligned, a.limit, a.out});
   if (c.M > 64 && c.N > 512 && c.K > 512 && c.epilogue != JG_DENSE_GLU)
-    return launch_pair<DensePairEpi<false>>(dev, "dense_pair", c.x, c.ldx, c.w[0], c.w[0], c.ldw, c.M, c.N, c.K, true, a.w_late, {a.y, a.y32, a.b0, a.b1, a.ldy, aligned, a.limit, a.out});
+    return launch_pair<DensePairEpi<false>>(dev, "dense_pair", c.x, c.ldx, c.w[0], c.w[0], c.ldw, c.M, c.N, c.K, true, a.w_late,
+                                            {a.y, a.y32, a.b0, a.b1, a.ldy, aligned, a.limit, a.out});
   if (c.epilogue == JG_DENSE_GLU) {
     if (c.M <= 16) return launch_dt<16, true, false>(dev, c, a);
     if (c.M <= 32) return launch_dt<32, true, false>(dev, c, a);

@@ -1,6 +1,7 @@
 // Dense projection on the 5th-generation tensor cores for 3 rows and more (batched decode, prompt processing):
 // Y[m][n] = epilogue( sum_k X[m][k] * W[n][k] ) with tcgen05.mma, the accumulator in tensor memory and both operands
-// brought into 128-byte swizzled shared memory by TMA (cp.async.bulk.tensor).
+// brought into 128-byte swizzled shared memory by TMA (cp.async.bulk.tensor).  Fp16 weights of more than 64 rows (gate and up: 32) mostly
+// go to pairs of CTAs instead (gemm_pair.cuh, launch_tc_rows).
 //
 // The roles of the MMA are swapped with respect to the usual GEMM picture so that both operands are K-major exactly as
 // they lie in memory (nn.Linear keeps W as [out][in], jsgrad/nn/index.ts:403-412): A = 128 weight rows x 64 k,
@@ -317,7 +318,7 @@ struct TcPairEpi {
     const __half* residual;
     int aligned;  // results (and residual) start on 16 bytes
   };
-  static __device__ __forceinline__ bool wide(const Args& e, const PairPlan& a, int feat) { return e.aligned && feat + 32 <= a.N; }
+  static __device__ __forceinline__ bool wide(const Args& e, const PairPlan& a, int feat) { return e.aligned && feat + (GLU ? 16 : 32) <= a.N; }
   static __device__ __forceinline__ bool f32(const Args&) { return EPI == TC_PARTIAL; }
   static __device__ __forceinline__ float* out32(const Args& e, const PairPlan& a, int tok, int feat) { return e.y32 + (size_t)tok * a.N + feat; }
   static __device__ __forceinline__ __half* out(const Args& e, const PairPlan& a, int tok, int feat) { return e.y + (size_t)tok * a.N + feat; }
@@ -414,12 +415,13 @@ static int launch_tc(jg_dev* dev, const void* x, const void* w0, const void* w1,
 
 template <int EPI>
 static int launch_tc_rows(jg_dev* dev, const void* x, const void* w0, const void* w1, const TcArgs& a) {
-  // more than 64 rows, gate and up more than 32: pairs of CTAs.  us per launch, one tile per CTA / pairs: 8B shapes, 45 rows qkv 19 / 15,
-  // wo 12 / 13, gate and up 45 / 44, down 25 / 28; 100 rows 23 / 17, 16 / 15, 48 / 48, 29 / 31; 512 rows 37 / 24, 35 / 19, 140 / 102,
-  // 70 / 54; 1B shapes, 45 rows 8 / 9, 9 / 10, 22 / 16, 15 / 15; 100 rows 11 / 10, 11 / 10, 25 / 18, 17 / 16
+  // more than 64 rows, gate and up more than 32 (see cta_per_tile): pairs of CTAs.  us per launch, weights from HBM, one tile per CTA /
+  // pairs: 8B shapes, 100 rows qkv 26.2 / 17.1, wo 17.0 / 14.9, down 31.0 / 32.2; 300 rows 26.4 / 19.9, 24.0 / 19.0, 53.5 / 40.5; 512
+  // rows 26.8 / 26.4, 24.4 / 21.5, 59.0 / 55.4, gate and up 119 / 105; 1B shapes, 100 rows 12.4 / 10.0, 13.3 / 10.0, 26.8 / 19.8,
+  // 20.6 / 16.1; 512 rows 15.7 / 11.7, 18.4 / 11.4, 40.3 / 34.5, 33.6 / 23.1
   if (a.s0 == nullptr && a.M > (EPI == TC_SWIGLU ? 32 : 64) && !(EPI == TC_SWIGLU && cta_per_tile(dev, a.M, a.N)))
-    return launch_pair<TcPairEpi<EPI>>(dev, "gemm_pair", x, a.K, w0, w1, a.K, a.M, a.N, a.K, false, a.w_late, 
-                                        {a.y, a.y32, a.residual, (uintptr_t)a.y % 16 == 0 && (uintptr_t)a.residual % 16 == 0});
+    return launch_pair<TcPairEpi<EPI>>(dev, "gemm_pair", x, a.K, w0, w1, a.K, a.M, a.N, a.K, false, a.w_late,
+                                       {a.y, a.y32, a.residual, (uintptr_t)a.y % 16 == 0 && (uintptr_t)a.residual % 16 == 0});
   if (a.s0 != nullptr) {  // int8 weights: used from 20 rows on (fewer go to the mma.sync kernel)
     if (a.M <= 32) return launch_tc<32, EPI, true>(dev, x, w0, w1, a);
     if (a.M <= 128) return launch_tc<128, EPI, true>(dev, x, w0, w1, a);

@@ -117,7 +117,7 @@ def NF4Linear(block_size: int):
 
         @property
         def scale_ptr(self) -> int:
-            return 0  # the projection kernels see the dequantised fp16 copy
+            return 0  # per-row scales are int8's; these weights have one per block (`scale`)
 
         def row_views(self, r0: int, r1: int) -> dict:
             k = self.in_features
