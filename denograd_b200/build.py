@@ -18,7 +18,7 @@ COMPONENTS = {"hybrid": CORE + DENSE + RECURRENT + BRANCHES, "hybrid_recurrent":
 # which of them a mixer of the layer-list models is in
 MIXER_COMPONENT = {"mingru": "hybrid_recurrent", "delta": "hybrid_recurrent", "latent_attention": "hybrid_recurrent", "mlstm": "hybrid_branches",
                    "parallel": "hybrid_branches", "window_attention": "hybrid_branches", "lightning": "hybrid_branches"}
-SOURCES = CORE + ["gemv.cu", "matvec_w8.cu", "matvec_nf4.cu", "gemm_small.cu", "gemm_tc.cu", "attention.cu", "attention_chunk.cu", "step.cu", "program.cu",
+SOURCES = CORE + ["gemv.cu", "matvec_w8.cu", "matvec_nf4.cu", "gemm_small.cu", "skinny.cu", "gemm_tc.cu", "attention.cu", "attention_chunk.cu", "step.cu", "program.cu",
                   *DENSE, *RECURRENT, *BRANCHES]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-fvisibility=hidden", "--expt-relaxed-constexpr"]

@@ -11,6 +11,7 @@
 
 #include "dense.cuh"
 #include "gemm_pair.cuh"
+#include "skinny.cuh"
 
 constexpr int DT_BM = 128, DT_BK = 64;
 
@@ -287,6 +288,38 @@ struct DensePairEpi {
   }
 };
 
+// ... and the kernel for few rows (skinny.cuh).
+struct SkDense {
+  struct Args {
+    bf16* y;
+    float* y32;
+    const float *b0, *b1;
+    int ldy, glu;
+    float limit;
+    DenseOut out;
+  };
+  struct Pre { float b0, b1, side; };
+  static __device__ __forceinline__ unsigned long long* keys(const Args&) { return nullptr; }
+  static __device__ __forceinline__ Pre fetch(const Args& e, int n, int m) {
+    return {e.b0 ? e.b0[n] : 0.f, e.glu && e.b1 ? e.b1[n] : 0.f, dense_side<bf16>(e.out, m, n)};
+  }
+  static __device__ __forceinline__ void store(const Args& e, int n, int m, float s, float u, const Pre& p, unsigned long long&) {
+    const size_t o = (size_t)m * e.ldy + n;
+    if (e.glu) { e.y[o] = __float2bfloat16_rn(clamped_glu(s + p.b0, u + p.b1, e.limit)); return; }
+    const float v = dense_act(e.out, n, s + p.b0, p.side);
+    if (n >= e.out.split) e.out.y2[(size_t)m * e.out.ld2 + n - e.out.split] = v;
+    else if (e.y32) e.y32[o] = v;
+    else e.y[o] = __float2bfloat16_rn(v);
+  }
+};
+template <bool GLU>
+static int launch_dense_skinny(jg_dev* dev, const DenseCall& c, const DtArgs& d) {
+  SkArgs a = {};
+  a.err = dev->err_word; a.M = c.M; a.N = c.N; a.w_late = d.w_late;
+  const SkOperands o = {c.x, c.w[0], c.w[GLU ? 1 : 0], c.K, c.ldx, c.ldw};
+  return launch_skinny_as<SK_BF16, 1, GLU, SkDense>(dev, "dense_skinny", o, a, {d.y, d.y32, d.b0, d.b1, d.ldy, GLU, d.limit, d.out});
+}
+
 int jg_dense_tc(jg_dev* dev, const DenseCall& c) {
   JG_REQUIRE(((uintptr_t)c.x % 16) == 0 && c.ldx % 8 == 0 && c.ldw % 8 == 0, "dense: operands must be 16-byte aligned with row strides of a multiple of 8");
   DtArgs a = {};
@@ -294,6 +327,10 @@ int jg_dense_tc(jg_dev* dev, const DenseCall& c) {
   else a.y = (bf16*)c.y;
   a.b0 = c.bias[0]; a.b1 = c.bias[1]; a.err = dev->err_word; a.M = c.M; a.N = c.N; a.K = c.K; a.ldy = c.ldy; a.limit = c.limit; a.out = c.out;
   a.w_late = jg_is_fresh(dev, c.w[0]) || jg_is_fresh(dev, c.w[1]);
+  // up to 8 rows: the kernel around the weight stream, but for gate and up whose 128-row tiles keep two thirds of the SMs busy here (both sides
+  // measured in skinny.cu; a Rigazen of 1B sizes, 8 rows: 1.49 / 1.31 ms a token with tiles of 128 rows / with that kernel)
+  if (c.M <= 8 && c.K % 64 == 0 && !(c.epilogue == JG_DENSE_GLU && c.N / DT_BM * 3 >= dev->sm_count * 2))
+    return c.epilogue == JG_DENSE_GLU ? launch_dense_skinny<true>(dev, c, a) : launch_dense_skinny<false>(dev, c, a);
   const int aligned = (uintptr_t)c.y % 16 == 0 && c.ldy % (c.out_f32 ? 4 : 8) == 0;
   // more than 64 rows, GLU more than 32 (see cta_per_tile): pairs of CTAs (gemm_pair.cuh; both sides measured in gemm_tc.cu), but for few
   // features or a short K, where tiles of theirs are too few or over too soon (prompts of 1999 tokens at 8B sizes, a 128 x 256 tile per

@@ -486,6 +486,11 @@ int jg_matvec_w8(jg_dev* dev, int epi, const void* x, const void* norm_w, float 
                  const void* s0, const void* s1, void* y, const void* residual, void* key, int M, int N, int K, int row_offset);
 bool jg_matvec_w8_fits(const jg_dev* dev, int M, int K);
 
+// skinny.cu: a few rows (activations already normalised)
+int jg_skinny(jg_dev* dev, int epi, const void* x, const void* w0, const void* w1, const void* s0, const void* s1, void* y, const void* residual,
+              void* key, int M, int N, int K, int row_offset);
+bool jg_skinny_fits(const jg_dev* dev, bool w8, int epi, int M, int N, int K);
+
 // gemm_tc.cu: tcgen05 / TMA projection (fp16 weights, N % 128 == 0, K % 64 == 0), any number of rows
 int jg_gemm_tc(jg_dev* dev, int epi, const void* x, const void* w0, const void* w1, void* y, const void* residual, int M, int N, int K,
                const void* s0, const void* s1);
@@ -535,6 +540,8 @@ static int dispatch_m(jg_dev* dev, const GemvArgs& a, const char* name) {
     jg_set_error("%s: the projection fused with its all-reduce takes at most 8 rows (M=%d)", name, a.M);
     return JG_ENOTSUP;
   }
+  if (!NORM && jg_skinny_fits(dev, W8, EPI, a.M, a.N, a.K))
+    return jg_skinny(dev, EPI, a.x, a.w0, a.w1, a.s0, a.s1, EPI == EPI_PARTIAL ? (void*)a.y32 : (void*)a.y, a.residual, a.key, a.M, a.N, a.K, a.row_offset);
   if (!W8 && !NORM && EPI != EPI_LOGITS && (a.M > 64 || (a.M >= tc_min_rows() && jg_gemm_tc_fits(a.N, a.K))))
     return jg_gemm_tc(dev, EPI, a.x, a.w0, a.w1, EPI == EPI_PARTIAL ? (void*)a.y32 : (void*)a.y, a.residual, a.M, a.N, a.K, nullptr, nullptr);
   // int8 weights and enough rows: the tcgen05 kernel with the conversion inside it

@@ -2,8 +2,10 @@
 // y[m][n] = half( sum_k float( x[m][k] * half(CODE[code] * scale) ) ), fp32 accumulation, one fp16 scale per `block`
 // consecutive elements of the flattened matrix.
 //
+// The kernel here takes the shapes that skinny.cuh does not (n4_skinny).
+//
 // The matrix crosses HBM once, packed.  (Writing an fp16 copy first and projecting from that moves 9 bytes per pair of
-// weights instead of 1: 10.0 ms per token for the 8B shapes, 2.8 now.)  At that rate the unpacking is what
+// weights instead of 1: 10.0 ms per token for the 8B shapes, 2.8 with this kernel.)  At that rate the unpacking is what
 // counts: a byte holds two codes, and the pair's fp16 values come out of a 256-entry table in shared memory, one word of
 // it per lane and byte in the lane's own bank (32 KB; a table shared by the lanes would meet 3-4 conflicts per access),
 // so a pair of weights takes a shift, a mask, a load and a half2 product with the block's scale (one rounding, as the
@@ -14,7 +16,7 @@
 // A warp walks its (tile, k block) pairs with U loads of each row in flight, refilled across the ends of tiles; KS warps
 // share a tile and add their sums in a fixed order at a barrier of their own, two copies of the sums taking turns.
 // Epilogues: STORE, RESIDUAL (fp16 add), SWIGLU (two matrices).
-#include "common.cuh"
+#include "skinny.cuh"
 #include "transcendental.cuh"
 
 enum { N4_STORE = 0, N4_RESIDUAL = 1, N4_SWIGLU = 2 };
@@ -187,6 +189,36 @@ static int launch_n4_ks(jg_dev* dev, const Nf4Args& a, const char* name) {
   return launch_n4<EPI, 8>(dev, a, name);
 }
 
+// What skinny.cuh does with a sum: the roundings above.
+struct SkNf4 {
+  struct Args {
+    __half* y;
+    const __half* residual;
+    int N, glu;
+  };
+  typedef __half Pre;
+  static __device__ __forceinline__ unsigned long long* keys(const Args&) { return nullptr; }
+  static __device__ __forceinline__ __half fetch(const Args& e, int n, int m) { return e.residual ? e.residual[(size_t)m * e.N + n] : __float2half_rn(0.f); }
+  static __device__ __forceinline__ void store(const Args& e, int n, int m, float s, float u, __half pre, unsigned long long&) {
+    __half v = __float2half_rn(s);
+    if (e.residual) v = hadd1(pre, v);
+    if (e.glu) v = jg_silu_mul(v, __float2half_rn(u));
+    e.y[(size_t)m * e.N + n] = v;
+  }
+};
+// Rows of whole 128-byte runs and blocks whose scales come in 16-byte pieces: the kernel around the weight stream (skinny.cuh).
+static bool n4_skinny(const Nf4Args& a) {
+  return a.block_shift >= 5 && a.block_shift <= 8 && a.K % (8 << a.block_shift) == 0 && a.K % 256 == 0 && (uintptr_t)a.s0 % 16 == 0 && (uintptr_t)a.s1 % 16 == 0;
+}
+template <bool GLU>
+static int launch_n4_skinny(jg_dev* dev, const Nf4Args& n, const char* name) {
+  SkArgs a = {};
+  a.s0 = n.s0; a.s1 = n.s1; a.err = dev->err_word; a.M = n.M; a.N = n.N; a.block_shift = n.block_shift; a.w_late = n.late;
+  const SkOperands o = {n.x, n.w0, n.w1, n.K, n.K, n.K};
+  const SkNf4::Args e = {n.y, n.residual, n.N, GLU};
+  return launch_skinny_as<SK_NF4, 1, GLU, SkNf4>(dev, name, o, a, e);
+}
+
 // Rows a call takes.  One n-tile of the MMA: up to 8 rows cost what one does.  Beyond, a dequantised copy and the
 // tensor-core projection are used (jg_dequant_nf4_f16, jg_linear).
 constexpr int N4_MAX_ROWS = 8;
@@ -211,9 +243,10 @@ JG_API int jg_linear_nf4(jg_dev* dev, uint64_t y, uint64_t x, uint64_t w, uint64
   if (rc) return rc;
   a.late = jg_is_fresh(dev, a.w0) || jg_is_fresh(dev, a.s0);
   jg_mark_fresh(dev, y, (uint64_t)M * N * 2);
-  if (!residual) return launch_n4_ks<N4_STORE>(dev, a, "linear_nf4");
-  JG_REQUIRE(jg_aligned(residual, 2), "linear_nf4: misaligned residual pointer");
+  JG_REQUIRE(residual == 0 || jg_aligned(residual, 2), "linear_nf4: misaligned residual pointer");
   a.residual = (const __half*)residual;
+  if (n4_skinny(a)) return launch_n4_skinny<false>(dev, a, "linear_nf4");
+  if (!residual) return launch_n4_ks<N4_STORE>(dev, a, "linear_nf4");
   return launch_n4_ks<N4_RESIDUAL>(dev, a, "linear_nf4");
 }
 
@@ -227,5 +260,6 @@ JG_API int jg_swiglu_nf4(jg_dev* dev, uint64_t y, uint64_t x, uint64_t w_gate, u
   a.w1 = (const uint8_t*)w_up; a.s1 = (const __half*)s_up;
   a.late = jg_is_fresh(dev, a.w0) || jg_is_fresh(dev, a.s0) || jg_is_fresh(dev, a.w1) || jg_is_fresh(dev, a.s1);
   jg_mark_fresh(dev, y, (uint64_t)M * N * 2);
+  if (n4_skinny(a)) return launch_n4_skinny<true>(dev, a, "swiglu_nf4");
   return launch_n4_ks<N4_SWIGLU>(dev, a, "swiglu_nf4");
 }

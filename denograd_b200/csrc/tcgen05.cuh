@@ -66,6 +66,11 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
                ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
                : "memory");
 }
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+               ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
+}
 // K-major operand tile in 128-byte swizzled shared memory: rows of 128 bytes, 8-row groups 1024 bytes apart.
 __device__ __forceinline__ uint64_t umma_desc(const void* tile) {
   const uint32_t lo = ((smem_u32(tile) & 0x3FFFFu) >> 4) | (1u << 16);  // start address, leading byte offset = 1 (unused)
@@ -119,5 +124,7 @@ __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
 // Tensor map of a row-major [rows][cols] matrix of 16-bit elements (or int8 when bytes == 1) with `ld` elements between
 // rows, cut into boxes of box_rows x 64; out-of-range elements read as zero.  Maps are kept per argument set; `out` is a
 // copy, because the next call may reuse the slot this one came from.
+// groups > 0: boxes of box_rows x `groups` runs of 128 bytes, [run][row][128 bytes] in shared memory (rows of a whole number of
+// runs); groups < 0: boxes of box_rows x -groups elements, as they lie.
 int jg_tensor_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows,
-                  const char* what, int bytes = 2, bool bf16 = false);
+                  const char* what, int bytes = 2, bool bf16 = false, int groups = 0);

@@ -1,0 +1,74 @@
+"""The projections of a few rows around the weight stream (skinny.cuh) at the edges of their tiles: outputs fewer than CTAs, a row more
+than a tile, one and two tiles to a warp, a second pass; K of one run, and with a last stage that is not full."""
+import numpy as np
+import pytest
+
+from denograd_b200 import Device
+from denograd_b200.device import Tensor
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    return Device["CUDA"]
+
+
+def weights(rng, kind, N, K, dev):
+    """(pointers of matrix and scales, dequantised values in 64 bits)"""
+    if kind == "int8":
+        q, s = rng.integers(-127, 128, (N, K), dtype=np.int8), (rng.uniform(0.5, 1.5, N) * 3e-4).astype(np.float16)
+        return (Tensor(q, device=dev), Tensor(s, device=dev)), (q.astype(np.float16) * s[:, None]).astype(np.float64)
+    w = (rng.standard_normal((N, K)) * 0.02).astype(np.float16)
+    return (Tensor(w, device=dev), None), w.astype(np.float64)
+
+
+@pytest.mark.parametrize("kind", ["float16", "int8"])
+@pytest.mark.parametrize("M,N,K", [(3, 5, 128), (8, 149, 256), (4, 148 * 16 + 3, 1152), (7, 148 * 64 + 130, 384), (8, 148 * 136 + 9, 128), (5, 148 * 256 + 77, 128), (16, 700, 2048)])
+def test_edges_of_tiles(dev, kind, M, N, K):
+    """Tolerance: the fp32 sum of K exact products (relative to the sum of their magnitudes) and an fp16 rounding per elementwise op."""
+    rng = np.random.default_rng(M * 7 + N + K)
+    x, res = rng.standard_normal((M, K)).astype(np.float16), rng.standard_normal((M, N)).astype(np.float16)
+    (w, s), dw = weights(rng, kind, N, K, dev)
+    (w3, s3), dw3 = weights(rng, kind, N, K, dev)
+    sp, sp3 = s.ptr if s else 0, s3.ptr if s3 else 0
+    xt, rt, y = Tensor(x, device=dev), Tensor(res, device=dev), Tensor.zeros((M, N), "float16", dev)
+    x64, ulp, eps = x.astype(np.float64), 2.0 ** -11, 2.0 ** -20
+    g, u, mg, mu = x64 @ dw.T, x64 @ dw3.T, np.abs(x64) @ np.abs(dw).T, np.abs(x64) @ np.abs(dw3).T
+
+    def check(want, bound):
+        assert (np.abs(y.numpy().astype(np.float64) - want) <= bound + 1e-7).all()
+
+    dev.call("jg_linear", y.ptr, xt.ptr, w.ptr, sp, 0, M, N, K)
+    check(g, eps * mg + ulp * np.abs(g) * 1.01)
+    dev.call("jg_linear", y.ptr, xt.ptr, w.ptr, sp, rt.ptr, M, N, K)
+    check(g + res, eps * mg + ulp * (np.abs(g) + np.abs(g + res)) * 1.01)
+    dev.call("jg_norm_swiglu", y.ptr, xt.ptr, 0, 1e-5, w.ptr, sp, w3.ptr, sp3, M, N, K)
+    want = g / (1 + np.exp(-g)) * u
+    check(want, 8 * ulp * np.abs(want) + 1.2 * np.abs(u) * (eps * mg + ulp * np.abs(g)) + np.abs(g) * eps * mu + 1e-4)
+    p32 = Tensor.zeros((M, N), "float32", dev)
+    dev.call("jg_linear_partial", p32.ptr, xt.ptr, w.ptr, sp, M, N, K)
+    assert (np.abs(p32.numpy() - g) <= eps * mg + 1e-7).all()
+    key, tok = Tensor.zeros((M,), "uint64", dev), Tensor.empty((M,), "int32", dev)
+    dev.call("jg_norm_logits_argmax", y.ptr, key.ptr, xt.ptr, 0, 1e-5, w.ptr, sp, M, N, K)
+    dev.call("jg_argmax_finalize", tok.ptr, key.ptr, M)
+    check(g, eps * mg + ulp * np.abs(g) * 1.01)
+    assert tok.numpy().tolist() == [O.argmax_f16(r) for r in y.numpy()]
+
+
+@pytest.mark.parametrize("M,N,K,block", [(1, 148 * 72 + 5, 512, 64), (8, 150, 256, 32), (2, 33, 2048, 256), (1, 14, 8192, 64)])
+def test_nf4_blocks_and_stages(dev, M, N, K, block):
+    """Blocks of 32 to 256: the scales of a stage take 16 bytes a row at least."""
+    rng = np.random.default_rng(N + block)
+    code = np.array([-1.0, -0.6961928009986877, -0.5250730514526367, -0.39491748809814453, -0.28444138169288635, -0.18477343022823334,
+                     -0.09105003625154495, 0.0, 0.07958029955625534, 0.16093020141124725, 0.24611230194568634, 0.33791524171829224,
+                     0.44070982933044434, 0.5626170039176941, 0.7229568362236023, 1.0]).astype(np.float16)
+    x, c = rng.standard_normal((M, K)).astype(np.float16), rng.integers(0, 16, N * K).astype(np.uint8)
+    s = (0.02 + 0.05 * rng.random(N * K // block)).astype(np.float16)
+    d = (code[c].reshape(-1, block) * s[:, None]).astype(np.float16).reshape(N, K).astype(np.float64)
+    xt, y = Tensor(x, device=dev), Tensor.zeros((M, N), "float16", dev)
+    wt, st = Tensor(c[0::2] * 16 + c[1::2], device=dev), Tensor(s, device=dev)
+    dev.call("jg_linear_nf4", y.ptr, xt.ptr, wt.ptr, st.ptr, 0, M, N, K, block)
+    want, mag = x.astype(np.float64) @ d.T, np.abs(x.astype(np.float64)) @ np.abs(d).T
+    assert (np.abs(y.numpy().astype(np.float64) - want) <= 2.0 ** -20 * mag + 2.0 ** -11 * np.abs(want) * 1.01 + 1e-7).all()
