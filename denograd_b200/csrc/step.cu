@@ -17,15 +17,14 @@
 //               P6 h += W2 ffn                                                          | barrier
 //   per step    x = RMSNorm(h) * g;  logits = Wout x, (value, lowest index) max key     | barrier, pick, feed back
 //
-// The point of the arrangement is that the weight stream never stops at a phase boundary: weights do not depend on
-// activations, so before a CTA arrives at a barrier it has already issued the first two passes of the NEXT projection
-// into registers (128 KB per SM in flight), and while the two attention phases run (which move 1 MB at short contexts)
-// every CTA has its share of Wo and the head of its W1 / W3 rows brought into L2.
+// The point of the arrangement is that the weight stream never stops at a phase boundary: weights do not depend on activations, so
+// one warp of every CTA walks the step's matrices in order and keeps 128 to 192 KB of passes in flight as bulk copies into a ring in
+// shared memory, while the others stage activations, wait at a barrier or work on attention.
 //
-// A projection phase: the CTA owns a contiguous run of output rows; its 16 warps split K (thread t owns the 16-byte
-// chunks t, t + 512, ... of every row), a pass is 8 loads per lane (R rows x NI chunks x NW matrices), two passes are
-// in flight (register double buffer), the per-warp partial sums of a pass meet in shared memory at one barrier per
-// pass and are finished in warp order (fixed summation order: results do not depend on timing).
+// A projection phase: passes of a few whole rows are dealt to the CTAs in turn; the 16 computing warps share a pass by rows and by K,
+// run through the ring at their own pace and meet once per batch of passes (st_project).  Fixed summation order: results do not
+// depend on timing.  us per step, with a barrier of all warps per pass / so: 1B 856 / 792 (one row), 1090 / 880 (two), 8B 3.61 / 3.36 ms
+// (two rows; one row waits for HBM either way: 6.46 TB/s in the gate and up phase), 3B 2.10 / 1.93 (two rows).
 // Arithmetic is that of the stand-alone kernels (gemv.cu, attention.cu): exact fp16 products accumulated in fp32,
 // every elementwise fp16 operation rounded once, softmax probabilities formed from the global max and sum and rounded
 // to fp16 before they meet v (jsgrad/tensor.ts:2186-2214, 2593-2605; jsgrad/nn/index.ts:586-588).
@@ -39,9 +38,9 @@
 #include "peer.cuh"
 #include "transcendental.cuh"
 
-constexpr int ST_THREADS = 512;
+constexpr int ST_THREADS = 512;  // that compute; one more warp requests the weights
 constexpr int ST_WARPS = ST_THREADS / 32;
-constexpr int ST_PART = 16;  // partial sums per warp and pass: NW * R * MT <= 16
+constexpr int ST_PART = 384;  // partial sums of a batch of passes
 
 struct StepLayer {
   const __half* attn_norm;
@@ -127,12 +126,15 @@ __device__ __forceinline__ bool st_mbar_wait(uint64_t* bar, uint32_t parity, uns
   }
 }
 
+// Barrier of the CTA's computing warps (the warp that requests the weights goes its own way).
+__device__ __forceinline__ void st_sync() { asm volatile("bar.sync 1, %0;" ::"n"(ST_THREADS) : "memory"); }
+
 // Grid-wide barrier: every CTA adds one to a counter the host zeroed before the launch and waits until the counter
 // reaches the barrier's ordinal times the grid size.  All CTAs are resident (cooperative launch).  Returns false when
 // the wait ran out; the caller leaves the kernel.
 __device__ __forceinline__ bool st_grid_sync(const StepArgs& a, unsigned& nbar) {
   __shared__ int s_ok;
-  __syncthreads();
+  st_sync();
   if (threadIdx.x == 0) {
     int ok = 1;
     nbar++;
@@ -154,13 +156,13 @@ __device__ __forceinline__ bool st_grid_sync(const StepArgs& a, unsigned& nbar) 
     s_ok = ok;
     if (!ok) atomicCAS(a.err, 0, 4);
   }
-  __syncthreads();
+  st_sync();
   return s_ok != 0;
 }
 
-// ---- the weight stream.  Thread 0 of the CTA walks the step's projections in order (qkv, wo, gate/up, down of every
+// ---- the weight stream.  The CTA's last warp walks the step's projections in order (qkv, wo, gate/up, down of every
 // layer, then the output matrix, then the next step) and keeps `nslot` passes in flight as bulk copies into a ring of
-// shared-memory slots; the copy of pass q + nslot is issued the moment pass q has been consumed.  The walk does not stop
+// shared-memory slots; the copy of pass q + nslot is issued the moment pass q has been read by all computing warps.  The walk does not stop
 // at phase boundaries: while the CTA stages activations, waits at a grid barrier or works on attention, the first
 // passes of the next projection are landing.
 // How an N-row matrix is dealt to the CTAs in passes of rs rows: CTA c takes passes c, c + grid, c + 2 grid, ... (at
@@ -223,7 +225,7 @@ __device__ __forceinline__ void st_stream_next_phase(StepStream& st, const StepA
     st_stream_enter<RS_D, RS_G, RS_H>(st, a, qkv_dim);
   } while (st.left <= 0);
 }
-// Request the next pass of the walk into the slot that has just been consumed (the CTA's producer thread only).
+// Request the next pass of the walk into the next slot (the CTA's producer thread only).
 template <int RS_D, int RS_G, int RS_H>
 __device__ __forceinline__ void st_stream_issue(StepStream& st, const StepArgs& a, int qkv_dim, unsigned char* ring, uint64_t* full) {
   if (st.step >= a.n_steps) return;
@@ -248,88 +250,89 @@ __device__ __forceinline__ void st_stream_issue(StepStream& st, const StepArgs& 
 // Where the consumer is in the ring: slot of the next pass and the parity of that slot's barrier.
 struct StepRing { uint32_t slot, parity; };
 
-constexpr int ST_PRODUCER = ST_THREADS - 32;  // the thread that requests the weight passes (lane 0 of the last warp)
-
-// One projection phase of this CTA: its passes of RS rows (of each of NW matrices) of an N-row matrix; thread t multiplies
-// the 16-byte chunks t, t + 512, ... of every row of the pass (read from the slot) with the activations; the per-warp
-// partial sums meet in shared memory at one barrier per pass, after which the producer thread refills the slot and
-// output o of the pass (o < RS * MT) is finished by lane 0 of warp o, in warp order (fixed summation order) — one
-// output per warp, so that no warp carries the whole epilogue.  `pre(row, m)` fetches what the epilogue needs from
-// global memory (the residual) before the pass is multiplied.  A data wait that runs out is recorded and the pass is
-// carried on with whatever the slot holds (the launch's results are void then).
-template <int RS, int NI, int NW, int MT, class Pre, class Epi, class Refill>
-__device__ __forceinline__ void st_project(int N, int KC, const __half* xs, int M, const unsigned char* ring, uint64_t* full,
-                                           StepRing& rg, unsigned& seq, float (*part)[ST_PART * ST_WARPS], const StepArgs& a, int tid,
-                                           Pre pre, Epi epi, Refill refill) {
-  static_assert(RS * NW * MT <= ST_PART && RS * MT <= ST_WARPS, "partial sums per warp; one output per finishing warp");
+// One projection phase of this CTA: its passes of RS rows (of each of NW matrices) of an N-row matrix.  The warps share a pass by
+// rows and by K: of ROWS rows, RG groups of RPW rows go to KSP warps each, which have every KSP-th run of 32 16-byte chunks (8 rows: 4
+// groups of 2 rows, K over 4 warps, whose lanes read an activation chunk once for both rows and reduce two sums instead of eight).
+// Each warp goes through the ring at its own pace: it waits for a pass's bytes and arrives at the slot's second mbarrier when it has
+// read them.  (With a barrier of all warps per pass, a pass took 2000 cycles even when its bytes had landed long before: wait,
+// products, reductions and finishing one after the other.)  The sums of a batch of
+// passes meet in shared memory at one barrier, after which thread o finishes output o of the batch, adding in a fixed order.
+// `pre(row, m)` fetches what the epilogue needs from global memory (the residual) when the batch begins.  A data wait that runs out is
+// recorded and the pass is carried on with whatever the slot holds (the launch's results are void then).
+template <int RS, int NI, int NW, int MT, class Pre, class Epi>
+__device__ __forceinline__ void st_project(int N, int KC, const __half* xs, int M, const unsigned char* ring, uint64_t* full, uint64_t* empty,
+                                           StepRing& rg, unsigned& batch, float (*part)[ST_PART], const StepArgs& a, int tid,
+                                           Pre pre, Epi epi) {
+  constexpr int ROWS = RS * NW, RG = ROWS % 8 == 0 ? 4 : ROWS % 4 == 0 ? 2 : 1, KSP = ST_WARPS / RG, RPW = ROWS / RG;
+  constexpr int SUMS = ROWS * MT * KSP, BATCH = ST_PART / SUMS < 16 ? ST_PART / SUMS : 16;  // of a pass; passes of a batch
+  static_assert(BATCH >= 1 && BATCH * RS * MT <= ST_THREADS, "a thread per output of a batch");
   const int K = KC * 8;
   const uint32_t row_bytes = (uint32_t)KC * 16u;
   const int bid = blockIdx.x, nb = gridDim.x;
-  const StepSplit sp = st_split(N, RS);
-  const int np = sp.passes;
-  const int lane = tid & 31, warp = tid >> 5;
-  const int fr = warp / MT, fm = warp % MT;  // the output lane 0 of this warp finishes (warp < RS * MT)
-  for (int p = 0; p < np; p++) {
-    const int frow = (bid + p * nb) * RS + fr;
-    const bool fin = lane == 0 && warp < RS * MT && fm < M && frow < N;
+  const int np = st_split(N, RS).passes;
+  const int lane = tid & 31, warp = tid >> 5, kpart = warp % KSP, r0 = warp / KSP * RPW;
+  const int fp = tid / (RS * MT), fr = tid / MT % RS, fm = tid % MT;  // the output of a batch that this thread finishes
+  for (int p0 = 0; p0 < np; p0 += BATCH) {
+    const int n_batch = min(BATCH, np - p0), frow = (bid + (p0 + fp) * nb) * RS + fr;
+    const bool fin = fp < n_batch && fm < M && frow < N;
     __half prev = __float2half_rn(0.f);
     if (fin) prev = pre(frow, fm);
-    if (!st_mbar_wait(full + rg.slot, rg.parity, a.timeout_ns)) atomicCAS(a.err, 0, 5);
-    const unsigned char* sl = ring + (size_t)rg.slot * a.slot_bytes;
-    float acc[NW * RS][MT];
+    float* pp = part[batch & 1u];  // [pass][row][m][k part]
+    for (int p = 0; p < n_batch; p++) {
+      if (!st_mbar_wait(full + rg.slot, rg.parity, a.timeout_ns)) atomicCAS(a.err, 0, 5);
+      const unsigned char* sl = ring + (size_t)rg.slot * a.slot_bytes + (size_t)r0 * row_bytes;
+      float acc[RPW][MT];
 #pragma unroll
-    for (int j = 0; j < NW * RS; j++)
+      for (int j = 0; j < RPW; j++)
 #pragma unroll
-      for (int m = 0; m < MT; m++) acc[j][m] = 0.f;
+        for (int m = 0; m < MT; m++) acc[j][m] = 0.f;
+#pragma unroll (RG * NI <= 8 ? RG * NI : 4)
+      for (int i = 0; i < RG * NI; i++) {
+        const int c = kpart * 32 + lane + i * KSP * 32;
+        if (c < KC) {
+          float xf[MT][8];
 #pragma unroll
-    for (int i = 0; i < NI; i++) {
-      const int c = tid + ST_THREADS * i;
-      if (c < KC) {
-        float xf[MT][8];
+          for (int m = 0; m < MT; m++) unpack8(*reinterpret_cast<const uint4*>(xs + (size_t)m * K + (size_t)c * 8), xf[m]);
 #pragma unroll
-        for (int m = 0; m < MT; m++) unpack8(*reinterpret_cast<const uint4*>(xs + (size_t)m * K + (size_t)c * 8), xf[m]);
+          for (int j = 0; j < RPW; j++) {
+            const uint4 wv = *reinterpret_cast<const uint4*>(sl + (size_t)j * row_bytes + (size_t)c * 16);
 #pragma unroll
-        for (int j = 0; j < NW * RS; j++) {
-          const uint4 wv = *reinterpret_cast<const uint4*>(sl + (size_t)j * row_bytes + (size_t)c * 16);
-#pragma unroll
-          for (int m = 0; m < MT; m++) acc[j][m] = dot8_acc(acc[j][m], wv, xf[m]);
+            for (int m = 0; m < MT; m++) acc[j][m] = dot8_acc(acc[j][m], wv, xf[m]);
+          }
         }
       }
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(st_smem_u32(empty + rg.slot)) : "memory");
+#pragma unroll
+      for (int j = 0; j < RPW; j++)
+#pragma unroll
+        for (int m = 0; m < MT; m++) {
+          const float v = warp_sum(acc[j][m]);
+          if (lane == 0) pp[((p * ROWS + r0 + j) * MT + m) * KSP + kpart] = v;
+        }
+      if (++rg.slot == (uint32_t)a.nslot) { rg.slot = 0; rg.parity ^= 1u; }
     }
-    float* pp = part[seq & 1u];  // [value][warp]
-#pragma unroll
-    for (int j = 0; j < NW * RS; j++)
-#pragma unroll
-      for (int m = 0; m < MT; m++) {
-        const float v = warp_sum(acc[j][m]);
-        if (lane == 0) pp[(j * MT + m) * ST_WARPS + warp] = v;
-      }
-    __syncthreads();
-    if (tid == ST_PRODUCER) refill();
+    batch++;
+    st_sync();
     if (fin) {
-      auto sum16 = [&](int value) {
-        const float4* q = reinterpret_cast<const float4*>(pp + value * ST_WARPS);
+      auto sum = [&](int row) {
+        const float* q = pp + ((fp * ROWS + row) * MT + fm) * KSP;
         float t = 0.f;
 #pragma unroll
-        for (int w = 0; w < ST_WARPS / 4; w++) {
-          const float4 v = q[w];
-          t += v.x; t += v.y; t += v.z; t += v.w;
-        }
+        for (int w = 0; w < KSP; w++) t += q[w];
         return t;
       };
-      const float s_a = sum16(fr * MT + fm);
-      const float s_b = NW == 2 ? sum16((RS + fr) * MT + fm) : 0.f;
+      const float s_a = sum(fr);
+      const float s_b = NW == 2 ? sum(RS + fr) : 0.f;
       epi(frow, fm, s_a, s_b, prev);
     }
-    seq++;
-    if (++rg.slot == (uint32_t)a.nslot) { rg.slot = 0; rg.parity ^= 1u; }
   }
 }
 
 // RS_D / RS_G / RS_H: rows per pass of a projection with K = dim (one matrix), of the gate / up pair (rows of each), with
 // K = hidden; NI_D / NI_H: 16-byte chunks per thread and row (K / 8 chunks over 512 threads).
 template <int MT, int HD, int NREP, int RS_D, int RS_G, int RS_H, int NI_D, int NI_H>
-__global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a) {
+__global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepArgs a) {
   static_assert(NREP <= 4 && MT <= 2, "register budget of 128 per thread");
   constexpr int LPR = HD / 8;    // lanes per K / V row
   constexpr int RPW = 32 / LPR;  // rows per warp pass
@@ -342,8 +345,9 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
   float* sc = reinterpret_cast<float*>(st_smem);                     // [NREP][chunk_cap]
   float* pv_part = sc + (size_t)NREP * a.chunk_cap;                   // [ST_WARPS / 2][NREP][HD]
   unsigned char* ring = st_smem + a.ring_offset;                     // [nslot][slot_bytes] weight passes in flight
-  __shared__ __align__(8) uint64_t full[ST_MAX_SLOTS];
-  __shared__ __align__(16) float part[2][ST_PART * ST_WARPS];
+  __shared__ __align__(8) uint64_t full[ST_MAX_SLOTS], empty[ST_MAX_SLOTS];
+  __shared__ int s_quit;  // the computing warps have left: no more passes
+  __shared__ __align__(16) float part[2][ST_PART];
   __shared__ float red[ST_WARPS][4];
   __shared__ float s_rs[MT];
   __shared__ float s_m[4], s_M[4], s_rL[4];
@@ -366,30 +370,50 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
   const float log2e = 1.4426950408889634f;
 
   unsigned gen = 0;  // grid barriers passed
-  unsigned seq = 0;  // weight passes consumed
+  unsigned batch = 0;  // batches of weight passes finished
 
   // the weight stream starts before anything else: nslot passes are on their way while the first rows are staged
-  StepStream st;
   StepRing rg;
   rg.slot = 0; rg.parity = 0;
-  unsigned issued = 0;  // passes requested (producer thread)
-  if (tid == ST_PRODUCER) {
-    for (int i = 0; i < a.nslot; i++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(st_smem_u32(full + i)) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    st.step = 0; st.layer = 0; st.phase = 0; st.slot = 0;
-    st_stream_enter<RS_D, RS_G, RS_H>(st, a, qkv_dim);
-    if (st.left <= 0) st_stream_next_phase<RS_D, RS_G, RS_H>(st, a, qkv_dim);
-    for (int i = 0; i < a.nslot; i++) {
-      if (st.step < a.n_steps) issued++;
-      st_stream_issue<RS_D, RS_G, RS_H>(st, a, qkv_dim, ring, full);
+  if (warp == ST_WARPS) {
+    StepStream st;
+    if (lane == 0) {
+      s_quit = 0;
+      for (int i = 0; i < a.nslot; i++) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(st_smem_u32(full + i)) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(st_smem_u32(empty + i)), "n"(ST_WARPS) : "memory");
+      }
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      st.step = 0; st.layer = 0; st.phase = 0; st.slot = 0;
+      st_stream_enter<RS_D, RS_G, RS_H>(st, a, qkv_dim);
+      if (st.left <= 0) st_stream_next_phase<RS_D, RS_G, RS_H>(st, a, qkv_dim);
+      for (int i = 0; i < a.nslot; i++) st_stream_issue<RS_D, RS_G, RS_H>(st, a, qkv_dim, ring, full);
     }
+    __syncthreads();  // the barriers are there
+    if (lane == 0) {
+      // The computing warps may stand at a grid barrier for as long as its limit allows; if they leave, they say so.
+      const unsigned limit = (unsigned)(a.timeout_ns / 250000ull) + 4u;  // milliseconds: four times theirs
+      uint32_t slot = 0, parity = 0;
+      unsigned left = 0;  // passes whose landing is still to be seen
+      bool quit = false;
+      while (st.step < a.n_steps && !quit) {
+        for (unsigned ms = 0; !quit && !st_mbar_wait(empty + slot, parity, 1000000ull); ms++)
+          if (*(volatile int*)&s_quit || ms > limit) quit = true;
+        if (quit) break;
+        st_stream_issue<RS_D, RS_G, RS_H>(st, a, qkv_dim, ring, full);
+        if (++slot == (uint32_t)a.nslot) { slot = 0; parity ^= 1u; }
+      }
+      if (quit) {  // none of the copies in flight may land in the memory of a CTA that has gone: the slots from `slot` on hold the last nslot passes
+        for (left = 0; left < (unsigned)a.nslot; left++) {
+          st_mbar_wait(full + slot, parity, a.timeout_ns);
+          if (++slot == (uint32_t)a.nslot) { slot = 0; parity ^= 1u; }
+        }
+      }
+    }
+    return;
   }
   __syncthreads();
-  auto refill = [&]() {
-    if (st.step < a.n_steps) issued++;
-    st_stream_issue<RS_D, RS_G, RS_H>(st, a, qkv_dim, ring, full);
-  };
   auto no_pre = [](int, int) { return __float2half_rn(0.f); };
   auto residual = [&](int row, int m) { return __ldcg(a.h + (size_t)m * dim + row); };
   const uint32_t ex_per_step = (uint32_t)(2 * a.n_layers + 1);  // exchanges of a step: Wo and W2 of every layer, the pick
@@ -439,18 +463,12 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
     }
     if (!ok) atomicCAS(a.peer.err, 0, 1);  // a rank never arrived: the launch's results are void, nobody is waited for
   };
-  // a wait ran out: record it, let the copies still in flight land (bounded) so that none writes into shared memory of
-  // a CTA that has gone, and leave
+  // a wait ran out: record it, send the producer home (it lets the copies in flight land) and leave
   auto give_up = [&](int code) {
-    if (tid == ST_PRODUCER) {
+    if (tid == 0) {
       atomicCAS(a.err, 0, code);
-      StepRing r = rg;
-      for (unsigned q = seq; q < issued; q++) {
-        st_mbar_wait(full + r.slot, r.parity, a.timeout_ns);
-        if (++r.slot == (uint32_t)a.nslot) { r.slot = 0; r.parity ^= 1u; }
-      }
+      *(volatile int*)&s_quit = 1;
     }
-    __syncthreads();
   };
 
   // x <- RMSNorm(rows) * g into shared memory (rows beyond M are zero); src(m) = the row's address
@@ -473,13 +491,13 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
       ss[m] = warp_sum(ss[m]);
       if (lane == 0) red[warp][m] = ss[m];
     }
-    __syncthreads();
+    st_sync();
     if (tid < MT) {
       float t = 0.f;
       for (int i = 0; i < ST_WARPS; i++) t += red[i][tid];
       s_rs[tid] = sqrtf(__fdiv_rn(1.0f, __fadd_rn(__fmul_rn(t, a.recip_dim), a.eps)));
     }
-    __syncthreads();
+    st_sync();
 #pragma unroll
     for (int m = 0; m < MT; m++) {
       const float rs = s_rs[m];
@@ -498,7 +516,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
         }
       }
     }
-    __syncthreads();
+    st_sync();
   };
   // x <- rows of a [M][K] buffer another phase wrote
   auto stage_copy = [&](const __half* src, int K) {
@@ -506,7 +524,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
     for (int m = 0; m < MT; m++)
       for (int c = tid; c < kc; c += ST_THREADS)
         reinterpret_cast<uint4*>(xs + (size_t)m * K)[c] = (m < M) ? ld_cg_128(src + (size_t)m * K + (size_t)c * 8) : make_uint4(0, 0, 0, 0);
-    __syncthreads();
+    st_sync();
   };
 
   int tok[MT], posv[MT];
@@ -584,9 +602,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
       } else {
         stage_norm([&](int m) -> const __half* { return a.h + (size_t)m * dim; }, L->attn_norm);
       }
-      st_project<RS_D, NI_D, 1, MT>(qkv_dim, KC_D, xs, M, ring, full, rg, seq, part, a, tid, no_pre,
-                                         [&](int row, int m, float s, float, __half) { a.qkv[(size_t)m * qkv_dim + row] = __float2half_rn(s); },
-                                         refill);
+      st_project<RS_D, NI_D, 1, MT>(qkv_dim, KC_D, xs, M, ring, full, empty, rg, batch, part, a, tid, no_pre,
+                                         [&](int row, int m, float s, float, __half) { a.qkv[(size_t)m * qkv_dim + row] = __float2half_rn(s); });
       // the first K and V rows of this CTA's context slice are requested now, ahead of the barrier: cached rows do not
       // depend on this step's projection (the new position's row does and is fetched again once it has been written)
       uint4 k0[AU], v0[AU];
@@ -618,7 +635,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
         float qf[NREP][8];
 #pragma unroll
         for (int r = 0; r < NREP; r++) unpack8(rope8(ld_cg_128(xrow + (size_t)(g * NREP + r) * HD + sub * 8), traw), qf[r]);
-        __syncthreads();  // the new K / V rows are visible to this CTA's loads below
+        st_sync();  // the new K / V rows are visible to this CTA's loads below
         float lmax[NREP];
 #pragma unroll
         for (int r = 0; r < NREP; r++) lmax[r] = -INFINITY;
@@ -656,13 +673,13 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
           const float mx = warp_max(lmax[r]);
           if (lane == 0) red[warp][r] = mx;
         }
-        __syncthreads();
+        st_sync();
         if (tid < NREP) {
           float mx = red[0][tid];
           for (int w = 1; w < ST_WARPS; w++) mx = fmaxf(mx, red[w][tid]);
           s_m[tid] = mx;
         }
-        __syncthreads();
+        st_sync();
         float lsum[NREP];
 #pragma unroll
         for (int r = 0; r < NREP; r++) lsum[r] = 0.f;
@@ -676,7 +693,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
           const float v = warp_sum(lsum[r]);
           if (lane == 0) red[warp][r] = v;
         }
-        __syncthreads();
+        st_sync();
         if (tid < NREP) {
           float v = 0.f;
           for (int w = 0; w < ST_WARPS; w++) v += red[w][tid];
@@ -700,7 +717,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
           ml_s[2 * tid] = v.x;
           ml_s[2 * tid + 1] = v.y;
         }
-        __syncthreads();
+        st_sync();
         if (tid < NREP) {
           const float* ml = ml_s + (size_t)tid * S * 2;
           float Mx = -INFINITY;
@@ -711,7 +728,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
           s_M[tid] = Mx;
           s_rL[tid] = __fdiv_rn(1.0f, Ls);
         }
-        __syncthreads();
+        st_sync();
         float acc[NREP][8];
 #pragma unroll
         for (int r = 0; r < NREP; r++)
@@ -759,14 +776,14 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
 #pragma unroll
             for (int i = 0; i < 8; i++) pv_part[((size_t)(warp - ST_WARPS / 2) * NREP + r) * HD + sub * 8 + i] = acc[r][i];
         }
-        __syncthreads();
+        st_sync();
         if (rgrp == 0 && warp < ST_WARPS / 2) {
 #pragma unroll
           for (int r = 0; r < NREP; r++)
 #pragma unroll
             for (int i = 0; i < 8; i++) pv_part[((size_t)warp * NREP + r) * HD + sub * 8 + i] += acc[r][i];
         }
-        __syncthreads();
+        st_sync();
         float* po = a.att_o + ((size_t)pair * a.slices + slice) * (NREP * HD);
         for (int idx = tid; idx < NREP * HD; idx += ST_THREADS) {
           float s = 0.f;
@@ -776,7 +793,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
         }
         // the last CTA of the pair to get here folds the slices in slice order (the ticket's release covers the whole
         // CTA's stores: they are ordered before it by the barrier)
-        __syncthreads();
+        st_sync();
         if (tid == 0) {
           unsigned prev;
           asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(prev) : "l"(a.tickets + pair) : "memory");
@@ -784,7 +801,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
           if (s_last) a.tickets[pair] = 0;
           __threadfence();
         }
-        __syncthreads();
+        st_sync();
         if (s_last) {
           const float* pall = a.att_o + (size_t)pair * a.slices * (NREP * HD);
           for (int idx = tid; idx < NREP * HD; idx += ST_THREADS) {
@@ -809,8 +826,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
       stage_copy(a.attn, a.q_dim);
       {
         const uint32_t ex = peer_base + (uint32_t)step * ex_per_step + 2u * (uint32_t)l;
-        st_project<RS_D, NI_D, 1, MT>(dim, KC_Q, xs, M, ring, full, rg, seq, part, a, tid, residual,
-                                      [&](int row, int m, float s, float, __half prev) { rowpar_epi(ex, row, m, s, prev); }, refill);
+        st_project<RS_D, NI_D, 1, MT>(dim, KC_Q, xs, M, ring, full, empty, rg, batch, part, a, tid, residual,
+                                      [&](int row, int m, float s, float, __half prev) { rowpar_epi(ex, row, m, s, prev); });
         rowpar_gather(ex, RS_D);
       }
       stamp(6);
@@ -819,11 +836,10 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
 
       // ================================================================ P5: norm -> silu(W1 x) * (W3 x)
       stage_norm([&](int m) -> const __half* { return a.h + (size_t)m * dim; }, L->ffn_norm);
-      st_project<RS_G, NI_D, 2, MT>(hidden, KC_D, xs, M, ring, full, rg, seq, part, a, tid, no_pre,
+      st_project<RS_G, NI_D, 2, MT>(hidden, KC_D, xs, M, ring, full, empty, rg, batch, part, a, tid, no_pre,
                                          [&](int row, int m, float sa, float sb, __half) {
                                            a.ffn[(size_t)m * hidden + row] = jg_silu_mul(__float2half_rn(sa), __float2half_rn(sb));
-                                         },
-                                         refill);
+                                         });
       stamp(8);
       if (!st_grid_sync(a, gen)) { give_up(4); return; }
       stamp(9);
@@ -832,8 +848,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
       stage_copy(a.ffn, hidden);
       {
         const uint32_t ex = peer_base + (uint32_t)step * ex_per_step + 2u * (uint32_t)l + 1u;
-        st_project<RS_H, NI_H, 1, MT>(dim, KC_H, xs, M, ring, full, rg, seq, part, a, tid, residual,
-                                      [&](int row, int m, float s, float, __half prev) { rowpar_epi(ex, row, m, s, prev); }, refill);
+        st_project<RS_H, NI_H, 1, MT>(dim, KC_H, xs, M, ring, full, empty, rg, batch, part, a, tid, residual,
+                                      [&](int row, int m, float s, float, __half prev) { rowpar_epi(ex, row, m, s, prev); });
         rowpar_gather(ex, RS_H);
       }
       stamp(10);
@@ -845,16 +861,20 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
     stage_norm([&](int m) -> const __half* { return a.h + (size_t)m * dim; }, a.out_norm);
     {
       unsigned long long best = 0ull;
-      st_project<RS_D, NI_D, 1, MT>(a.vocab, KC_D, xs, M, ring, full, rg, seq, part, a, tid, no_pre,
+      st_project<RS_D, NI_D, 1, MT>(a.vocab, KC_D, xs, M, ring, full, empty, rg, batch, part, a, tid, no_pre,
                                          [&](int row, int m, float s, float, __half) {
                                            const __half v = __float2half_rn(s);
                                            a.logits[(size_t)m * a.vocab + row] = v;
                                            const unsigned long long k = argmax_key(v, (uint32_t)(row + a.vocab_offset));
                                            best = k > best ? k : best;
-                                         },
-                                         refill);
-      // lane 0 of warp o finished output o = r * MT + m of every pass
-      if (lane == 0 && warp < RS_D * MT && (warp % MT) < M && best != 0ull) atomicMax(a.key + (warp % MT), best);
+                                         });
+      // thread o finished outputs of activation row o % MT
+#pragma unroll
+      for (int o = 16; o >= MT; o >>= 1) {
+        const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
+        best = other > best ? other : best;
+      }
+      if (lane < MT && lane < M && best != 0ull) atomicMax(a.key + lane, best);
     }
     stamp(12);
     if (!st_grid_sync(a, gen)) { give_up(4); return; }
@@ -883,7 +903,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) jg_step_kernel(const StepArgs a
         if (!ok) atomicCAS(a.peer.err, 0, 1);
         s_key[tid] = best;
       }
-      __syncthreads();
+      st_sync();
     }
 #pragma unroll
     for (int m = 0; m < MT; m++) {
@@ -1013,17 +1033,18 @@ JG_API int jg_step_create(jg_dev* dev, jg_kvcache* kv, const jg_step_desc* desc,
     const size_t x_bytes = (size_t)mt * (d.dim > d.hidden_dim ? d.dim : d.hidden_dim) * sizeof(__half);
     const size_t head = ((att_bytes > x_bytes ? att_bytes : x_bytes) + 127) & ~(size_t)127;
     const long long room = (long long)dev->prop.sharedMemPerBlockOptin - 4096 - (long long)head;  // 4 KB: the kernel's static arrays
-    // 64 KB passes (half the barriers and epilogues per byte of 32 KB ones) where at least two of them fit: three beside
-    // one activation row, two beside two rows (8B shapes, two rows: 516 tok/s against 491 with five 32 KB passes)
-    int sb = room >= 2 * 65536 ? 65536 : 32768;
-    if (ke && atoi(ke) == 32) sb = 32768;
+    // 64 KB passes where at least two of them fit and eight rows (the most a pass has) fill them, else 32 KB (two rows, us per step with
+    // passes of 64 / 32 KB: 1B 947 / 880, 3B 1931 / 2006, 8B 3373 / 3373; one row: 1B 792 / 792, 8B 3012 / 3038)
+    int sb = room >= 2 * 65536 && 8 * d.dim * 2 > 32768 ? 65536 : 32768;
+    if (ke && (atoi(ke) == 32 || atoi(ke) == 64)) sb = atoi(ke) * 1024;
+    const int q_dim = k.n_heads * k.head_dim;  // Wo's columns: all heads on one GPU, a rank's share under tensor parallelism
+    const bool heads_ok = d.comm != 0 ? (q_dim <= d.dim && q_dim % 8 == 0) : q_dim == d.dim;
+    int vi = (heads_ok && nrep <= 4) ? find_variant(mt, k.head_dim, nrep, d.dim, d.hidden_dim, sb) : -1;
+    if (heads_ok && nrep <= 4 && vi < 0 && sb == 32768 && room >= 2 * 65536) vi = find_variant(mt, k.head_dim, nrep, d.dim, d.hidden_dim, sb = 65536);
     int ns = (int)(room / sb);
     if (ns > ST_MAX_SLOTS) ns = ST_MAX_SLOTS;
     const char* se = getenv("JG_STEP_SLOTS");
     if (se && atoi(se) >= 2 && atoi(se) < ns) ns = atoi(se);
-    const int q_dim = k.n_heads * k.head_dim;  // Wo's columns: all heads on one GPU, a rank's share under tensor parallelism
-    const bool heads_ok = d.comm != 0 ? (q_dim <= d.dim && q_dim % 8 == 0) : q_dim == d.dim;
-    const int vi = (heads_ok && nrep <= 4) ? find_variant(mt, k.head_dim, nrep, d.dim, d.hidden_dim, sb) : -1;
     if (ns < 2 || vi < 0) {
       jg_set_error("step_create: no single-kernel step for dim %d, hidden %d, head_dim %d, %d query heads per kv head (%d slots of %d bytes)",
                    d.dim, d.hidden_dim, k.head_dim, nrep, ns, sb);
@@ -1038,7 +1059,7 @@ JG_API int jg_step_create(jg_dev* dev, jg_kvcache* kv, const jg_step_desc* desc,
   for (int i = 0; i < 2; i++) {
     JG_CUDA(cudaFuncSetAttribute(g_step_variants[variant[i]].kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[i]));
     int per_sm = 0;
-    JG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, g_step_variants[variant[i]].kern, ST_THREADS, smem[i]));
+    JG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, g_step_variants[variant[i]].kern, ST_THREADS + 32, smem[i]));
     if (per_sm < 1) { jg_set_error("step_create: the step kernel does not fit an SM"); return JG_ENOTSUP; }
   }
   jg_step* s = new jg_step();
@@ -1140,7 +1161,7 @@ JG_API int jg_step_run(jg_step* s, uint64_t tokens, uint64_t pos, uint64_t h, ui
   JG_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned int), dev->stream));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(s->grid);
-  cfg.blockDim = dim3(ST_THREADS);
+  cfg.blockDim = dim3(ST_THREADS + 32);
   cfg.dynamicSmemBytes = s->smem[vi];
   cfg.stream = dev->stream;
   cudaLaunchAttribute attr[1];

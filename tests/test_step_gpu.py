@@ -83,3 +83,24 @@ def test_unsupported_shapes_keep_the_launch_per_op_path():
     greedy_with_logits(llm, prompt, 3)
     assert llm.model._single_kernel_step(1) is None
 
+
+
+@pytest.mark.parametrize("B", [1, 2])
+@pytest.mark.parametrize("size", [{"dim": 4096, "n_heads": 32, "hidden_dim": 14336}, {"dim": 3072, "n_heads": 24, "hidden_dim": 8192}])
+def test_passes_of_64_kb_equal_the_launch_per_op_path(monkeypatch, B, size):
+    """One layer of the 8B and 3B widths: passes of 8, 4 + 4 and 2 or 4 rows, shared by 16 warps by rows and K, batches of passes that do
+    not divide a CTA's; contexts that start in one slice and end in several, and one that no longer fits a CTA's shared memory whole."""
+    args = dict(SMALL, n_layers=1, n_kv_heads=8, vocab_size=9001, **size)
+    for positions, steps in ((14, 40), (830, 3)):
+        prompt = synth.prompt_tokens(positions, args["vocab_size"], batch=B, seed=80)
+        got = []
+        for kernel in ("1", "0"):
+            monkeypatch.setenv("JG_STEP_KERNEL", kernel)
+            llm = make("1B", args=args, max_context=1024, max_batch=2, tied_output=True)
+            got.append(greedy_with_logits(llm, prompt, steps))
+            assert (llm.model._single_kernel_step(B) is not None) == (kernel == "1")
+        (ids, logits), (ids2, logits2) = got
+        for b in range(B):  # up to the first step at which a near-tie was decided otherwise
+            n = steps if (ids[b] == ids2[b]).all() else int(np.argmin(ids[b] == ids2[b]))
+            assert n >= 1
+            assert np.abs(logits[:n, b] - logits2[:n, b]).max() <= 1e-2  # summation order only
