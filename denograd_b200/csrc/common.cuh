@@ -151,6 +151,14 @@ static inline int jg_launch(jg_dev* dev, const char* name, void (*kern)(KArgs...
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Parameters that a launch reads behind its dependency wait (norm weights, scales: in HBM, a step has 15 GB of weights between two uses)
+// are asked into L2 ahead of it, each line by one thread of the grid.  A hint only: what the load itself sees is in order.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ __forceinline__ void prefetch_lines(const void* p, unsigned bytes) {
+  if (p != nullptr)
+    for (unsigned i = (threadIdx.x * gridDim.x + blockIdx.x) * 128u; i < bytes; i += blockDim.x * gridDim.x * 128u) prefetch_l2((const char*)p + i);
+}
+
 // 128-bit streaming load of read-only weights: bypass L1 allocation, they are read exactly once per launch.
 __device__ __forceinline__ uint4 ld_stream_128(const void* p) {
   uint4 v;

@@ -79,6 +79,8 @@ __global__ void __launch_bounds__(MV_THREADS, 2) dense_mv_kernel(const MvArgs<T>
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(wrow(w, min(rem0 * RW + r, N - 1)) + off), "r"(512u) : "memory");
     }
   }
+  if (FROM == ROWS_STREAM) { prefetch_lines(a.st.y ? a.st.w_add : nullptr, a.st.D * 4u); prefetch_lines(a.st.plain ? nullptr : a.st.w_norm, a.st.D * 4u); }
+  if (FROM == ROWS_GATED) prefetch_lines(a.gated.w, a.gated.H * a.gated.vd * 4u);
   pdl_wait();
   if (EPI == JG_DENSE_STORE && a.out.act == JG_ACT_GELU_SIDE && tid < a.M && u0 < u1)  // this CTA's part of the tokens' rows
     prefetch_l2(dense_side_ptr<T>(a.out, a.out.tokens[tid], u0 * RW));
@@ -382,6 +384,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) stream_step_kernel(const StreamArgs a, T* __restrict__ h, int ldh) {
   extern __shared__ __align__(16) float sbuf[];
   pdl_launch();
+  prefetch_lines(a.y ? a.w_add : nullptr, a.D * 4u);
+  prefetch_lines(a.plain ? nullptr : a.w_norm, a.D * 4u);
   pdl_wait();
   const size_t r = blockIdx.x, src = a.rows ? (size_t)a.rows[r] : r;
   T* hr = h + r * ldh;
@@ -529,6 +533,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) gated_norm_kernel(const GatedArgs<T> a, T* __restrict__ out, int ldo) {
   extern __shared__ __align__(16) float sbuf[];
   pdl_launch();
+  prefetch_lines(a.w, a.H * a.vd * 4u);
   pdl_wait();
   const size_t r = blockIdx.x;
   gated_row<256>(a, r, sbuf, [&](int i, const auto& v) {

@@ -23,7 +23,6 @@ __device__ __forceinline__ float dense_side(const DenseOut& o, int row, int col)
   const float v = to_f32(*dense_side_ptr<T>(o, tok, col));
   return tok >= 0 && tok < o.vocab ? v : 0.f;
 }
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 // side: dense_side of the same row and column, which the caller may have loaded ahead
 __device__ __forceinline__ float dense_act(const DenseOut& o, int col, float v, float side) {
   if (o.act == JG_ACT_NONE || col < o.lo || col >= o.hi) return v;

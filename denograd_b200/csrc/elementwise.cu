@@ -72,14 +72,26 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(__half* __restrict__ y, co
   const int row = blockIdx.x;
   const __half* xr = x + (size_t)row * dim;
   if (early) pdl_launch();
+  prefetch_lines(w, dim * 2u);
   pdl_wait();
+  constexpr int C = 4;  // chunks of a thread that stay in registers: rows of up to 8192 values are read once, and all at once
+  uint4 xv[C], wv[C];
+#pragma unroll
+  for (int c = 0; c < C; c++) {
+    const int i = threadIdx.x + 256 * c;
+    xv[c] = i < dim / 8 ? ld_128(xr + (size_t)i * 8) : make_uint4(0, 0, 0, 0);
+    wv[c] = i < dim / 8 ? ld_128(w + (size_t)i * 8) : make_uint4(0, 0, 0, 0);
+  }
   float ss = 0.f;
-  for (int c = threadIdx.x; c < dim / 8; c += 256) {
+  auto squares = [&](const uint4& x) {
     float v[8];
-    unpack8(ld_128(xr + (size_t)c * 8), v);
+    unpack8(x, v);
 #pragma unroll
     for (int k = 0; k < 8; k++) ss = fmaf(v[k], v[k], ss);
-  }
+  };
+#pragma unroll
+  for (int c = 0; c < C; c++) squares(xv[c]);
+  for (int i = threadIdx.x + 256 * C; i < dim / 8; i += 256) squares(ld_128(xr + (size_t)i * 8));
   ss = warp_sum(ss);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
   __syncthreads();
@@ -90,16 +102,19 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(__half* __restrict__ y, co
   }
   __syncthreads();
   const float rs = s_rs;
-  for (int c = threadIdx.x; c < dim / 8; c += 256) {
+  auto finish = [&](int i, const uint4& x, const uint4& g) {
     float v[8];
-    unpack8(ld_128(xr + (size_t)c * 8), v);
-    uint4 wv = ld_128(w + (size_t)c * 8);
-    const __half* wh = reinterpret_cast<const __half*>(&wv);
+    unpack8(x, v);
+    const __half* wh = reinterpret_cast<const __half*>(&g);
     __align__(16) __half o[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) o[k] = hmul1(__float2half_rn(__fmul_rn(v[k], rs)), wh[k]);
-    reinterpret_cast<uint4*>(y + (size_t)row * dim)[c] = *reinterpret_cast<uint4*>(o);
-  }
+    reinterpret_cast<uint4*>(y + (size_t)row * dim)[i] = *reinterpret_cast<uint4*>(o);
+  };
+#pragma unroll
+  for (int c = 0; c < C; c++)
+    if (threadIdx.x + 256 * c < dim / 8) finish(threadIdx.x + 256 * c, xv[c], wv[c]);
+  for (int i = threadIdx.x + 256 * C; i < dim / 8; i += 256) finish(i, ld_128(xr + (size_t)i * 8), ld_128(w + (size_t)i * 8));
 }
 
 JG_API int jg_rmsnorm(jg_dev* dev, uint64_t y, uint64_t x, uint64_t w, int32_t rows, int32_t dim, float eps) {

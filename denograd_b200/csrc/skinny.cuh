@@ -88,6 +88,11 @@ __device__ __forceinline__ void sk_dequant16(const uint4& raw, __half2 s2, uint3
   }
 }
 
+// What this CTA alone will read, asked into L2.
+__device__ __forceinline__ void prefetch_run(const void* p, int bytes) {
+  for (int i = threadIdx.x * 128; i < bytes + 127; i += SK_WARPS * 32 * 128) prefetch_l2((const char*)p + min(i, bytes - 1));
+}
+
 // E: what happens to a finished sum.  E::Pre is what it needs from global memory.
 template <int TYPE, int NT, int TP, bool GLU, class E>
 __global__ void __launch_bounds__(SK_THREADS, 1)
@@ -158,6 +163,10 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
     }
   }
   const uint32_t lut_lane = lut + lane * 4;
+  if (TYPE == SK_W8 && !a.w_late) {  // the run's scales
+    prefetch_run(a.s0 + n0, cnt * 2);
+    if (GLU) prefetch_run(a.s1 + n0, cnt * 2);
+  }
   __syncthreads();
   pdl_wait();
   // This warp's run of a stage and its row tile, and where their fragments lie: rows g and g + 8 of the tile (of a gated pair row g of

@@ -557,6 +557,9 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
   for (int step = 0; step < a.n_steps; step++) {
     for (int l = 0; l < a.n_layers; l++) {
       const StepLayer* L = a.layers + l;
+      // the next norms' weights come into L2 in time, a line from each CTA (they are read once a step, from HBM otherwise)
+      if (tid < 2 && bid * 64 < dim)
+        prefetch_l2((tid == 0 ? L->ffn_norm : l + 1 < a.n_layers ? L[1].attn_norm : a.out_norm) + bid * 64);
       // this CTA's share of attention: context slice `slice` of (row b, kv head g); the pages of its first rows are looked
       // up now, so that the rows themselves can be requested without a dependent load when the projection is over
       const int n_pairs = M * a.G;

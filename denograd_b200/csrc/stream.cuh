@@ -104,6 +104,60 @@ __device__ __forceinline__ void stream_row_v(const StreamArgs& a, size_t src, fl
     for (int p = 0; p < P; p++) t += s[g * P + p];
     return 1.0f / sqrtf(t / (float)gs + a.eps);
   };
+  // A unit or less to a warp, no more than C chunks of it to a lane: the row stays in registers, and everything is asked for at once (one
+  // trip to L2 instead of three; stream_step_kernel, 8 rows of 2048: 3.9 -> 2.7 us between launches).
+  constexpr int C = 4;
+  if (V == 4 && units <= W && plen <= 32 * V * C) {
+    const bool on = warp < units;
+    const int g = warp / P, lo = on ? g * gs + (warp % P) * plen : 0, hi = on ? min((g + 1) * gs, lo + plen) : 0;
+    float x[C][V], y[C][V], wa[C][V], wn[C][V];
+    const bool norm = a.w_norm != nullptr && !a.plain;
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      const int i = lo + (lane + 32 * c) * V;
+#pragma unroll
+      for (int k = 0; k < V; k++) x[c][k] = y[c][k] = wa[c][k] = wn[c][k] = 0.f;
+      if (i < hi) {
+        load(xr + i, x[c]);
+        if (yr) { load(yr + i, y[c]); load(a.w_add + i, wa[c]); }
+        if (norm) load(a.w_norm + i, wn[c]);
+      }
+    }
+    auto squares = [&](const float (&v)[C][V], float* to) {
+      float ss = 0.f;
+#pragma unroll
+      for (int c = 0; c < C; c++)
+#pragma unroll
+        for (int k = 0; k < V; k++) ss = fmaf(v[c][k], v[c][k], ss);
+      ss = warp_sum(ss);
+      if (on && lane == 0) to[warp] = ss;
+      __syncthreads();
+    };
+    if (yr) {
+      squares(y, red);
+      const float r = on ? rstd(red, g) : 0.f;
+#pragma unroll
+      for (int c = 0; c < C; c++) {
+        const int i = lo + (lane + 32 * c) * V;
+#pragma unroll
+        for (int k = 0; k < V; k++) x[c][k] = fmaf(y[c][k] * r, wa[c][k], x[c][k]);
+        if (x_out_row && i < hi) put(x_out_row + i, x[c]);
+      }
+    }
+    if (!a.plain && a.w_norm == nullptr) return;
+    if (norm) {
+      squares(x, red2);
+      const float r = on ? rstd(red2, g) : 0.f;
+#pragma unroll
+      for (int c = 0; c < C; c++)
+#pragma unroll
+        for (int k = 0; k < V; k++) x[c][k] = x[c][k] * r * wn[c][k];
+    }
+#pragma unroll
+    for (int c = 0; c < C; c++)
+      if (lo + (lane + 32 * c) * V < hi) store(lo + (lane + 32 * c) * V, x[c]);
+    return;
+  }
   for (int u = warp; u < units; u += W) {  // a thread meets the same elements again below: buf needs no barrier
     const int g = u / P, lo = g * gs + (u % P) * plen, hi = min((g + 1) * gs, lo + plen);
     float ss = 0.f;
@@ -188,26 +242,40 @@ __device__ __forceinline__ void gated_row_v(const GatedArgs<T>& a, size_t r, flo
   const float *o = a.o + r * n, *den = a.den ? a.den + r * a.H : nullptr;
   const T* gate = a.gate + r * a.ldp;
   float *fac = buf + n4, *red = fac + n4;
-#pragma unroll 4
-  for (int i = threadIdx.x * V; i < n; i += NT * V) {
-    const float d = den ? den[i / a.vd] : 1.f;
+  constexpr int C = 4;  // chunks of a thread that are on their way together
+  for (int i0 = threadIdx.x * V; i0 < n; i0 += C * NT * V) {
     if constexpr (V == 4) {
-      float4 x = *reinterpret_cast<const float4*>(o + i), w = *reinterpret_cast<const float4*>(a.w + i);
-      float g[4];
-      if constexpr (sizeof(T) == 2) {
-        const uint2 t = *reinterpret_cast<const uint2*>(gate + i);
-        g[0] = __uint_as_float(t.x << 16); g[1] = __uint_as_float(t.x & 0xFFFF0000u); g[2] = __uint_as_float(t.y << 16); g[3] = __uint_as_float(t.y & 0xFFFF0000u);
-      } else {
-        const float4 t = *reinterpret_cast<const float4*>(gate + i);
-        g[0] = t.x; g[1] = t.y; g[2] = t.z; g[3] = t.w;
+      float4 x[C], w[C], gt[C];
+      float d[C];
+#pragma unroll
+      for (int c = 0; c < C; c++) {
+        const int i = i0 + c * NT * V;
+        if (i >= n) continue;
+        x[c] = *reinterpret_cast<const float4*>(o + i);
+        w[c] = *reinterpret_cast<const float4*>(a.w + i);
+        d[c] = den ? den[i / a.vd] : 1.f;
+        if constexpr (sizeof(T) == 2) {
+          const uint2 t = *reinterpret_cast<const uint2*>(gate + i);
+          gt[c] = make_float4(__uint_as_float(t.x << 16), __uint_as_float(t.x & 0xFFFF0000u), __uint_as_float(t.y << 16), __uint_as_float(t.y & 0xFFFF0000u));
+        } else {
+          gt[c] = *reinterpret_cast<const float4*>(gate + i);
+        }
       }
-      if (den) { x.x /= d; x.y /= d; x.z /= d; x.w /= d; }
-      w.x *= sigmoid_f32(g[0]); w.y *= sigmoid_f32(g[1]); w.z *= sigmoid_f32(g[2]); w.w *= sigmoid_f32(g[3]);
-      *reinterpret_cast<float4*>(buf + i) = x;
-      *reinterpret_cast<float4*>(fac + i) = w;
+#pragma unroll
+      for (int c = 0; c < C; c++) {
+        const int i = i0 + c * NT * V;
+        if (i >= n) continue;
+        if (den) { x[c].x /= d[c]; x[c].y /= d[c]; x[c].z /= d[c]; x[c].w /= d[c]; }
+        w[c].x *= sigmoid_f32(gt[c].x); w[c].y *= sigmoid_f32(gt[c].y); w[c].z *= sigmoid_f32(gt[c].z); w[c].w *= sigmoid_f32(gt[c].w);
+        *reinterpret_cast<float4*>(buf + i) = x[c];
+        *reinterpret_cast<float4*>(fac + i) = w[c];
+      }
     } else {
-      buf[i] = den ? o[i] / d : o[i];
-      fac[i] = a.w[i] * sigmoid_f32(to_f32(gate[i]));
+      for (int i = i0; i < min(n, i0 + C * NT * V); i += NT * V) {
+        const float d = den ? den[i / a.vd] : 1.f;
+        buf[i] = den ? o[i] / d : o[i];
+        fac[i] = a.w[i] * sigmoid_f32(to_f32(gate[i]));
+      }
     }
   }
   __syncthreads();
