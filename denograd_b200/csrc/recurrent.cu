@@ -122,6 +122,7 @@ struct DeltaArgs {
   T* out;
   const int32_t *pos, *seq;
   int B, Sc, H, G, dim, vd, taps, ldp, ldo, lds;  // lds: dim rounded up to 4
+  int conv_vec;  // the taps of a channel (four) lie on 16 bytes
   float eps;
   __device__ __forceinline__ int channels() const { return 2 * G * dim + H * vd; }
   // column of the projection that holds b / a of head h, and the output gate
@@ -145,12 +146,14 @@ __device__ __forceinline__ float delta_conv_silu(const DeltaArgs<T>& a, int b, i
   }
   return silu_f32(acc);
 }
+// decay and beta of a token and head
+__device__ __forceinline__ float2 delta_gates(float beta_in, float decay_in, float dt_bias, float a_log) {
+  return make_float2(expf(-expf(a_log) * softplus_f32(decay_in + dt_bias)), sigmoid_f32(beta_in));
+}
 template <typename T>
 __device__ __forceinline__ float2 delta_gates(const DeltaArgs<T>& a, size_t row, int h) {
   const T* p = a.proj + row * a.ldp;
-  const float beta = sigmoid_f32(to_f32(p[a.col_b() + h]));
-  const float dt = softplus_f32(to_f32(p[a.col_a() + h]) + a.dt_bias[h]);
-  return make_float2(expf(-expf(a.a_log[h]) * dt), beta);
+  return delta_gates(to_f32(p[a.col_b() + h]), to_f32(p[a.col_a() + h]), a.dt_bias[h], a.a_log[h]);
 }
 constexpr float DELTA_UNIT_EPS = 1e-6f;
 
@@ -520,7 +523,11 @@ __global__ void __launch_bounds__(256) delta_out_kernel(const DeltaArgs<T> a, in
 // S; the sum of squares of the output norm crosses through distributed shared memory.
 constexpr int DD_THREADS = 256, DD_COLS = DD_THREADS / DL_LPC, DD_MAX_CLUSTER = 8;
 
-template <typename T, int E>
+//
+// Bound by its chain of loads (12 us for 1 MB of state at 1B sizes when every tap of every channel was a trip of its own), so whatever
+// does not hang on something computed is asked for first: gates, output gate and norm, then the inputs and taps (TAPS = 4; 0: any
+// number, one after the other) of two channels per thread at a time.
+template <typename T, int E, int TAPS>
 __global__ void __launch_bounds__(DD_THREADS) delta_step_kernel(const DeltaArgs<T> a) {
   constexpr int DP = E * DL_LPC;
   extern __shared__ __align__(16) float dyn[];  // this CTA's columns: v, then o
@@ -542,23 +549,68 @@ __global__ void __launch_bounds__(DD_THREADS) delta_step_kernel(const DeltaArgs<
   DeltaCol<DL_LPC, E> S;
   float* st0 = a.state + ((size_t)slot * a.H + h) * a.vd * a.lds;
   S.load(st0 + (size_t)min(j0 + col, a.vd - 1) * a.lds, l, a.lds, p0 > 0);
-  float qv = 0.f, kv = 0.f, pq = 0.f, pk = 0.f, pqk = 0.f;
-  for (int i = tid; i < DP; i += DD_THREADS) {
-    if (i < a.dim) {
-      const int cq = g * a.dim + i, ck = (a.G + g) * a.dim + i;
-      qv = delta_conv_silu(a, r, 0, cq, p0, tail);
-      kv = delta_conv_silu(a, r, 0, ck, p0, tail);
-      pq = fmaf(qv, qv, pq); pk = fmaf(kv, kv, pk); pqk = fmaf(qv, kv, pqk);
-      sq[i] = qv; sk[i] = kv;
-      if (cr == 0 && h % (a.H / a.G) == 0) { tail_now[cq] = row[cq]; tail_now[ck] = row[ck]; }
-    } else {
-      sq[i] = 0.f; sk[i] = 0.f;
+  const T beta_in = row[a.col_b() + h], decay_in = row[a.col_a() + h];
+  const float dt_bias = a.dt_bias[h], a_log = a.a_log[h];
+  const T* gate = row + a.col_g() + h * a.vd;
+  const bool first = j0 + tid < j1;  // this thread's first column of the result
+  const T gate_in = first ? gate[j0 + tid] : from_f32<T>(0.f);
+  const float norm_in = first ? a.norm_w[j0 + tid] : 0.f;
+  float pq = 0.f, pk = 0.f, pqk = 0.f;
+  if (TAPS == 4) {
+    const int total = 2 * a.dim + j1 - j0;  // channels: the query head's, the key head's, this CTA's columns of the values
+    const bool writes = cr == 0 && h % (a.H / a.G) == 0;
+    for (int i0 = tid; i0 < total; i0 += 2 * DD_THREADS) {
+      float4 w[2];
+      float x[2][4];
+      int ch[2];
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const int i = i0 + u * DD_THREADS;
+        ch[u] = i < a.dim ? g * a.dim + i : i < 2 * a.dim ? a.G * a.dim + g * a.dim + i - a.dim : 2 * a.G * a.dim + h * a.vd + j0 + i - 2 * a.dim;
+        if (i >= total) continue;
+        const float* wp = a.conv_w + (size_t)ch[u] * 4;
+        if (a.conv_vec) w[u] = *reinterpret_cast<const float4*>(wp);
+        else w[u] = make_float4(wp[0], wp[1], wp[2], wp[3]);
+        x[u][3] = to_f32(row[ch[u]]);
+#pragma unroll
+        for (int j = 0; j < 3; j++) x[u][j] = p0 + j >= 3 ? to_f32(tail[(size_t)((p0 + j - 3) & 3) * C + ch[u]]) : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const int i = i0 + u * DD_THREADS;
+        if (i >= total) continue;
+        const float v = silu_f32(fmaf(w[u].w, x[u][3], fmaf(w[u].z, x[u][2], fmaf(w[u].y, x[u][1], fmaf(w[u].x, x[u][0], 0.f)))));
+        if (i < a.dim) sq[i] = v;
+        else if (i < 2 * a.dim) sk[i - a.dim] = v;
+        else dyn[i - 2 * a.dim] = v;
+        if (writes || i >= 2 * a.dim) tail_now[ch[u]] = row[ch[u]];
+      }
     }
-  }
-  for (int j = j0 + tid; j < j1; j += DD_THREADS) {
-    const int c = 2 * a.G * a.dim + h * a.vd + j;
-    dyn[j - j0] = delta_conv_silu(a, r, 0, c, p0, tail);
-    tail_now[c] = row[c];
+    for (int i = a.dim + tid; i < DP; i += DD_THREADS) { sq[i] = 0.f; sk[i] = 0.f; }
+    __syncthreads();
+    for (int i = tid; i < DP; i += DD_THREADS) {
+      const float qv = sq[i], kv = sk[i];
+      pq = fmaf(qv, qv, pq); pk = fmaf(kv, kv, pk); pqk = fmaf(qv, kv, pqk);
+    }
+  } else {
+    float qv = 0.f, kv = 0.f;
+    for (int i = tid; i < DP; i += DD_THREADS) {
+      if (i < a.dim) {
+        const int cq = g * a.dim + i, ck = (a.G + g) * a.dim + i;
+        qv = delta_conv_silu(a, r, 0, cq, p0, tail);
+        kv = delta_conv_silu(a, r, 0, ck, p0, tail);
+        pq = fmaf(qv, qv, pq); pk = fmaf(kv, kv, pk); pqk = fmaf(qv, kv, pqk);
+        sq[i] = qv; sk[i] = kv;
+        if (cr == 0 && h % (a.H / a.G) == 0) { tail_now[cq] = row[cq]; tail_now[ck] = row[ck]; }
+      } else {
+        sq[i] = 0.f; sk[i] = 0.f;
+      }
+    }
+    for (int j = j0 + tid; j < j1; j += DD_THREADS) {
+      const int c = 2 * a.G * a.dim + h * a.vd + j;
+      dyn[j - j0] = delta_conv_silu(a, r, 0, c, p0, tail);
+      tail_now[c] = row[c];
+    }
   }
   pq = warp_sum(pq); pk = warp_sum(pk); pqk = warp_sum(pqk);
   if (lane == 0) { red[0][warp] = pq; red[1][warp] = pk; red[2][warp] = pqk; }
@@ -567,7 +619,7 @@ __global__ void __launch_bounds__(DD_THREADS) delta_step_kernel(const DeltaArgs<
 #pragma unroll
   for (int w = 0; w < DD_THREADS / 32; w++) { tq += red[0][w]; tk += red[1][w]; tqk += red[2][w]; }
   const float rq = 1.0f / sqrtf(tq + DELTA_UNIT_EPS) * (1.0f / sqrtf((float)a.dim)), rk = 1.0f / sqrtf(tk + DELTA_UNIT_EPS);
-  const float2 gt = delta_gates(a, r, h);
+  const float2 gt = delta_gates(to_f32(beta_in), to_f32(decay_in), dt_bias, a_log);
   float4 k4[E / 4], q4[E / 4];
 #pragma unroll
   for (int i = 0; i < E / 4; i++) {
@@ -605,8 +657,8 @@ __global__ void __launch_bounds__(DD_THREADS) delta_step_kernel(const DeltaArgs<
   float tot = 0.f;
   for (int c = 0; c < cs; c++) tot += s_ss[c];
   const float rs = 1.0f / sqrtf(tot / (float)a.vd + a.eps);
-  const T* gate = row + a.col_g() + h * a.vd;
-  for (int j = j0 + tid; j < j1; j += DD_THREADS)
+  if (first) a.out[(size_t)r * a.ldo + h * a.vd + j0 + tid] = from_f32<T>(dyn[tid] * rs * norm_in * silu_f32(to_f32(gate_in)));
+  for (int j = j0 + tid + DD_THREADS; j < j1; j += DD_THREADS)
     a.out[(size_t)r * a.ldo + h * a.vd + j] = from_f32<T>(dyn[j - j0] * rs * a.norm_w[j] * silu_f32(to_f32(gate[j])));
 }
 
@@ -624,7 +676,7 @@ static int delta_launch(jg_dev* dev, const DeltaArgs<T>& a) {
     int cs = 1;
     while (cs < DD_MAX_CLUSTER && cs * DD_COLS < a.vd && R * a.H * cs < 2 * dev->sm_count) cs *= 2;
     const size_t smem = (size_t)((a.vd + cs - 1) / cs) * sizeof(float);
-    return jg_launch_cluster(dev, "delta_step", delta_step_kernel<T, DP / DL_LPC>, dim3((unsigned)cs, (unsigned)a.H, (unsigned)R), dim3(DD_THREADS), smem, cs, a);
+    return jg_launch_cluster(dev, "delta_step", a.taps == 4 ? delta_step_kernel<T, DP / DL_LPC, 4> : delta_step_kernel<T, DP / DL_LPC, 0>, dim3((unsigned)cs, (unsigned)a.H, (unsigned)R), dim3(DD_THREADS), smem, cs, a);
   }
   constexpr int E = DP / DS_LPC, NI = DP <= 128 ? 4 : 8;
   const dim3 pg((unsigned)((2 * a.G + (a.H * a.vd + NI * 32 - 1) / (NI * 32) + 1 + 7) / 8), (unsigned)((a.Sc + DP_TOK - 1) / DP_TOK), (unsigned)a.B);
@@ -648,7 +700,7 @@ static int delta_run(jg_dev* dev, const jg_batch* b, const jg_delta_desc* d) {
   a.norm_w = (const float*)d->norm_w; a.state = (float*)d->state; a.tail = (T*)d->tail; a.out = (T*)d->out;
   a.pos = (const int32_t*)b->pos; a.seq = (const int32_t*)b->seq;
   a.B = b->B; a.Sc = b->Sc; a.H = d->heads; a.G = d->kv_heads; a.dim = d->dim; a.vd = d->vdim; a.taps = d->taps;
-  a.ldp = d->ldp; a.ldo = d->ldo; a.lds = (d->dim + 3) & ~3; a.eps = d->eps;
+  a.ldp = d->ldp; a.ldo = d->ldo; a.lds = (d->dim + 3) & ~3; a.eps = d->eps; a.conv_vec = d->taps == 4 && d->conv_w % 16 == 0;
   const size_t R = (size_t)b->B * b->Sc;
   a.qk = (float*)d->scratch;  // 16-byte rows first, 8-byte pairs next
   a.gates = a.qk + R * d->kv_heads * 2 * a.lds;
