@@ -1,4 +1,4 @@
-// bf16 projection on the 5th-generation tensor cores for 3 rows and more: y = epilogue(x W^T + b), any N and K.
+// bf16 projection on the 5th-generation tensor cores for 3 rows and more (fewer, and up to 8 mostly: skinny.cuh): y = epilogue(x W^T + b), any N and K.
 //
 // The scheme of gemm_tc.cu on bf16 operands: A = 128 weight rows x 64 k, B = TN activation rows x 64 k, both K-major and
 // brought into 128-byte swizzled shared memory by TMA, D = 128 x TN fp32 in tensor memory; warp 0 issues the loads, warp 1
