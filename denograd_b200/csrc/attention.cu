@@ -266,48 +266,47 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_pv_kernel(const AttnArgs a) 
 // ------------------------------------------------------------------------------------------------ RoPE + cache write
 // apply_rotary_emb / complex_mult (jsgrad/models/llama.ts:17-32) on the interleaved pairs of Q and K, every op in
 // fp16; K and V of the new token go to their page (cache assign, jsgrad/models/llama.ts:87).
-// One thread handles 8 consecutive halves (4 pairs) of one head.
-__global__ void rope_kvwrite_kernel(__half* __restrict__ qkv, const __half* __restrict__ table,
+// A CTA per row: position, page and sequence are looked up once, and a thread's pieces of 8 halves (4 pairs) of the row's heads are on
+// their way together.  (A thread per piece, which divided its way to row and head in 64 bits: 64 us for 3800 rows of the 8B's 6144
+// values, 9.6 us for 512; now 20 and 4.)
+constexpr int RK_THREADS = 256;
+__global__ void __launch_bounds__(RK_THREADS) rope_kvwrite_kernel(__half* __restrict__ qkv, const __half* __restrict__ table,
                                     const int32_t* __restrict__ pos, const int32_t* __restrict__ block_table,
-                                    __half* __restrict__ k_layer, __half* __restrict__ v_layer, int B, int H, int G,
+                                    __half* __restrict__ k_layer, __half* __restrict__ v_layer, int H, int G,
                                     int hd, int page, int page_shift, int max_pages_per_seq, int table_rows,
                                     const int32_t* __restrict__ seq, int n_seq) {
+  constexpr int U = 4;
   pdl_launch();
   pdl_wait();
-  const int per_head = hd / 8;
-  const int heads = H + 2 * G;
-  const long long total = (long long)B * heads * per_head;
-  for (long long it = blockIdx.x * (long long)blockDim.x + threadIdx.x; it < total; it += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(it % per_head);
-    const int h = (int)((it / per_head) % heads);
-    const int b = (int)(it / ((long long)per_head * heads));
-    const int p = pos[b];
-    if (p < 0 || p >= max_pages_per_seq * page || p >= table_rows) continue;  // out-of-range position: leave the row untouched
-    const int sq = seq ? seq[b] : b;
-    if ((unsigned)sq >= (unsigned)n_seq) continue;  // row mapped to a sequence the block table does not have: skipped too
-    __half* src = qkv + ((size_t)b * heads + h) * hd + (size_t)c * 8;
-    uint4 raw = *reinterpret_cast<uint4*>(src);
-    if (h < H + G) {
-      uint4 traw = ld_128(table + ((size_t)p * (hd / 2) + (size_t)c * 4) * 2);
-      const __half* x = reinterpret_cast<const __half*>(&raw);
-      const __half* t = reinterpret_cast<const __half*>(&traw);
-      __align__(16) __half o[8];
+  const int b = blockIdx.x, shift = hd == 128 ? 4 : 3, heads = H + 2 * G, total = heads << shift;  // hd: 64 or 128
+  const int p = pos[b], sq = seq ? seq[b] : b;
+  if (p < 0 || p >= max_pages_per_seq * page || p >= table_rows) return;  // out-of-range position: leave the row untouched
+  if ((unsigned)sq >= (unsigned)n_seq) return;  // row mapped to a sequence the block table does not have: skipped too
+  const int pg = block_table[(size_t)sq * max_pages_per_seq + (p >> page_shift)], slot = p & (page - 1);
+  __half* row = qkv + (size_t)b * heads * hd;
+  const __half* trow = table + (size_t)p * hd;
+  for (int i0 = threadIdx.x; i0 < total; i0 += U * RK_THREADS) {
+    uint4 raw[U], traw[U];
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const __half xa = x[2 * i], xb = x[2 * i + 1], co = t[2 * i], si = t[2 * i + 1];
-        o[2 * i] = hsub1(hmul1(xa, co), hmul1(xb, si));
-        o[2 * i + 1] = hadd1(hmul1(xa, si), hmul1(xb, co));
+    for (int u = 0; u < U; u++) {
+      const int i = i0 + u * RK_THREADS, h = i >> shift, c = i & ((1 << shift) - 1);
+      raw[u] = traw[u] = make_uint4(0, 0, 0, 0);
+      if (i < total) {
+        raw[u] = ld_128(row + (size_t)i * 8);
+        if (h < H + G) traw[u] = ld_128(trow + c * 8);
       }
-      raw = *reinterpret_cast<uint4*>(o);
     }
-    if (h < H) {
-      *reinterpret_cast<uint4*>(src) = raw;
-    } else {
-      const int g = (h < H + G) ? (h - H) : (h - H - G);
-      __half* layer = (h < H + G) ? k_layer : v_layer;
-      const int pg = block_table[(size_t)sq * max_pages_per_seq + (p >> page_shift)];
-      const int slot = p & (page - 1);
-      *reinterpret_cast<uint4*>(layer + (((size_t)pg * G + g) * page + slot) * hd + (size_t)c * 8) = raw;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int i = i0 + u * RK_THREADS, h = i >> shift, c = i & ((1 << shift) - 1);
+      if (i >= total) continue;
+      if (h < H + G) raw[u] = rope8(raw[u], traw[u]);
+      if (h < H) {
+        *reinterpret_cast<uint4*>(row + (size_t)i * 8) = raw[u];
+      } else {
+        const int g = h < H + G ? h - H : h - H - G;
+        *reinterpret_cast<uint4*>((h < H + G ? k_layer : v_layer) + (((size_t)pg * G + g) * page + slot) * hd + (size_t)c * 8) = raw[u];
+      }
     }
   }
 }
@@ -666,12 +665,9 @@ static int rope_kvwrite_impl(jg_dev* dev, jg_kvcache* kv, int32_t layer, uint64_
   JG_REQUIRE(B > 0 && (seq != 0 || B <= kv->d.max_batch) && B <= 65535 && H == kv->d.n_heads, "rope_kvwrite: B=%d H=%d do not match the cache (max_batch %d, n_heads %d)", B, H, kv->d.max_batch, kv->d.n_heads);
   JG_REQUIRE(jg_aligned(qkv, 16) && jg_aligned(table, 16) && jg_aligned(pos, 4), "rope_kvwrite: null or misaligned pointer");
   const int G = kv->d.n_kv_heads, hd = kv->d.head_dim;
-  const long long total = (long long)B * (H + 2 * G) * (hd / 8);
-  int blocks = (int)((total + 127) / 128);
-  if (blocks > dev->sm_count * 8) blocks = dev->sm_count * 8;
-  return jg_launch(dev, "rope_kvwrite", rope_kvwrite_kernel, dim3(blocks), dim3(128), 0, (__half*)qkv, (const __half*)table,
+  return jg_launch(dev, "rope_kvwrite", rope_kvwrite_kernel, dim3((unsigned)B), dim3(RK_THREADS), 0, (__half*)qkv, (const __half*)table,
                    (const int32_t*)pos, (const int32_t*)kv->block_table, kv->k_pool + kv->layer_elems * layer,
-                   kv->v_pool + kv->layer_elems * layer, B, H, G, hd, kv->d.page_size, ilog2(kv->d.page_size),
+                   kv->v_pool + kv->layer_elems * layer, H, G, hd, kv->d.page_size, ilog2(kv->d.page_size),
                    kv->d.max_pages_per_seq, table_rows, (const int32_t*)seq, kv->d.max_batch);
 }
 
