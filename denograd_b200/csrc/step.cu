@@ -12,13 +12,15 @@
 //               P2 RoPE(q, k), cache write, scores of this CTA's context slice, slice max / sum -> scratch      | barrier
 //               P3 global max / sum, p = half(softmax), p.v partial -> scratch; the last CTA of a (row, kv head)
 //                  folds the slices in order into attn                                  | barrier
+//                  (a cache of up to about 2000 positions: P2's scores themselves -> scratch, a counter per (row, kv head), then
+//                  softmax and p.v of 16 of the head's dimensions per CTA                | barrier)
 //               P4 h += Wo attn                                                         | barrier
 //               P5 x = RMSNorm(h) * g;  ffn = silu(W1 x) * (W3 x)                       | barrier
 //               P6 h += W2 ffn                                                          | barrier
 //   per step    x = RMSNorm(h) * g;  logits = Wout x, (value, lowest index) max key     | barrier, pick, feed back
 //
 // The point of the arrangement is that the weight stream never stops at a phase boundary: weights do not depend on activations, so
-// one warp of every CTA walks the step's matrices in order and keeps 128 to 192 KB of passes in flight as bulk copies into a ring in
+// one warp of every CTA walks the step's matrices in order and keeps 128 to 176 KB of passes in flight as bulk copies into a ring in
 // shared memory, while the others stage activations, wait at a barrier or work on attention.
 //
 // A projection phase: passes of a few whole rows are dealt to the CTAs in turn; the 16 computing warps share a pass by rows and by K,
@@ -40,6 +42,7 @@
 
 constexpr int ST_THREADS = 512;  // that compute; one more warp requests the weights
 constexpr int ST_WARPS = ST_THREADS / 32;
+constexpr int ST_SHORT_MAX = 2048;  // four positions to a thread
 constexpr int ST_PART = 384;  // partial sums of a batch of passes
 
 struct StepLayer {
@@ -72,6 +75,8 @@ struct StepArgs {
   unsigned long long* key;  // [2] (value, lowest index) max keys of the step's rows (scratch of the plan)
   float* att_ml;          // [M * G][NREP][slices][2]
   float* att_o;           // [M * G][slices][NREP * hd]
+  float* att_s;           // [M * G][NREP][ST_SHORT_MAX] scores of short contexts
+  unsigned int* att_n;    // [M * G] slices whose scores are there, since the launch began
   unsigned int* tickets;  // [M * G]
   unsigned int* bar;      // [0] arrivals of the barrier in progress, [32] generation
   int* err;
@@ -132,14 +137,18 @@ __device__ __forceinline__ void st_sync() { asm volatile("bar.sync 1, %0;" ::"n"
 // Grid-wide barrier: every CTA adds one to a counter the host zeroed before the launch and waits until the counter
 // reaches the barrier's ordinal times the grid size.  All CTAs are resident (cooperative launch).  Returns false when
 // the wait ran out; the caller leaves the kernel.
-__device__ __forceinline__ bool st_grid_sync(const StepArgs& a, unsigned& nbar) {
+template <class Meanwhile>
+__device__ __forceinline__ bool st_grid_sync(const StepArgs& a, unsigned& nbar, Meanwhile meanwhile) {
   __shared__ int s_ok;
   st_sync();
+  const unsigned target = (nbar + 1) * gridDim.x;
+  if (threadIdx.x == 0) {
+    nbar++;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+  }
+  meanwhile();  // by all threads, between arrival and wait
   if (threadIdx.x == 0) {
     int ok = 1;
-    nbar++;
-    const unsigned target = nbar * gridDim.x;
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
     // (several polls in flight per CTA were measured: two change nothing, four slow the counter's line down: 1.44 -> 2.26 us)
     unsigned long long t0 = 0;
     for (unsigned polls = 1;; polls++) {
@@ -159,6 +168,8 @@ __device__ __forceinline__ bool st_grid_sync(const StepArgs& a, unsigned& nbar) 
   st_sync();
   return s_ok != 0;
 }
+
+__device__ __forceinline__ bool st_grid_sync(const StepArgs& a, unsigned& nbar) { return st_grid_sync(a, nbar, [] {}); }
 
 // ---- the weight stream.  The CTA's last warp walks the step's projections in order (qkv, wo, gate/up, down of every
 // layer, then the output matrix, then the next step) and keeps `nslot` passes in flight as bulk copies into a ring of
@@ -331,7 +342,7 @@ __device__ __forceinline__ void st_project(int N, int KC, const __half* xs, int 
 
 // RS_D / RS_G / RS_H: rows per pass of a projection with K = dim (one matrix), of the gate / up pair (rows of each), with
 // K = hidden; NI_D / NI_H: 16-byte chunks per thread and row (K / 8 chunks over 512 threads).
-template <int MT, int HD, int NREP, int RS_D, int RS_G, int RS_H, int NI_D, int NI_H>
+template <int MT, int HD, int NREP, int RS_D, int RS_G, int RS_H, int NI_D, int NI_H, bool BRIEF>
 __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepArgs a) {
   static_assert(NREP <= 4 && MT <= 2, "register budget of 128 per thread");
   constexpr int LPR = HD / 8;    // lanes per K / V row
@@ -370,6 +381,7 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
   const float log2e = 1.4426950408889634f;
 
   unsigned gen = 0;  // grid barriers passed
+  unsigned scored = 0;  // slices of this CTA's pair whose scores are to be there, since the launch began
   unsigned batch = 0;  // batches of weight passes finished
 
   // the weight stream starts before anything else: nslot passes are on their way while the first rows are staged
@@ -581,6 +593,12 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
       const int32_t* bt_row = a.block_table + (size_t)b * a.max_pages_per_seq;
       __half* k_layer = a.k_pool + (size_t)l * a.layer_elems;
       __half* v_layer = a.v_pool + (size_t)l * a.layer_elems;
+      constexpr int DS = HD / 16;  // BRIEF: CTAs of a pair that share the head's dimensions
+      constexpr bool brief = BRIEF;
+      const bool dims = brief && mine && slice < DS;
+      const int T16 = (T + 15) & ~15;
+      __half* vs = reinterpret_cast<__half*>(st_smem);  // [T16][16], behind it the probabilities [NREP][T16 + 8]
+      __half* ps = vs + (size_t)T16 * 16;
       int pg0[AU];
 #pragma unroll
       for (int u = 0; u < AU; u++) {
@@ -616,10 +634,21 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
         const bool ld = att && t < t1 && t != pnew;
         const size_t off = (((size_t)pg0[u] * a.G + g) * a.page + (t & (a.page - 1))) * HD + sub * 8;
         k0[u] = ld ? ld_cg_128(k_layer + off) : make_uint4(0, 0, 0, 0);
-        v0[u] = ld ? ld_cg_128(v_layer + off) : make_uint4(0, 0, 0, 0);
+        v0[u] = ld && !brief ? ld_cg_128(v_layer + off) : make_uint4(0, 0, 0, 0);
       }
       stamp(0);
-      if (!st_grid_sync(a, gen)) { give_up(4); return; }
+      // this CTA's 16 dimensions of every cached row, where the projection's last activations were (all warps have read them)
+      auto values = [&] {
+        if (BRIEF && dims)
+          for (int i = tid; i < 2 * T16; i += ST_THREADS) {
+            const int t = i >> 1;
+            if (t == pnew) continue;
+            const bool ld = t < T;  // zeros behind the context
+            const __half* src = ld ? kv_row(v_layer, bt_row, t, g, a.G, a.page, a.page_shift, HD) + slice * 16 + (i & 1) * 8 : v_layer;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(st_smem_u32(vs + (size_t)i * 8)), "l"(src), "r"(ld ? 16 : 0) : "memory");
+          }
+      };
+      if (!st_grid_sync(a, gen, values)) { give_up(4); return; }
       stamp(1);
       if (l == 0 && bid == 0 && tid < M) a.key[tid] = 0ull;  // every CTA has read the previous step's key by now
 
@@ -666,162 +695,267 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
               const float s = __fmul_rn(d, a.scale);
               if (t < t1) {
                 lmax[r] = fmaxf(lmax[r], s);
-                if (sub == (r % LPR)) sc[(size_t)r * a.chunk_cap + (t - t0)] = s;
+                if (sub == (r % LPR)) *(brief ? a.att_s + ((size_t)pair * NREP + r) * ST_SHORT_MAX + t : sc + (size_t)r * a.chunk_cap + (t - t0)) = s;
               }
             }
           }
         }
+        if (!brief) {
 #pragma unroll
-        for (int r = 0; r < NREP; r++) {
-          const float mx = warp_max(lmax[r]);
-          if (lane == 0) red[warp][r] = mx;
-        }
-        st_sync();
-        if (tid < NREP) {
-          float mx = red[0][tid];
-          for (int w = 1; w < ST_WARPS; w++) mx = fmaxf(mx, red[w][tid]);
-          s_m[tid] = mx;
-        }
-        st_sync();
-        float lsum[NREP];
+          for (int r = 0; r < NREP; r++) {
+            const float mx = warp_max(lmax[r]);
+            if (lane == 0) red[warp][r] = mx;
+          }
+          st_sync();
+          if (tid < NREP) {
+            float mx = red[0][tid];
+            for (int w = 1; w < ST_WARPS; w++) mx = fmaxf(mx, red[w][tid]);
+            s_m[tid] = mx;
+          }
+          st_sync();
+          float lsum[NREP];
 #pragma unroll
-        for (int r = 0; r < NREP; r++) lsum[r] = 0.f;
-        for (int t = t0 + tid; t < t1; t += ST_THREADS) {
+          for (int r = 0; r < NREP; r++) lsum[r] = 0.f;
+          for (int t = t0 + tid; t < t1; t += ST_THREADS) {
 #pragma unroll
-          for (int r = 0; r < NREP; r++)
-            lsum[r] = __fadd_rn(lsum[r], jg_xexp2_f32(__fmul_rn(__fsub_rn(sc[(size_t)r * a.chunk_cap + (t - t0)], s_m[r]), log2e)));
-        }
+            for (int r = 0; r < NREP; r++)
+              lsum[r] = __fadd_rn(lsum[r], jg_xexp2_f32(__fmul_rn(__fsub_rn(sc[(size_t)r * a.chunk_cap + (t - t0)], s_m[r]), log2e)));
+          }
 #pragma unroll
-        for (int r = 0; r < NREP; r++) {
-          const float v = warp_sum(lsum[r]);
-          if (lane == 0) red[warp][r] = v;
-        }
-        st_sync();
-        if (tid < NREP) {
-          float v = 0.f;
-          for (int w = 0; w < ST_WARPS; w++) v += red[w][tid];
-          float* ml = a.att_ml + (((size_t)pair * NREP + tid) * a.slices + slice) * 2;
-          ml[0] = s_m[tid];
-          ml[1] = v;
+          for (int r = 0; r < NREP; r++) {
+            const float v = warp_sum(lsum[r]);
+            if (lane == 0) red[warp][r] = v;
+          }
+          st_sync();
+          if (tid < NREP) {
+            float v = 0.f;
+            for (int w = 0; w < ST_WARPS; w++) v += red[w][tid];
+            float* ml = a.att_ml + (((size_t)pair * NREP + tid) * a.slices + slice) * 2;
+            ml[0] = s_m[tid];
+            ml[1] = v;
+          }
         }
       }
       stamp(2);
-      if (!st_grid_sync(a, gen)) { give_up(4); return; }
-      stamp(3);
-
-      // ================================================================ P3: probabilities, p.v, fold over the slices
-      if (att) {
-        // every (head, slice) pair of statistics is fetched by its own thread (one round trip to L2 for all of them), then
-        // one thread per head combines them in slice order
-        float* ml_s = pv_part;  // [NREP][slices][2], free until the p.v partials are stored
-        if (tid < NREP * S) {
-          const int r = tid / S, j = tid % S;
-          const float2 v = __ldcg(reinterpret_cast<const float2*>(a.att_ml + (((size_t)pair * NREP + r) * a.slices + j) * 2));
-          ml_s[2 * tid] = v.x;
-          ml_s[2 * tid + 1] = v.y;
-        }
+      if constexpr (BRIEF) {
+        // A context that fits: the slices' scores go to the pair's CTAs as they are (an arrival counter of the pair in place of a grid
+        // barrier), and DS of them work out the whole softmax and finish 16 of the head's dimensions each, V read by dimensions instead
+        // of positions: no statistics to combine, no partial outputs to fold, one grid barrier less.  us per step, with the general form
+        // below / so: 8B 3027 / 2850 (547 positions), 3067 / 2873 (900), 3171 / 3011 (2000), 1B 820 / 756 (1000), 822 / 790 (2000), 3B
+        // 1667 / 1548 (600); two rows 8B 3594 / 3331 (900), 1B 904 / 850 (900).
         st_sync();
-        if (tid < NREP) {
-          const float* ml = ml_s + (size_t)tid * S * 2;
-          float Mx = -INFINITY;
-          for (int j = 0; j < S; j++) Mx = fmaxf(Mx, ml[2 * j]);
-          float Ls = 0.f;
-          for (int j = 0; j < S; j++)
-            Ls = __fadd_rn(Ls, __fmul_rn(ml[2 * j + 1], jg_xexp2_f32(__fmul_rn(__fsub_rn(ml[2 * j], Mx), log2e))));
-          s_M[tid] = Mx;
-          s_rL[tid] = __fdiv_rn(1.0f, Ls);
+        if (mine) {
+          scored += (unsigned)S;
+          if (tid == 0 && att) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.att_n + pair) : "memory");
         }
-        st_sync();
-        float acc[NREP][8];
-#pragma unroll
-        for (int r = 0; r < NREP; r++)
-#pragma unroll
-          for (int i = 0; i < 8; i++) acc[r][i] = 0.f;
-        const int my_r = sub < NREP ? sub : 0;
-        const float myM = s_M[my_r], myrL = s_rL[my_r];
-        for (int base = t0; base < t1; base += ROWS_IT) {
-          const int tb = base + warp * RPW + rgrp;
-          uint4 vv[AU];
-#pragma unroll
-          for (int u = 0; u < AU; u++) {
-            const int t = tb + u * ST_WARPS * RPW;
-            if (base == t0) vv[u] = v0[u];
-            else vv[u] = (t < t1) ? ld_cg_128(kv_row(v_layer, bt_row, t, g, a.G, a.page, a.page_shift, HD) + sub * 8) : make_uint4(0, 0, 0, 0);
+        if (dims) {
+          if (tid < 2)  // the new position's values
+            reinterpret_cast<uint4*>(vs + (size_t)pnew * 16)[tid] = ld_cg_128(a.qkv + (size_t)b * qkv_dim + (size_t)(a.H + a.G + g) * HD + slice * 16 + tid * 8);
+          if (tid == 0) {
+            unsigned long long w0 = 0;
+            for (unsigned polls = 1;; polls++) {
+              unsigned v;
+              asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.att_n + pair) : "memory");
+              if (v >= scored) break;
+              if ((polls & 255u) == 0) {
+                const unsigned long long now = st_now();
+                if (w0 == 0) w0 = now;
+                else if (now - w0 > a.timeout_ns) { atomicCAS(a.err, 0, 4); break; }  // the results are void; the next barrier ends the launch
+              }
+            }
+            asm volatile("fence.acq_rel.gpu;" ::: "memory");
           }
+          st_sync();
+          constexpr int UT = ST_SHORT_MAX / ST_THREADS;
+          float e[NREP][UT];
 #pragma unroll
-          for (int u = 0; u < AU; u++) {
-            const int t = tb + u * ST_WARPS * RPW;
-            const float s = (t < t1 && sub < NREP) ? sc[(size_t)my_r * a.chunk_cap + (t - t0)] : -INFINITY;
-            const float e = jg_xexp2_f32(__fmul_rn(__fsub_rn(s, myM), log2e));
-            const float pr = __half2float(__float2half_rn(__fmul_rn(e, myrL)));
-            float vf[8];
-            unpack8(vv[u], vf);
+          for (int r = 0; r < NREP; r++) {
+            float mx = -INFINITY;
 #pragma unroll
-            for (int r = 0; r < NREP; r++) {
-              const float p_r = __shfl_sync(0xffffffffu, pr, rgrp * LPR + r);
+            for (int u = 0; u < UT; u++) {
+              const int t = tid + u * ST_THREADS;
+              e[r][u] = t < T ? __ldcg(a.att_s + ((size_t)pair * NREP + r) * ST_SHORT_MAX + t) : -INFINITY;
+              mx = fmaxf(mx, e[r][u]);
+            }
+            mx = warp_max(mx);
+            if (lane == 0) red[warp][r] = mx;
+          }
+          st_sync();
+          if (tid < NREP) {
+            float mx = red[0][tid];
+            for (int w = 1; w < ST_WARPS; w++) mx = fmaxf(mx, red[w][tid]);
+            s_M[tid] = mx;
+          }
+          st_sync();
 #pragma unroll
-              for (int i = 0; i < 8; i++) acc[r][i] = fmaf(p_r, vf[i], acc[r][i]);
+          for (int r = 0; r < NREP; r++) {
+            float ls = 0.f;
+#pragma unroll
+            for (int u = 0; u < UT; u++) {
+              e[r][u] = tid + u * ST_THREADS < T ? jg_xexp2_f32(__fmul_rn(__fsub_rn(e[r][u], s_M[r]), log2e)) : 0.f;
+              ls = __fadd_rn(ls, e[r][u]);
+            }
+            ls = warp_sum(ls);
+            if (lane == 0) red[warp][r] = ls;
+          }
+          st_sync();
+          if (tid < NREP) {
+            float ls = 0.f;
+            for (int w = 0; w < ST_WARPS; w++) ls = __fadd_rn(ls, red[w][tid]);
+            s_rL[tid] = __fdiv_rn(1.0f, ls);
+          }
+          st_sync();
+#pragma unroll
+          for (int r = 0; r < NREP; r++)
+#pragma unroll
+            for (int u = 0; u < UT; u++) {
+              const int t = tid + u * ST_THREADS;
+              if (t < T16) ps[(size_t)r * (T16 + 8) + t] = __float2half_rn(__fmul_rn(e[r][u], s_rL[r]));
+            }
+          asm volatile("cp.async.wait_all;" ::: "memory");
+          st_sync();
+          // out^T [16 dims x heads] = V^T [16 x 16 positions] p^T: a warp takes every 16th run of 16 positions
+          float o4[4] = {0.f, 0.f, 0.f, 0.f};
+          const __half* pw = ps + (size_t)min(lane >> 2, NREP - 1) * (T16 + 8) + (lane & 3) * 2;
+          for (int kk = warp * 16; kk < T16; kk += ST_WARPS * 16) {
+            uint32_t a0, a1, a2, a3;
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(a0), "=r"(a1), "=r"(a2), "=r"(a3)
+                         : "r"(st_smem_u32(vs + (size_t)(kk + ((lane >> 4) << 3) + (lane & 7)) * 16 + (((lane >> 3) & 1) << 3))));
+            const uint32_t b0 = *reinterpret_cast<const uint32_t*>(pw + kk), b1 = *reinterpret_cast<const uint32_t*>(pw + kk + 8);
+            asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                         : "+f"(o4[0]), "+f"(o4[1]), "+f"(o4[2]), "+f"(o4[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+          }
+          st_sync();  // V has been read: its place takes the warps' sums
+          float* ow = reinterpret_cast<float*>(st_smem);  // [warp][4][32]
+#pragma unroll
+          for (int i = 0; i < 4; i++) ow[(warp * 4 + i) * 32 + lane] = o4[i];
+          st_sync();
+          if (tid < 16 * NREP) {
+            const int h = tid >> 4, d = tid & 15, i = (h & 1) + ((d >> 3) << 1), ln = (d & 7) * 4 + (h >> 1);
+            float sum = 0.f;
+            for (int w = 0; w < ST_WARPS; w++) sum += ow[(w * 4 + i) * 32 + ln];
+            a.attn[(size_t)b * a.H * HD + (size_t)(g * NREP + h) * HD + slice * 16 + d] = __float2half_rn(sum);
+          }
+        }
+        stamp(4);
+      } else {
+        if (!st_grid_sync(a, gen)) { give_up(4); return; }
+        stamp(3);
+
+        // ================================================================ P3: probabilities, p.v, fold over the slices
+        if (att) {
+          // every (head, slice) pair of statistics is fetched by its own thread (one round trip to L2 for all of them), then
+          // one thread per head combines them in slice order
+          float* ml_s = pv_part;  // [NREP][slices][2], free until the p.v partials are stored
+          if (tid < NREP * S) {
+            const int r = tid / S, j = tid % S;
+            const float2 v = __ldcg(reinterpret_cast<const float2*>(a.att_ml + (((size_t)pair * NREP + r) * a.slices + j) * 2));
+            ml_s[2 * tid] = v.x;
+            ml_s[2 * tid + 1] = v.y;
+          }
+          st_sync();
+          if (tid < NREP) {
+            const float* ml = ml_s + (size_t)tid * S * 2;
+            float Mx = -INFINITY;
+            for (int j = 0; j < S; j++) Mx = fmaxf(Mx, ml[2 * j]);
+            float Ls = 0.f;
+            for (int j = 0; j < S; j++)
+              Ls = __fadd_rn(Ls, __fmul_rn(ml[2 * j + 1], jg_xexp2_f32(__fmul_rn(__fsub_rn(ml[2 * j], Mx), log2e))));
+            s_M[tid] = Mx;
+            s_rL[tid] = __fdiv_rn(1.0f, Ls);
+          }
+          st_sync();
+          float acc[NREP][8];
+#pragma unroll
+          for (int r = 0; r < NREP; r++)
+#pragma unroll
+            for (int i = 0; i < 8; i++) acc[r][i] = 0.f;
+          const int my_r = sub < NREP ? sub : 0;
+          const float myM = s_M[my_r], myrL = s_rL[my_r];
+          for (int base = t0; base < t1; base += ROWS_IT) {
+            const int tb = base + warp * RPW + rgrp;
+            uint4 vv[AU];
+#pragma unroll
+            for (int u = 0; u < AU; u++) {
+              const int t = tb + u * ST_WARPS * RPW;
+              if (base == t0) vv[u] = v0[u];
+              else vv[u] = (t < t1) ? ld_cg_128(kv_row(v_layer, bt_row, t, g, a.G, a.page, a.page_shift, HD) + sub * 8) : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int u = 0; u < AU; u++) {
+              const int t = tb + u * ST_WARPS * RPW;
+              const float s = (t < t1 && sub < NREP) ? sc[(size_t)my_r * a.chunk_cap + (t - t0)] : -INFINITY;
+              const float e = jg_xexp2_f32(__fmul_rn(__fsub_rn(s, myM), log2e));
+              const float pr = __half2float(__float2half_rn(__fmul_rn(e, myrL)));
+              float vf[8];
+              unpack8(vv[u], vf);
+#pragma unroll
+              for (int r = 0; r < NREP; r++) {
+                const float p_r = __shfl_sync(0xffffffffu, pr, rgrp * LPR + r);
+#pragma unroll
+                for (int i = 0; i < 8; i++) acc[r][i] = fmaf(p_r, vf[i], acc[r][i]);
+              }
             }
           }
-        }
 #pragma unroll
-        for (int r = 0; r < NREP; r++)
+          for (int r = 0; r < NREP; r++)
 #pragma unroll
-          for (int i = 0; i < 8; i++) {
+            for (int i = 0; i < 8; i++) {
 #pragma unroll
-            for (int o = 16; o >= LPR; o >>= 1) acc[r][i] += __shfl_xor_sync(0xffffffffu, acc[r][i], o);
+              for (int o = 16; o >= LPR; o >>= 1) acc[r][i] += __shfl_xor_sync(0xffffffffu, acc[r][i], o);
+            }
+          // the warps' partials meet in two rounds (upper half of the warps stores, lower half adds its own on top), which
+          // halves the scratch
+          if (rgrp == 0 && warp >= ST_WARPS / 2) {
+#pragma unroll
+            for (int r = 0; r < NREP; r++)
+#pragma unroll
+              for (int i = 0; i < 8; i++) pv_part[((size_t)(warp - ST_WARPS / 2) * NREP + r) * HD + sub * 8 + i] = acc[r][i];
           }
-        // the warps' partials meet in two rounds (upper half of the warps stores, lower half adds its own on top), which
-        // halves the scratch
-        if (rgrp == 0 && warp >= ST_WARPS / 2) {
+          st_sync();
+          if (rgrp == 0 && warp < ST_WARPS / 2) {
 #pragma unroll
-          for (int r = 0; r < NREP; r++)
+            for (int r = 0; r < NREP; r++)
 #pragma unroll
-            for (int i = 0; i < 8; i++) pv_part[((size_t)(warp - ST_WARPS / 2) * NREP + r) * HD + sub * 8 + i] = acc[r][i];
-        }
-        st_sync();
-        if (rgrp == 0 && warp < ST_WARPS / 2) {
-#pragma unroll
-          for (int r = 0; r < NREP; r++)
-#pragma unroll
-            for (int i = 0; i < 8; i++) pv_part[((size_t)warp * NREP + r) * HD + sub * 8 + i] += acc[r][i];
-        }
-        st_sync();
-        float* po = a.att_o + ((size_t)pair * a.slices + slice) * (NREP * HD);
-        for (int idx = tid; idx < NREP * HD; idx += ST_THREADS) {
-          float s = 0.f;
-#pragma unroll
-          for (int w = 0; w < ST_WARPS / 2; w++) s += pv_part[(size_t)w * NREP * HD + idx];
-          po[idx] = s;
-        }
-        // the last CTA of the pair to get here folds the slices in slice order (the ticket's release covers the whole
-        // CTA's stores: they are ordered before it by the barrier)
-        st_sync();
-        if (tid == 0) {
-          unsigned prev;
-          asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(prev) : "l"(a.tickets + pair) : "memory");
-          s_last = (prev == (unsigned)S - 1u);
-          if (s_last) a.tickets[pair] = 0;
-          __threadfence();
-        }
-        st_sync();
-        if (s_last) {
-          const float* pall = a.att_o + (size_t)pair * a.slices * (NREP * HD);
+              for (int i = 0; i < 8; i++) pv_part[((size_t)warp * NREP + r) * HD + sub * 8 + i] += acc[r][i];
+          }
+          st_sync();
+          float* po = a.att_o + ((size_t)pair * a.slices + slice) * (NREP * HD);
           for (int idx = tid; idx < NREP * HD; idx += ST_THREADS) {
             float s = 0.f;
-            for (int j0 = 0; j0 < S; j0 += 8) {  // eight slices' values requested together, added in slice order
-              float v[8];
 #pragma unroll
-              for (int jj = 0; jj < 8; jj++) v[jj] = (j0 + jj < S) ? __ldcg(pall + (size_t)(j0 + jj) * (NREP * HD) + idx) : 0.f;
+            for (int w = 0; w < ST_WARPS / 2; w++) s += pv_part[(size_t)w * NREP * HD + idx];
+            po[idx] = s;
+          }
+          // the last CTA of the pair to get here folds the slices in slice order (the ticket's release covers the whole
+          // CTA's stores: they are ordered before it by the barrier)
+          st_sync();
+          if (tid == 0) {
+            unsigned prev;
+            asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(prev) : "l"(a.tickets + pair) : "memory");
+            s_last = (prev == (unsigned)S - 1u);
+            if (s_last) a.tickets[pair] = 0;
+            __threadfence();
+          }
+          st_sync();
+          if (s_last) {
+            const float* pall = a.att_o + (size_t)pair * a.slices * (NREP * HD);
+            for (int idx = tid; idx < NREP * HD; idx += ST_THREADS) {
+              float s = 0.f;
+              for (int j0 = 0; j0 < S; j0 += 8) {  // eight slices' values requested together, added in slice order
+                float v[8];
 #pragma unroll
-              for (int jj = 0; jj < 8; jj++)
-                if (j0 + jj < S) s = __fadd_rn(s, v[jj]);
+                for (int jj = 0; jj < 8; jj++) v[jj] = (j0 + jj < S) ? __ldcg(pall + (size_t)(j0 + jj) * (NREP * HD) + idx) : 0.f;
+#pragma unroll
+                for (int jj = 0; jj < 8; jj++)
+                  if (j0 + jj < S) s = __fadd_rn(s, v[jj]);
+              }
+              a.attn[(size_t)b * a.H * HD + (size_t)g * NREP * HD + idx] = __float2half_rn(s);
             }
-            a.attn[(size_t)b * a.H * HD + (size_t)g * NREP * HD + idx] = __float2half_rn(s);
           }
         }
+        stamp(4);
       }
-      stamp(4);
       if (!st_grid_sync(a, gen)) { give_up(4); return; }
       stamp(5);
 
@@ -939,14 +1073,14 @@ struct jg_step {
   int grid;
   int max_rows;
   size_t smem[2];      // dynamic shared memory of the 1-row and the 2-row kernel
-  int nslot[2], ring_offset[2], slot_bytes[2];
+  int nslot[2], ring_offset[2], slot_bytes[2], short_ctx[2];
   int max_slices;
   uint64_t steps_run, launches_run;
 };
 
 typedef void (*StepKernel)(const StepArgs);
-struct StepVariant { int mt, hd, nrep, rs_d, rs_g, rs_h, ni_d, ni_h; StepKernel kern; };
-#define ST_VARIANT(MT, HD, NREP, RSD, RSG, RSH, NID, NIH) {MT, HD, NREP, RSD, RSG, RSH, NID, NIH, jg_step_kernel<MT, HD, NREP, RSD, RSG, RSH, NID, NIH>}
+struct StepVariant { int mt, hd, nrep, rs_d, rs_g, rs_h, ni_d, ni_h; StepKernel kern[2]; };  // any context; short ones
+#define ST_VARIANT(MT, HD, NREP, RSD, RSG, RSH, NID, NIH) {MT, HD, NREP, RSD, RSG, RSH, NID, NIH, {jg_step_kernel<MT, HD, NREP, RSD, RSG, RSH, NID, NIH, false>, jg_step_kernel<MT, HD, NREP, RSD, RSG, RSH, NID, NIH, true>}}
 // Per model shape: the 1-row and the 2-row kernel, each with 64 KB and with 32 KB passes.
 static const StepVariant g_step_variants[] = {
     // Llama-3.1-8B: dim 4096, hidden 14336
@@ -989,6 +1123,7 @@ static void step_destroy_now(void* p) {
   if (s->d_layers) cudaFree(s->d_layers);
   if (s->args.att_ml) cudaFree(s->args.att_ml);
   if (s->args.att_o) cudaFree(s->args.att_o);
+  if (s->args.att_s) cudaFree(s->args.att_s);
   if (s->args.tickets) cudaFree(s->args.tickets);
   if (s->args.bar) cudaFree(s->args.bar);
   if (s->args.key) cudaFree(s->args.key);
@@ -1030,15 +1165,18 @@ JG_API int jg_step_create(jg_dev* dev, jg_kvcache* kv, const jg_step_desc* desc,
   const int chunk_cap = ((kv->max_ctx + slices_min - 1) / slices_min + 31) & ~31;
   const size_t att_bytes = ((size_t)nrep * chunk_cap + (size_t)(ST_WARPS / 2) * nrep * k.head_dim) * sizeof(float);
   size_t smem[2];
-  int nslot[2], ring_offset[2], slot_bytes[2], variant[2];
+  int nslot[2], ring_offset[2], slot_bytes[2], variant[2], short_ctx[2] = {0, 0};
   const char* ke = getenv("JG_STEP_SLOT_KB");
   for (int mt = 1; mt <= 2; mt++) {
     const size_t x_bytes = (size_t)mt * (d.dim > d.hidden_dim ? d.dim : d.hidden_dim) * sizeof(__half);
     const size_t head = ((att_bytes > x_bytes ? att_bytes : x_bytes) + 127) & ~(size_t)127;
     const long long room = (long long)dev->prop.sharedMemPerBlockOptin - 4096 - (long long)head;  // 4 KB: the kernel's static arrays
-    // 64 KB passes where at least two of them fit and eight rows (the most a pass has) fill them, else 32 KB (two rows, us per step with
-    // passes of 64 / 32 KB: 1B 947 / 880, 3B 1931 / 2006, 8B 3373 / 3373; one row: 1B 792 / 792, 8B 3012 / 3038)
-    int sb = room >= 2 * 65536 && 8 * d.dim * 2 > 32768 ? 65536 : 32768;
+    // A CTA's passes in flight: about 128 KB with one row, 160 KB with two (whose passes take longer to work through).  More only wait
+    // in the memory system, out of order: 8B, one row, context 547, us per step with 3 / 4 / 5 / 6 passes of 32 KB 2903 / 2851 / 2887 /
+    // 2933, two or three of 64 KB 2952 / 2920; two rows 3373 / 3315 / 3267 / 3277 and 3258 / 3251 (context 4000: 4184 / 4070 / 4050 with
+    // 3 / 4 / 5, 4106 / 4116).  32 KB a pass, unless that cuts the eight rows a pass can have to five, which the warps share badly (3B,
+    // one row: 4 passes of 5 rows 1566, 3 of 8 rows 1546).  What the ring does not take is the attention phases'.
+    int sb = 8 * d.dim * 2 > 32768 && 8 * d.dim * 2 <= 49152 && room >= 2 * 65536 ? 65536 : 32768;
     if (ke && (atoi(ke) == 32 || atoi(ke) == 64)) sb = atoi(ke) * 1024;
     const int q_dim = k.n_heads * k.head_dim;  // Wo's columns: all heads on one GPU, a rank's share under tensor parallelism
     const bool heads_ok = d.comm != 0 ? (q_dim <= d.dim && q_dim % 8 == 0) : q_dim == d.dim;
@@ -1046,23 +1184,32 @@ JG_API int jg_step_create(jg_dev* dev, jg_kvcache* kv, const jg_step_desc* desc,
     if (heads_ok && nrep <= 4 && vi < 0 && sb == 32768 && room >= 2 * 65536) vi = find_variant(mt, k.head_dim, nrep, d.dim, d.hidden_dim, sb = 65536);
     int ns = (int)(room / sb);
     if (ns > ST_MAX_SLOTS) ns = ST_MAX_SLOTS;
+    const int used = (sb / (d.dim * 2) < 8 ? sb / (d.dim * 2) : 8) * d.dim * 2;  // bytes of a slot that a pass over `dim` columns fills
+    const int deep = used > 0 ? (mt == 1 ? 144 : 176) * 1024 / used : 2;
     const char* se = getenv("JG_STEP_SLOTS");
-    if (se && atoi(se) >= 2 && atoi(se) < ns) ns = atoi(se);
+    const int want = se && atoi(se) >= 2 ? atoi(se) : deep < 2 ? 2 : deep;
+    if (want < ns) ns = want;
     if (ns < 2 || vi < 0) {
       jg_set_error("step_create: no single-kernel step for dim %d, hidden %d, head_dim %d, %d query heads per kv head (%d slots of %d bytes)",
                    d.dim, d.hidden_dim, k.head_dim, nrep, ns, sb);
       return JG_ENOTSUP;
     }
-    nslot[mt - 1] = ns; ring_offset[mt - 1] = (int)head; slot_bytes[mt - 1] = sb; variant[mt - 1] = vi;
-    smem[mt - 1] = head + (size_t)ns * sb;
+    // what the slots leave over goes to the attention phases: a context of which a CTA holds 32 bytes of V and the probabilities a position
+    const size_t head_all = head + (size_t)((room - (long long)ns * sb) & ~127ll);
+    if (grid / (mt * k.n_kv_heads) >= k.head_dim / 16 && getenv("JG_STEP_SLICES") == nullptr)
+      while (short_ctx[mt - 1] + 16 <= ST_SHORT_MAX && (size_t)(short_ctx[mt - 1] + 16) * 32 + (size_t)nrep * (short_ctx[mt - 1] + 24) * 2 <= head_all) short_ctx[mt - 1] += 16;
+    if (getenv("JG_STEP_SHORT") != nullptr && atoi(getenv("JG_STEP_SHORT")) < short_ctx[mt - 1]) short_ctx[mt - 1] = atoi(getenv("JG_STEP_SHORT"));
+    nslot[mt - 1] = ns; ring_offset[mt - 1] = (int)head_all; slot_bytes[mt - 1] = sb; variant[mt - 1] = vi;
+    smem[mt - 1] = head_all + (size_t)ns * sb;
   }
   int coop = 0;
   JG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev->ordinal));
   if (!coop) { jg_set_error("step_create: the device does not support cooperative launches"); return JG_ENOTSUP; }
   for (int i = 0; i < 2; i++) {
-    JG_CUDA(cudaFuncSetAttribute(g_step_variants[variant[i]].kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[i]));
+    const StepKernel kern = g_step_variants[variant[i]].kern[kv->max_ctx <= short_ctx[i]];
+    JG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[i]));
     int per_sm = 0;
-    JG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, g_step_variants[variant[i]].kern, ST_THREADS + 32, smem[i]));
+    JG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, ST_THREADS + 32, smem[i]));
     if (per_sm < 1) { jg_set_error("step_create: the step kernel does not fit an SM"); return JG_ENOTSUP; }
   }
   jg_step* s = new jg_step();
@@ -1071,7 +1218,7 @@ JG_API int jg_step_create(jg_dev* dev, jg_kvcache* kv, const jg_step_desc* desc,
   if (getenv("JG_STEP_SLICES") != nullptr && atoi(getenv("JG_STEP_SLICES")) >= slices_min) s->max_slices = atoi(getenv("JG_STEP_SLICES"));
   s->args.slice_len = (getenv("JG_STEP_SLICE_LEN") != nullptr && atoi(getenv("JG_STEP_SLICE_LEN")) > 0) ? atoi(getenv("JG_STEP_SLICE_LEN")) : 48;
   for (int i = 0; i < 2; i++) {
-    s->smem[i] = smem[i]; s->nslot[i] = nslot[i]; s->ring_offset[i] = ring_offset[i]; s->slot_bytes[i] = slot_bytes[i]; s->variant[i] = variant[i];
+    s->smem[i] = smem[i]; s->nslot[i] = nslot[i]; s->ring_offset[i] = ring_offset[i]; s->slot_bytes[i] = slot_bytes[i]; s->variant[i] = variant[i]; s->short_ctx[i] = short_ctx[i];
   }
   StepArgs& a = s->args;
   a.tok_emb = (const __half*)d.tok_embeddings; a.out_norm = (const __half*)d.out_norm; a.out_w = (const __half*)d.output;
@@ -1102,14 +1249,15 @@ JG_API int jg_step_create(jg_dev* dev, jg_kvcache* kv, const jg_step_desc* desc,
   if (e == cudaSuccess) e = cudaMalloc(&a.att_ml, pairs * nrep * 32 * 2 * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&a.att_o, pairs * 32 * nrep * k.head_dim * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&a.tickets, pairs * sizeof(unsigned int));
-  if (e == cudaSuccess) e = cudaMalloc(&a.bar, 64 * sizeof(unsigned int));
+  if (e == cudaSuccess) e = cudaMalloc(&a.bar, (64 + pairs) * sizeof(unsigned int));
+  if (e == cudaSuccess) e = cudaMalloc(&a.att_s, pairs * nrep * ST_SHORT_MAX * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&a.key, 2 * sizeof(unsigned long long));
   if (e == cudaSuccess && getenv("JG_STEP_PROF") != nullptr && atoi(getenv("JG_STEP_PROF")) != 0) {
     e = cudaMalloc(&a.prof, 32 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemsetAsync(a.prof, 0, 32 * sizeof(unsigned long long), dev->stream);
   }
   if (e == cudaSuccess) e = cudaMemsetAsync(a.tickets, 0, pairs * sizeof(unsigned int), dev->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(a.bar, 0, 64 * sizeof(unsigned int), dev->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(a.bar, 0, (64 + pairs) * sizeof(unsigned int), dev->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(dev->stream);
   delete[] hl;
   if (e != cudaSuccess) {
@@ -1118,6 +1266,7 @@ JG_API int jg_step_create(jg_dev* dev, jg_kvcache* kv, const jg_step_desc* desc,
     return jg_cuda_fail(e, "step_create", __FILE__, __LINE__);
   }
   a.layers = s->d_layers;
+  a.att_n = a.bar + 64;
   a.err = dev->err_word;
   *out = s;
   return JG_OK;
@@ -1161,7 +1310,7 @@ JG_API int jg_step_run(jg_step* s, uint64_t tokens, uint64_t pos, uint64_t h, ui
   a.slot_bytes = s->slot_bytes[vi];
   a.ring_offset = s->ring_offset[vi];
   // the arrival count starts at zero whatever an earlier launch that ran out of time left behind
-  JG_CUDA(cudaMemsetAsync(a.bar, 0, sizeof(unsigned int), dev->stream));
+  JG_CUDA(cudaMemsetAsync(a.bar, 0, (size_t)(64 + s->max_rows * a.G) * sizeof(unsigned int), dev->stream));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(s->grid);
   cfg.blockDim = dim3(ST_THREADS + 32);
@@ -1172,7 +1321,7 @@ JG_API int jg_step_run(jg_step* s, uint64_t tokens, uint64_t pos, uint64_t h, ui
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, v.kern, (const StepArgs)a);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, v.kern[a.max_ctx <= s->short_ctx[vi]], (const StepArgs)a);
   if (e != cudaSuccess) return jg_cuda_fail(e, "step", __FILE__, __LINE__);
   s->steps_run += (uint64_t)n_steps;
   s->launches_run++;

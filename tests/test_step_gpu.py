@@ -84,23 +84,29 @@ def test_unsupported_shapes_keep_the_launch_per_op_path():
     assert llm.model._single_kernel_step(1) is None
 
 
+WIDTHS = {"8B": {"dim": 4096, "n_heads": 32, "hidden_dim": 14336}, "3B": {"dim": 3072, "n_heads": 24, "hidden_dim": 8192},
+          "1B": {"dim": 2048, "n_heads": 32, "hidden_dim": 8192}}
+
 
 @pytest.mark.parametrize("B", [1, 2])
-@pytest.mark.parametrize("size", [{"dim": 4096, "n_heads": 32, "hidden_dim": 14336}, {"dim": 3072, "n_heads": 24, "hidden_dim": 8192}])
-def test_passes_of_64_kb_equal_the_launch_per_op_path(monkeypatch, B, size):
-    """One layer of the 8B and 3B widths: passes of 8, 4 + 4 and 2 or 4 rows, shared by 16 warps by rows and K, batches of passes that do
-    not divide a CTA's; contexts that start in one slice and end in several, and one that no longer fits a CTA's shared memory whole."""
-    args = dict(SMALL, n_layers=1, n_kv_heads=8, vocab_size=9001, **size)
-    for positions, steps in ((14, 40), (830, 3)):
-        prompt = synth.prompt_tokens(positions, args["vocab_size"], batch=B, seed=80)
-        got = []
-        for kernel in ("1", "0"):
-            monkeypatch.setenv("JG_STEP_KERNEL", kernel)
-            llm = make("1B", args=args, max_context=1024, max_batch=2, tied_output=True)
-            got.append(greedy_with_logits(llm, prompt, steps))
-            assert (llm.model._single_kernel_step(B) is not None) == (kernel == "1")
-        (ids, logits), (ids2, logits2) = got
-        for b in range(B):  # up to the first step at which a near-tie was decided otherwise
-            n = steps if (ids[b] == ids2[b]).all() else int(np.argmin(ids[b] == ids2[b]))
-            assert n >= 1
-            assert np.abs(logits[:n, b] - logits2[:n, b]).max() <= 1e-2  # summation order only
+@pytest.mark.parametrize("size", list(WIDTHS))
+@pytest.mark.parametrize("max_context,positions,steps,slot_kb", [(1024, 14, 40, "64"), (1024, 1019, 6, None), (2048, 2043, 6, None), (4096, 14, 40, None), (4096, 2043, 6, "64")])
+def test_widths_and_contexts_equal_the_launch_per_op_path(monkeypatch, size, B, max_context, positions, steps, slot_kb):
+    """One layer of each width: passes of 2 to 8 rows in slots of 32 and 64 KB, shared by 16 warps by rows and K, batches of passes that do
+    not divide a CTA's; caches whose attention takes the form for short contexts (over two and three runs of 16 positions, and up to the
+    last position that fits) and the general one (one slice, several, and a context that no longer fits a CTA's shared memory whole)."""
+    args = dict(SMALL, n_layers=1, n_kv_heads=8, vocab_size=9001, **WIDTHS[size])
+    if slot_kb is not None:
+        monkeypatch.setenv("JG_STEP_SLOT_KB", slot_kb)
+    prompt = synth.prompt_tokens(positions, args["vocab_size"], batch=B, seed=80)
+    got = []
+    for kernel in ("1", "0"):
+        monkeypatch.setenv("JG_STEP_KERNEL", kernel)
+        llm = make("1B", args=args, max_context=max_context, max_batch=2, tied_output=True)
+        got.append(greedy_with_logits(llm, prompt, steps))
+        assert (llm.model._single_kernel_step(B) is not None) == (kernel == "1")
+    (ids, logits), (ids2, logits2) = got
+    for b in range(B):  # up to the first step at which a near-tie was decided otherwise
+        n = steps if (ids[b] == ids2[b]).all() else int(np.argmin(ids[b] == ids2[b]))
+        assert n >= 1
+        assert np.abs(logits[:n, b] - logits2[:n, b]).max() <= 1e-2  # summation order only
