@@ -42,7 +42,7 @@
 
 constexpr int ST_THREADS = 512;  // that compute; one more warp requests the weights
 constexpr int ST_WARPS = ST_THREADS / 32;
-constexpr int ST_SHORT_MAX = 2048;  // four positions to a thread
+constexpr int ST_SHORT_MAX = 2560;  // five positions to a thread
 constexpr int ST_PART = 384;  // partial sums of a batch of passes
 
 struct StepLayer {
@@ -75,6 +75,7 @@ struct StepArgs {
   unsigned long long* key;  // [2] (value, lowest index) max keys of the step's rows (scratch of the plan)
   float* att_ml;          // [M * G][NREP][slices][2]
   float* att_o;           // [M * G][slices][NREP * hd]
+  int kv_offset, kv_rows;  // K / V rows of a context slice in shared memory: where, how many
   float* att_s;           // [M * G][NREP][ST_SHORT_MAX] scores of short contexts
   unsigned int* att_n;    // [M * G] slices whose scores are there, since the launch began
   unsigned int* tickets;  // [M * G]
@@ -347,7 +348,7 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
   static_assert(NREP <= 4 && MT <= 2, "register budget of 128 per thread");
   constexpr int LPR = HD / 8;    // lanes per K / V row
   constexpr int RPW = 32 / LPR;  // rows per warp pass
-  constexpr int AU = 2;          // attention row passes in flight
+  constexpr int AU = BRIEF ? 2 : 4;  // attention row passes in flight
   constexpr int ROWS_IT = ST_WARPS * RPW * AU;
 
   extern __shared__ __align__(16) unsigned char st_smem[];
@@ -477,6 +478,7 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
   };
   // a wait ran out: record it, send the producer home (it lets the copies in flight land) and leave
   auto give_up = [&](int code) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
     if (tid == 0) {
       atomicCAS(a.err, 0, code);
       *(volatile int*)&s_quit = 1;
@@ -599,11 +601,27 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
       const int T16 = (T + 15) & ~15;
       __half* vs = reinterpret_cast<__half*>(st_smem);  // [T16][16], behind it the probabilities [NREP][T16 + 8]
       __half* ps = vs + (size_t)T16 * 16;
+      // otherwise: the slice's K rows are requested between the arrival at the barrier ahead of the scores and its end, its V rows when
+      // K is there, or, where there is no room for both, after K has been read, in its place.  Rows that do not fit are read as they are
+      // needed.  us per step of one row, both through registers 64 rows at a time / so: 8B 3385 / 3200 (4000 positions), 3304 / 3175 (3000,
+      // where requesting V along with K took as long as before), 3B 1937 / 1875 (4000), 1B 878 / 866.
+      __half* kv_s = reinterpret_cast<__half*>(st_smem + a.kv_offset);  // [a.kv_rows][HD]
+      const int staged = min(t1 - t0, a.kv_rows), v_at = 2 * (t1 - t0) <= a.kv_rows ? staged : 0;
+      auto request = [&](const __half* layer, int at) {
+        for (int i = tid; i < staged * LPR; i += ST_THREADS) {
+          const int t = t0 + i / LPR;
+          if (t == pnew) continue;  // written in the phase of the scores
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(st_smem_u32(kv_s + (size_t)at * HD + (size_t)i * 8)),
+                       "l"(kv_row(layer, bt_row, t, g, a.G, a.page, a.page_shift, HD) + i % LPR * 8) : "memory");
+        }
+      };
       int pg0[AU];
+      if constexpr (BRIEF) {
 #pragma unroll
-      for (int u = 0; u < AU; u++) {
-        const int t = t0 + warp * RPW + rgrp + u * ST_WARPS * RPW;
-        pg0[u] = (att && t < t1) ? bt_row[t >> a.page_shift] : 0;
+        for (int u = 0; u < AU; u++) {
+          const int t = t0 + warp * RPW + rgrp + u * ST_WARPS * RPW;
+          pg0[u] = (att && t < t1) ? bt_row[t >> a.page_shift] : 0;
+        }
       }
       // ================================================================ P1: norm -> qkv
       if (l == 0) {
@@ -625,30 +643,34 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
       }
       st_project<RS_D, NI_D, 1, MT>(qkv_dim, KC_D, xs, M, ring, full, empty, rg, batch, part, a, tid, no_pre,
                                          [&](int row, int m, float s, float, __half) { a.qkv[(size_t)m * qkv_dim + row] = __float2half_rn(s); });
-      // the first K and V rows of this CTA's context slice are requested now, ahead of the barrier: cached rows do not
-      // depend on this step's projection (the new position's row does and is fetched again once it has been written)
-      uint4 k0[AU], v0[AU];
+      // a short context's first K rows are requested now, ahead of the barrier: cached rows do not depend on this step's projection (the
+      // new position's row does and is fetched once it has been written)
+      uint4 k0[AU];
+      if constexpr (BRIEF) {
 #pragma unroll
-      for (int u = 0; u < AU; u++) {
-        const int t = t0 + warp * RPW + rgrp + u * ST_WARPS * RPW;
-        const bool ld = att && t < t1 && t != pnew;
-        const size_t off = (((size_t)pg0[u] * a.G + g) * a.page + (t & (a.page - 1))) * HD + sub * 8;
-        k0[u] = ld ? ld_cg_128(k_layer + off) : make_uint4(0, 0, 0, 0);
-        v0[u] = ld && !brief ? ld_cg_128(v_layer + off) : make_uint4(0, 0, 0, 0);
+        for (int u = 0; u < AU; u++) {
+          const int t = t0 + warp * RPW + rgrp + u * ST_WARPS * RPW;
+          const bool ld = att && t < t1 && t != pnew;
+          const size_t off = (((size_t)pg0[u] * a.G + g) * a.page + (t & (a.page - 1))) * HD + sub * 8;
+          k0[u] = ld ? ld_cg_128(k_layer + off) : make_uint4(0, 0, 0, 0);
+        }
       }
       stamp(0);
-      // this CTA's 16 dimensions of every cached row, where the projection's last activations were (all warps have read them)
-      auto values = [&] {
-        if (BRIEF && dims)
-          for (int i = tid; i < 2 * T16; i += ST_THREADS) {
-            const int t = i >> 1;
-            if (t == pnew) continue;
-            const bool ld = t < T;  // zeros behind the context
-            const __half* src = ld ? kv_row(v_layer, bt_row, t, g, a.G, a.page, a.page_shift, HD) + slice * 16 + (i & 1) * 8 : v_layer;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(st_smem_u32(vs + (size_t)i * 8)), "l"(src), "r"(ld ? 16 : 0) : "memory");
-          }
+      auto rows = [&] {
+        if constexpr (BRIEF) {  // this CTA's 16 dimensions of every cached row, where the projection's last activations were (all warps have read them)
+          if (dims)
+            for (int i = tid; i < 2 * T16; i += ST_THREADS) {
+              const int t = i >> 1;
+              if (t == pnew) continue;
+              const bool ld = t < T;  // zeros behind the context
+              const __half* src = ld ? kv_row(v_layer, bt_row, t, g, a.G, a.page, a.page_shift, HD) + slice * 16 + (i & 1) * 8 : v_layer;
+              asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(st_smem_u32(vs + (size_t)i * 8)), "l"(src), "r"(ld ? 16 : 0) : "memory");
+            }
+        } else if (att) {
+          request(k_layer, 0);
+        }
       };
-      if (!st_grid_sync(a, gen, values)) { give_up(4); return; }
+      if (!st_grid_sync(a, gen, rows)) { give_up(4); return; }
       stamp(1);
       if (l == 0 && bid == 0 && tid < M) a.key[tid] = 0ull;  // every CTA has read the previous step's key by now
 
@@ -661,12 +683,21 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
           const uint4 vraw = ld_cg_128(xrow + (size_t)(a.H + a.G + g) * HD + lane * 8);
           const int pg = bt_row[pnew >> a.page_shift], slot = pnew & (a.page - 1);
           const size_t off = (((size_t)pg * a.G + g) * a.page + slot) * HD + (size_t)lane * 8;
-          *reinterpret_cast<uint4*>(k_layer + off) = rope8(kraw, traw);
+          const uint4 krot = rope8(kraw, traw);
+          *reinterpret_cast<uint4*>(k_layer + off) = krot;
           *reinterpret_cast<uint4*>(v_layer + off) = vraw;
+          if (!brief && pnew - t0 < staged) {
+            reinterpret_cast<uint4*>(kv_s + (size_t)(pnew - t0) * HD)[lane] = krot;
+            if (v_at > 0) reinterpret_cast<uint4*>(kv_s + (size_t)(v_at + pnew - t0) * HD)[lane] = vraw;
+          }
         }
         float qf[NREP][8];
 #pragma unroll
         for (int r = 0; r < NREP; r++) unpack8(rope8(ld_cg_128(xrow + (size_t)(g * NREP + r) * HD + sub * 8), traw), qf[r]);
+        if constexpr (!BRIEF) {  // the K rows are here
+          asm volatile("cp.async.wait_all;" ::: "memory");
+          if (v_at > 0) request(v_layer, v_at);
+        }
         st_sync();  // the new K / V rows are visible to this CTA's loads below
         float lmax[NREP];
 #pragma unroll
@@ -677,12 +708,9 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
 #pragma unroll
           for (int u = 0; u < AU; u++) {
             const int t = tb + u * ST_WARPS * RPW;
-            if (base == t0 && t != pnew) {
-              kk[u] = k0[u];  // requested before the barrier
-            } else {
-              kk[u] = (t < t1) ? ld_cg_128(kv_row(k_layer, bt_row, t, g, a.G, a.page, a.page_shift, HD) + sub * 8) : make_uint4(0, 0, 0, 0);
-              if (base == t0) v0[u] = (t < t1) ? ld_cg_128(kv_row(v_layer, bt_row, t, g, a.G, a.page, a.page_shift, HD) + sub * 8) : make_uint4(0, 0, 0, 0);
-            }
+            if (brief && base == t0 && t != pnew) kk[u] = k0[u];  // requested before the barrier
+            else if (!brief && t - t0 < staged) kk[u] = *reinterpret_cast<const uint4*>(kv_s + (size_t)(t - t0) * HD + sub * 8);
+            else kk[u] = (t < t1) ? ld_cg_128(kv_row(k_layer, bt_row, t, g, a.G, a.page, a.page_shift, HD) + sub * 8) : make_uint4(0, 0, 0, 0);
           }
 #pragma unroll
           for (int u = 0; u < AU; u++) {
@@ -839,7 +867,10 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
         }
         stamp(4);
       } else {
-        if (!st_grid_sync(a, gen)) { give_up(4); return; }
+        auto values = [&] {
+          if (att && v_at == 0) request(v_layer, 0);
+        };
+        if (!st_grid_sync(a, gen, values)) { give_up(4); return; }
         stamp(3);
 
         // ================================================================ P3: probabilities, p.v, fold over the slices
@@ -864,6 +895,9 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
             s_M[tid] = Mx;
             s_rL[tid] = __fdiv_rn(1.0f, Ls);
           }
+          if (v_at == 0 && t0 <= pnew && pnew - t0 < staged && tid < LPR)
+            reinterpret_cast<uint4*>(kv_s + (size_t)(pnew - t0) * HD)[tid] = ld_cg_128(a.qkv + (size_t)b * qkv_dim + (size_t)(a.H + a.G + g) * HD + tid * 8);
+          asm volatile("cp.async.wait_all;" ::: "memory");
           st_sync();
           float acc[NREP][8];
 #pragma unroll
@@ -878,7 +912,7 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
 #pragma unroll
             for (int u = 0; u < AU; u++) {
               const int t = tb + u * ST_WARPS * RPW;
-              if (base == t0) vv[u] = v0[u];
+              if (t - t0 < staged) vv[u] = *reinterpret_cast<const uint4*>(kv_s + (size_t)(v_at + t - t0) * HD + sub * 8);
               else vv[u] = (t < t1) ? ld_cg_128(kv_row(v_layer, bt_row, t, g, a.G, a.page, a.page_shift, HD) + sub * 8) : make_uint4(0, 0, 0, 0);
             }
 #pragma unroll
@@ -1073,7 +1107,7 @@ struct jg_step {
   int grid;
   int max_rows;
   size_t smem[2];      // dynamic shared memory of the 1-row and the 2-row kernel
-  int nslot[2], ring_offset[2], slot_bytes[2], short_ctx[2];
+  int nslot[2], ring_offset[2], slot_bytes[2], short_ctx[2], kv_offset[2], kv_rows[2];
   int max_slices;
   uint64_t steps_run, launches_run;
 };
@@ -1165,7 +1199,7 @@ JG_API int jg_step_create(jg_dev* dev, jg_kvcache* kv, const jg_step_desc* desc,
   const int chunk_cap = ((kv->max_ctx + slices_min - 1) / slices_min + 31) & ~31;
   const size_t att_bytes = ((size_t)nrep * chunk_cap + (size_t)(ST_WARPS / 2) * nrep * k.head_dim) * sizeof(float);
   size_t smem[2];
-  int nslot[2], ring_offset[2], slot_bytes[2], variant[2], short_ctx[2] = {0, 0};
+  int nslot[2], ring_offset[2], slot_bytes[2], variant[2], short_ctx[2] = {0, 0}, kv_offset[2], kv_rows[2];
   const char* ke = getenv("JG_STEP_SLOT_KB");
   for (int mt = 1; mt <= 2; mt++) {
     const size_t x_bytes = (size_t)mt * (d.dim > d.hidden_dim ? d.dim : d.hidden_dim) * sizeof(__half);
@@ -1174,31 +1208,41 @@ JG_API int jg_step_create(jg_dev* dev, jg_kvcache* kv, const jg_step_desc* desc,
     // A CTA's passes in flight: about 128 KB with one row, 160 KB with two (whose passes take longer to work through).  More only wait
     // in the memory system, out of order: 8B, one row, context 547, us per step with 3 / 4 / 5 / 6 passes of 32 KB 2903 / 2851 / 2887 /
     // 2933, two or three of 64 KB 2952 / 2920; two rows 3373 / 3315 / 3267 / 3277 and 3258 / 3251 (context 4000: 4184 / 4070 / 4050 with
-    // 3 / 4 / 5, 4106 / 4116).  32 KB a pass, unless that cuts the eight rows a pass can have to five, which the warps share badly (3B,
-    // one row: 4 passes of 5 rows 1566, 3 of 8 rows 1546).  What the ring does not take is the attention phases'.
-    int sb = 8 * d.dim * 2 > 32768 && 8 * d.dim * 2 <= 49152 && room >= 2 * 65536 ? 65536 : 32768;
+    // 3 / 4 / 5, 4106 / 4116).  What the ring does not take is the attention phases'.
+    auto slots = [&](int bytes) {
+      const int used = (bytes / (d.dim * 2) < 8 ? bytes / (d.dim * 2) : 8) * d.dim * 2;  // bytes of a slot that a pass over `dim` columns fills
+      const int deep = used > 0 ? (mt == 1 ? 144 : 176) * 1024 / used : 2;
+      const int fit = room / bytes < ST_MAX_SLOTS ? (int)(room / bytes) : ST_MAX_SLOTS;
+      const char* se = getenv("JG_STEP_SLOTS");
+      const int want = se && atoi(se) >= 2 ? atoi(se) : deep < 2 ? 2 : deep;
+      return want < fit ? want : fit;
+    };
+    auto front = [&](int bytes) { return head + (size_t)((room - (long long)slots(bytes) * bytes) & ~127ll); };  // ahead of the ring
+    // the longest cache that takes the short contexts' form: a CTA of it holds 32 bytes of V and the probabilities of a position
+    auto brief_up_to = [&](int bytes) {
+      int n = 0;
+      if (grid / (mt * k.n_kv_heads) >= k.head_dim / 16 && getenv("JG_STEP_SLICES") == nullptr)
+        while (n + 16 <= ST_SHORT_MAX && (size_t)(n + 16) * 32 + (size_t)nrep * (n + 24) * 2 <= front(bytes)) n += 16;
+      return getenv("JG_STEP_SHORT") != nullptr && atoi(getenv("JG_STEP_SHORT")) < n ? atoi(getenv("JG_STEP_SHORT")) : n;
+    };
+    // 32 KB a pass, unless that cuts the eight rows a pass can have to five, which the warps share badly (3B, us per step, 5 / 8 rows: one
+    // row 1567 / 1544 at 600 positions, two 1924 / 1854, 2304 / 2218 at 3000); with one row the larger passes are given up where they
+    // leave too little for the short contexts' form or for K and V (1632 / 1738 at 1500, 1838 / 1875 at 4000).
+    int sb = 8 * d.dim * 2 > 32768 && 8 * d.dim * 2 <= 49152 && room >= 2 * 65536 && (mt > 1 || kv->max_ctx <= brief_up_to(65536)) ? 65536 : 32768;
     if (ke && (atoi(ke) == 32 || atoi(ke) == 64)) sb = atoi(ke) * 1024;
     const int q_dim = k.n_heads * k.head_dim;  // Wo's columns: all heads on one GPU, a rank's share under tensor parallelism
     const bool heads_ok = d.comm != 0 ? (q_dim <= d.dim && q_dim % 8 == 0) : q_dim == d.dim;
     int vi = (heads_ok && nrep <= 4) ? find_variant(mt, k.head_dim, nrep, d.dim, d.hidden_dim, sb) : -1;
     if (heads_ok && nrep <= 4 && vi < 0 && sb == 32768 && room >= 2 * 65536) vi = find_variant(mt, k.head_dim, nrep, d.dim, d.hidden_dim, sb = 65536);
-    int ns = (int)(room / sb);
-    if (ns > ST_MAX_SLOTS) ns = ST_MAX_SLOTS;
-    const int used = (sb / (d.dim * 2) < 8 ? sb / (d.dim * 2) : 8) * d.dim * 2;  // bytes of a slot that a pass over `dim` columns fills
-    const int deep = used > 0 ? (mt == 1 ? 144 : 176) * 1024 / used : 2;
-    const char* se = getenv("JG_STEP_SLOTS");
-    const int want = se && atoi(se) >= 2 ? atoi(se) : deep < 2 ? 2 : deep;
-    if (want < ns) ns = want;
+    const int ns = slots(sb);
     if (ns < 2 || vi < 0) {
       jg_set_error("step_create: no single-kernel step for dim %d, hidden %d, head_dim %d, %d query heads per kv head (%d slots of %d bytes)",
                    d.dim, d.hidden_dim, k.head_dim, nrep, ns, sb);
       return JG_ENOTSUP;
     }
-    // what the slots leave over goes to the attention phases: a context of which a CTA holds 32 bytes of V and the probabilities a position
-    const size_t head_all = head + (size_t)((room - (long long)ns * sb) & ~127ll);
-    if (grid / (mt * k.n_kv_heads) >= k.head_dim / 16 && getenv("JG_STEP_SLICES") == nullptr)
-      while (short_ctx[mt - 1] + 16 <= ST_SHORT_MAX && (size_t)(short_ctx[mt - 1] + 16) * 32 + (size_t)nrep * (short_ctx[mt - 1] + 24) * 2 <= head_all) short_ctx[mt - 1] += 16;
-    if (getenv("JG_STEP_SHORT") != nullptr && atoi(getenv("JG_STEP_SHORT")) < short_ctx[mt - 1]) short_ctx[mt - 1] = atoi(getenv("JG_STEP_SHORT"));
+    const size_t head_all = front(sb);
+    short_ctx[mt - 1] = brief_up_to(sb);
+    kv_offset[mt - 1] = (int)head; kv_rows[mt - 1] = (int)((head_all - head) / (k.head_dim * sizeof(__half)));
     nslot[mt - 1] = ns; ring_offset[mt - 1] = (int)head_all; slot_bytes[mt - 1] = sb; variant[mt - 1] = vi;
     smem[mt - 1] = head_all + (size_t)ns * sb;
   }
@@ -1219,6 +1263,7 @@ JG_API int jg_step_create(jg_dev* dev, jg_kvcache* kv, const jg_step_desc* desc,
   s->args.slice_len = (getenv("JG_STEP_SLICE_LEN") != nullptr && atoi(getenv("JG_STEP_SLICE_LEN")) > 0) ? atoi(getenv("JG_STEP_SLICE_LEN")) : 48;
   for (int i = 0; i < 2; i++) {
     s->smem[i] = smem[i]; s->nslot[i] = nslot[i]; s->ring_offset[i] = ring_offset[i]; s->slot_bytes[i] = slot_bytes[i]; s->variant[i] = variant[i]; s->short_ctx[i] = short_ctx[i];
+    s->kv_offset[i] = kv_offset[i]; s->kv_rows[i] = kv_rows[i];
   }
   StepArgs& a = s->args;
   a.tok_emb = (const __half*)d.tok_embeddings; a.out_norm = (const __half*)d.out_norm; a.out_w = (const __half*)d.output;
@@ -1308,6 +1353,7 @@ JG_API int jg_step_run(jg_step* s, uint64_t tokens, uint64_t pos, uint64_t h, ui
   const StepVariant& v = g_step_variants[s->variant[vi]];
   a.nslot = s->nslot[vi];
   a.slot_bytes = s->slot_bytes[vi];
+  a.kv_offset = s->kv_offset[vi]; a.kv_rows = s->kv_rows[vi];
   a.ring_offset = s->ring_offset[vi];
   // the arrival count starts at zero whatever an earlier launch that ran out of time left behind
   JG_CUDA(cudaMemsetAsync(a.bar, 0, (size_t)(64 + s->max_rows * a.G) * sizeof(unsigned int), dev->stream));

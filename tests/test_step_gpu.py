@@ -90,11 +90,11 @@ WIDTHS = {"8B": {"dim": 4096, "n_heads": 32, "hidden_dim": 14336}, "3B": {"dim":
 
 @pytest.mark.parametrize("B", [1, 2])
 @pytest.mark.parametrize("size", list(WIDTHS))
-@pytest.mark.parametrize("max_context,positions,steps,slot_kb", [(1024, 14, 40, "64"), (1024, 1019, 6, None), (2048, 2043, 6, None), (4096, 14, 40, None), (4096, 2043, 6, "64")])
+@pytest.mark.parametrize("max_context,positions,steps,slot_kb", [(1024, 14, 40, "64"), (1024, 1019, 6, None), (2048, 2043, 6, None), (4096, 14, 40, None), (4096, 4000, 6, "64"), (8192, 8100, 3, None)])
 def test_widths_and_contexts_equal_the_launch_per_op_path(monkeypatch, size, B, max_context, positions, steps, slot_kb):
     """One layer of each width: passes of 2 to 8 rows in slots of 32 and 64 KB, shared by 16 warps by rows and K, batches of passes that do
     not divide a CTA's; caches whose attention takes the form for short contexts (over two and three runs of 16 positions, and up to the
-    last position that fits) and the general one (one slice, several, and a context that no longer fits a CTA's shared memory whole)."""
+    last position that fits) and the general one (one slice, several; K and V of a slice in shared memory both, one after the other, and in part)."""
     args = dict(SMALL, n_layers=1, n_kv_heads=8, vocab_size=9001, **WIDTHS[size])
     if slot_kb is not None:
         monkeypatch.setenv("JG_STEP_SLOT_KB", slot_kb)
