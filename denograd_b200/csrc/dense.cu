@@ -5,7 +5,8 @@
 //              from the fp32 residual stream — post-norm of the previous sublayer, residual sum and pre-norm (stream.cuh) —
 //              so that a decode step has no launch of its own for them; every CTA recomputes the row, CTA 0 writes the
 //              new stream to a second buffer.
-//   more rows  bf16: tcgen05 kernel (dense_tc.cu); float: a register-tiled fp32 kernel (no reduced-precision modes).
+//              Given rows of bf16 that are only stored go to the kernel around the weight stream (skinny.cuh).
+//   more rows  bf16: tcgen05 kernel or skinny.cuh (dense_tc.cu); float: a register-tiled fp32 kernel (no reduced-precision modes).
 //
 // The prologue can also finish a linear recurrence (division, norm and output gate of jg_gated_norm).
 //
