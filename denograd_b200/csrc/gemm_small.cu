@@ -22,6 +22,7 @@
 #include <stdlib.h>
 
 #include "common.cuh"
+#include "skinny_plan.h"
 #include "transcendental.cuh"
 
 enum { GS_STORE = 0, GS_RESIDUAL = 1, GS_SWIGLU = 2, GS_LOGITS = 3, GS_PARTIAL = 4 };
@@ -42,14 +43,9 @@ struct GemmSmallArgs {
 
 constexpr int GS_THREADS = 256;
 constexpr int GS_WARPS = 8;
-// Activation k tile (halves).  A lane holds the weights of one k tile at a time, and K slices divide the tile among the warps:
-// with int8 weights and 512 halves, eight slices leave a lane 32 bytes in flight, 2 MB on the whole GPU, and the kernel waits
-// for memory at 1.4 to 2 TB/s (8B shapes, 8 rows).  So many slices take longer tiles, as far as two CTAs' activations fit an SM.
-template <int MT, int KS, bool W8>
-constexpr int gs_kt() { return !W8 || KS < 4 || MT > 16 ? 512 : MT <= 8 ? 2048 : 1024; }
 // bytes of a padded row: rows g and g+1 land 4 x 16 B apart modulo 128 B; int8 weights read 32 B per lane, rows 16 B apart
 template <int MT, int KS, bool W8>
-constexpr int gs_row_bytes() { return gs_kt<MT, KS, W8>() * 2 + (W8 ? 16 : 64); }
+constexpr int gs_row_bytes() { return gs_k_tile(MT, KS, W8) * 2 + (W8 ? 16 : 64); }
 
 // int8 x16 (one uint4) -> eight half2 words of half(q) * s in k order, each product rounded once.  Bytes become halves
 // exactly through the 0x6400 (1024.0) exponent trick.
@@ -87,7 +83,7 @@ template <int MT, int KS, int EPI, bool W8>
 __global__ void __launch_bounds__(GS_THREADS, (MT <= 32 ? 2 : 1)) gemm_small_kernel(const GemmSmallArgs a) {
   constexpr int KBLK = W8 ? 64 : 32;         // k block: 4 lanes x one 16-byte weight load each
   constexpr int CH = KBLK / 4;               // weights per lane and block
-  constexpr int GS_KT = gs_kt<MT, KS, W8>(), ROWB = gs_row_bytes<MT, KS, W8>();
+  constexpr int GS_KT = gs_k_tile(MT, KS, W8), ROWB = gs_row_bytes<MT, KS, W8>();
   constexpr int WB = W8 ? 1 : 2;             // bytes per weight
   constexpr int NT = MT / 8;                 // 8-row activation tiles
   constexpr int NW = (EPI == GS_SWIGLU) ? 2 : 1;
@@ -300,13 +296,11 @@ static int launch_gs(jg_dev* dev, const GemmSmallArgs& a, const char* name) {
 template <int MT, int EPI, bool W8>
 static int dispatch_ks(jg_dev* dev, const GemmSmallArgs& a, const char* name) {
   const long long tiles = (a.N + 15) / 16;
-  if (W8 && MT <= 16 && a.K >= 8 * 256) {
-    // int8 weights: no more slices than it takes to have a CTA and a quarter per SM, so that the launch stays one round of two CTAs
-    // per SM and fewer CTAs fetch the same activations (8B shapes, 8 rows, us with 2 / 4 / 8 slices: gate and up 25.6 / 29.8 / 31.3,
-    // qkv 13.1 / 9.0 / 11.4, wo 12.8 / 9.2 / 8.0, down 39 / 27 / 20)
-    for (int ks = 1, per = GS_WARPS; ks < GS_WARPS; ks *= 2, per /= 2) {
-      if ((tiles + per - 1) / per * 4 < 5ll * dev->sm_count) continue;
-      return ks == 1 ? launch_gs<MT, 1, EPI, W8>(dev, a, name) : ks == 2 ? launch_gs<MT, 2, EPI, W8>(dev, a, name) : launch_gs<MT, 4, EPI, W8>(dev, a, name);
+  if (W8 && MT <= 16) {
+    switch (w8_slices(a.N, a.K, dev->sm_count)) {
+      case 1: return launch_gs<MT, 1, EPI, W8>(dev, a, name);
+      case 2: return launch_gs<MT, 2, EPI, W8>(dev, a, name);
+      case 4: return launch_gs<MT, 4, EPI, W8>(dev, a, name);
     }
     return launch_gs<MT, 8, EPI, W8>(dev, a, name);
   }

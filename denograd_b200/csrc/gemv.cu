@@ -35,6 +35,7 @@
 //                       reads only 1/cluster of the entries; the first cluster also writes the new residual stream
 #include "common.cuh"
 #include "peer.cuh"
+#include "skinny_plan.h"
 #include "transcendental.cuh"
 
 enum { EPI_STORE = 0, EPI_RESIDUAL = 1, EPI_SWIGLU = 2, EPI_LOGITS = 3, EPI_PARTIAL = 4, EPI_PEER = 5, EPI_PUSH = 6 };
@@ -487,9 +488,9 @@ int jg_matvec_w8(jg_dev* dev, int epi, const void* x, const void* norm_w, float 
 bool jg_matvec_w8_fits(const jg_dev* dev, int M, int K);
 
 // skinny.cu: a few rows (activations already normalised)
-int jg_skinny(jg_dev* dev, int epi, const void* x, const void* w0, const void* w1, const void* s0, const void* s1, void* y, const void* residual,
+int jg_skinny(jg_dev* dev, int type, int epi, const void* x, const void* w0, const void* w1, const void* s0, const void* s1, void* y, const void* residual,
               void* key, int M, int N, int K, int row_offset);
-bool jg_skinny_fits(const jg_dev* dev, bool w8, int epi, int M, int N, int K);
+bool jg_skinny_fits(const jg_dev* dev, int type, int epi, int M, int N, int K);
 
 // gemm_tc.cu: tcgen05 / TMA projection (fp16 weights, N % 128 == 0, K % 64 == 0), any number of rows
 int jg_gemm_tc(jg_dev* dev, int epi, const void* x, const void* w0, const void* w1, void* y, const void* residual, int M, int N, int K,
@@ -540,8 +541,10 @@ static int dispatch_m(jg_dev* dev, const GemvArgs& a, const char* name) {
     jg_set_error("%s: the projection fused with its all-reduce takes at most 8 rows (M=%d)", name, a.M);
     return JG_ENOTSUP;
   }
-  if (!NORM && jg_skinny_fits(dev, W8, EPI, a.M, a.N, a.K))
-    return jg_skinny(dev, EPI, a.x, a.w0, a.w1, a.s0, a.s1, EPI == EPI_PARTIAL ? (void*)a.y32 : (void*)a.y, a.residual, a.key, a.M, a.N, a.K, a.row_offset);
+  auto skinny = [&](int type) {
+    return jg_skinny(dev, type, EPI, a.x, a.w0, a.w1, a.s0, a.s1, EPI == EPI_PARTIAL ? (void*)a.y32 : (void*)a.y, a.residual, a.key, a.M, a.N, a.K, a.row_offset);
+  };
+  if (!W8 && !NORM && jg_skinny_fits(dev, SK_F16, EPI, a.M, a.N, a.K)) return skinny(SK_F16);
   if (!W8 && !NORM && EPI != EPI_LOGITS && (a.M > 64 || (a.M >= tc_min_rows() && jg_gemm_tc_fits(a.N, a.K))))
     return jg_gemm_tc(dev, EPI, a.x, a.w0, a.w1, EPI == EPI_PARTIAL ? (void*)a.y32 : (void*)a.y, a.residual, a.M, a.N, a.K, nullptr, nullptr);
   // int8 weights and enough rows: the tcgen05 kernel with the conversion inside it
@@ -555,7 +558,8 @@ static int dispatch_m(jg_dev* dev, const GemvArgs& a, const char* name) {
   // int8 weights: the CUDA-core kernel spends its issue slots on dequantisation (half(q) * scale, widen, FMA: about 80
   // instructions per 16 bytes) and reaches half of the HBM rate; on the tensor cores the widening and the FMAs are
   // gone, so pre-normalised int8 projections of any row count go to the mma.sync kernel (JG_W8_MMA=0 keeps the
-  // CUDA-core kernel)
+  // CUDA-core kernel), few rows of them with the same sums around the weight stream
+  if (W8 && !NORM && a.K >= 256 && w8_mma() && jg_skinny_fits(dev, SK_W8, EPI, a.M, a.N, a.K)) return skinny(SK_W8);
   if (W8 && !NORM && a.K >= 256 && w8_mma()) return jg_gemm_small(dev, EPI, a.x, a.w0, a.w1, a.s0, a.s1, EPI == EPI_PARTIAL ? (void*)a.y32 : (void*)a.y, a.residual, a.key, a.M, a.N, a.K, a.row_offset);
   if (a.M == 1) return launch_gemv<1, W8, EPI, NORM>(dev, a, name);
   if (a.M == 2) return launch_gemv<2, W8, EPI, NORM>(dev, a, name);

@@ -31,16 +31,26 @@ struct SkLlama {
   }
 };
 
-// Which calls come here.  int8: up to 8 rows all, 9 to 16 the single matrices with an fp16 result (gate and up of the 8B at 16 rows, us
-// here / in gemm_small.cu: 34.1 / 32.8, logits 126.7 / 130.3 at 16 and 122.4 / 115.6 at 9 rows; the others as in skinny.cuh).  fp16: 3 to
-// 8 rows, logits to 16 (8B: 171.9 / 186.7), but for gate and up where gemm_tc.cu's 128-row tiles keep two thirds of the SMs busy
+// Which calls come here.
+//
+// int8: of those that would go to gemm_small.cu up to 8 rows the single matrices and logits, gate and up from 5 rows on where they are not
+// small, 9 to 16 rows the single matrices with an fp16 result.  Their sums are gemm_small.cu's to the bit (skinny_plan.h): a token drawn
+// from the flat tail of a quantised model's distribution moves with the last bit of a logit.  ms a step with gate and up there / here: 1B 2
+// rows 0.631 / 0.667, 8 rows 0.673 / 0.679; 3B 4 rows 1.500 / 1.604, 5 to 8 rows 1.637 / 1.607 on average; 8B 3 rows 2.26 / 2.30, 4 rows
+// 2.29 / 2.29, 8 rows 2.39 / 2.28; with the single matrices there / here 1B 0.80 / 0.67, 3B 1.90 / 1.60, 8B 2.66 / 2.30 (4 rows).  At 16
+// rows, us: gate and up of the 8B 32.8 / 34.1, logits 130.3 / 126.7 (9 rows 115.6 / 122.4).
+//
+// fp16: 3 to 8 rows, logits to 16 (8B: 171.9 / 186.7), but for gate and up where gemm_tc.cu's 128-row tiles keep two thirds of the SMs busy
 // (8B: 40.4 / 39.0); at 9 to 16 rows that kernel's MMAs cost no more while these read twice the activations (8B step, 16 rows: 3.90 /
 // 3.74 ms with all projections here / there).
-bool jg_skinny_fits(const jg_dev* dev, bool w8, int epi, int M, int N, int K) {
-  if (w8) return K % 128 == 0 && (M <= 8 || (M <= 16 && epi != SKE_SWIGLU && epi != SKE_LOGITS));
-  if (K % 64 != 0 || M < 3) return false;
-  if (epi == SKE_LOGITS) return M <= 16;
-  return M <= 8 && !(epi == SKE_SWIGLU && N % 128 == 0 && N / 128 * 3 >= dev->sm_count * 2);
+bool jg_skinny_fits(const jg_dev* dev, int type, int epi, int M, int N, int K) {
+  const bool glu = epi == SKE_SWIGLU;
+  if (type == SK_W8) {
+    if (glu ? M < 5 || M > 8 || (long long)N * K < 20ll << 20 : M > (epi == SKE_LOGITS ? 8 : 16)) return false;
+  } else {
+    if (M < 3 || M > (epi == SKE_LOGITS ? 16 : 8) || (glu && N % 128 == 0 && N / 128 * 3 >= dev->sm_count * 2)) return false;
+  }
+  return sk_plan(type, glu, M, N, K, 0, dev->sm_count).ok;
 }
 
 template <int TYPE>
@@ -49,8 +59,8 @@ static int launch_skinny(jg_dev* dev, int epi, const SkOperands& o, const SkArgs
   return a.M <= 8 ? launch_skinny_as<TYPE, 1, false, SkLlama>(dev, "skinny", o, a, e) : launch_skinny_as<TYPE, 2, false, SkLlama>(dev, "skinny", o, a, e);
 }
 
-// Entry used by gemv.cu's public functions; s0 / s1 non-null = int8 weights with per-row scales.
-int jg_skinny(jg_dev* dev, int epi, const void* x, const void* w0, const void* w1, const void* s0, const void* s1, void* y, const void* residual,
+// Entry used by gemv.cu's public functions, which ask jg_skinny_fits first; s0, s1: the scales of int8 weights.
+int jg_skinny(jg_dev* dev, int type, int epi, const void* x, const void* w0, const void* w1, const void* s0, const void* s1, void* y, const void* residual,
               void* key, int M, int N, int K, int row_offset) {
   const SkOperands o = {x, w0, w1, K, K, K};
   SkArgs a = {};
@@ -59,5 +69,5 @@ int jg_skinny(jg_dev* dev, int epi, const void* x, const void* w0, const void* w
   SkLlama::Args e = {};
   e.y = (__half*)y; e.y32 = (float*)y; e.residual = (const __half*)residual; e.key = epi == SKE_LOGITS ? (unsigned long long*)key : nullptr;
   e.kind = epi; e.N = N; e.row_offset = row_offset;
-  return s0 ? launch_skinny<SK_W8>(dev, epi, o, a, e) : launch_skinny<SK_F16>(dev, epi, o, a, e);
+  return type == SK_W8 ? launch_skinny<SK_W8>(dev, epi, o, a, e) : launch_skinny<SK_F16>(dev, epi, o, a, e);
 }

@@ -5,16 +5,18 @@
 // a producer warp keeps a ring of stages in flight, each a TMA box of the run's rows x a few 128-byte runs of K (one instruction per
 // matrix; a bulk copy per row piece moved 512 bytes in 75 cycles and no more) with the same k of the activations beside it.  16 warps
 // share a stage: warp (tile, k) has one 128-byte run of one or two 16-row tiles, whose 16-byte chunks in shared memory *are* A
-// fragments of mma.sync.m16n8k16 (the k order inside a run may be permuted as long as the activations' is, too).  The warps run free
+// fragments of mma.sync.m16n8k16 (the k order inside a run may be permuted as long as the activations' is, too).  int8 has the sums of
+// gemm_small.cu to the bit: a warp has one of its K slices, and a stage's box one or two runs of each slice.  The warps run free
 // of each other through the ring (an mbarrier per stage in each direction) and meet once, at the end, to add the sums of the warps
 // that share a tile, in a fixed order.  The first stages' weights are requested before the dependency wait: up to 28 MB in all, most
 // small matrices whole.
 //
-// us per launch, weights from HBM, back to back, the kernels used before / this one: 8B int8, 8 rows qkv 8.8 / 9.0, wo 7.2 / 6.9, gate
-// and up 25.1 / 24.3, down 18.3 / 13.6, logits 94.6 / 89.1; 16 rows 13.6 / 9.7, 11.6 / 8.2, -, 27.7 / 18.7; 8B NF4, one row 8.9 / 9.0,
-// 5.9 / 7.1, 28.3 / 24.6, 14.5 / 13.7 (in a step all four gain: 2.56 / 2.42 ms a token); 1B fp16, 8 rows 6.2 / 5.5, 5.4 / 5.1, 15.2 /
-// 13.6, 11.2 / 8.4; 8B fp16 logits, 8 rows 163.9 / 155.9 (6.7 TB/s).  The stream alone would take 21 us for the 8B int8 gate and up:
-// what is left there is unpacking, at 40 % of the issue slots; a launch costs about 4 us beyond its stream.
+// us per launch, weights from HBM, back to back, the kernels used before / this one: 8B int8, 8 rows qkv 9.4 / 7.9, wo 7.6 / 6.7, gate
+// and up 24.8 / 26.3 (between its neighbours in a step it gains, see skinny.cu), down 19.8 / 13.9, logits 97.8 / 90.4; 16 rows 14.4 /
+// 9.7, 11.5 / 7.7, -, 30.1 / 18.5; 8B NF4, one row 8.9 / 9.0, 5.9 / 7.1, 28.3 / 24.6, 14.5 / 13.7 (in a step all four gain: 2.56 / 2.42
+// ms a token); 1B fp16, 8 rows 6.2 / 5.5, 5.4 / 5.1, 15.2 / 13.6, 11.2 / 8.4; 8B fp16 logits, 8 rows 163.9 / 155.9 (6.7 TB/s).  The
+// stream alone would take 21 us for the 8B int8 gate and up: what is left there is unpacking, at 40 % of the issue slots, and requests
+// of 128 bytes a row where slices lie apart (24.3 us with whole rows of a stage); a launch costs about 4 us beyond its stream.
 //
 // Weights: fp16, bf16, int8 (half(q) * scale of the row, one rounding) or NF4 (half(code * scale of the block) out of a table of byte
 // -> two codes, one copy of it per lane and so per bank).  Products are exact, sums fp32.
@@ -23,31 +25,29 @@
 // reports JG_ETIMEDOUT at the next synchronisation); the producer stops requesting and lets the copies in flight land.
 #pragma once
 #include "common.cuh"
+#include "skinny_plan.h"
 #include "tcgen05.cuh"
-
-enum { SK_F16 = 0, SK_BF16 = 1, SK_W8 = 2, SK_NF4 = 3 };
 
 struct SkArgs {
   const __half *s0, *s1;  // int8: a scale per row
   int* err;
-  int M, N, row_bytes;    // bytes of a weight row: a multiple of 128
+  int M, N;
   int tr, sp;             // outputs of a pass; NF4: bytes of a row's scales in a stage
   int tiles, ks, units;   // 16-row tiles of a pass, warps that share one along K, runs of a warp in a stage
+  int runs, pieces, slice;  // runs of a stage, stages of a pass; W8: runs of a slice
   int stages, stage_bytes, block_shift;
   int w_late;             // the weights were written by a launch that may still be running
 };
 
-constexpr int SK_WARPS = 16, SK_THREADS = 32 * (SK_WARPS + 1), SK_MAX_STAGES = 12;
+constexpr int SK_THREADS = 32 * (SK_WARPS + 1);
 // NT tiles of 8 activation rows x TP tiles of 16 weight rows to a warp
 template <int TYPE, int NT, int TP> struct SkCfg {
-  static constexpr int CPL = TYPE == SK_NF4 ? 4 : TYPE == SK_W8 ? 2 : 1;  // runs of activations to one of weights
-  static constexpr int LUT = TYPE == SK_NF4 ? 256 * 32 * 4 : 0;
-  static constexpr int PERW = TP * NT * 4;                                     // sums of a lane
-  static constexpr int PART = SK_WARPS * PERW * 32 * 4;
-  static constexpr int HEAD = LUT ? 2 * LUT : PART + 1024;                // before the ring; the table lies on a multiple of its size
-  static constexpr int EPT = 4 * NT;                                      // sums a thread finishes at most
+  static constexpr int CPL = sk_runs_x(TYPE);
+  static constexpr int LUT = TYPE == SK_NF4 ? SK_TABLE : 0;
+  static constexpr int PERW = TP * NT * 4;  // sums of a lane
+  static constexpr int PART = sk_part(NT, TP);
+  static constexpr int EPT = 4 * NT;        // sums a thread finishes at most
 };
-__host__ __device__ constexpr int sk_align(int n, int to) { return (n + to - 1) / to * to; }
 
 #ifdef __CUDACC__
 __constant__ float c_sk_nf4[16] = {-1.0f, -0.6961928009986877f, -0.5250730514526367f, -0.39491748809814453f, -0.28444138169288635f, -0.18477343022823334f,
@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
                   const __grid_constant__ CUtensorMap tm_s0, const __grid_constant__ CUtensorMap tm_s1, const SkArgs a, const typename E::Args e) {
   using C = SkCfg<TYPE, NT, TP>;
   constexpr int CPL = C::CPL, NW = GLU ? 2 : 1, PERW = C::PERW, EPT = C::EPT;
+  constexpr bool W8 = TYPE == SK_W8;
   extern __shared__ __align__(1024) unsigned char sk_raw[];
   // [sums | table | ring]
   const uint32_t raw = smem_u32(sk_raw), lut = C::LUT ? (raw + C::PART + C::LUT - 1) & ~(uint32_t)(C::LUT - 1) : 0;
@@ -107,9 +108,9 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
   unsigned char* ring = sk_raw + ((C::LUT ? lut + C::LUT : (raw + C::PART + 1023) & ~1023u) - raw);
   __shared__ __align__(8) uint64_t full[SK_MAX_STAGES], empty[SK_MAX_STAGES];
   const int warp = uniform_warp(), lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int S = a.stages, M = a.M, tr = a.tr, KS = a.ks, U = a.units, RUNS = KS * U;
+  const int S = a.stages, M = a.M, tr = a.tr, KS = a.ks, U = a.units, RUNS = a.runs;
   const int n0 = (int)((long long)blockIdx.x * a.N / gridDim.x), cnt = (int)((long long)(blockIdx.x + 1) * a.N / gridDim.x) - n0;
-  const int passes = (cnt + tr - 1) / tr, np = (a.row_bytes / 128 + RUNS - 1) / RUNS, total = passes * np;
+  const int passes = (cnt + tr - 1) / tr, np = a.pieces, total = passes * np;
   const int w_al = sk_align(RUNS * tr * 128, 1024), x_al = sk_align(RUNS * CPL * M * 128, 1024), s_al = sk_align(tr * a.sp, 128);
   pdl_launch();
 
@@ -121,10 +122,21 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncwarp();
+    // W8: a stage has the next U runs of every slice: run of the slice, first slice
+    auto slice_at = [&](int piece) {
+      const int per = a.slice / U;
+      return make_int2(piece % per * U, piece / per * KS);
+    };
     auto load_w = [&](int i) {
       const int pass = i / np, piece = i - pass * np, s = i % S, row = n0 + pass * tr;
       unsigned char* st = ring + s * a.stage_bytes;
       mbar_expect_tx(&full[s], NW * tr * (RUNS * 128 + a.sp) + M * CPL * RUNS * 128);
+      if (W8) {
+        const int2 at = slice_at(piece);
+        tma_load_4d(st, &tm_w0, 0, row, at.x, at.y, &full[s]);
+        if (GLU) tma_load_4d(st + w_al, &tm_w1, 0, row, at.x, at.y, &full[s]);
+        return;
+      }
       tma_load_3d(st, &tm_w0, 0, row, piece * RUNS, &full[s]);
       if (GLU) tma_load_3d(st + w_al, &tm_w1, 0, row, piece * RUNS, &full[s]);
       if (TYPE == SK_NF4) {
@@ -132,7 +144,15 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
         if (GLU) tma_load_2d(st + NW * w_al + x_al + s_al, &tm_s1, piece * (a.sp / 2), row, &full[s]);
       }
     };
-    auto load_x = [&](int i) { tma_load_3d(ring + (i % S) * a.stage_bytes + NW * w_al, &tm_x, 0, 0, i % np * (RUNS * CPL), &full[i % S]); };
+    auto load_x = [&](int i) {
+      unsigned char* st = ring + (i % S) * a.stage_bytes + NW * w_al;
+      if (W8) {
+        const int2 at = slice_at(i % np);
+        tma_load_4d(st, &tm_x, 0, 0, at.x * CPL, at.y, &full[i % S]);
+      } else {
+        tma_load_3d(st, &tm_x, 0, 0, i % np * (RUNS * CPL), &full[i % S]);
+      }
+    };
     const int pre = min(S, total);
     if (a.w_late) pdl_wait();
     if (elect_one())
@@ -163,7 +183,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
     }
   }
   const uint32_t lut_lane = lut + lane * 4;
-  if (TYPE == SK_W8 && !a.w_late) {  // the run's scales
+  if (W8 && !a.w_late) {  // the run's scales
     prefetch_run(a.s0 + n0, cnt * 2);
     if (GLU) prefetch_run(a.s1 + n0, cnt * 2);
   }
@@ -174,20 +194,20 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
   const int my_tile = warp / KS * TP, my_k = warp % KS;
   const bool active = my_tile < a.tiles;
   // Offsets into a stage, worked out once: a run of a stage lies where it lay in the last one.
-  constexpr int UMAX = TYPE == SK_NF4 ? 2 : 1;
+  constexpr int UMAX = sk_units(TYPE, NT);
   uint32_t wo[UMAX][2], xo[UMAX][2][NT], so[UMAX][2];
   int xs[UMAX][2][NT];
 #pragma unroll
   for (int u = 0; u < UMAX; u++)
 #pragma unroll
     for (int h = 0; h < 2; h++) {  // blocks of 64 bytes of a weight row
-      const int run = u * KS + my_k, wr = run * tr + (GLU ? my_tile * 8 : my_tile * 16) + g;
+      const int run = W8 ? my_k * U + u : u * KS + my_k, wr = run * tr + (GLU ? my_tile * 8 : my_tile * 16) + g;
       wo[u][h] = wr * 128 + (((t + 4 * h) ^ (wr & 7)) << 4);
       so[u][h] = NW * w_al + x_al + ((GLU ? my_tile * 8 : my_tile * 16) + g) * a.sp + ((run * 256 + h * 128 + 32 * t) >> a.block_shift) * 2;
 #pragma unroll
       for (int n = 0; n < NT; n++) {
         // the k of these weights: half a run of the activations, a run, or two (lanes 0 and 1 in the first)
-        const int xr = (TYPE == SK_NF4 ? 4 * run + 2 * h + (t >> 1) : TYPE == SK_W8 ? 2 * run + h : run) * M + min(n * 8 + g, M - 1);
+        const int xr = (TYPE == SK_NF4 ? 4 * run + 2 * h + (t >> 1) : W8 ? 2 * run + h : run) * M + min(n * 8 + g, M - 1);
         xs[u][h][n] = xr & 7;
         xo[u][h][n] = NW * w_al + xr * 128;
       }
@@ -206,7 +226,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
     typename E::Pre pre;
     if (finishes && warp < per && out_of(warp) < nr) pre = E::fetch(e, base + out_of(warp), m_out);
     __half2 s2[TP][2];
-    if (TYPE == SK_W8) {
+    if (W8) {
 #pragma unroll
       for (int p = 0; p < TP; p++)
 #pragma unroll
@@ -241,7 +261,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
           for (int n = 0; n < NT; n++)
 #pragma unroll
             for (int c = 0; c < CPL; c++) {
-              const int xc = TYPE == SK_NF4 ? 4 * (t & 1) + c : TYPE == SK_W8 ? 2 * t + c : t + 4 * h;
+              const int xc = TYPE == SK_NF4 ? 4 * (t & 1) + c : W8 ? 2 * t + c : t + 4 * h;
               const uint4 v = sk_lds(st + xo[u][h][n] + ((xc ^ xs[u][h][n]) << 4));
               xw[n][4 * c] = v.x; xw[n][4 * c + 1] = v.y; xw[n][4 * c + 2] = v.z; xw[n][4 * c + 3] = v.w;
             }
@@ -253,7 +273,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
                 sk_mma<TYPE == SK_BF16>(acc[p][n], va[p].x, vb[p].x, va[p].y, vb[p].y, xw[n][0], xw[n][1]);
                 sk_mma<TYPE == SK_BF16>(acc[p][n], va[p].z, vb[p].z, va[p].w, vb[p].w, xw[n][2], xw[n][3]);
               }
-            } else if (TYPE == SK_W8) {
+            } else if (W8) {
               uint32_t da[8], db[8];
               sk_dequant16(va[p], s2[p][0], da);
               sk_dequant16(vb[p], s2[p][1], db);
@@ -322,40 +342,21 @@ struct SkOperands {
   int K, ldx, ldw;  // elements (NF4: ldw = K)
 };
 template <int TYPE, int NT, int TP, bool GLU, class E>
-static int launch_skinny_tp(jg_dev* dev, const char* name, const SkOperands& o, SkArgs a, const typename E::Args& e) {
-  using C = SkCfg<TYPE, NT, TP>;
-  constexpr int NW = GLU ? 2 : 1;
-  a.row_bytes = TYPE == SK_NF4 ? o.K / 2 : TYPE == SK_W8 ? o.K : o.K * 2;
-  const int warps = (a.tiles + TP - 1) / TP;
-  a.ks = 1;
-  while (warps * a.ks * 2 <= SK_WARPS && a.ks * 128 < a.row_bytes) a.ks *= 2;
-  const int head = C::HEAD + 4096;  // fragments of a tile may reach up to 31 rows past the ring
-  for (;; a.ks /= 2) {
-    a.units = 1;
-    if (TYPE == SK_NF4) {  // at least 16 bytes of scales to a row and stage
-      const int run = 512 >> a.block_shift;
-      while (a.ks * a.units * run < 16) a.units *= 2;
-      a.sp = a.ks * a.units * run;
-    }
-    const int runs = a.ks * a.units;
-    a.stage_bytes = sk_align(NW * sk_align(runs * a.tr * 128, 1024) + sk_align(runs * C::CPL * a.M * 128, 1024) + NW * sk_align(a.tr * a.sp, 128), 1024);
-    a.stages = (200 * 1024 - head) / a.stage_bytes;
-    if (a.stages >= 3 || a.ks == 1) break;
-  }
-  if (a.stages > SK_MAX_STAGES) a.stages = SK_MAX_STAGES;
-  const int grid = a.N < dev->sm_count ? a.N : dev->sm_count, runs = a.ks * a.units;
-  const size_t smem = (size_t)head + (size_t)a.stages * a.stage_bytes;
+static int launch_skinny_tp(jg_dev* dev, const char* name, const SkOperands& o, const SkPlan& p, SkArgs a, const typename E::Args& e) {
+  a.tr = p.tr; a.tiles = p.tiles; a.ks = p.ks; a.units = p.units; a.runs = p.runs; a.sp = p.sp; a.slice = p.slice; a.pieces = p.pieces;
+  a.stages = p.stages; a.stage_bytes = p.stage_bytes;
+  const size_t smem = (size_t)p.smem;
   static size_t set[8] = {};
   if (smem > set[dev->ordinal & 7]) {
     JG_CUDA(cudaFuncSetAttribute(skinny_kernel<TYPE, NT, TP, GLU, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     set[dev->ordinal & 7] = smem;
   }
   CUtensorMap w0, w1, x, s0, s1;
-  const int wb = TYPE == SK_NF4 || TYPE == SK_W8 ? 1 : 2, div = TYPE == SK_NF4 ? 2 : 1;
+  const int wb = TYPE == SK_F16 || TYPE == SK_BF16 ? 2 : 1, div = TYPE == SK_NF4 ? 2 : 1, cpl = sk_runs_x(TYPE), slices = TYPE == SK_W8 ? p.ks : 1;
   const bool bf = TYPE == SK_BF16;
-  int rc = jg_tensor_map(&w0, o.w0, a.N, o.K / div, o.ldw / div, a.tr, "weights", wb, bf, runs);
-  if (!rc) rc = jg_tensor_map(&w1, GLU ? o.w1 : o.w0, a.N, o.K / div, o.ldw / div, a.tr, "weights (second matrix)", wb, bf, runs);
-  if (!rc) rc = jg_tensor_map(&x, o.x, a.M, o.K, o.ldx, a.M, "activations", 2, bf, runs * C::CPL);
+  int rc = jg_tensor_map(&w0, o.w0, a.N, o.K / div, o.ldw / div, a.tr, "weights", wb, bf, p.runs, p.slice, slices);
+  if (!rc) rc = jg_tensor_map(&w1, GLU ? o.w1 : o.w0, a.N, o.K / div, o.ldw / div, a.tr, "weights (second matrix)", wb, bf, p.runs, p.slice, slices);
+  if (!rc) rc = jg_tensor_map(&x, o.x, a.M, o.K, o.ldx, a.M, "activations", 2, bf, p.runs * cpl, p.slice * cpl, slices);
   if (rc) return rc;
   s0 = s1 = x;
   if (TYPE == SK_NF4) {
@@ -364,15 +365,12 @@ static int launch_skinny_tp(jg_dev* dev, const char* name, const SkOperands& o, 
     if (rc) return rc;
   }
   dev->tc_pending = true;
-  return jg_launch(dev, name, skinny_kernel<TYPE, NT, TP, GLU, E>, dim3((unsigned)grid), dim3(SK_THREADS), smem, w0, w1, x, s0, s1, a, e);
+  return jg_launch(dev, name, skinny_kernel<TYPE, NT, TP, GLU, E>, dim3((unsigned)p.grid), dim3(SK_THREADS), smem, w0, w1, x, s0, s1, a, e);
 }
 template <int TYPE, int NT, bool GLU, class E>
-static int launch_skinny_as(jg_dev* dev, const char* name, const SkOperands& o, SkArgs a, const typename E::Args& e) {
-  constexpr int TO = GLU ? 8 : 16;  // outputs of a 16-row tile
-  const int grid = a.N < dev->sm_count ? a.N : dev->sm_count, per = (a.N + grid - 1) / grid, passes = (per + 16 * TO - 1) / (16 * TO);
-  a.tr = (per + passes - 1) / passes;
-  a.tiles = (a.tr + TO - 1) / TO;
-  // more than 8 tiles: two to a warp, which share its activations' fragments
-  return a.tiles <= 8 ? launch_skinny_tp<TYPE, NT, 1, GLU, E>(dev, name, o, a, e) : launch_skinny_tp<TYPE, NT, 2, GLU, E>(dev, name, o, a, e);
+static int launch_skinny_as(jg_dev* dev, const char* name, const SkOperands& o, const SkArgs& a, const typename E::Args& e) {
+  const SkPlan p = sk_plan(TYPE, GLU, a.M, a.N, o.K, a.block_shift, dev->sm_count);
+  JG_REQUIRE(p.ok, "%s: no plan for %d rows, N=%d K=%d", name, a.M, a.N, o.K);
+  return p.tp == 1 ? launch_skinny_tp<TYPE, NT, 1, GLU, E>(dev, name, o, p, a, e) : launch_skinny_tp<TYPE, NT, 2, GLU, E>(dev, name, o, p, a, e);
 }
 #endif

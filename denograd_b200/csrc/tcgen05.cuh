@@ -71,6 +71,11 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
                ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
                : "memory");
 }
+__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+               ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+               : "memory");
+}
 // K-major operand tile in 128-byte swizzled shared memory: rows of 128 bytes, 8-row groups 1024 bytes apart.
 __device__ __forceinline__ uint64_t umma_desc(const void* tile) {
   const uint32_t lo = ((smem_u32(tile) & 0x3FFFFu) >> 4) | (1u << 16);  // start address, leading byte offset = 1 (unused)
@@ -125,6 +130,8 @@ __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
 // rows, cut into boxes of box_rows x 64; out-of-range elements read as zero.  Maps are kept per argument set; `out` is a
 // copy, because the next call may reuse the slot this one came from.
 // groups > 0: boxes of box_rows x `groups` runs of 128 bytes, [run][row][128 bytes] in shared memory (rows of a whole number of
-// runs); groups < 0: boxes of box_rows x -groups elements, as they lie.
+// runs); groups < 0: boxes of box_rows x -groups elements, as they lie.  slice > 0: a row is slices of that many runs, one more
+// dimension, and the box's groups are spread evenly over `slices` of them.
 int jg_tensor_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows,
-                  const char* what, int bytes = 2, bool bf16 = false, int groups = 0);
+                  const char* what, int bytes = 2, bool bf16 = false, int groups = 0,
+                  int slice = 0, int slices = 1);

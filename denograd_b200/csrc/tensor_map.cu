@@ -23,16 +23,17 @@ static int find_encoder() {
 }
 // `bytes` = element size: 2 for fp16 operands (128-byte swizzle, the layout the MMA descriptors name), 1 for int8
 // weight tiles, which land unswizzled (64-byte rows) for the converting warps
-static int make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, const char* what, int bytes, bool bf16, int groups) {
+static int make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, const char* what, int bytes, bool bf16, int groups,
+                    int slice, int slices) {
   const int rc = find_encoder();
   if (rc) return rc;
   const cuuint32_t run = 128 / bytes;
-  const cuuint64_t dims[3] = {groups > 0 ? run : cols, rows, cols / run};  // innermost first
-  const cuuint64_t strides[2] = {ld * (cuuint64_t)bytes, 128};             // bytes between rows, between runs
-  const cuuint32_t box[3] = {groups > 0 ? run : groups < 0 ? (cuuint32_t)-groups : 64, box_rows, (cuuint32_t)groups};
-  const cuuint32_t estr[3] = {1, 1, 1};
+  const cuuint64_t dims[4] = {groups > 0 ? run : cols, rows, slice > 0 ? slice : cols / run, slice > 0 ? cols / run / slice : 1};  // innermost first
+  const cuuint64_t strides[3] = {ld * (cuuint64_t)bytes, 128, 128ull * slice};  // bytes between rows, between runs, between slices
+  const cuuint32_t box[4] = {groups > 0 ? run : groups < 0 ? (cuuint32_t)-groups : 64, box_rows, (cuuint32_t)(groups / slices), (cuuint32_t)slices};
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
   const CUtensorMapDataType type = bytes == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : (bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16);
-  CUresult r = g_encode(m, type, groups > 0 ? 3 : 2, const_cast<void*>(base), dims,
+  CUresult r = g_encode(m, type, slice > 0 ? 4 : groups > 0 ? 3 : 2, const_cast<void*>(base), dims,
                         strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                         groups > 0 || (bytes == 2 && groups == 0) ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -45,32 +46,33 @@ static int make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t co
 
 // Encoded maps are kept per (base, rows, cols, box rows): a model's weights and workspaces keep their addresses, so a
 // step after the first finds all of its maps here instead of encoding three per launch.
-struct MapKey { const void* base; uint64_t rows, cols, ld; uint32_t box_rows; int bytes; bool bf16; int groups; };
+struct MapKey { const void* base; uint64_t rows, cols, ld; uint32_t box_rows; int bytes; bool bf16; int groups, slice, slices; };
 struct MapSlot { MapKey k; CUtensorMap m; bool used; };
 constexpr int MAP_SLOTS = 8192;
 static MapSlot g_maps[MAP_SLOTS];
 
 int jg_tensor_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows, const char* what,
-                  int bytes, bool bf16, int groups) {
-  uint64_t h = (uint64_t)(uintptr_t)base * 0x9E3779B97F4A7C15ull ^ (rows * 0xBF58476D1CE4E5B9ull) ^ (cols << 20) ^ (ld << 4) ^ box_rows ^ ((uint64_t)bytes << 40) ^ ((uint64_t)bf16 << 43) ^ ((uint64_t)(uint32_t)groups << 44);
+                  int bytes, bool bf16, int groups, int slice, int slices) {
+  uint64_t h = (uint64_t)(uintptr_t)base * 0x9E3779B97F4A7C15ull ^ (rows * 0xBF58476D1CE4E5B9ull) ^ (cols << 20) ^ (ld << 4) ^ box_rows ^ ((uint64_t)bytes << 40) ^ ((uint64_t)bf16 << 43) ^ ((uint64_t)(uint32_t)groups << 44) ^
+               ((uint64_t)slice << 48) ^ ((uint64_t)slices << 58);
   h ^= h >> 29;
   for (int probe = 0; probe < 8; probe++) {
     MapSlot& s = g_maps[(h + probe) % MAP_SLOTS];
     if (s.used && s.k.base == base && s.k.rows == rows && s.k.cols == cols && s.k.ld == ld && s.k.box_rows == box_rows && s.k.bytes == bytes &&
-        s.k.bf16 == bf16 && s.k.groups == groups) { *out = s.m; return JG_OK; }
+        s.k.bf16 == bf16 && s.k.groups == groups && s.k.slice == slice && s.k.slices == slices) { *out = s.m; return JG_OK; }
     if (!s.used) {
-      int rc = make_map(&s.m, base, rows, cols, ld, box_rows, what, bytes, bf16, groups);
+      int rc = make_map(&s.m, base, rows, cols, ld, box_rows, what, bytes, bf16, groups, slice, slices);
       if (rc) return rc;
-      s.k = MapKey{base, rows, cols, ld, box_rows, bytes, bf16, groups};
+      s.k = MapKey{base, rows, cols, ld, box_rows, bytes, bf16, groups, slice, slices};
       s.used = true;
       *out = s.m;
       return JG_OK;
     }
   }
   MapSlot& s = g_maps[h % MAP_SLOTS];  // neighbourhood full: replace
-  int rc = make_map(&s.m, base, rows, cols, ld, box_rows, what, bytes, bf16, groups);
+  int rc = make_map(&s.m, base, rows, cols, ld, box_rows, what, bytes, bf16, groups, slice, slices);
   if (rc) { s.used = false; return rc; }
-  s.k = MapKey{base, rows, cols, ld, box_rows, bytes, bf16, groups};
+  s.k = MapKey{base, rows, cols, ld, box_rows, bytes, bf16, groups, slice, slices};
   s.used = true;
   *out = s.m;
   return JG_OK;

@@ -72,3 +72,52 @@ def test_nf4_blocks_and_stages(dev, M, N, K, block):
     dev.call("jg_linear_nf4", y.ptr, xt.ptr, wt.ptr, st.ptr, 0, M, N, K, block)
     want, mag = x.astype(np.float64) @ d.T, np.abs(x.astype(np.float64)) @ np.abs(d).T
     assert (np.abs(y.numpy().astype(np.float64) - want) <= 2.0 ** -20 * mag + 2.0 ** -11 * np.abs(want) * 1.01 + 1e-7).all()
+
+
+def int8_matrix(rng, N, K, dev):
+    q, s = rng.integers(-127, 128, (N, K), dtype=np.int8), (rng.uniform(0.5, 1.5, N) * 3e-4).astype(np.float16)
+    return q, Tensor(q, device=dev), Tensor(s, device=dev)
+
+
+@pytest.mark.parametrize("M", [2, 5, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(1000, 512), (300, 2048), (6000, 2176), (4096, 5120), (6144, 3584), (12000, 2048), (24001, 2304)])
+def test_int8_sums_are_the_general_kernels_to_the_bit(dev, M, N, K):
+    """64 columns of zeros more keep a call off the kernel around the weight stream and add nothing: the same bits, so that a token drawn
+    from a quantised model does not hang on which of the two ran."""
+    rng = np.random.default_rng(N + K + M)
+    x = rng.standard_normal((M, K)).astype(np.float16)
+    pad = lambda a: np.pad(a, ((0, 0), (0, 64)))
+    (q, w, s), (q3, w3, s3) = int8_matrix(rng, N, K, dev), int8_matrix(rng, N, K, dev)
+    outs = []
+    for xa, wa, w3a in ((x, w, w3), (pad(x), Tensor(pad(q), device=dev), Tensor(pad(q3), device=dev))):
+        xt, k = Tensor(xa, device=dev), xa.shape[1]
+        y32, y, z = Tensor.zeros((M, N), "float32", dev), Tensor.zeros((M, N), "float16", dev), Tensor.zeros((M, N), "float16", dev)
+        key = Tensor.zeros((M,), "uint64", dev)
+        dev.call("jg_linear_partial", y32.ptr, xt.ptr, wa.ptr, s.ptr, M, N, k)
+        dev.call("jg_norm_swiglu", y.ptr, xt.ptr, 0, 1e-5, wa.ptr, s.ptr, w3a.ptr, s3.ptr, M, N, k)
+        dev.call("jg_norm_logits_argmax", z.ptr, key.ptr, xt.ptr, 0, 1e-5, wa.ptr, s.ptr, M, N, k)
+        outs.append([t.numpy() for t in (y32, y, z, key)])
+    for a, b in zip(*outs):
+        assert (a.view(np.uint8) == b.view(np.uint8)).all()
+
+
+@pytest.mark.parametrize("N,K", [(14336, 4096), (6144, 4096), (4096, 14336), (8192, 2048), (1003, 512), (24001, 1536)])
+def test_int8_sums_of_one_row_do_not_depend_on_where_it_is_normalised(dev, N, K):
+    """A row of ones and minus ones is its own norm at eps = 0, so the launch that normalises and the one that is given the row multiply
+    the same numbers: the same bits."""
+    rng = np.random.default_rng(N + K)
+    xt = Tensor(rng.choice(np.array([-1, 1], np.float16), (1, K)), device=dev)
+    ones = Tensor(np.ones(K, np.float16), device=dev)
+    (_, w, s), (_, w3, s3) = int8_matrix(rng, N, K, dev), int8_matrix(rng, N, K, dev)
+    outs = []
+    for norm in (0, ones.ptr):
+        y, g, z, key = Tensor.zeros((1, N), "float16", dev), Tensor.zeros((1, N), "float16", dev), Tensor.zeros((1, N), "float16", dev), Tensor.zeros((1,), "uint64", dev)
+        if norm:
+            dev.call("jg_norm_linear", y.ptr, xt.ptr, norm, 0.0, w.ptr, s.ptr, 1, N, K)
+        else:
+            dev.call("jg_linear", y.ptr, xt.ptr, w.ptr, s.ptr, 0, 1, N, K)
+        dev.call("jg_norm_swiglu", g.ptr, xt.ptr, norm, 0.0, w.ptr, s.ptr, w3.ptr, s3.ptr, 1, N, K)
+        dev.call("jg_norm_logits_argmax", z.ptr, key.ptr, xt.ptr, norm, 0.0, w.ptr, s.ptr, 1, N, K)
+        outs.append([t.numpy() for t in (y, g, z, key)])
+    for a, b in zip(*outs):
+        assert (a.view(np.uint8) == b.view(np.uint8)).all()
