@@ -206,9 +206,11 @@ struct SkNf4 {
     e.y[(size_t)m * e.N + n] = v;
   }
 };
-// Rows of whole 128-byte runs and blocks whose scales come in 16-byte pieces: the kernel around the weight stream (skinny.cuh).
-static bool n4_skinny(const Nf4Args& a) {
-  return a.block_shift >= 5 && a.block_shift <= 8 && a.K % (8 << a.block_shift) == 0 && a.K % 256 == 0 && (uintptr_t)a.s0 % 16 == 0 && (uintptr_t)a.s1 % 16 == 0;
+// Rows of whole 128-byte runs and blocks whose scales come in 16-byte pieces: the kernel around the weight stream (skinny.cuh), where it
+// has a plan.
+static bool n4_skinny(const jg_dev* dev, const Nf4Args& a, bool glu) {
+  return a.block_shift >= 5 && a.block_shift <= 8 && a.K % (8 << a.block_shift) == 0 && a.K % 256 == 0 && (uintptr_t)a.s0 % 16 == 0 &&
+         (uintptr_t)a.s1 % 16 == 0 && sk_plan(SK_NF4, glu, a.M, a.N, a.K, a.block_shift, dev->sm_count).ok;
 }
 template <bool GLU>
 static int launch_n4_skinny(jg_dev* dev, const Nf4Args& n, const char* name) {
@@ -245,7 +247,7 @@ JG_API int jg_linear_nf4(jg_dev* dev, uint64_t y, uint64_t x, uint64_t w, uint64
   jg_mark_fresh(dev, y, (uint64_t)M * N * 2);
   JG_REQUIRE(residual == 0 || jg_aligned(residual, 2), "linear_nf4: misaligned residual pointer");
   a.residual = (const __half*)residual;
-  if (n4_skinny(a)) return launch_n4_skinny<false>(dev, a, "linear_nf4");
+  if (n4_skinny(dev, a, false)) return launch_n4_skinny<false>(dev, a, "linear_nf4");
   if (!residual) return launch_n4_ks<N4_STORE>(dev, a, "linear_nf4");
   return launch_n4_ks<N4_RESIDUAL>(dev, a, "linear_nf4");
 }
@@ -260,6 +262,6 @@ JG_API int jg_swiglu_nf4(jg_dev* dev, uint64_t y, uint64_t x, uint64_t w_gate, u
   a.w1 = (const uint8_t*)w_up; a.s1 = (const __half*)s_up;
   a.late = jg_is_fresh(dev, a.w0) || jg_is_fresh(dev, a.s0) || jg_is_fresh(dev, a.w1) || jg_is_fresh(dev, a.s1);
   jg_mark_fresh(dev, y, (uint64_t)M * N * 2);
-  if (n4_skinny(a)) return launch_n4_skinny<true>(dev, a, "swiglu_nf4");
+  if (n4_skinny(dev, a, true)) return launch_n4_skinny<true>(dev, a, "swiglu_nf4");
   return launch_n4_ks<N4_SWIGLU>(dev, a, "swiglu_nf4");
 }

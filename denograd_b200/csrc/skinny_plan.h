@@ -95,6 +95,6 @@ inline SkPlan sk_plan(int type, bool glu, int M, int N, int K, int block_shift, 
     stage(p.ks * p.units);
     if (p.stages >= 3 || p.ks == 1) break;
   }
-  p.ok = true;
+  p.ok = p.units <= sk_units(type, nt) && p.stages >= 2;  // blocks of 128 and 256 may ask for more runs to a stage, and for more memory
   return p;
 }

@@ -81,6 +81,9 @@ int main() {
             if (K % 64 == 0 && (M <= 8 || !glu)) walk(SK_F16, glu, M, N, K, 0, sms), plans++;
             if (K % 128 == 0 && (M <= 8 || !glu)) walk(SK_W8, glu, M, N, K, 0, sms), plans++;
           }
+          for (int block = 32; block <= 256; block *= 2)
+            if (K % (8 * block) == 0 && K % 256 == 0)
+              for (int M : {1, 2, 4, 5, 8}) walk(SK_NF4, glu, M, N, K, block, sms), plans++;
         }
   printf("%lld plans, %d findings\n", plans, findings);
   return findings != 0;

@@ -9,6 +9,9 @@ from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
+CODES = [-1.0, -0.6961928009986877, -0.5250730514526367, -0.39491748809814453, -0.28444138169288635, -0.18477343022823334, -0.09105003625154495, 0.0,
+         0.07958029955625534, 0.16093020141124725, 0.24611230194568634, 0.33791524171829224, 0.44070982933044434, 0.5626170039176941, 0.7229568362236023, 1.0]
+
 
 @pytest.fixture(scope="module")
 def dev():
@@ -61,9 +64,7 @@ def test_edges_of_tiles(dev, kind, M, N, K):
 def test_nf4_blocks_and_stages(dev, M, N, K, block):
     """Blocks of 32 to 256: the scales of a stage take 16 bytes a row at least."""
     rng = np.random.default_rng(N + block)
-    code = np.array([-1.0, -0.6961928009986877, -0.5250730514526367, -0.39491748809814453, -0.28444138169288635, -0.18477343022823334,
-                     -0.09105003625154495, 0.0, 0.07958029955625534, 0.16093020141124725, 0.24611230194568634, 0.33791524171829224,
-                     0.44070982933044434, 0.5626170039176941, 0.7229568362236023, 1.0]).astype(np.float16)
+    code = np.array(CODES).astype(np.float16)
     x, c = rng.standard_normal((M, K)).astype(np.float16), rng.integers(0, 16, N * K).astype(np.uint8)
     s = (0.02 + 0.05 * rng.random(N * K // block)).astype(np.float16)
     d = (code[c].reshape(-1, block) * s[:, None]).astype(np.float16).reshape(N, K).astype(np.float64)
@@ -121,3 +122,34 @@ def test_int8_sums_of_one_row_do_not_depend_on_where_it_is_normalised(dev, N, K)
         outs.append([t.numpy() for t in (y, g, z, key)])
     for a, b in zip(*outs):
         assert (a.view(np.uint8) == b.view(np.uint8)).all()
+
+
+@pytest.mark.parametrize("M", [1, 8])
+@pytest.mark.parametrize("N,K", [(8192, 2048), (14336, 4096), (12289, 2048), (4096, 14336)])
+@pytest.mark.parametrize("block", [32, 64, 128, 256])
+def test_nf4_wide_matrices_of_every_block(dev, block, M, N, K):
+    """One matrix and two, against the products of the dequantised matrix in 64 bits: fp32 sums of K exact products and one fp16 rounding
+    per output and elementwise op.  Wide matrices leave few warps to a tile, so that large blocks need many runs for 16 bytes of scales."""
+    import torch
+
+    rng = np.random.default_rng(N + K + block)
+    code = torch.tensor(CODES, dtype=torch.float64, device="cuda").half()
+    x = rng.standard_normal((M, K)).astype(np.float16)
+    ws, sums, mags = [], [], []
+    x64 = torch.from_numpy(x).cuda().double()
+    for _ in range(2):
+        c = rng.integers(0, 256, N * K // 2).astype(np.uint8)
+        s = (0.02 + 0.05 * rng.random(N * K // block)).astype(np.float16)
+        ws.append((Tensor(c, device=dev), Tensor(s, device=dev)))
+        ct = torch.from_numpy(c).cuda()
+        d = (code[torch.stack([ct >> 4, ct & 15], -1).reshape(-1, block).long()] * torch.from_numpy(s).cuda()[:, None]).reshape(N, K).double()
+        sums.append((x64 @ d.T).cpu().numpy())
+        mags.append((x64.abs() @ d.abs().T).cpu().numpy())
+    (g, u), eps, ulp = sums, 2.0 ** -20, 2.0 ** -11
+    xt, y = Tensor(x, device=dev), Tensor.zeros((M, N), "float16", dev)
+    dev.call("jg_linear_nf4", y.ptr, xt.ptr, ws[0][0].ptr, ws[0][1].ptr, 0, M, N, K, block)
+    assert (np.abs(y.numpy().astype(np.float64) - g) <= eps * mags[0] + ulp * np.abs(g) * 1.01 + 1e-7).all()
+    dev.call("jg_swiglu_nf4", y.ptr, xt.ptr, ws[0][0].ptr, ws[0][1].ptr, ws[1][0].ptr, ws[1][1].ptr, M, N, K, block)
+    want = g / (1 + np.exp(-g)) * u
+    bound = 8 * ulp * np.abs(want) + 1.2 * np.abs(u) * (eps * mags[0] + ulp * np.abs(g)) + np.abs(g) * eps * mags[1] + 1e-4
+    assert (np.abs(y.numpy().astype(np.float64) - want) <= bound).all()
