@@ -201,6 +201,7 @@ struct StepStream {
   const unsigned char* src1;
   uint32_t slot;           // ring slot the next pass goes to
   size_t stride;           // bytes from one pass of this CTA to its next
+  unsigned sent;           // passes requested
 };
 
 // Position (step, layer, phase) -> matrix, this CTA's rows, passes (0 when the CTA has no rows in the phase).
@@ -255,6 +256,7 @@ __device__ __forceinline__ void st_stream_issue(StepStream& st, const StepArgs& 
     st.src1 += st.stride;
   }
   st.src0 += st.stride;
+  st.sent++;
   st.slot = (st.slot + 1 == (uint32_t)a.nslot) ? 0u : st.slot + 1;
   if (--st.left == 0) st_stream_next_phase<RS_D, RS_G, RS_H>(st, a, qkv_dim);
 }
@@ -398,7 +400,7 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
       }
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      st.step = 0; st.layer = 0; st.phase = 0; st.slot = 0;
+      st.step = 0; st.layer = 0; st.phase = 0; st.slot = 0; st.sent = 0;
       st_stream_enter<RS_D, RS_G, RS_H>(st, a, qkv_dim);
       if (st.left <= 0) st_stream_next_phase<RS_D, RS_G, RS_H>(st, a, qkv_dim);
       for (int i = 0; i < a.nslot; i++) st_stream_issue<RS_D, RS_G, RS_H>(st, a, qkv_dim, ring, full);
@@ -408,7 +410,6 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
       // The computing warps may stand at a grid barrier for as long as its limit allows; if they leave, they say so.
       const unsigned limit = (unsigned)(a.timeout_ns / 250000ull) + 4u;  // milliseconds: four times theirs
       uint32_t slot = 0, parity = 0;
-      unsigned left = 0;  // passes whose landing is still to be seen
       bool quit = false;
       while (st.step < a.n_steps && !quit) {
         for (unsigned ms = 0; !quit && !st_mbar_wait(empty + slot, parity, 1000000ull); ms++)
@@ -417,12 +418,11 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
         st_stream_issue<RS_D, RS_G, RS_H>(st, a, qkv_dim, ring, full);
         if (++slot == (uint32_t)a.nslot) { slot = 0; parity ^= 1u; }
       }
-      if (quit) {  // none of the copies in flight may land in the memory of a CTA that has gone: the slots from `slot` on hold the last nslot passes
-        for (left = 0; left < (unsigned)a.nslot; left++) {
-          st_mbar_wait(full + slot, parity, a.timeout_ns);
-          if (++slot == (uint32_t)a.nslot) { slot = 0; parity ^= 1u; }
-        }
-      }
+      // None of the copies in flight may land in the memory of a CTA that has gone.  The walk is over long before the computing warps
+      // are (a narrow model's last passes are requested phases ahead), and they may leave at any barrier: so on every way out.  The copies
+      // wait for nobody, whatever the limit of the other waits is.
+      const unsigned ns = (unsigned)a.nslot;
+      for (unsigned i = st.sent > ns ? st.sent - ns : 0u; i < st.sent; i++) st_mbar_wait(full + i % ns, (i / ns) & 1u, a.timeout_ns + 1000000000ull);
     }
     return;
   }

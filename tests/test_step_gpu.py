@@ -110,3 +110,23 @@ def test_widths_and_contexts_equal_the_launch_per_op_path(monkeypatch, size, B, 
         n = steps if (ids[b] == ids2[b]).all() else int(np.argmin(ids[b] == ids2[b]))
         assert n >= 1
         assert np.abs(logits[:n, b] - logits2[:n, b]).max() <= 1e-2  # summation order only
+
+
+@pytest.mark.parametrize("slots", ["2", "6"])
+@pytest.mark.parametrize("B", [1, 2])
+def test_a_walk_over_the_weights_that_ends_phases_before_the_last_barrier(monkeypatch, B, slots):
+    """One layer, fewer than a pass per CTA in most phases: the warp that requests the weights has nothing left to request while the others
+    still have barriers ahead, and leaves when the last pass has landed.  Runs of one step and of several, in two launches each."""
+    args = dict(SMALL, n_layers=1)
+    monkeypatch.setenv("JG_STEP_SLOTS", slots)
+    prompt = synth.prompt_tokens(7, args["vocab_size"], batch=B, seed=82)
+    llm = make("1B", args=args, max_context=128, max_batch=2, tied_output=True)
+    ids, logits = greedy_with_logits(llm, prompt, 9)
+    assert llm.model._single_kernel_step(B) is not None
+    llm2 = make("1B", args=args, max_context=128, max_batch=2, tied_output=True)
+    first = llm2._prefill(prompt).numpy()
+    assert (llm2.model.decode_loop(first, llm2.start_pos, 4) == ids[:, 1:5]).all()
+    assert (llm2.model.decode_loop(first, llm2.start_pos + 4, 4, resume=True) == ids[:, 5:9]).all()
+    m = build_oracle(args, max_context=128, max_batch=B, tied=True)
+    _, ref_logits, _ = oracle_greedy(m, prompt, 9)
+    assert np.abs(logits - ref_logits).max() <= LOGIT_TOL
