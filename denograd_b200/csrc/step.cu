@@ -407,8 +407,9 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
     }
     __syncthreads();  // the barriers are there
     if (lane == 0) {
-      // The computing warps may stand at a grid barrier for as long as its limit allows; if they leave, they say so.
-      const unsigned limit = (unsigned)(a.timeout_ns / 250000ull) + 4u;  // milliseconds: four times theirs
+      // Between two passes the computing warps may stand at four grid barriers and wait for a peer's part of a sum and of the pick, each
+      // for as long as its limit allows; if they leave, they say so.
+      const unsigned limit = (unsigned)((4ull * a.timeout_ns + (world > 1 ? 2ull * a.peer.timeout_ns : 0ull)) / 1000000ull) + 4u;  // milliseconds
       uint32_t slot = 0, parity = 0;
       bool quit = false;
       while (st.step < a.n_steps && !quit) {
