@@ -12,7 +12,7 @@
 //               P2 RoPE(q, k), cache write, scores of this CTA's context slice, slice max / sum -> scratch      | barrier
 //               P3 global max / sum, p = half(softmax), p.v partial -> scratch; the last CTA of a (row, kv head)
 //                  folds the slices in order into attn                                  | barrier
-//                  (a cache of up to about 2000 positions: P2's scores themselves -> scratch, a counter per (row, kv head), then
+//                  (contexts of up to about 2400 positions, 1600 with two rows: P2's scores themselves -> scratch, a counter per (row, kv head), then
 //                  softmax and p.v of 16 of the head's dimensions per CTA                | barrier)
 //               P4 h += Wo attn                                                         | barrier
 //               P5 x = RMSNorm(h) * g;  ffn = silu(W1 x) * (W3 x)                       | barrier
@@ -86,6 +86,7 @@ struct StepArgs {
   int n_layers, dim, hidden, H, G, vocab, M, table_rows, page, page_shift, max_pages_per_seq, max_ctx;
   int slices, chunk_cap;  // most context slices per (row, kv head) and the scores one slice can hold
   int slice_len;          // positions a slice aims at
+  int short_ctx;          // contexts of up to so many positions take the short contexts' form of attention
   int advance, n_steps;
   int nslot;        // slots of the weight ring (passes in flight per CTA)
   int q_dim;        // H * head_dim: columns of Wo (a rank's share of the heads under tensor parallelism)
@@ -101,6 +102,12 @@ struct StepArgs {
 };
 
 constexpr int ST_MAX_SLOTS = 6;
+// Forms of attention that a kernel has: the short contexts' alone (whatever the cache holds takes it), or both, chosen by the rows' positions.
+// A cache that fits has a kernel of its own, since both forms in the registers of one cost up to 5 % (us per step of one row at position
+// 67, that kernel / with both: 1B 730 / 767, 3B 1529 / 1533, 8B 2881 / 2862, two rows of 8B 3199 / 3341; the general form at 4000 alone / with
+// both: 1B 866 / 878, 3B 1817 / 1827, 8B 3185 / 3203).  (The short form as a function of its own: 5 us more a layer.)  In a cache of 8192
+// one row at 67 / 547 positions takes, with the general form / so: 1B 815 / 767, 830 / 780; 3B 1643 / 1533, 1675 / 1554; 8B 2961 / 2862, 3013 / 2927.
+enum { ST_FITS = 0, ST_BY_POSITION = 1 };
 
 __device__ __forceinline__ unsigned long long st_now() {
   unsigned long long t;
@@ -343,14 +350,216 @@ __device__ __forceinline__ void st_project(int N, int KC, const __half* xs, int 
   }
 }
 
+// What a CTA brings to the attention of one layer (its slice of one (row, kv head) pair), and takes on from it.
+struct StShort {
+  int l, pair, slice, b, g, T, S, t0, t1;
+  bool mine, att;
+  int pg0, pg1;  // pages of this thread's first two rows
+  unsigned gen, scored;
+  bool prof;
+  unsigned long long t_prev;
+  float (*red)[4];  // scratch of the CTA: a sum or maximum per warp and head, per head
+  float *s_M, *s_rL;
+};
+__device__ __forceinline__ void st_stamp(const StepArgs& a, bool prof, unsigned long long& t_prev, int i) {
+  if (prof) {
+    const unsigned long long t = st_now();
+    a.prof[(blockIdx.x == 0 ? 0 : 16) + i] += t - t_prev;
+    t_prev = t;
+  }
+}
+
+// Attention of a short context, from the finished qkv projection to the barrier ahead of the output projection: false = a wait ran out.
+template <int HD, int NREP>
+__device__ __forceinline__ bool st_attend_short(const StepArgs& a, StShort& c) {
+  constexpr int LPR = HD / 8, RPW = 32 / LPR, AU = 2, ROWS_IT = ST_WARPS * RPW * AU;  // lanes of a K row, rows of a warp's pass, passes in flight
+  constexpr int DS = HD / 16;  // CTAs of a pair that share the head's dimensions
+  extern __shared__ __align__(16) unsigned char st_smem[];
+  float (*red)[4] = c.red;
+  float *s_M = c.s_M, *s_rL = c.s_rL;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = lane % LPR, rgrp = lane / LPR;
+  const int pair = c.pair, slice = c.slice, b = c.b, g = c.g, T = c.T, S = c.S, t0 = c.t0, t1 = c.t1, pnew = T - 1;
+  const bool mine = c.mine, att = c.att, dims = mine && slice < DS;
+  const float log2e = 1.4426950408889634f;
+  const int qkv_dim = (a.H + 2 * a.G) * HD, T16 = (T + 15) & ~15;
+  const int32_t* bt_row = a.block_table + (size_t)b * a.max_pages_per_seq;
+  __half* k_layer = a.k_pool + (size_t)c.l * a.layer_elems;
+  __half* v_layer = a.v_pool + (size_t)c.l * a.layer_elems;
+  __half* vs = reinterpret_cast<__half*>(st_smem);  // [T16][16], behind it the probabilities [NREP][T16 + 8]
+  __half* ps = vs + (size_t)T16 * 16;
+  // the first K rows are requested now, ahead of the barrier: cached rows do not depend on this step's projection (the new position's row
+  // does and is fetched once it has been written)
+  uint4 k0[AU];
+#pragma unroll
+  for (int u = 0; u < AU; u++) {
+    const int t = t0 + warp * RPW + rgrp + u * ST_WARPS * RPW;
+    const bool ld = att && t < t1 && t != pnew;
+    const size_t off = (((size_t)(u == 0 ? c.pg0 : c.pg1) * a.G + g) * a.page + (t & (a.page - 1))) * HD + sub * 8;
+    k0[u] = ld ? ld_cg_128(k_layer + off) : make_uint4(0, 0, 0, 0);
+  }
+  st_stamp(a, c.prof, c.t_prev, 0);
+  auto rows = [&] {  // this CTA's 16 dimensions of every cached row, where the projection's last activations were (all warps have read them)
+    if (dims)
+      for (int i = tid; i < 2 * T16; i += ST_THREADS) {
+        const int t = i >> 1;
+        if (t == pnew) continue;
+        const bool ld = t < T;  // zeros behind the context
+        const __half* src = ld ? kv_row(v_layer, bt_row, t, g, a.G, a.page, a.page_shift, HD) + slice * 16 + (i & 1) * 8 : v_layer;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(st_smem_u32(vs + (size_t)i * 8)), "l"(src), "r"(ld ? 16 : 0) : "memory");
+      }
+  };
+  if (!st_grid_sync(a, c.gen, rows)) return false;
+  st_stamp(a, c.prof, c.t_prev, 1);
+  if (c.l == 0 && blockIdx.x == 0 && tid < a.M) a.key[tid] = 0ull;  // every CTA has read the previous step's key by now
+  if (att) {
+    const __half* xrow = a.qkv + (size_t)b * qkv_dim;
+    const uint4 traw = ld_128(a.table + ((size_t)min(pnew, a.table_rows - 1) * (HD / 2) + (size_t)sub * 4) * 2);
+    if (t0 <= pnew && pnew < t1 && warp == 0 && lane < LPR) {
+      const uint4 kraw = ld_cg_128(xrow + (size_t)(a.H + g) * HD + lane * 8);
+      const uint4 vraw = ld_cg_128(xrow + (size_t)(a.H + a.G + g) * HD + lane * 8);
+      const int pg = bt_row[pnew >> a.page_shift], slot = pnew & (a.page - 1);
+      const size_t off = (((size_t)pg * a.G + g) * a.page + slot) * HD + (size_t)lane * 8;
+      *reinterpret_cast<uint4*>(k_layer + off) = rope8(kraw, traw);
+      *reinterpret_cast<uint4*>(v_layer + off) = vraw;
+    }
+    float qf[NREP][8];
+#pragma unroll
+    for (int r = 0; r < NREP; r++) unpack8(rope8(ld_cg_128(xrow + (size_t)(g * NREP + r) * HD + sub * 8), traw), qf[r]);
+    st_sync();  // the new K / V rows are visible to this CTA's loads below
+    for (int base = t0; base < t1; base += ROWS_IT) {
+      const int tb = base + warp * RPW + rgrp;
+      uint4 kk[AU];
+#pragma unroll
+      for (int u = 0; u < AU; u++) {
+        const int t = tb + u * ST_WARPS * RPW;
+        if (base == t0 && t != pnew) kk[u] = k0[u];  // requested before the barrier
+        else kk[u] = (t < t1) ? ld_cg_128(kv_row(k_layer, bt_row, t, g, a.G, a.page, a.page_shift, HD) + sub * 8) : make_uint4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (int u = 0; u < AU; u++) {
+        const int t = tb + u * ST_WARPS * RPW;
+#pragma unroll
+        for (int r = 0; r < NREP; r++) {
+          float d = dot8_acc(0.f, kk[u], qf[r]);
+#pragma unroll
+          for (int o = LPR / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+          if (t < t1 && sub == (r % LPR)) a.att_s[((size_t)pair * NREP + r) * ST_SHORT_MAX + t] = __fmul_rn(d, a.scale);
+        }
+      }
+    }
+  }
+  st_stamp(a, c.prof, c.t_prev, 2);
+  // A context that fits: the slices' scores go to the pair's CTAs as they are (an arrival counter of the pair in place of a grid
+  // barrier), and DS of them work out the whole softmax and finish 16 of the head's dimensions each, V read by dimensions instead
+  // of positions: no statistics to combine, no partial outputs to fold, one grid barrier less.  us per step in
+  // caches that fit, with the general form / so: 8B 3027 / 2850 (547 positions), 3067 / 2873 (900), 3171 / 3011 (2000), 1B 820 / 756 (1000), 822 / 790 (2000), 3B
+  // 1667 / 1548 (600); two rows 8B 3594 / 3331 (900), 1B 904 / 850 (900).
+  st_sync();
+  if (mine) {
+    c.scored += (unsigned)S;
+    if (tid == 0 && att) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.att_n + pair) : "memory");
+  }
+  if (dims) {
+    if (tid < 2)  // the new position's values
+      reinterpret_cast<uint4*>(vs + (size_t)pnew * 16)[tid] = ld_cg_128(a.qkv + (size_t)b * qkv_dim + (size_t)(a.H + a.G + g) * HD + slice * 16 + tid * 8);
+    if (tid == 0) {
+      unsigned long long w0 = 0;
+      for (unsigned polls = 1;; polls++) {
+        unsigned v;
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.att_n + pair) : "memory");
+        if (v >= c.scored) break;
+        if ((polls & 255u) == 0) {
+          const unsigned long long now = st_now();
+          if (w0 == 0) w0 = now;
+          else if (now - w0 > a.timeout_ns) { atomicCAS(a.err, 0, 4); break; }  // the results are void; the next barrier ends the launch
+        }
+      }
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    }
+    st_sync();
+    constexpr int UT = ST_SHORT_MAX / ST_THREADS;
+    float e[NREP][UT];
+#pragma unroll
+    for (int r = 0; r < NREP; r++) {
+      float mx = -INFINITY;
+#pragma unroll
+      for (int u = 0; u < UT; u++) {
+        const int t = tid + u * ST_THREADS;
+        e[r][u] = t < T ? __ldcg(a.att_s + ((size_t)pair * NREP + r) * ST_SHORT_MAX + t) : -INFINITY;
+        mx = fmaxf(mx, e[r][u]);
+      }
+      mx = warp_max(mx);
+      if (lane == 0) red[warp][r] = mx;
+    }
+    st_sync();
+    if (tid < NREP) {
+      float mx = red[0][tid];
+      for (int w = 1; w < ST_WARPS; w++) mx = fmaxf(mx, red[w][tid]);
+      s_M[tid] = mx;
+    }
+    st_sync();
+#pragma unroll
+    for (int r = 0; r < NREP; r++) {
+      float ls = 0.f;
+#pragma unroll
+      for (int u = 0; u < UT; u++) {
+        e[r][u] = tid + u * ST_THREADS < T ? jg_xexp2_f32(__fmul_rn(__fsub_rn(e[r][u], s_M[r]), log2e)) : 0.f;
+        ls = __fadd_rn(ls, e[r][u]);
+      }
+      ls = warp_sum(ls);
+      if (lane == 0) red[warp][r] = ls;
+    }
+    st_sync();
+    if (tid < NREP) {
+      float ls = 0.f;
+      for (int w = 0; w < ST_WARPS; w++) ls = __fadd_rn(ls, red[w][tid]);
+      s_rL[tid] = __fdiv_rn(1.0f, ls);
+    }
+    st_sync();
+#pragma unroll
+    for (int r = 0; r < NREP; r++)
+#pragma unroll
+      for (int u = 0; u < UT; u++) {
+        const int t = tid + u * ST_THREADS;
+        if (t < T16) ps[(size_t)r * (T16 + 8) + t] = __float2half_rn(__fmul_rn(e[r][u], s_rL[r]));
+      }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    st_sync();
+    // out^T [16 dims x heads] = V^T [16 x 16 positions] p^T: a warp takes every 16th run of 16 positions
+    float o4[4] = {0.f, 0.f, 0.f, 0.f};
+    const __half* pw = ps + (size_t)min(lane >> 2, NREP - 1) * (T16 + 8) + (lane & 3) * 2;
+    for (int kk = warp * 16; kk < T16; kk += ST_WARPS * 16) {
+      uint32_t a0, a1, a2, a3;
+      asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(a0), "=r"(a1), "=r"(a2), "=r"(a3)
+                   : "r"(st_smem_u32(vs + (size_t)(kk + ((lane >> 4) << 3) + (lane & 7)) * 16 + (((lane >> 3) & 1) << 3))));
+      const uint32_t b0 = *reinterpret_cast<const uint32_t*>(pw + kk), b1 = *reinterpret_cast<const uint32_t*>(pw + kk + 8);
+      asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                   : "+f"(o4[0]), "+f"(o4[1]), "+f"(o4[2]), "+f"(o4[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+    }
+    st_sync();  // V has been read: its place takes the warps' sums
+    float* ow = reinterpret_cast<float*>(st_smem);  // [warp][4][32]
+#pragma unroll
+    for (int i = 0; i < 4; i++) ow[(warp * 4 + i) * 32 + lane] = o4[i];
+    st_sync();
+    if (tid < 16 * NREP) {
+      const int h = tid >> 4, d = tid & 15, i = (h & 1) + ((d >> 3) << 1), ln = (d & 7) * 4 + (h >> 1);
+      float sum = 0.f;
+      for (int w = 0; w < ST_WARPS; w++) sum += ow[(w * 4 + i) * 32 + ln];
+      a.attn[(size_t)b * a.H * HD + (size_t)(g * NREP + h) * HD + slice * 16 + d] = __float2half_rn(sum);
+    }
+  }
+  st_stamp(a, c.prof, c.t_prev, 4);
+  return true;
+}
+
 // RS_D / RS_G / RS_H: rows per pass of a projection with K = dim (one matrix), of the gate / up pair (rows of each), with
 // K = hidden; NI_D / NI_H: 16-byte chunks per thread and row (K / 8 chunks over 512 threads).
-template <int MT, int HD, int NREP, int RS_D, int RS_G, int RS_H, int NI_D, int NI_H, bool BRIEF>
+template <int MT, int HD, int NREP, int RS_D, int RS_G, int RS_H, int NI_D, int NI_H, int FORM>
 __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepArgs a) {
-  static_assert(NREP <= 4 && MT <= 2, "register budget of 128 per thread");
+  static_assert(NREP <= 4 && MT <= 2, "register budget of 96 per thread");
   constexpr int LPR = HD / 8;    // lanes per K / V row
   constexpr int RPW = 32 / LPR;  // rows per warp pass
-  constexpr int AU = BRIEF ? 2 : 4;  // attention row passes in flight
+  constexpr int AU = 4;          // attention row passes in flight
   constexpr int ROWS_IT = ST_WARPS * RPW * AU;
 
   extern __shared__ __align__(16) unsigned char st_smem[];
@@ -556,13 +765,7 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
     t_prev = st_now();
     if (bid == 0) { a.prof[14] += 1ull; a.prof[30] += (unsigned long long)a.n_steps; }  // launches and steps, replays included
   }
-  auto stamp = [&](int i) {
-    if (prof) {
-      const unsigned long long t = st_now();
-      a.prof[(bid == 0 ? 0 : 16) + i] += t - t_prev;
-      t_prev = t;
-    }
-  };
+  auto stamp = [&](int i) { st_stamp(a, prof, t_prev, i); };
 
   if (a.prof != nullptr && a.bar_probe > 0) {  // diagnostic: the cost of a grid barrier nobody arrives late at
     for (int i = 0; i < a.bar_probe; i++)
@@ -570,12 +773,16 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
     stamp(15);
   }
   for (int step = 0; step < a.n_steps; step++) {
+    int last = posv[0];
+#pragma unroll
+    for (int m = 1; m < MT; m++) last = m < M ? max(last, posv[m]) : last;
+    const bool brief = FORM == ST_FITS || min(last, a.max_ctx - 1) < a.short_ctx;  // every row's context takes the short contexts' form
     for (int l = 0; l < a.n_layers; l++) {
       const StepLayer* L = a.layers + l;
       // the next norms' weights come into L2 in time, a line from each CTA (they are read once a step, from HBM otherwise)
       if (tid < 2 && bid * 64 < dim)
         prefetch_l2((tid == 0 ? L->ffn_norm : l + 1 < a.n_layers ? L[1].attn_norm : a.out_norm) + bid * 64);
-      // this CTA's share of attention: context slice `slice` of (row b, kv head g); the pages of its first rows are looked
+      // this CTA's share of attention: context slice `slice` of (row b, kv head g); the pages of a short context's first rows are looked
       // up now, so that the rows themselves can be requested without a dependent load when the projection is over
       const int n_pairs = M * a.G;
       const bool mine = bid < n_pairs * a.slices;  // a.slices: the most slices a pair can have (the scratch's stride)
@@ -596,13 +803,7 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
       const int32_t* bt_row = a.block_table + (size_t)b * a.max_pages_per_seq;
       __half* k_layer = a.k_pool + (size_t)l * a.layer_elems;
       __half* v_layer = a.v_pool + (size_t)l * a.layer_elems;
-      constexpr int DS = HD / 16;  // BRIEF: CTAs of a pair that share the head's dimensions
-      constexpr bool brief = BRIEF;
-      const bool dims = brief && mine && slice < DS;
-      const int T16 = (T + 15) & ~15;
-      __half* vs = reinterpret_cast<__half*>(st_smem);  // [T16][16], behind it the probabilities [NREP][T16 + 8]
-      __half* ps = vs + (size_t)T16 * 16;
-      // otherwise: the slice's K rows are requested between the arrival at the barrier ahead of the scores and its end, its V rows when
+      // The general form: the slice's K rows are requested between the arrival at the barrier ahead of the scores and its end, its V rows when
       // K is there, or, where there is no room for both, after K has been read, in its place.  Rows that do not fit are read as they are
       // needed.  us per step of one row, both through registers 64 rows at a time / so: 8B 3385 / 3200 (4000 positions), 3304 / 3175 (3000,
       // where requesting V along with K took as long as before), 3B 1937 / 1875 (4000), 1B 878 / 866.
@@ -616,10 +817,10 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
                        "l"(kv_row(layer, bt_row, t, g, a.G, a.page, a.page_shift, HD) + i % LPR * 8) : "memory");
         }
       };
-      int pg0[AU];
-      if constexpr (BRIEF) {
+      int pg0[2] = {0, 0};
+      if (brief) {  // the pages of its first rows
 #pragma unroll
-        for (int u = 0; u < AU; u++) {
+        for (int u = 0; u < 2; u++) {
           const int t = t0 + warp * RPW + rgrp + u * ST_WARPS * RPW;
           pg0[u] = (att && t < t1) ? bt_row[t >> a.page_shift] : 0;
         }
@@ -644,92 +845,71 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
       }
       st_project<RS_D, NI_D, 1, MT>(qkv_dim, KC_D, xs, M, ring, full, empty, rg, batch, part, a, tid, no_pre,
                                          [&](int row, int m, float s, float, __half) { a.qkv[(size_t)m * qkv_dim + row] = __float2half_rn(s); });
-      // a short context's first K rows are requested now, ahead of the barrier: cached rows do not depend on this step's projection (the
-      // new position's row does and is fetched once it has been written)
-      uint4 k0[AU];
-      if constexpr (BRIEF) {
-#pragma unroll
-        for (int u = 0; u < AU; u++) {
-          const int t = t0 + warp * RPW + rgrp + u * ST_WARPS * RPW;
-          const bool ld = att && t < t1 && t != pnew;
-          const size_t off = (((size_t)pg0[u] * a.G + g) * a.page + (t & (a.page - 1))) * HD + sub * 8;
-          k0[u] = ld ? ld_cg_128(k_layer + off) : make_uint4(0, 0, 0, 0);
-        }
-      }
-      stamp(0);
-      auto rows = [&] {
-        if constexpr (BRIEF) {  // this CTA's 16 dimensions of every cached row, where the projection's last activations were (all warps have read them)
-          if (dims)
-            for (int i = tid; i < 2 * T16; i += ST_THREADS) {
-              const int t = i >> 1;
-              if (t == pnew) continue;
-              const bool ld = t < T;  // zeros behind the context
-              const __half* src = ld ? kv_row(v_layer, bt_row, t, g, a.G, a.page, a.page_shift, HD) + slice * 16 + (i & 1) * 8 : v_layer;
-              asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(st_smem_u32(vs + (size_t)i * 8)), "l"(src), "r"(ld ? 16 : 0) : "memory");
-            }
-        } else if (att) {
-          request(k_layer, 0);
-        }
-      };
-      if (!st_grid_sync(a, gen, rows)) { give_up(4); return; }
-      stamp(1);
-      if (l == 0 && bid == 0 && tid < M) a.key[tid] = 0ull;  // every CTA has read the previous step's key by now
+      if (brief) {
+        StShort c = {l, pair, slice, b, g, T, S, t0, t1, mine, att, pg0[0], pg0[1], gen, scored, prof, t_prev, red, s_M, s_rL};
+        const bool ok = st_attend_short<HD, NREP>(a, c);
+        gen = c.gen; scored = c.scored; t_prev = c.t_prev;
+        if (!ok) { give_up(4); return; }
+      } else if constexpr (FORM != ST_FITS) {
+        stamp(0);
+        auto rows = [&] {
+          if (att) request(k_layer, 0);
+        };
+        if (!st_grid_sync(a, gen, rows)) { give_up(4); return; }
+        stamp(1);
+        if (l == 0 && bid == 0 && tid < M) a.key[tid] = 0ull;  // every CTA has read the previous step's key by now
 
-      // ================================================================ P2: RoPE, cache write, scores of a context slice
-      if (att) {
-        const __half* xrow = a.qkv + (size_t)b * qkv_dim;
-        const uint4 traw = ld_128(a.table + ((size_t)min(pnew, a.table_rows - 1) * (HD / 2) + (size_t)sub * 4) * 2);
-        if (t0 <= pnew && pnew < t1 && warp == 0 && lane < LPR) {
-          const uint4 kraw = ld_cg_128(xrow + (size_t)(a.H + g) * HD + lane * 8);
-          const uint4 vraw = ld_cg_128(xrow + (size_t)(a.H + a.G + g) * HD + lane * 8);
-          const int pg = bt_row[pnew >> a.page_shift], slot = pnew & (a.page - 1);
-          const size_t off = (((size_t)pg * a.G + g) * a.page + slot) * HD + (size_t)lane * 8;
-          const uint4 krot = rope8(kraw, traw);
-          *reinterpret_cast<uint4*>(k_layer + off) = krot;
-          *reinterpret_cast<uint4*>(v_layer + off) = vraw;
-          if (!brief && pnew - t0 < staged) {
-            reinterpret_cast<uint4*>(kv_s + (size_t)(pnew - t0) * HD)[lane] = krot;
-            if (v_at > 0) reinterpret_cast<uint4*>(kv_s + (size_t)(v_at + pnew - t0) * HD)[lane] = vraw;
+        // ================================================================ P2: RoPE, cache write, scores of a context slice
+        if (att) {
+          const __half* xrow = a.qkv + (size_t)b * qkv_dim;
+          const uint4 traw = ld_128(a.table + ((size_t)min(pnew, a.table_rows - 1) * (HD / 2) + (size_t)sub * 4) * 2);
+          if (t0 <= pnew && pnew < t1 && warp == 0 && lane < LPR) {
+            const uint4 kraw = ld_cg_128(xrow + (size_t)(a.H + g) * HD + lane * 8);
+            const uint4 vraw = ld_cg_128(xrow + (size_t)(a.H + a.G + g) * HD + lane * 8);
+            const int pg = bt_row[pnew >> a.page_shift], slot = pnew & (a.page - 1);
+            const size_t off = (((size_t)pg * a.G + g) * a.page + slot) * HD + (size_t)lane * 8;
+            const uint4 krot = rope8(kraw, traw);
+            *reinterpret_cast<uint4*>(k_layer + off) = krot;
+            *reinterpret_cast<uint4*>(v_layer + off) = vraw;
+            if (pnew - t0 < staged) {
+              reinterpret_cast<uint4*>(kv_s + (size_t)(pnew - t0) * HD)[lane] = krot;
+              if (v_at > 0) reinterpret_cast<uint4*>(kv_s + (size_t)(v_at + pnew - t0) * HD)[lane] = vraw;
+            }
           }
-        }
-        float qf[NREP][8];
+          float qf[NREP][8];
 #pragma unroll
-        for (int r = 0; r < NREP; r++) unpack8(rope8(ld_cg_128(xrow + (size_t)(g * NREP + r) * HD + sub * 8), traw), qf[r]);
-        if constexpr (!BRIEF) {  // the K rows are here
-          asm volatile("cp.async.wait_all;" ::: "memory");
+          for (int r = 0; r < NREP; r++) unpack8(rope8(ld_cg_128(xrow + (size_t)(g * NREP + r) * HD + sub * 8), traw), qf[r]);
+          asm volatile("cp.async.wait_all;" ::: "memory");  // the K rows are here
           if (v_at > 0) request(v_layer, v_at);
-        }
-        st_sync();  // the new K / V rows are visible to this CTA's loads below
-        float lmax[NREP];
+          st_sync();  // the new K / V rows are visible to this CTA's loads below
+          float lmax[NREP];
 #pragma unroll
-        for (int r = 0; r < NREP; r++) lmax[r] = -INFINITY;
-        for (int base = t0; base < t1; base += ROWS_IT) {
-          const int tb = base + warp * RPW + rgrp;
-          uint4 kk[AU];
+          for (int r = 0; r < NREP; r++) lmax[r] = -INFINITY;
+          for (int base = t0; base < t1; base += ROWS_IT) {
+            const int tb = base + warp * RPW + rgrp;
+            uint4 kk[AU];
 #pragma unroll
-          for (int u = 0; u < AU; u++) {
-            const int t = tb + u * ST_WARPS * RPW;
-            if (brief && base == t0 && t != pnew) kk[u] = k0[u];  // requested before the barrier
-            else if (!brief && t - t0 < staged) kk[u] = *reinterpret_cast<const uint4*>(kv_s + (size_t)(t - t0) * HD + sub * 8);
-            else kk[u] = (t < t1) ? ld_cg_128(kv_row(k_layer, bt_row, t, g, a.G, a.page, a.page_shift, HD) + sub * 8) : make_uint4(0, 0, 0, 0);
-          }
+            for (int u = 0; u < AU; u++) {
+              const int t = tb + u * ST_WARPS * RPW;
+              if (t - t0 < staged) kk[u] = *reinterpret_cast<const uint4*>(kv_s + (size_t)(t - t0) * HD + sub * 8);
+              else kk[u] = (t < t1) ? ld_cg_128(kv_row(k_layer, bt_row, t, g, a.G, a.page, a.page_shift, HD) + sub * 8) : make_uint4(0, 0, 0, 0);
+            }
 #pragma unroll
-          for (int u = 0; u < AU; u++) {
-            const int t = tb + u * ST_WARPS * RPW;
+            for (int u = 0; u < AU; u++) {
+              const int t = tb + u * ST_WARPS * RPW;
 #pragma unroll
-            for (int r = 0; r < NREP; r++) {
-              float d = dot8_acc(0.f, kk[u], qf[r]);
+              for (int r = 0; r < NREP; r++) {
+                float d = dot8_acc(0.f, kk[u], qf[r]);
 #pragma unroll
-              for (int o = LPR / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-              const float s = __fmul_rn(d, a.scale);
-              if (t < t1) {
-                lmax[r] = fmaxf(lmax[r], s);
-                if (sub == (r % LPR)) *(brief ? a.att_s + ((size_t)pair * NREP + r) * ST_SHORT_MAX + t : sc + (size_t)r * a.chunk_cap + (t - t0)) = s;
+                for (int o = LPR / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+                const float s = __fmul_rn(d, a.scale);
+                if (t < t1) {
+                  lmax[r] = fmaxf(lmax[r], s);
+                  if (sub == (r % LPR)) sc[(size_t)r * a.chunk_cap + (t - t0)] = s;
+                }
               }
             }
           }
-        }
-        if (!brief) {
 #pragma unroll
           for (int r = 0; r < NREP; r++) {
             const float mx = warp_max(lmax[r]);
@@ -764,110 +944,7 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
             ml[1] = v;
           }
         }
-      }
-      stamp(2);
-      if constexpr (BRIEF) {
-        // A context that fits: the slices' scores go to the pair's CTAs as they are (an arrival counter of the pair in place of a grid
-        // barrier), and DS of them work out the whole softmax and finish 16 of the head's dimensions each, V read by dimensions instead
-        // of positions: no statistics to combine, no partial outputs to fold, one grid barrier less.  us per step, with the general form
-        // below / so: 8B 3027 / 2850 (547 positions), 3067 / 2873 (900), 3171 / 3011 (2000), 1B 820 / 756 (1000), 822 / 790 (2000), 3B
-        // 1667 / 1548 (600); two rows 8B 3594 / 3331 (900), 1B 904 / 850 (900).
-        st_sync();
-        if (mine) {
-          scored += (unsigned)S;
-          if (tid == 0 && att) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.att_n + pair) : "memory");
-        }
-        if (dims) {
-          if (tid < 2)  // the new position's values
-            reinterpret_cast<uint4*>(vs + (size_t)pnew * 16)[tid] = ld_cg_128(a.qkv + (size_t)b * qkv_dim + (size_t)(a.H + a.G + g) * HD + slice * 16 + tid * 8);
-          if (tid == 0) {
-            unsigned long long w0 = 0;
-            for (unsigned polls = 1;; polls++) {
-              unsigned v;
-              asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.att_n + pair) : "memory");
-              if (v >= scored) break;
-              if ((polls & 255u) == 0) {
-                const unsigned long long now = st_now();
-                if (w0 == 0) w0 = now;
-                else if (now - w0 > a.timeout_ns) { atomicCAS(a.err, 0, 4); break; }  // the results are void; the next barrier ends the launch
-              }
-            }
-            asm volatile("fence.acq_rel.gpu;" ::: "memory");
-          }
-          st_sync();
-          constexpr int UT = ST_SHORT_MAX / ST_THREADS;
-          float e[NREP][UT];
-#pragma unroll
-          for (int r = 0; r < NREP; r++) {
-            float mx = -INFINITY;
-#pragma unroll
-            for (int u = 0; u < UT; u++) {
-              const int t = tid + u * ST_THREADS;
-              e[r][u] = t < T ? __ldcg(a.att_s + ((size_t)pair * NREP + r) * ST_SHORT_MAX + t) : -INFINITY;
-              mx = fmaxf(mx, e[r][u]);
-            }
-            mx = warp_max(mx);
-            if (lane == 0) red[warp][r] = mx;
-          }
-          st_sync();
-          if (tid < NREP) {
-            float mx = red[0][tid];
-            for (int w = 1; w < ST_WARPS; w++) mx = fmaxf(mx, red[w][tid]);
-            s_M[tid] = mx;
-          }
-          st_sync();
-#pragma unroll
-          for (int r = 0; r < NREP; r++) {
-            float ls = 0.f;
-#pragma unroll
-            for (int u = 0; u < UT; u++) {
-              e[r][u] = tid + u * ST_THREADS < T ? jg_xexp2_f32(__fmul_rn(__fsub_rn(e[r][u], s_M[r]), log2e)) : 0.f;
-              ls = __fadd_rn(ls, e[r][u]);
-            }
-            ls = warp_sum(ls);
-            if (lane == 0) red[warp][r] = ls;
-          }
-          st_sync();
-          if (tid < NREP) {
-            float ls = 0.f;
-            for (int w = 0; w < ST_WARPS; w++) ls = __fadd_rn(ls, red[w][tid]);
-            s_rL[tid] = __fdiv_rn(1.0f, ls);
-          }
-          st_sync();
-#pragma unroll
-          for (int r = 0; r < NREP; r++)
-#pragma unroll
-            for (int u = 0; u < UT; u++) {
-              const int t = tid + u * ST_THREADS;
-              if (t < T16) ps[(size_t)r * (T16 + 8) + t] = __float2half_rn(__fmul_rn(e[r][u], s_rL[r]));
-            }
-          asm volatile("cp.async.wait_all;" ::: "memory");
-          st_sync();
-          // out^T [16 dims x heads] = V^T [16 x 16 positions] p^T: a warp takes every 16th run of 16 positions
-          float o4[4] = {0.f, 0.f, 0.f, 0.f};
-          const __half* pw = ps + (size_t)min(lane >> 2, NREP - 1) * (T16 + 8) + (lane & 3) * 2;
-          for (int kk = warp * 16; kk < T16; kk += ST_WARPS * 16) {
-            uint32_t a0, a1, a2, a3;
-            asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(a0), "=r"(a1), "=r"(a2), "=r"(a3)
-                         : "r"(st_smem_u32(vs + (size_t)(kk + ((lane >> 4) << 3) + (lane & 7)) * 16 + (((lane >> 3) & 1) << 3))));
-            const uint32_t b0 = *reinterpret_cast<const uint32_t*>(pw + kk), b1 = *reinterpret_cast<const uint32_t*>(pw + kk + 8);
-            asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                         : "+f"(o4[0]), "+f"(o4[1]), "+f"(o4[2]), "+f"(o4[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-          }
-          st_sync();  // V has been read: its place takes the warps' sums
-          float* ow = reinterpret_cast<float*>(st_smem);  // [warp][4][32]
-#pragma unroll
-          for (int i = 0; i < 4; i++) ow[(warp * 4 + i) * 32 + lane] = o4[i];
-          st_sync();
-          if (tid < 16 * NREP) {
-            const int h = tid >> 4, d = tid & 15, i = (h & 1) + ((d >> 3) << 1), ln = (d & 7) * 4 + (h >> 1);
-            float sum = 0.f;
-            for (int w = 0; w < ST_WARPS; w++) sum += ow[(w * 4 + i) * 32 + ln];
-            a.attn[(size_t)b * a.H * HD + (size_t)(g * NREP + h) * HD + slice * 16 + d] = __float2half_rn(sum);
-          }
-        }
-        stamp(4);
-      } else {
+        stamp(2);
         auto values = [&] {
           if (att && v_at == 0) request(v_layer, 0);
         };
@@ -1114,8 +1191,8 @@ struct jg_step {
 };
 
 typedef void (*StepKernel)(const StepArgs);
-struct StepVariant { int mt, hd, nrep, rs_d, rs_g, rs_h, ni_d, ni_h; StepKernel kern[2]; };  // any context; short ones
-#define ST_VARIANT(MT, HD, NREP, RSD, RSG, RSH, NID, NIH) {MT, HD, NREP, RSD, RSG, RSH, NID, NIH, {jg_step_kernel<MT, HD, NREP, RSD, RSG, RSH, NID, NIH, false>, jg_step_kernel<MT, HD, NREP, RSD, RSG, RSH, NID, NIH, true>}}
+struct StepVariant { int mt, hd, nrep, rs_d, rs_g, rs_h, ni_d, ni_h; StepKernel kern[2]; };  // ST_FITS, ST_BY_POSITION
+#define ST_VARIANT(MT, HD, NREP, RSD, RSG, RSH, NID, NIH) {MT, HD, NREP, RSD, RSG, RSH, NID, NIH, {jg_step_kernel<MT, HD, NREP, RSD, RSG, RSH, NID, NIH, ST_FITS>, jg_step_kernel<MT, HD, NREP, RSD, RSG, RSH, NID, NIH, ST_BY_POSITION>}}
 // Per model shape: the 1-row and the 2-row kernel, each with 64 KB and with 32 KB passes.
 static const StepVariant g_step_variants[] = {
     // Llama-3.1-8B: dim 4096, hidden 14336
@@ -1251,7 +1328,7 @@ JG_API int jg_step_create(jg_dev* dev, jg_kvcache* kv, const jg_step_desc* desc,
   JG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev->ordinal));
   if (!coop) { jg_set_error("step_create: the device does not support cooperative launches"); return JG_ENOTSUP; }
   for (int i = 0; i < 2; i++) {
-    const StepKernel kern = g_step_variants[variant[i]].kern[kv->max_ctx <= short_ctx[i]];
+    const StepKernel kern = g_step_variants[variant[i]].kern[kv->max_ctx > short_ctx[i]];
     JG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[i]));
     int per_sm = 0;
     JG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, ST_THREADS + 32, smem[i]));
@@ -1354,6 +1431,7 @@ JG_API int jg_step_run(jg_step* s, uint64_t tokens, uint64_t pos, uint64_t h, ui
   const StepVariant& v = g_step_variants[s->variant[vi]];
   a.nslot = s->nslot[vi];
   a.slot_bytes = s->slot_bytes[vi];
+  a.short_ctx = s->short_ctx[vi];
   a.kv_offset = s->kv_offset[vi]; a.kv_rows = s->kv_rows[vi];
   a.ring_offset = s->ring_offset[vi];
   // the arrival count starts at zero whatever an earlier launch that ran out of time left behind
@@ -1368,7 +1446,7 @@ JG_API int jg_step_run(jg_step* s, uint64_t tokens, uint64_t pos, uint64_t h, ui
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, v.kern[a.max_ctx <= s->short_ctx[vi]], (const StepArgs)a);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, v.kern[a.max_ctx > a.short_ctx], (const StepArgs)a);
   if (e != cudaSuccess) return jg_cuda_fail(e, "step", __FILE__, __LINE__);
   s->steps_run += (uint64_t)n_steps;
   s->launches_run++;
