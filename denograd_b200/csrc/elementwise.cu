@@ -65,8 +65,8 @@ JG_API int jg_embed(jg_dev* dev, uint64_t out, uint64_t tokens, uint64_t w, uint
 
 // ------------------------------------------------------------------------------------------------ RMSNorm
 // RMSNorm.call (jsgrad/nn/index.ts:586-588): y = half(float(x) * sqrt(1/(mean(x^2)+eps))) * w, one CTA per row.
-__global__ void __launch_bounds__(256) rmsnorm_kernel(__half* __restrict__ y, const __half* __restrict__ x,
-                                                      const __half* __restrict__ w, int dim, float eps, float recip_d, int early) {
+// (Plain pointers: the launch begins beside the one that writes x, which a pointer to const and __restrict__ would promise it does not.)
+__global__ void __launch_bounds__(256) rmsnorm_kernel(__half* y, const __half* x, const __half* w, int dim, float eps, float recip_d, int early) {
   __shared__ float red[8];
   __shared__ float s_rs;
   const int row = blockIdx.x;
