@@ -125,6 +125,7 @@ JG_API int jg_rmsnorm(jg_dev* dev, uint64_t y, uint64_t x, uint64_t w, int32_t r
   // up to 8 rows (8B NF4, one row: 2.52 -> 2.42 ms a token; int8, 8 rows: 2.74 -> 2.65), and to 128 where its weights are many (8B, 32 rows:
   // 4.18 -> 4.11 ms a step, a prompt of 100: 4.70 -> 4.67; 1B prompts of 20 / 45 / 100 with / without: 1.26 / 1.20, 1.34 / 1.24, 1.48 / 1.41).
   const int early = rows <= 8 || (rows <= 128 && dim > 2048);
+  jg_mark_fresh(dev, y, (uint64_t)rows * dim * 2);  // rows that the next call takes as its weights are not to be requested early
   return jg_launch(dev, "rmsnorm", rmsnorm_kernel, dim3(rows), dim3(256), 0, (__half*)y, (const __half*)x, (const __half*)w, dim, eps,
                    (float)(1.0 / (double)dim), early);
 }

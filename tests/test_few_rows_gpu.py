@@ -153,3 +153,20 @@ def test_nf4_wide_matrices_of_every_block(dev, block, M, N, K):
     want = g / (1 + np.exp(-g)) * u
     bound = 8 * ulp * np.abs(want) + 1.2 * np.abs(u) * (eps * mags[0] + ulp * np.abs(g)) + np.abs(g) * eps * mags[1] + 1e-4
     assert (np.abs(y.numpy().astype(np.float64) - want) <= bound).all()
+
+
+@pytest.mark.parametrize("rows,M,K", [(8, 4, 8192), (5, 8, 4096), (128, 3, 4096)])
+def test_normed_rows_as_the_next_calls_weights(dev, rows, M, K):
+    """The launch behind a norm starts beside it: where its weights are the norm's result it waits before it requests them."""
+    rng = np.random.default_rng(rows + K)
+    x, ones, y = rng.standard_normal((M, K)).astype(np.float16), Tensor(np.ones(K, np.float16), device=dev), Tensor.zeros((rows, K), "float16", dev)
+    xt, out = Tensor(x, device=dev), Tensor.zeros((M, rows), "float16", dev)
+    for scale in (1.0, 3.0, -2.0, 0.5):  # a stale matrix would show the sign or the rows of the turn before
+        h = (scale * rng.standard_normal((rows, K))).astype(np.float16)
+        ht = Tensor(h, device=dev)
+        dev.synchronize()
+        dev.call("jg_rmsnorm", y.ptr, ht.ptr, ones.ptr, rows, K, 1e-5)
+        dev.call("jg_linear", out.ptr, xt.ptr, y.ptr, 0, 0, M, rows, K)
+        w = y.numpy().astype(np.float64)
+        want, mag = x.astype(np.float64) @ w.T, np.abs(x.astype(np.float64)) @ np.abs(w).T
+        assert (np.abs(out.numpy() - want) <= 2.0 ** -20 * mag + 2.0 ** -11 * np.abs(want) * 1.01 + 1e-7).all()
