@@ -497,8 +497,14 @@ int jg_gemm_tc(jg_dev* dev, int epi, const void* x, const void* w0, const void* 
                const void* s0, const void* s1);
 bool jg_gemm_tc_fits(int N, int K);
 
-// Fewest rows that go to the tcgen05 kernel when the shape allows it (JG_TC_MIN_M overrides; above 64 rows it is
-// the only kernel).  Measured on the 8B shapes: 3.73 against 3.94 ms per step at 4 rows, 3.85 against 4.16 at 8.
+// Fewest rows that go to the tcgen05 kernel when the shape allows it and skinny.cu does not take them (above 64 rows it is the only
+// kernel; against gemm_small.cu, 8B shapes: 3.73 and 3.94 ms per step at 4 rows, 3.85 and 4.16 at 8).  JG_TC_MIN_M overrides, and leaves
+// the choice to these two.
+static bool tc_min_rows_given() {
+  static int v = -1;
+  if (v < 0) v = getenv("JG_TC_MIN_M") != nullptr;
+  return v != 0;
+}
 static int tc_min_rows() {
   static int v = -1;
   if (v < 0) {
@@ -523,8 +529,8 @@ static bool w8_tc() {  // JG_W8_TC=0: int8 projections of more than 64 rows are 
 }
 
 // int8 weights: from this many rows on the tcgen05 kernel with the conversion inside it is ahead of the mma.sync
-// kernel (8B int8 decode, ms per step, mma.sync / tcgen05: 8 rows 3.79 / 4.82, 16 rows 4.30 / 4.76, 24 rows 5.34 /
-// 4.87, 32 rows 5.73 / 4.96, 48 rows 10.7 / 6.65, 64 rows 11.3 / 6.84).  JG_W8_TC_MIN overrides.
+// kernels (8B int8 decode, ms per step, gemm_small.cu / tcgen05: 24 rows 5.34 / 4.87, 32 rows 5.73 / 4.96, 48 rows 10.7 /
+// 6.65, 64 rows 11.3 / 6.84; 16 rows, where skinny.cu has the single matrices, 2.90 / 4.76).  JG_W8_TC_MIN overrides.
 static int w8_tc_min_rows() {
   static int v = -1;
   if (v < 0) { const char* e = getenv("JG_W8_TC_MIN"); v = e ? atoi(e) : 20; if (v < 3) v = 3; }
@@ -544,7 +550,7 @@ static int dispatch_m(jg_dev* dev, const GemvArgs& a, const char* name) {
   auto skinny = [&](int type) {
     return jg_skinny(dev, type, EPI, a.x, a.w0, a.w1, a.s0, a.s1, EPI == EPI_PARTIAL ? (void*)a.y32 : (void*)a.y, a.residual, a.key, a.M, a.N, a.K, a.row_offset);
   };
-  if (!W8 && !NORM && jg_skinny_fits(dev, SK_F16, EPI, a.M, a.N, a.K)) return skinny(SK_F16);
+  if (!W8 && !NORM && (EPI == EPI_LOGITS || !tc_min_rows_given()) && jg_skinny_fits(dev, SK_F16, EPI, a.M, a.N, a.K)) return skinny(SK_F16);
   if (!W8 && !NORM && EPI != EPI_LOGITS && (a.M > 64 || (a.M >= tc_min_rows() && jg_gemm_tc_fits(a.N, a.K))))
     return jg_gemm_tc(dev, EPI, a.x, a.w0, a.w1, EPI == EPI_PARTIAL ? (void*)a.y32 : (void*)a.y, a.residual, a.M, a.N, a.K, nullptr, nullptr);
   // int8 weights and enough rows: the tcgen05 kernel with the conversion inside it

@@ -1,5 +1,9 @@
 """The projections of a few rows around the weight stream (skinny.cuh) at the edges of their tiles: outputs fewer than CTAs, a row more
 than a tile, one and two tiles to a warp, a second pass; K of one run, and with a last stage that is not full."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -170,3 +174,29 @@ def test_normed_rows_as_the_next_calls_weights(dev, rows, M, K):
         w = y.numpy().astype(np.float64)
         want, mag = x.astype(np.float64) @ w.T, np.abs(x.astype(np.float64)) @ np.abs(w).T
         assert (np.abs(out.numpy() - want) <= 2.0 ** -20 * mag + 2.0 ** -11 * np.abs(want) * 1.01 + 1e-7).all()
+
+
+SWITCH = """
+import numpy as np
+from denograd_b200 import Device
+from denograd_b200.device import Tensor
+dev, rng, M, N, K = Device["CUDA"], np.random.default_rng(3), 4, 14336, 4096
+x, w = rng.standard_normal((M, K)).astype(np.float16), (rng.standard_normal((N, K)) * 0.02).astype(np.float16)
+outs = []
+for pad in (0, 8):
+    xt, wt = (Tensor(np.pad(a, ((0, 0), (0, pad))), device=dev) for a in (x, w))
+    y = Tensor.zeros((M, N), "float32", dev)
+    dev.call("jg_linear_partial", y.ptr, xt.ptr, wt.ptr, 0, M, N, K + pad)
+    outs.append(y.numpy().view(np.uint32))
+print("same" if (outs[0] == outs[1]).all() else "differ")
+"""
+
+
+@pytest.mark.parametrize("rows,want", [("65", "same"), (None, "differ")])
+def test_the_switch_between_the_tensor_core_projections_decides_for_few_rows(rows, want):
+    """Eight columns of zeros more keep a call off every kernel but gemm_small.cu's.  JG_TC_MIN_M beyond the rows sends the call without
+    them there, too (the same bits); unset, they go to the kernel around the weight stream, which adds K in another order."""
+    env = {k: v for k, v in os.environ.items() if k != "JG_TC_MIN_M"}
+    env.update({"JG_TC_MIN_M": rows} if rows else {})
+    r = subprocess.run([sys.executable, "-c", SWITCH], capture_output=True, text=True, env=env, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.stdout.split()[-1:] == [want], (r.stdout, r.stderr[-2000:])
