@@ -88,28 +88,40 @@ WIDTHS = {"8B": {"dim": 4096, "n_heads": 32, "hidden_dim": 14336}, "3B": {"dim":
           "1B": {"dim": 2048, "n_heads": 32, "hidden_dim": 8192}}
 
 
+def logits_of_fed_tokens(llm, prompt, fed):
+    """(ids, logits) of every step behind the prompt, [steps][B], where the given tokens go in whatever is picked."""
+    llm.model.forward(prompt, 0)
+    ids, logits = [], []
+    for i in range(fed.shape[1]):
+        ids.append(np.asarray(llm.model.call_host(np.ascontiguousarray(fed[:, i:i + 1]), prompt.shape[1] + i)).reshape(-1).copy())
+        logits.append(llm.model.last_logits(len(fed)).astype(np.float32))
+    return np.array(ids), np.array(logits)
+
+
 @pytest.mark.parametrize("B", [1, 2])
 @pytest.mark.parametrize("size", list(WIDTHS))
-@pytest.mark.parametrize("max_context,positions,steps,slot_kb", [(1024, 14, 40, "64"), (1024, 1019, 6, None), (2048, 2043, 6, None), (4096, 14, 40, None), (4096, 4000, 6, "64"), (8192, 8100, 3, None)])
-def test_widths_and_contexts_equal_the_launch_per_op_path(monkeypatch, size, B, max_context, positions, steps, slot_kb):
+@pytest.mark.parametrize("max_context,positions,steps,slot_kb,short", [(1024, 14, 40, "64", None), (1024, 1019, 5, None, None), (2048, 2043, 5, None, None), (4096, 14, 40, None, None),
+                                                                             (4096, 14, 40, None, "0"), (4096, 4000, 6, "64", None), (8192, 8100, 3, None, None)])
+def test_widths_and_contexts_equal_the_launch_per_op_path(monkeypatch, size, B, max_context, positions, steps, slot_kb, short):
     """One layer of each width: passes of 2 to 8 rows in slots of 32 and 64 KB, shared by 16 warps by rows and K, batches of passes that do
-    not divide a CTA's; caches whose attention takes the form for short contexts (over two and three runs of 16 positions, and up to the
-    last position that fits) and the general one (one slice, several; K and V of a slice in shared memory both, one after the other, and in part)."""
+    not divide a CTA's; contexts whose attention takes the short form (over two and three runs of 16 positions, up to the last position
+    that fits, and in a cache that does not) and the general one (one slice, several; K and V of a slice in shared memory both, one after the other, and in part)."""
     args = dict(SMALL, n_layers=1, n_kv_heads=8, vocab_size=9001, **WIDTHS[size])
     if slot_kb is not None:
         monkeypatch.setenv("JG_STEP_SLOT_KB", slot_kb)
-    prompt = synth.prompt_tokens(positions, args["vocab_size"], batch=B, seed=80)
+    if short is not None:
+        monkeypatch.setenv("JG_STEP_SHORT", short)
+    prompt, fed = synth.prompt_tokens(positions, args["vocab_size"], batch=B, seed=80), synth.prompt_tokens(steps, args["vocab_size"], batch=B, seed=81)
     got = []
     for kernel in ("1", "0"):
         monkeypatch.setenv("JG_STEP_KERNEL", kernel)
         llm = make("1B", args=args, max_context=max_context, max_batch=2, tied_output=True)
-        got.append(greedy_with_logits(llm, prompt, steps))
+        got.append(logits_of_fed_tokens(llm, prompt, fed))
         assert (llm.model._single_kernel_step(B) is not None) == (kernel == "1")
     (ids, logits), (ids2, logits2) = got
-    for b in range(B):  # up to the first step at which a near-tie was decided otherwise
-        n = steps if (ids[b] == ids2[b]).all() else int(np.argmin(ids[b] == ids2[b]))
-        assert n >= 1
-        assert np.abs(logits[:n, b] - logits2[:n, b]).max() <= 1e-2  # summation order only
+    assert np.abs(logits - logits2).max() <= 1e-2  # summation order only
+    top = np.sort(logits2, axis=2)
+    assert ((ids == ids2) | (top[..., -1] - top[..., -2] <= 2e-2)).all()  # another pick only at a near-tie
 
 
 @pytest.mark.parametrize("slots", ["2", "6"])
@@ -146,12 +158,7 @@ def test_form_of_attention_follows_the_position(monkeypatch, size, B, limit, max
     for kernel in ("1", "0"):
         monkeypatch.setenv("JG_STEP_KERNEL", kernel)
         llm = make("1B", args=args, max_context=max_context, max_batch=2, tied_output=True)
-        llm.model.forward(prompt, 0)
-        rows, ids = [], []
-        for i in range(steps):
-            ids.append(llm.model.call_host(fed[:, i:i + 1], positions + i))
-            rows.append(llm.model.last_logits(B).copy())
-        got.append(np.array(rows))
+        got.append(logits_of_fed_tokens(llm, prompt, fed)[1])
         assert (llm.model._single_kernel_step(B) is not None) == (kernel == "1")
         if kernel == "1":
             run = llm.model.decode_loop(fed[:, 0], positions, steps)
