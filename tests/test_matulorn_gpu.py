@@ -365,6 +365,39 @@ def test_first_tokens_of_a_sequence():
             assert error(run(m, toks, cuts), want) < F32_TOL
 
 
+def test_taps_of_the_delta_rule_need_no_alignment():
+    """One token at a time, four taps: those of a channel come in one load where they lie on 16 bytes, one by one elsewhere: the same bits."""
+    import ctypes as C
+
+    from denograd_b200 import Device, ffi
+    from denograd_b200.device import Tensor
+
+    dev, rng = Device["CUDA"], np.random.default_rng(5)
+    R, H, G, d, v, taps, ld = 2, 4, 2, 20, 28, 4, 4 * 28 * 2 + 2 * 2 * 20 + 8
+    ch = 2 * G * d + H * v
+    par = {n: (rng.standard_normal(k) * 0.3).astype(np.float32) for n, k in (("a_log", H), ("dt_bias", H), ("norm_w", v), ("conv", ch * taps))}
+    rows = [rng.standard_normal((R, ld)).astype(np.float32) for _ in range(6)]
+    t = {n: Tensor(x, device=dev) for n, x in par.items()}
+    outs = []
+    for off in (0, 1, 2):
+        conv = Tensor(np.concatenate([np.zeros(off, np.float32), par["conv"]]), device=dev)
+        state, tail = Tensor.zeros((R, H, v, d), "float32", dev), Tensor.zeros((R, taps, ch), "float32", dev)
+        n = C.c_uint64()
+        ffi.call("jg_delta_scratch_floats", C.byref(ffi.DeltaDesc(0, H, G, d, v, taps)), R, C.byref(n))
+        scratch, out, seq = Tensor.zeros((max(n.value, 4),), "float32", dev), Tensor.zeros((R, H * v), "float32", dev), Tensor(np.arange(R, dtype=np.int32), device=dev)
+        for i, x in enumerate(rows):
+            xt, pos = Tensor(x, device=dev), Tensor(np.full(R, i, np.int32), device=dev)
+            desc = ffi.DeltaDesc(0, H, G, d, v, taps, ld, H * v, 1e-5, 0, xt.ptr, conv.ptr + 4 * off, t["a_log"].ptr, t["dt_bias"].ptr, t["norm_w"].ptr, state.ptr,
+                                 tail.ptr, scratch.ptr, out.ptr)
+            dev.call("jg_delta_rule", C.byref(ffi.Batch(R, 1, pos.ptr, seq.ptr, i, 0)), C.byref(desc))
+            outs.append(out.numpy())
+    n = len(rows)
+    assert np.isfinite(outs).all() and np.abs(outs[n - 1]).max() > 0
+    for i in range(n):
+        for k in (1, 2):
+            assert (outs[i].view(np.uint32) == outs[k * n + i].view(np.uint32)).all()
+
+
 # ------------------------------------------------------------------------------------------------ drivers
 def driver(cfg, params, dtype="float32", **kw):
     from denograd_b200.matulorn import Matulorn
