@@ -4,6 +4,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "quant.cuh"
 #include "stream.cuh"
 #include "transcendental.cuh"
 
@@ -358,15 +359,10 @@ JG_API int jg_dequant_i8_f16(jg_dev* dev, uint64_t dst, uint64_t w, uint64_t sca
 // NF4Linear's dequantised matrix (jsgrad/models/llama3.ts:88-94): element i of the flattened [out][in] matrix is
 // half(CODE[code_i] * scale[i / block]) with code_2j in the high nibble of byte j and code_2j+1 in the low one, the 16
 // code values rounded to fp16 first (:81).  One thread turns 16 packed bytes into 32 halves.
-__constant__ float c_nf4_code[16] = {-1.0f, -0.6961928009986877f, -0.5250730514526367f, -0.39491748809814453f,
-                                     -0.28444138169288635f, -0.18477343022823334f, -0.09105003625154495f, 0.0f,
-                                     0.07958029955625534f, 0.16093020141124725f, 0.24611230194568634f,
-                                     0.33791524171829224f, 0.44070982933044434f, 0.5626170039176941f,
-                                     0.7229568362236023f, 1.0f};
 __global__ void dequant_nf4_f16_kernel(__half* __restrict__ dst, const uint8_t* __restrict__ w, const __half* __restrict__ scale,
                                        long long n32, int block) {
   __shared__ __half code[16];
-  if (threadIdx.x < 16) code[threadIdx.x] = __float2half_rn(c_nf4_code[threadIdx.x]);
+  if (threadIdx.x < 16) code[threadIdx.x] = __float2half_rn(c_nf4[threadIdx.x]);
   pdl_launch();
   pdl_wait();
   __syncthreads();

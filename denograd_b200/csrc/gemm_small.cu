@@ -1,5 +1,6 @@
-// Weight-streaming projection for up to 64 activation rows (batched decode, short prefill chunks) — int8 weights of more rows
-// than skinny.cu takes, shapes off the other kernels' tile grids, and the logits of 17 rows and more with their argmax keys:
+// Weight-streaming projection for up to 64 activation rows (batched decode, short prefill chunks) — int8 weights that skinny.cu does not
+// take (gate and up of up to 4 rows, or small ones, and everything of 17 to 19 rows), shapes off the other kernels' tile grids, and the
+// logits with their argmax keys (fp16 from 17 rows on, int8 from 9):
 //   y[m][n] = epilogue( sum_k x[m][k] * W[n][k] ),  fp16 operands, fp32 accumulation on the tensor cores.
 //
 // At these row counts the projection is still bound by reading W once from HBM, but the multiply-accumulate work no
@@ -21,7 +22,7 @@
 // LOGITS (store + per-row (value, lowest index) key, jsgrad/tensor.ts:2314-2320).
 #include <stdlib.h>
 
-#include "common.cuh"
+#include "quant.cuh"
 #include "skinny_plan.h"
 #include "transcendental.cuh"
 
@@ -46,23 +47,6 @@ constexpr int GS_WARPS = 8;
 // bytes of a padded row: rows g and g+1 land 4 x 16 B apart modulo 128 B; int8 weights read 32 B per lane, rows 16 B apart
 template <int MT, int KS, bool W8>
 constexpr int gs_row_bytes() { return gs_k_tile(MT, KS, W8) * 2 + (W8 ? 16 : 64); }
-
-// int8 x16 (one uint4) -> eight half2 words of half(q) * s in k order, each product rounded once.  Bytes become halves
-// exactly through the 0x6400 (1024.0) exponent trick.
-__device__ __forceinline__ void dequant16_h2(const uint4& raw, __half2 s2, uint32_t (&out)[8]) {
-  const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
-  const __half2 bias = __floats2half2_rn(1152.0f, 1152.0f);  // 1024 + 128
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const uint32_t v = words[i] ^ 0x80808080u;                  // signed -> offset-binary
-    uint32_t lo = __byte_perm(v, 0x64646464u, 0x4140);          // bytes 0,1 -> halves 0x64b0, 0x64b1
-    uint32_t hi = __byte_perm(v, 0x64646464u, 0x4342);          // bytes 2,3
-    const __half2 a = __hmul2_rn(__hsub2(*reinterpret_cast<__half2*>(&lo), bias), s2);
-    const __half2 b = __hmul2_rn(__hsub2(*reinterpret_cast<__half2*>(&hi), bias), s2);
-    out[2 * i] = *reinterpret_cast<const uint32_t*>(&a);
-    out[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&b);
-  }
-}
 
 __device__ __forceinline__ void cp_async_16(void* smem, const void* gmem) {
   const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
@@ -184,7 +168,7 @@ __global__ void __launch_bounds__(GS_THREADS, (MT <= 32 ? 2 : 1)) gemm_small_ker
         } else {
           uint32_t da[NW][8], db[NW][8];  // the lane's 16 weights of rows g and g+8 as fp16 pairs
 #pragma unroll
-          for (int w = 0; w < NW; w++) { dequant16_h2(fa[w][b], sa[w], da[w]); dequant16_h2(fb[w][b], sb[w], db[w]); }
+          for (int w = 0; w < NW; w++) { w8_to_half2(fa[w][b], sa[w], da[w]); w8_to_half2(fb[w][b], sb[w], db[w]); }
 #pragma unroll
           for (int j = 0; j < NT; j++) {
             const uint4* xp = reinterpret_cast<const uint4*>(xs + (size_t)(j * 8 + g) * ROWB + koff);

@@ -29,6 +29,7 @@
 
 #include "common.cuh"
 #include "gemm_pair.cuh"
+#include "quant.cuh"
 #include "transcendental.cuh"
 
 enum { TC_STORE = 0, TC_RESIDUAL = 1, TC_SWIGLU = 2, TC_PARTIAL = 4 };
@@ -82,22 +83,6 @@ struct TcCfg {
   // split-K peers park their accumulators ([column][128 lanes] fp32 each) in rank 0's pipeline buffers
   static constexpr int MAX_KS = 1 + (int)(((size_t)STAGES * STAGE_BYTES) / ((size_t)NCOL * TC_BM * 4));
 };
-
-// int8 x16 -> sixteen halves of half(q) * s (eight half2 registers in k order), each product rounded once
-__device__ __forceinline__ void tc_dequant16(const uint4& raw, __half2 s2, uint32_t (&out)[8]) {
-  const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
-  const __half2 bias = __floats2half2_rn(1152.0f, 1152.0f);  // 1024 + 128
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const uint32_t v = words[i] ^ 0x80808080u;          // signed -> offset-binary
-    uint32_t lo = __byte_perm(v, 0x64646464u, 0x4140);  // bytes 0,1 -> halves 1024 + b
-    uint32_t hi = __byte_perm(v, 0x64646464u, 0x4342);  // bytes 2,3
-    const __half2 p = __hmul2_rn(__hsub2(*reinterpret_cast<__half2*>(&lo), bias), s2);
-    const __half2 q = __hmul2_rn(__hsub2(*reinterpret_cast<__half2*>(&hi), bias), s2);
-    out[2 * i] = *reinterpret_cast<const uint32_t*>(&p);
-    out[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&q);
-  }
-}
 
 template <int TN, int EPI, bool W8 = false, bool HALF = false>
 __global__ void __launch_bounds__(TcCfg<TN, EPI, W8, HALF>::THREADS, HALF ? 2 : 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w0,
@@ -223,7 +208,7 @@ __global__ void __launch_bounds__(TcCfg<TN, EPI, W8, HALF>::THREADS, HALF ? 2 : 
 #pragma unroll
         for (int j = 0; j < 4; j++) {  // 16 weights -> two 16-byte chunks (2j, 2j + 1) of the row
           uint32_t d[8];
-          tc_dequant16(src[j], sc, d);
+          w8_to_half2(src[j], sc, d);
           *reinterpret_cast<uint4*>(dst + (((2 * j) ^ (r & 7)) << 4)) = make_uint4(d[0], d[1], d[2], d[3]);
           *reinterpret_cast<uint4*>(dst + (((2 * j + 1) ^ (r & 7)) << 4)) = make_uint4(d[4], d[5], d[6], d[7]);
         }

@@ -35,6 +35,7 @@
 //                       reads only 1/cluster of the entries; the first cluster also writes the new residual stream
 #include "common.cuh"
 #include "peer.cuh"
+#include "quant.cuh"
 #include "skinny_plan.h"
 #include "transcendental.cuh"
 
@@ -63,20 +64,14 @@ constexpr int GEMV_THREADS = 256;
 constexpr int GEMV_WARPS = GEMV_THREADS / 32;
 
 // int8 x16 (one uint4) -> sixteen fp32 values of half(q) * s, the fp16 product rounded once (Int8Linear:
-// jsgrad/models/llama3.ts:35).  Bytes are turned into halves exactly through the 0x6400 (1024.0) exponent trick.
+// jsgrad/models/llama3.ts:35).
 __device__ __forceinline__ void dequant16(const uint4& raw, __half2 s2, float (&w)[16]) {
-  const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
-  const __half2 bias = __floats2half2_rn(1152.0f, 1152.0f);  // 1024 + 128
+  uint32_t h[8];
+  w8_to_half2(raw, s2, h);
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    uint32_t v = words[i] ^ 0x80808080u;                  // signed -> offset-binary
-    uint32_t lo = __byte_perm(v, 0x64646464u, 0x4140);    // bytes 0,1 -> halves 0x64b0, 0x64b1
-    uint32_t hi = __byte_perm(v, 0x64646464u, 0x4342);    // bytes 2,3
-    __half2 a = __hsub2(*reinterpret_cast<__half2*>(&lo), bias);  // exact: integers below 2048
-    __half2 b = __hsub2(*reinterpret_cast<__half2*>(&hi), bias);
-    float2 fa = __half22float2(__hmul2_rn(a, s2));
-    float2 fb = __half22float2(__hmul2_rn(b, s2));
-    w[i * 4 + 0] = fa.x; w[i * 4 + 1] = fa.y; w[i * 4 + 2] = fb.x; w[i * 4 + 3] = fb.y;
+  for (int i = 0; i < 8; i++) {
+    const float2 f = h2_to_f2(h[i]);
+    w[2 * i] = f.x; w[2 * i + 1] = f.y;
   }
 }
 

@@ -32,12 +32,6 @@ struct Nf4Args {
 
 constexpr int N4_THREADS = 256, N4_WARPS = 8;
 
-__constant__ float c_n4_code[16] = {-1.0f, -0.6961928009986877f, -0.5250730514526367f, -0.39491748809814453f,
-                                    -0.28444138169288635f, -0.18477343022823334f, -0.09105003625154495f, 0.0f,
-                                    0.07958029955625534f, 0.16093020141124725f, 0.24611230194568634f,
-                                    0.33791524171829224f, 0.44070982933044434f, 0.5626170039176941f,
-                                    0.7229568362236023f, 1.0f};
-
 __device__ __forceinline__ void n4_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
@@ -59,7 +53,7 @@ __global__ void __launch_bounds__(N4_THREADS, 2) jg_matvec_nf4_kernel(const Nf4A
   const size_t row_bytes = (size_t)K / 2, row_blocks = (size_t)(K >> a.block_shift);
   pdl_launch();
   for (int b = warp; b < 256; b += N4_WARPS) {
-    const __half2 h = __halves2half2(__float2half_rn(c_n4_code[b >> 4]), __float2half_rn(c_n4_code[b & 15]));
+    const __half2 h = __halves2half2(__float2half_rn(c_nf4[b >> 4]), __float2half_rn(c_nf4[b & 15]));
     lut[b * 32 + lane] = *reinterpret_cast<const uint32_t*>(&h);
   }
   if (a.late) pdl_wait();  // the weights were written by a launch that may still be running

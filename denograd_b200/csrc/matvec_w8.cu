@@ -17,7 +17,7 @@
 //     that meet at a barrier of their own once per tile and add their sums in a fixed order.
 // Tiles are dealt to the warp groups as contiguous runs.
 // Epilogues: STORE, RESIDUAL, SWIGLU (two matrices), LOGITS (+ greedy key), PARTIAL (fp32), as in gemv.cu.
-#include "common.cuh"
+#include "quant.cuh"
 #include "transcendental.cuh"
 
 enum { W8_STORE = 0, W8_RESIDUAL = 1, W8_SWIGLU = 2, W8_LOGITS = 3, W8_PARTIAL = 4 };
@@ -41,21 +41,6 @@ struct MatvecW8Args {
 
 constexpr int W8_THREADS = 256;
 constexpr int W8_WARPS = 8;
-
-__device__ __forceinline__ void w8_dequant16(const uint4& raw, __half2 s2, uint32_t (&out)[8]) {
-  const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
-  const __half2 bias = __floats2half2_rn(1152.0f, 1152.0f);  // 1024 + 128
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const uint32_t v = words[i] ^ 0x80808080u;                  // signed -> offset-binary
-    uint32_t lo = __byte_perm(v, 0x64646464u, 0x4140);          // bytes 0,1 -> halves 1024 + b
-    uint32_t hi = __byte_perm(v, 0x64646464u, 0x4342);          // bytes 2,3
-    const __half2 a = __hmul2_rn(__hsub2(*reinterpret_cast<__half2*>(&lo), bias), s2);  // exact integer, one rounding
-    const __half2 b = __hmul2_rn(__hsub2(*reinterpret_cast<__half2*>(&hi), bias), s2);
-    out[2 * i] = *reinterpret_cast<const uint32_t*>(&a);
-    out[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&b);
-  }
-}
 
 __device__ __forceinline__ void w8_mma(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
   // rows 8..15 of the activation tile are zero (a1 = a3 = 0)
@@ -213,7 +198,7 @@ __global__ void __launch_bounds__(W8_THREADS, 2) jg_matvec_w8_kernel(const Matve
 #pragma unroll
         for (int w = 0; w < NW; w++) {
           uint32_t d[8];
-          w8_dequant16(cur[w], sc[w], d);
+          w8_to_half2(cur[w], sc[w], d);
 #pragma unroll
           for (int q = 0; q < 4; q++) w8_mma(acc[w][q & 1], xw[2 * q], xw[2 * q + 1], d[2 * q], d[2 * q + 1]);
         }

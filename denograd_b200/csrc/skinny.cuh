@@ -3,13 +3,13 @@
 // Bound by the weight stream and, for small matrices, by a launch's fixed latencies, so the kernel is built around the stream.  One
 // CTA per SM has an equal run of outputs (whole weight rows, N / SMs of them, not rounded to a tile) and walks K once for all of them:
 // a producer warp keeps a ring of stages in flight, each a TMA box of the run's rows x a few 128-byte runs of K (one instruction per
-// matrix; a bulk copy per row piece moved 512 bytes in 75 cycles and no more) with the same k of the activations beside it.  16 warps
-// share a stage: warp (tile, k) has one 128-byte run of one or two 16-row tiles, whose 16-byte chunks in shared memory *are* A
+// matrix; a bulk copy per row piece moved 512 bytes in 75 cycles and no more) with the same k of the activations beside it.  Up to 16
+// warps share a stage: warp (tile, k) has one 128-byte run of one or two 16-row tiles, whose 16-byte chunks in shared memory *are* A
 // fragments of mma.sync.m16n8k16 (the k order inside a run may be permuted as long as the activations' is, too).  int8 has the sums of
 // gemm_small.cu to the bit: a warp has one of its K slices, and a stage's box one or two runs of each slice.  The warps run free
 // of each other through the ring (an mbarrier per stage in each direction) and meet once, at the end, to add the sums of the warps
 // that share a tile, in a fixed order.  The first stages' weights are requested before the dependency wait: up to 28 MB in all, most
-// small matrices whole.
+// small matrices whole.  Activations travel with each stage.
 //
 // us per launch, weights from HBM, back to back, the kernels used before / this one: 8B int8, 8 rows qkv 9.4 / 7.9, wo 7.6 / 6.7, gate
 // and up 24.8 / 26.3 (between its neighbours in a step it gains, see skinny.cu), down 19.8 / 13.9, logits 97.8 / 90.4; 16 rows 14.4 /
@@ -24,7 +24,7 @@
 // Every mbarrier wait is bounded: a warp whose wait gives up records it and goes on without waiting (the results are void, the host
 // reports JG_ETIMEDOUT at the next synchronisation); the producer stops requesting and lets the copies in flight land.
 #pragma once
-#include "common.cuh"
+#include "quant.cuh"
 #include "skinny_plan.h"
 #include "tcgen05.cuh"
 
@@ -50,10 +50,6 @@ template <int TYPE, int NT, int TP> struct SkCfg {
 };
 
 #ifdef __CUDACC__
-__constant__ float c_sk_nf4[16] = {-1.0f, -0.6961928009986877f, -0.5250730514526367f, -0.39491748809814453f, -0.28444138169288635f, -0.18477343022823334f,
-                                   -0.09105003625154495f, 0.0f, 0.07958029955625534f, 0.16093020141124725f, 0.24611230194568634f, 0.33791524171829224f,
-                                   0.44070982933044434f, 0.5626170039176941f, 0.7229568362236023f, 1.0f};
-
 template <bool BF>
 __device__ __forceinline__ void sk_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   if (BF)
@@ -72,20 +68,6 @@ __device__ __forceinline__ __half sk_lds_half(uint32_t p) {
   uint16_t v;
   asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(p) : "memory");
   return __ushort_as_half(v);
-}
-// int8 x16 -> eight half2 words of half(q) * s in k order, each product rounded once (bytes become halves through 1024 + b)
-__device__ __forceinline__ void sk_dequant16(const uint4& raw, __half2 s2, uint32_t (&out)[8]) {
-  const uint32_t words[4] = {raw.x, raw.y, raw.z, raw.w};
-  const __half2 bias = __floats2half2_rn(1152.0f, 1152.0f);  // 1024 + 128
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const uint32_t v = words[i] ^ 0x80808080u;
-    uint32_t lo = __byte_perm(v, 0x64646464u, 0x4140), hi = __byte_perm(v, 0x64646464u, 0x4342);
-    const __half2 a = __hmul2_rn(__hsub2(*reinterpret_cast<__half2*>(&lo), bias), s2);
-    const __half2 b = __hmul2_rn(__hsub2(*reinterpret_cast<__half2*>(&hi), bias), s2);
-    out[2 * i] = *reinterpret_cast<const uint32_t*>(&a);
-    out[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&b);
-  }
 }
 
 // What this CTA alone will read, asked into L2.
@@ -178,7 +160,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
   if (TYPE == SK_NF4) {  // [byte][lane]: half2(code of the high nibble, of the low one)
     uint32_t* table = reinterpret_cast<uint32_t*>(sk_raw + (lut - raw));
     for (int b = warp; b < 256; b += SK_WARPS) {
-      const __half2 h = __halves2half2(__float2half_rn(c_sk_nf4[b >> 4]), __float2half_rn(c_sk_nf4[b & 15]));
+      const __half2 h = __halves2half2(__float2half_rn(c_nf4[b >> 4]), __float2half_rn(c_nf4[b & 15]));
       table[b * 32 + lane] = *reinterpret_cast<const uint32_t*>(&h);
     }
   }
@@ -275,8 +257,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
               }
             } else if (W8) {
               uint32_t da[8], db[8];
-              sk_dequant16(va[p], s2[p][0], da);
-              sk_dequant16(vb[p], s2[p][1], db);
+              w8_to_half2(va[p], s2[p][0], da);
+              w8_to_half2(vb[p], s2[p][1], db);
 #pragma unroll
               for (int n = 0; n < NT; n++)
 #pragma unroll
