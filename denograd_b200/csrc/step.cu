@@ -103,10 +103,11 @@ struct StepArgs {
 
 constexpr int ST_MAX_SLOTS = 6;
 // Forms of attention that a kernel has: the short contexts' alone (whatever the cache holds takes it), or both, chosen by the rows' positions.
-// A cache that fits has a kernel of its own, since both forms in the registers of one cost up to 5 % (us per step of one row at position
-// 67, that kernel / with both: 1B 730 / 767, 3B 1529 / 1533, 8B 2881 / 2862, two rows of 8B 3199 / 3341; the general form at 4000 alone / with
-// both: 1B 866 / 878, 3B 1817 / 1827, 8B 3185 / 3203).  (The short form as a function of its own: 5 us more a layer.)  In a cache of 8192
-// one row at 67 / 547 positions takes, with the general form / so: 1B 815 / 767, 830 / 780; 3B 1643 / 1533, 1675 / 1554; 8B 2961 / 2862, 3013 / 2927.
+// A cache that fits has a kernel of its own, since both forms in the registers of one cost up to 6 % (us per step of one row at position
+// 67, that kernel / with both: 1B 726 / 769, 3B 1542 / 1555, 8B 2871 / 2879, two rows of 8B 3262 / 3413; the general form at 4000
+// positions, alone / with both: 1B 864 / 875, 3B 1834 / 1852, 8B 3199 / 3216, two rows of 8B 3998 / 4064).  (The short form as a function
+// that is called: 5 us more a layer.)  In a cache of 8192 one row at 67 / 547 positions takes, with the general form / so: 1B 810 / 769,
+// 828 / 779; 3B 1663 / 1555, 1690 / 1574; 8B 2954 / 2879, 3034 / 2952.
 enum { ST_FITS = 0, ST_BY_POSITION = 1 };
 
 __device__ __forceinline__ unsigned long long st_now() {
@@ -208,7 +209,6 @@ struct StepStream {
   const unsigned char* src1;
   uint32_t slot;           // ring slot the next pass goes to
   size_t stride;           // bytes from one pass of this CTA to its next
-  unsigned sent;           // passes requested
 };
 
 // Position (step, layer, phase) -> matrix, this CTA's rows, passes (0 when the CTA has no rows in the phase).
@@ -263,7 +263,6 @@ __device__ __forceinline__ void st_stream_issue(StepStream& st, const StepArgs& 
     st.src1 += st.stride;
   }
   st.src0 += st.stride;
-  st.sent++;
   st.slot = (st.slot + 1 == (uint32_t)a.nslot) ? 0u : st.slot + 1;
   if (--st.left == 0) st_stream_next_phase<RS_D, RS_G, RS_H>(st, a, qkv_dim);
 }
@@ -350,17 +349,33 @@ __device__ __forceinline__ void st_project(int N, int KC, const __half* xs, int 
   }
 }
 
-// What a CTA brings to the attention of one layer (its slice of one (row, kv head) pair), and takes on from it.
-struct StShort {
-  int l, pair, slice, b, g, T, S, t0, t1;
-  bool mine, att;
-  int pg0, pg1;  // pages of this thread's first two rows
-  unsigned gen, scored;
-  bool prof;
-  unsigned long long t_prev;
-  float (*red)[4];  // scratch of the CTA: a sum or maximum per warp and head, per head
-  float *s_M, *s_rL;
+// A CTA's share of attention: context slice `slice` of a (row, kv head) pair.
+struct StShare {
+  int pair, slice, b, g, T, S, t0, t1;  // T positions in S slices, [t0, t1) of them here
+  bool mine, att;                       // the pair has a CTA here, its slice has positions
 };
+template <int MT>
+__device__ __forceinline__ StShare st_share(const StepArgs& a, const int (&posv)[MT], int slices) {  // slices: the most a pair can have (the scratch's stride)
+  StShare s;
+  const int bid = blockIdx.x;
+  s.mine = bid < a.M * a.G * slices;
+  s.pair = s.mine ? bid / slices : 0;
+  s.slice = s.mine ? bid % slices : 0;
+  s.b = s.pair / a.G;
+  s.g = s.pair % a.G;
+  int pb = posv[0];
+#pragma unroll
+  for (int m = 1; m < MT; m++) pb = (s.b == m) ? posv[m] : pb;
+  s.T = min(max(pb + 1, 1), a.max_ctx);
+  // slices of this pair: about a.slice_len positions each (a short context keeps few CTAs busy and the exchanges of
+  // statistics and partials short), never more positions than a slice's scores have room for
+  s.S = min(slices, max((s.T + a.slice_len - 1) / a.slice_len, (s.T + a.chunk_cap - 1) / a.chunk_cap));
+  s.att = s.mine && s.slice < s.S;
+  const int chunk = (s.T + s.S - 1) / s.S;
+  s.t0 = s.slice * chunk;
+  s.t1 = s.att ? min(s.T, s.t0 + chunk) : s.t0;
+  return s;
+}
 __device__ __forceinline__ void st_stamp(const StepArgs& a, bool prof, unsigned long long& t_prev, int i) {
   if (prof) {
     const unsigned long long t = st_now();
@@ -371,20 +386,19 @@ __device__ __forceinline__ void st_stamp(const StepArgs& a, bool prof, unsigned 
 
 // Attention of a short context, from the finished qkv projection to the barrier ahead of the output projection: false = a wait ran out.
 template <int HD, int NREP>
-__device__ __forceinline__ bool st_attend_short(const StepArgs& a, StShort& c) {
+__device__ __forceinline__ bool st_attend_short(const StepArgs& a, const StShare c, int l, const int (&pg0)[2], unsigned& gen, unsigned& scored, float (*red)[4], float* s_M, float* s_rL,
+                                                bool prof, unsigned long long& t_prev) {
   constexpr int LPR = HD / 8, RPW = 32 / LPR, AU = 2, ROWS_IT = ST_WARPS * RPW * AU;  // lanes of a K row, rows of a warp's pass, passes in flight
   constexpr int DS = HD / 16;  // CTAs of a pair that share the head's dimensions
   extern __shared__ __align__(16) unsigned char st_smem[];
-  float (*red)[4] = c.red;
-  float *s_M = c.s_M, *s_rL = c.s_rL;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = lane % LPR, rgrp = lane / LPR;
   const int pair = c.pair, slice = c.slice, b = c.b, g = c.g, T = c.T, S = c.S, t0 = c.t0, t1 = c.t1, pnew = T - 1;
   const bool mine = c.mine, att = c.att, dims = mine && slice < DS;
   const float log2e = 1.4426950408889634f;
   const int qkv_dim = (a.H + 2 * a.G) * HD, T16 = (T + 15) & ~15;
   const int32_t* bt_row = a.block_table + (size_t)b * a.max_pages_per_seq;
-  __half* k_layer = a.k_pool + (size_t)c.l * a.layer_elems;
-  __half* v_layer = a.v_pool + (size_t)c.l * a.layer_elems;
+  __half* k_layer = a.k_pool + (size_t)l * a.layer_elems;
+  __half* v_layer = a.v_pool + (size_t)l * a.layer_elems;
   __half* vs = reinterpret_cast<__half*>(st_smem);  // [T16][16], behind it the probabilities [NREP][T16 + 8]
   __half* ps = vs + (size_t)T16 * 16;
   // the first K rows are requested now, ahead of the barrier: cached rows do not depend on this step's projection (the new position's row
@@ -394,10 +408,10 @@ __device__ __forceinline__ bool st_attend_short(const StepArgs& a, StShort& c) {
   for (int u = 0; u < AU; u++) {
     const int t = t0 + warp * RPW + rgrp + u * ST_WARPS * RPW;
     const bool ld = att && t < t1 && t != pnew;
-    const size_t off = (((size_t)(u == 0 ? c.pg0 : c.pg1) * a.G + g) * a.page + (t & (a.page - 1))) * HD + sub * 8;
+    const size_t off = (((size_t)pg0[u] * a.G + g) * a.page + (t & (a.page - 1))) * HD + sub * 8;
     k0[u] = ld ? ld_cg_128(k_layer + off) : make_uint4(0, 0, 0, 0);
   }
-  st_stamp(a, c.prof, c.t_prev, 0);
+  st_stamp(a, prof, t_prev, 0);
   auto rows = [&] {  // this CTA's 16 dimensions of every cached row, where the projection's last activations were (all warps have read them)
     if (dims)
       for (int i = tid; i < 2 * T16; i += ST_THREADS) {
@@ -408,9 +422,9 @@ __device__ __forceinline__ bool st_attend_short(const StepArgs& a, StShort& c) {
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(st_smem_u32(vs + (size_t)i * 8)), "l"(src), "r"(ld ? 16 : 0) : "memory");
       }
   };
-  if (!st_grid_sync(a, c.gen, rows)) return false;
-  st_stamp(a, c.prof, c.t_prev, 1);
-  if (c.l == 0 && blockIdx.x == 0 && tid < a.M) a.key[tid] = 0ull;  // every CTA has read the previous step's key by now
+  if (!st_grid_sync(a, gen, rows)) return false;
+  st_stamp(a, prof, t_prev, 1);
+  if (l == 0 && blockIdx.x == 0 && tid < a.M) a.key[tid] = 0ull;  // every CTA has read the previous step's key by now
   if (att) {
     const __half* xrow = a.qkv + (size_t)b * qkv_dim;
     const uint4 traw = ld_128(a.table + ((size_t)min(pnew, a.table_rows - 1) * (HD / 2) + (size_t)sub * 4) * 2);
@@ -448,7 +462,7 @@ __device__ __forceinline__ bool st_attend_short(const StepArgs& a, StShort& c) {
       }
     }
   }
-  st_stamp(a, c.prof, c.t_prev, 2);
+  st_stamp(a, prof, t_prev, 2);
   // A context that fits: the slices' scores go to the pair's CTAs as they are (an arrival counter of the pair in place of a grid
   // barrier), and DS of them work out the whole softmax and finish 16 of the head's dimensions each, V read by dimensions instead
   // of positions: no statistics to combine, no partial outputs to fold, one grid barrier less.  us per step in
@@ -456,7 +470,7 @@ __device__ __forceinline__ bool st_attend_short(const StepArgs& a, StShort& c) {
   // 1667 / 1548 (600); two rows 8B 3594 / 3331 (900), 1B 904 / 850 (900).
   st_sync();
   if (mine) {
-    c.scored += (unsigned)S;
+    scored += (unsigned)S;
     if (tid == 0 && att) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.att_n + pair) : "memory");
   }
   if (dims) {
@@ -467,7 +481,7 @@ __device__ __forceinline__ bool st_attend_short(const StepArgs& a, StShort& c) {
       for (unsigned polls = 1;; polls++) {
         unsigned v;
         asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.att_n + pair) : "memory");
-        if (v >= c.scored) break;
+        if (v >= scored) break;
         if ((polls & 255u) == 0) {
           const unsigned long long now = st_now();
           if (w0 == 0) w0 = now;
@@ -548,7 +562,7 @@ __device__ __forceinline__ bool st_attend_short(const StepArgs& a, StShort& c) {
       a.attn[(size_t)b * a.H * HD + (size_t)(g * NREP + h) * HD + slice * 16 + d] = __float2half_rn(sum);
     }
   }
-  st_stamp(a, c.prof, c.t_prev, 4);
+  st_stamp(a, prof, t_prev, 4);
   return true;
 }
 
@@ -601,6 +615,7 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
   rg.slot = 0; rg.parity = 0;
   if (warp == ST_WARPS) {
     StepStream st;
+    int sent = 0;  // slots that hold a pass
     if (lane == 0) {
       s_quit = 0;
       for (int i = 0; i < a.nslot; i++) {
@@ -609,10 +624,10 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
       }
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      st.step = 0; st.layer = 0; st.phase = 0; st.slot = 0; st.sent = 0;
+      st.step = 0; st.layer = 0; st.phase = 0; st.slot = 0;
       st_stream_enter<RS_D, RS_G, RS_H>(st, a, qkv_dim);
       if (st.left <= 0) st_stream_next_phase<RS_D, RS_G, RS_H>(st, a, qkv_dim);
-      for (int i = 0; i < a.nslot; i++) st_stream_issue<RS_D, RS_G, RS_H>(st, a, qkv_dim, ring, full);
+      for (int i = 0; i < a.nslot && st.step < a.n_steps; i++, sent++) st_stream_issue<RS_D, RS_G, RS_H>(st, a, qkv_dim, ring, full);
     }
     __syncthreads();  // the barriers are there
     if (lane == 0) {
@@ -631,8 +646,10 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
       // None of the copies in flight may land in the memory of a CTA that has gone.  The walk is over long before the computing warps
       // are (a narrow model's last passes are requested phases ahead), and they may leave at any barrier: so on every way out.  The copies
       // wait for nobody, whatever the limit of the other waits is.
-      const unsigned ns = (unsigned)a.nslot;
-      for (unsigned i = st.sent > ns ? st.sent - ns : 0u; i < st.sent; i++) st_mbar_wait(full + i % ns, (i / ns) & 1u, a.timeout_ns + 1000000000ull);
+      for (; sent > 0; sent--) {  // the slots from `slot` on hold the last passes
+        st_mbar_wait(full + slot, parity, a.timeout_ns + 1000000000ull);
+        if (++slot == (uint32_t)a.nslot) { slot = 0; parity ^= 1u; }
+      }
     }
     return;
   }
@@ -784,22 +801,10 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
         prefetch_l2((tid == 0 ? L->ffn_norm : l + 1 < a.n_layers ? L[1].attn_norm : a.out_norm) + bid * 64);
       // this CTA's share of attention: context slice `slice` of (row b, kv head g); the pages of a short context's first rows are looked
       // up now, so that the rows themselves can be requested without a dependent load when the projection is over
-      const int n_pairs = M * a.G;
-      const bool mine = bid < n_pairs * a.slices;  // a.slices: the most slices a pair can have (the scratch's stride)
-      const int pair = mine ? bid / a.slices : 0, slice = mine ? bid % a.slices : 0;
-      const int b = pair / a.G, g = pair % a.G;
+      const StShare share = st_share<MT>(a, posv, a.slices);
+      const int pair = share.pair, slice = share.slice, b = share.b, g = share.g, T = share.T, S = share.S, t0 = share.t0, t1 = share.t1, pnew = T - 1;
+      const bool att = share.att;
       const int sub = lane % LPR, rgrp = lane / LPR;
-      int pb = posv[0];
-#pragma unroll
-      for (int m = 1; m < MT; m++) pb = (b == m) ? posv[m] : pb;
-      const int T = min(max(pb + 1, 1), a.max_ctx);
-      const int pnew = T - 1;
-      // slices of this pair: about a.slice_len positions each (a short context keeps few CTAs busy and the exchanges of
-      // statistics and partials short), never more positions than a slice's scores have room for
-      const int S = min(a.slices, max((T + a.slice_len - 1) / a.slice_len, (T + a.chunk_cap - 1) / a.chunk_cap));
-      const bool att = mine && slice < S;
-      const int chunk = (T + S - 1) / S;
-      const int t0 = slice * chunk, t1 = att ? min(T, t0 + chunk) : t0;
       const int32_t* bt_row = a.block_table + (size_t)b * a.max_pages_per_seq;
       __half* k_layer = a.k_pool + (size_t)l * a.layer_elems;
       __half* v_layer = a.v_pool + (size_t)l * a.layer_elems;
@@ -846,10 +851,9 @@ __global__ void __launch_bounds__(ST_THREADS + 32, 1) jg_step_kernel(const StepA
       st_project<RS_D, NI_D, 1, MT>(qkv_dim, KC_D, xs, M, ring, full, empty, rg, batch, part, a, tid, no_pre,
                                          [&](int row, int m, float s, float, __half) { a.qkv[(size_t)m * qkv_dim + row] = __float2half_rn(s); });
       if (brief) {
-        StShort c = {l, pair, slice, b, g, T, S, t0, t1, mine, att, pg0[0], pg0[1], gen, scored, prof, t_prev, red, s_M, s_rL};
-        const bool ok = st_attend_short<HD, NREP>(a, c);
-        gen = c.gen; scored = c.scored; t_prev = c.t_prev;
-        if (!ok) { give_up(4); return; }
+        int slices = a.slices;  // the share is worked out anew: nothing of it stays in registers through a projection
+        asm volatile("" : "+r"(slices));
+        if (!st_attend_short<HD, NREP>(a, st_share<MT>(a, posv, slices), l, pg0, gen, scored, red, s_M, s_rL, prof, t_prev)) { give_up(4); return; }
       } else if constexpr (FORM != ST_FITS) {
         stamp(0);
         auto rows = [&] {
