@@ -4,7 +4,7 @@
 #include <math.h>
 
 #include "common.cuh"
-#include "quant.cuh"
+#include "nf4.cuh"
 #include "stream.cuh"
 #include "transcendental.cuh"
 
@@ -362,7 +362,7 @@ JG_API int jg_dequant_i8_f16(jg_dev* dev, uint64_t dst, uint64_t w, uint64_t sca
 __global__ void dequant_nf4_f16_kernel(__half* __restrict__ dst, const uint8_t* __restrict__ w, const __half* __restrict__ scale,
                                        long long n32, int block) {
   __shared__ __half code[16];
-  if (threadIdx.x < 16) code[threadIdx.x] = __float2half_rn(c_nf4[threadIdx.x]);
+  if (threadIdx.x < 16) code[threadIdx.x] = __float2half_rn(nf4_code(threadIdx.x));
   pdl_launch();
   pdl_wait();
   __syncthreads();

@@ -52,8 +52,9 @@ __global__ void __launch_bounds__(N4_THREADS, 2) jg_matvec_nf4_kernel(const Nf4A
   const int total = (tile1 - tile0) * per;
   const size_t row_bytes = (size_t)K / 2, row_blocks = (size_t)(K >> a.block_shift);
   pdl_launch();
+  const float lane_code = nf4_code(lane & 15);
   for (int b = warp; b < 256; b += N4_WARPS) {
-    const __half2 h = __halves2half2(__float2half_rn(c_nf4[b >> 4]), __float2half_rn(c_nf4[b & 15]));
+    const __half2 h = nf4_pair(lane_code, b);
     lut[b * 32 + lane] = *reinterpret_cast<const uint32_t*>(&h);
   }
   if (a.late) pdl_wait();  // the weights were written by a launch that may still be running

@@ -24,6 +24,7 @@
 // Every mbarrier wait is bounded: a warp whose wait gives up records it and goes on without waiting (the results are void, the host
 // reports JG_ETIMEDOUT at the next synchronisation); the producer stops requesting and lets the copies in flight land.
 #pragma once
+#include "nf4.cuh"
 #include "quant.cuh"
 #include "skinny_plan.h"
 #include "tcgen05.cuh"
@@ -157,10 +158,11 @@ __global__ void __launch_bounds__(SK_THREADS, 1)
     return;
   }
 
-  if (TYPE == SK_NF4) {  // [byte][lane]: half2(code of the high nibble, of the low one)
+  if constexpr (TYPE == SK_NF4) {  // [byte][lane]: half2(code of the high nibble, of the low one)
     uint32_t* table = reinterpret_cast<uint32_t*>(sk_raw + (lut - raw));
+    const float lane_code = nf4_code(lane & 15);
     for (int b = warp; b < 256; b += SK_WARPS) {
-      const __half2 h = __halves2half2(__float2half_rn(c_nf4[b >> 4]), __float2half_rn(c_nf4[b & 15]));
+      const __half2 h = nf4_pair(lane_code, b);
       table[b * 32 + lane] = *reinterpret_cast<const uint32_t*>(&h);
     }
   }
